@@ -15,6 +15,9 @@
 //                        A product may take its k in any order as long as both operands
 //                        do, so a lane's 16 contiguous bytes of a row serve as the k's of
 //                        two instructions: no shared memory, no shuffles.
+//   group_stream_kernel  row groups of few rows each (experts in decoding and in short
+//                        portions): tcgen05 with the weights as the 128-row operand, a
+//                        persistent CTA per SM with a TMA ring that runs on across tiles
 //   group_large_kernel   many rows: tcgen05, 128 rows x 256 weight rows, TMA-fed,
 //                        accumulators double-buffered in tensor memory
 #include "fk_tcgen05.cuh"
@@ -344,6 +347,41 @@ __device__ __forceinline__ GgTile gg_tile(const GroupParams& p, const int* first
   return t;
 }
 
+// first_tile[g] = tiles of the groups ahead of g, ROWS rows by one column block each; one
+// warp.
+template <int ROWS>
+__device__ __forceinline__ void gg_count_tiles(const GroupParams& p, int* first_tile,
+                                               int n_tiles) {
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  for (int g0 = 0; g0 < p.groups; g0 += 32) {
+    int64_t f = 0, c = 0;
+    const int g = g0 + lane;
+    if (g < p.groups) {
+      if (p.offsets) {
+        f = p.offsets[g];
+        c = p.offsets[g + 1] - f;
+        if (f < 0 || c < 0 || f + c > p.rows) {
+          if (p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
+          c = 0;
+        }
+      } else {
+        c = p.rows;
+      }
+    }
+    const int mine = (int)((c + ROWS - 1) / ROWS) * n_tiles;
+    int run = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += up;
+    }
+    if (g < p.groups) first_tile[g] = base + run - mine;
+    base += __shfl_sync(0xffffffffu, run, 31);
+  }
+  if (lane == 0) first_tile[p.groups] = base;
+}
+
 // Adds bias[from + c .. from + c + 3]; columns beyond n are not stored.
 __device__ __forceinline__ void gg_add_bias(const GroupParams& p, int from, int c, float& a,
                                             float& b, float& d, float& e) {
@@ -398,36 +436,7 @@ group_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
   }
   if (warp == 1) tmem_alloc(tmem_slot, 512);
   pdl_wait();
-  // running tile count of the groups
-  if (warp == 0) {
-    int base = 0;
-    for (int g0 = 0; g0 < p.groups; g0 += 32) {
-      int64_t f = 0, c = 0;
-      const int g = g0 + lane;
-      if (g < p.groups) {
-        if (p.offsets) {
-          f = p.offsets[g];
-          c = p.offsets[g + 1] - f;
-          if (f < 0 || c < 0 || f + c > p.rows) {
-            if (p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
-            c = 0;
-          }
-        } else {
-          c = p.rows;
-        }
-      }
-      const int mine = (int)((c + Cfg::kRows - 1) / Cfg::kRows) * n_tiles;
-      int run = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, run, o);
-        if (lane >= o) run += up;
-      }
-      if (g < p.groups) first_tile[g] = base + run - mine;
-      base += __shfl_sync(0xffffffffu, run, 31);
-    }
-    if (lane == 0) first_tile[p.groups] = base;
-  }
+  if (warp == 0) gg_count_tiles<Cfg::kRows>(p, first_tile, n_tiles);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -596,6 +605,217 @@ group_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
   }
 }
 
+// -------------------------------------------------------------- few rows a group, streamed
+// Bound by the weights' bytes.  A tile is 128 weight rows (64 gate rows and the 64 up rows of
+// the same columns with ACT) of one group against up to NT of its rows: the weights are the
+// M operand, so a handful of rows costs N = 16 and not 128.  One CTA an SM walks tiles
+// (rows fastest: a group with more than NT rows finds its weights in L2), and the ring runs
+// on across tiles, so that the loads of the next one are under way while this one is stored.
+// Gathered rows come by tile::gather4, four rows an instruction, one lane of the loading warp
+// each.  64 experts, 384 rows, 4096 -> 2 x 1408 (1.48 GB of weights): 265 us, 225 at the copy rate;
+// 1408 -> 4096: 138 us (113).  A CTA for every 16 weight rows (group_skinny_kernel), which fills
+// and drains its loads for 256 KB of weights, takes 324 and 197.
+template <int NT, bool ACT>
+struct GtCfg {
+  static constexpr int kABytes = 128 * GG_BK * 2;
+  static constexpr int kBBytes = NT * GG_BK * 2;
+  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kStages = NT <= 16 ? 10 : NT <= 32 ? 9 : NT <= 64 ? 7 : 5;
+  static constexpr int kOffTiles = kStages * kStageBytes;
+  static constexpr int kOffBar = kOffTiles + (GG_MAX_GROUPS + 8) * 4;
+  static constexpr int kOffUp = kOffBar + 256;              // 2 x [16 rows][64 up values]
+  static constexpr int kSmem = kOffUp + (ACT ? 2 * 16 * 64 * 4 : 0) + 1024;
+  static constexpr int kTmemCols = 2 * NT;
+  static_assert(kSmem <= 232448, "shared memory budget");
+  static_assert(kTmemCols >= 32 && (kTmemCols & (kTmemCols - 1)) == 0, "tensor memory");
+};
+
+// rows r[0..3] of the tensor, 64 columns from col: 4 x 128 bytes, swizzled like a box of rows
+__device__ __forceinline__ void gt_gather4(void* dst, const CUtensorMap* m, uint64_t* bar,
+                                           int col, const int (&r)[4]) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_u32(dst)),
+      "l"(m), "r"(col), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(smem_u32(bar))
+      : "memory");
+}
+// whether `ok` holds in all 128 threads of the storing warps
+__device__ __forceinline__ bool gt_all(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, 2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r) : "r"(ok ? 1u : 0u) : "memory");
+  return r != 0;
+}
+
+template <int NT, bool ACT>
+__global__ void __launch_bounds__(GG_THREADS, 1)
+group_stream_kernel(const __grid_constant__ CUtensorMap tmap_x,
+                    const __grid_constant__ CUtensorMap tmap_w, const GroupParams p) {
+  using Cfg = GtCfg<NT, ACT>;
+  extern __shared__ uint8_t gg_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gg_raw) + 1023) &
+                                             ~uintptr_t(1023));
+  int* first_tile = reinterpret_cast<int*>(smem + Cfg::kOffTiles);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBar);
+  uint64_t* empty = full + Cfg::kStages;
+  uint64_t* acc_full = empty + Cfg::kStages;       // [2]
+  uint64_t* acc_empty = acc_full + 2;              // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(acc_empty + 3);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int TN = ACT ? 64 : 128;               // outputs per tile
+  const int n_tiles = (p.n + TN - 1) / TN;
+  const int kb_total = (p.k + GG_BK - 1) / GG_BK;
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < Cfg::kStages; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&acc_full[b], 1);
+      mbar_init(&acc_empty[b], 4);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmap_x);
+    tma_prefetch_desc(&tmap_w);
+  }
+  if (warp == 1) tmem_alloc(tmem_slot, Cfg::kTmemCols);
+  pdl_wait();
+  if (warp == 0) gg_count_tiles<NT>(p, first_tile, n_tiles);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int total = first_tile[p.groups];
+
+  if (warp == 0) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int ti = blockIdx.x; ti < total && ok; ti += gridDim.x) {
+      const GgTile t = gg_tile<NT>(p, first_tile, ti, n_tiles);
+      const int wrow = (int)(t.g * p.w_rows) + t.nt * TN;
+      int rows[4];
+      if (p.gather && lane < NT / 4) {
+        // rows beyond the group's last repeat it: multiplied, not stored
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          rows[i] = (int)group_x_row(p, t.row0 + min((int64_t)(lane * 4 + i), t.rows_left - 1));
+      }
+      for (int kb = 0; kb < kb_total; ++kb) {
+        uint8_t* dst = smem + stage * Cfg::kStageBytes;
+        if (lane == 0) {
+          ok = gg_wait(&empty[stage], phase ^ 1, abort_flag, p.status);
+          if (ok) {
+            mbar_arrive_expect_tx(&full[stage], (uint32_t)Cfg::kStageBytes);
+            tma_load_2d(dst, &tmap_w, &full[stage], kb * GG_BK, wrow);
+            if (ACT)
+              tma_load_2d(dst + Cfg::kABytes / 2, &tmap_w, &full[stage], kb * GG_BK,
+                          wrow + p.n);
+            if (!p.gather)
+              tma_load_2d(dst + Cfg::kABytes, &tmap_x, &full[stage], kb * GG_BK, (int)t.row0);
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        if (!ok) break;
+        if (p.gather && lane < NT / 4)
+          gt_gather4(dst + Cfg::kABytes + lane * 512, &tmap_x, &full[stage], kb * GG_BK, rows);
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                               ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    int stage = 0;
+    uint32_t phase = 0, done = 0;
+    bool ok = true;
+    for (int ti = blockIdx.x; ti < total && ok; ti += gridDim.x) {
+      const uint32_t buf = done & 1u, use = done >> 1;
+      if (use > 0) ok = gg_wait_warp(&acc_empty[buf], (use - 1) & 1u, abort_flag, p.status);
+      if (!ok) break;
+      tc_fence_after();
+      for (int kb = 0; kb < kb_total; ++kb) {
+        ok = gg_wait_warp(&full[stage], phase, abort_flag, p.status);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t a = smem_u32(smem + stage * Cfg::kStageBytes);
+        const uint32_t b = a + Cfg::kABytes;
+#pragma unroll
+        for (int kk = 0; kk < GG_BK / 16; ++kk)
+          tc_mma_bf16_elect(tmem + buf * NT, smem_desc_sw128(a + kk * 32),
+                            smem_desc_sw128(b + kk * 32), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+        tc_commit_elect(&empty[stage]);
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) break;
+      tc_commit_elect(&acc_full[buf]);
+      ++done;
+    }
+  } else {
+    // a lane has one weight row; 16 of the group's rows at a time
+    const int q = warp & 3;
+    const uint32_t lane_addr = tmem + ((uint32_t)(q * 32) << 16);
+    uint32_t done = 0, chunk = 0;
+    for (int ti = blockIdx.x; ti < total; ti += gridDim.x) {
+      const GgTile t = gg_tile<NT>(p, first_tile, ti, n_tiles);
+      const uint32_t buf = done & 1u, use = done >> 1;
+      // one answer for all four warps: with ACT they meet at barriers below
+      if (!gt_all(gg_wait(&acc_full[buf], use & 1u, abort_flag, p.status))) break;
+      tc_fence_after();
+      const int rows = (int)min((int64_t)NT, t.rows_left);
+      const int col = t.nt * TN + (ACT ? (q & 1) : q) * 32 + lane;
+      const bool on = col < p.n;
+      const float bias = p.bias && on ? p.bias[ACT && q >= 2 ? p.n + col : col] : 0.f;
+      uint16_t* y = static_cast<uint16_t*>(p.y) + t.row0 * p.y_stride + col;
+      for (int c0 = 0; c0 < rows; c0 += 16, ++chunk) {
+        uint32_t v[16];
+        tc_ld16(lane_addr + buf * NT + c0, v);
+        tc_wait_ld();
+        if (ACT) {
+          // the up half hands its values to the gate half; two buffers, so that one barrier
+          // a chunk is enough
+          float* up = reinterpret_cast<float*>(smem + Cfg::kOffUp) + (chunk & 1u) * 1024 +
+                      (q & 1) * 32 + lane;
+          if (q >= 2) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) up[i * 64] = __uint_as_float(v[i]) + bias;
+          }
+          asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+          if (q < 2) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (c0 + i < rows && on)
+                Elem<uint16_t>::store(y + (c0 + i) * p.y_stride,
+                                      group_act(__uint_as_float(v[i]) + bias, p.act) *
+                                          up[i * 64]);
+          }
+        } else if (on) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (c0 + i < rows)
+              Elem<uint16_t>::store(y + (c0 + i) * p.y_stride, __uint_as_float(v[i]) + bias);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      ++done;
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, Cfg::kTmemCols);
+  }
+}
+
 // ----------------------------------------------------------------------------- host
 struct GgKey {
   const void* ptr; int64_t rows, cols, stride; int box_rows;
@@ -704,6 +924,49 @@ static int launch_large(const GroupParams& p, int64_t x_cols, cudaStream_t s) {
   return launch_large_one<256, ACT, OUT>(p, x_cols, s);
 }
 
+template <int NT, bool ACT>
+static int launch_stream_one(const GroupParams& p, cudaStream_t s) {
+  using Cfg = GtCfg<NT, ACT>;
+  constexpr int TN = ACT ? 64 : 128;
+  const int64_t n_tiles = (p.n + TN - 1) / TN;
+  const int64_t bound = ((p.rows + NT - 1) / NT + p.groups) * n_tiles;
+  FK_REQUIRE(bound <= 0x7fffffff && p.rows < (1ll << 31) && p.x_rows < (1ll << 31) &&
+                 p.groups * p.w_rows < (1ll << 31),
+             FK_ERR_UNSUPPORTED, "fk_group_gemm: too many tiles");
+  CUtensorMap mx, mw;
+  int rc = gg_map(p.x, p.x_rows, p.k, p.x_stride, p.gather ? 1 : NT, &mx);
+  if (rc != FK_OK) return rc;
+  rc = gg_map(p.w, p.groups * p.w_rows, p.k, p.k, TN, &mw);
+  if (rc != FK_OK) return rc;
+  static PerDeviceOnce once;
+  FK_CUDA_OK(set_max_dynamic_smem(once, group_stream_kernel<NT, ACT>, Cfg::kSmem));
+  const int ctas = (int)(bound < sm_count() ? bound : sm_count());
+  FK_CUDA_OK(launch_kernel(group_stream_kernel<NT, ACT>, dim3((unsigned)ctas), dim3(GG_THREADS),
+                           (size_t)Cfg::kSmem, s, mx, mw, p));
+  count_launch();
+  return FK_OK;
+}
+// Row groups are streamed, except
+//  - where there are fewer tiles than two thirds of the SMs (one row of 16 experts, 1600 ->
+//    2560: 18.5 us against 14.3 in CTAs of 16 weight rows; two rows: 19.2 and 16.8; four rows:
+//    22.6 and 26.7, and from there on it is ahead);
+//  - gathered rows above 16 a group: the ring then waits for the gathers (64 experts, 29 rows
+//    each, 4096 -> 2 x 1408: 514 us against 447, where rows laid out beforehand take 270).
+static bool streams(const GroupParams& p, int64_t expect) {
+  if (!p.offsets || p.groups > GG_MAX_GROUPS || (p.gather && expect > 16)) return false;
+  const int64_t n_tiles = (p.n + (p.act >= 0 ? 63 : 127)) / (p.act >= 0 ? 64 : 128);
+  const int64_t used = p.rows < p.groups ? p.rows : p.groups;
+  return used * n_tiles * 3 >= 2ll * sm_count();
+}
+// Rows of a tile: twice what a group has on average, so that most groups are one tile.
+template <bool ACT>
+static int launch_stream(const GroupParams& p, int64_t expect, cudaStream_t s) {
+  if (expect <= 8) return launch_stream_one<16, ACT>(p, s);
+  if (expect <= 16) return launch_stream_one<32, ACT>(p, s);
+  if (expect <= 32) return launch_stream_one<64, ACT>(p, s);
+  return launch_stream_one<128, ACT>(p, s);
+}
+
 }  // namespace fk
 
 using namespace fk;
@@ -761,6 +1024,9 @@ int fk_group_gemm(const void* x, int64_t x_stride, int64_t x_group, int64_t x_ro
     return y_f32 ? launch_large<false, float>(p, x_cols, s)
                  : launch_large<false, uint16_t>(p, x_cols, s);
   }
+  if (!y_f32 && streams(p, expect_rows))
+    return act >= 0 ? launch_stream<true>(p, expect_rows, s)
+                    : launch_stream<false>(p, expect_rows, s);
   if (act >= 0) return launch_skinny<true, uint16_t>(p, expect_rows, s);
   return y_f32 ? launch_skinny<false, float>(p, expect_rows, s)
                : launch_skinny<false, uint16_t>(p, expect_rows, s);

@@ -205,6 +205,33 @@ def test_row_groups(counts, act, dtype):
             close(got, z, dtype, scale=np.abs(z).max())
 
 
+@pytest.mark.parametrize("act", [None, 0])
+@pytest.mark.parametrize("counts", [[16, 17, 0, 1], [32, 33, 64, 65, 0, 0, 128, 129, 300]])
+def test_row_groups_streamed(counts, act):
+    """Enough weight tiles for the streaming kernel: an odd number of columns, k that ends
+    inside a block of 64, groups around every size of its row tile, with a bias."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(len(counts))
+    groups, rows, n, k = len(counts), sum(counts), 3331, 72
+    x = values(rs, 40, k, dtype=BF16)
+    w = values(rs, groups, n if act is None else 2 * n, k, dtype=BF16) / 8
+    bias = values(rs, n if act is None else 2 * n)
+    source = rs.randint(0, 40, size=rows)
+    off = np.concatenate([[0], np.cumsum(counts)])
+    z = np.concatenate([x[source[a:b]] @ m.T + bias for a, b, m in zip(off, off[1:], w)])
+    if act is not None:
+        z = R.silu(z[:, :n]) * z[:, n:]
+    xd, wd, sd = dev(x, BF16), dev(w, BF16), i32(source)
+    for expect in (1, 12, 20, 50):
+        for gather in (True, False):
+            out = torch.full((rows, n + 3), 3.0, device="cuda", dtype=BF16)
+            ops.group_gemm(xd if gather else ops.gather_rows(xd, sd), wd, out=out[:, :n],
+                           offsets=i32(off), gather=sd if gather else None, bias=dev(bias), act=act,
+                           expect_rows=expect)
+            close(out[:, :n], z, BF16, scale=np.abs(z).max())
+            assert torch.all(out[:, n:] == 3.0)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("rows", [1, 37, 64, 300])
 @pytest.mark.parametrize("ff,bias", [(56, True), (200, False), (333, True)])
