@@ -27,7 +27,7 @@ COMPONENT_SOURCES = {"decode_attn": ["fk_attn.cu"], "delta": ["fk_delta.cu"],
                      "experts": ["fk_moe.cu"], "comm": ["fk_comm.cu"], "block": ["fk_block.cu"]}
 SOURCES = CORE_SOURCES + [s for c in COMPONENT_SOURCES.values() for s in c]
 HEADERS = [CSRC / "fk_common.cuh", CSRC / "fk_tcgen05.cuh", CSRC / "fk_rowops.cuh",
-           CSRC / "fk_types.cuh",
+           CSRC / "fk_types.cuh", CSRC / "fk_f32_tile.cuh",
            CSRC / "fk_gemm_shared.cuh", PKG.parent / "include" / "fk_b200.h"]
 
 NVCC_FLAGS = [

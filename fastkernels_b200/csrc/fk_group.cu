@@ -10,7 +10,7 @@
 // each with its part of the bias.
 // bf16 operands with fp32 accumulation and bf16 or fp32 results, or true fp32.
 //
-//   group_any_kernel     fp32 FMA, any sizes (fp32 operands)
+//   f32_product_kernel   fp32 FMA, any sizes (fp32 operands; fk_plain.cu)
 //   group_skinny_kernel  few rows: streams the weights straight into mma.sync fragments.
 //                        A product may take its k in any order as long as both operands
 //                        do, so a lane's 16 contiguous bytes of a row serve as the k's of
@@ -20,6 +20,7 @@
 //                        persistent CTA per SM with a TMA ring that runs on across tiles
 //   group_large_kernel   many rows: tcgen05, 128 rows x 256 weight rows, TMA-fed,
 //                        accumulators double-buffered in tensor memory
+#include "fk_f32_tile.cuh"
 #include "fk_tcgen05.cuh"
 #include "fk_types.cuh"
 
@@ -64,78 +65,6 @@ __device__ __forceinline__ int64_t group_x_row(const GroupParams& p, int64_t row
     return 0;
   }
   return r;
-}
-
-// ------------------------------------------------------------------------- any size
-constexpr int GA_M = 64, GA_N = 64, GA_K = 16;
-
-template <bool ACT>
-__global__ void __launch_bounds__(256) group_any_kernel(const GroupParams p) {
-  pdl_launch_dependents();
-  pdl_wait();
-  constexpr int NB = ACT ? 2 : 1;
-  __shared__ float xs[GA_K][GA_M + 4], ws[NB][GA_K][GA_N + 4];
-  const int g = blockIdx.z;
-  int64_t first, count;
-  group_range(p, g, &first, &count);
-  const int n0 = blockIdx.x * GA_N;
-  const int64_t m0 = (int64_t)blockIdx.y * GA_M;
-  if (m0 >= count) return;
-  const float* x = static_cast<const float*>(p.x) + (p.offsets ? 0 : g * p.x_group);
-  const float* w = static_cast<const float*>(p.w) + (int64_t)g * p.w_rows * p.k;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int lr = threadIdx.x >> 2, lc = (threadIdx.x & 3) * 4;
-  const bool x_on = m0 + lr < count, w_on = n0 + lr < p.n;
-  const float* xr = x + (x_on ? group_x_row(p, first + m0 + lr) : 0) * p.x_stride;
-  float acc[NB][4][4] = {};
-  for (int k0 = 0; k0 < p.k; k0 += GA_K) {
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b[NB];
-#pragma unroll
-    for (int e = 0; e < NB; ++e) b[e] = a;
-    if (k0 + lc < p.k) {
-      if (x_on) a = *reinterpret_cast<const float4*>(xr + k0 + lc);
-#pragma unroll
-      for (int e = 0; e < NB; ++e)
-        if (w_on)
-          b[e] = *reinterpret_cast<const float4*>(w + ((int64_t)e * p.n + n0 + lr) * p.k + k0 + lc);
-    }
-    __syncthreads();
-    xs[lc][lr] = a.x; xs[lc + 1][lr] = a.y; xs[lc + 2][lr] = a.z; xs[lc + 3][lr] = a.w;
-#pragma unroll
-    for (int e = 0; e < NB; ++e) {
-      ws[e][lc][lr] = b[e].x; ws[e][lc + 1][lr] = b[e].y;
-      ws[e][lc + 2][lr] = b[e].z; ws[e][lc + 3][lr] = b[e].w;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < GA_K; ++kk) {
-      const float4 av = *reinterpret_cast<const float4*>(&xs[kk][ty * 4]);
-      const float aa[4] = {av.x, av.y, av.z, av.w};
-#pragma unroll
-      for (int e = 0; e < NB; ++e) {
-        const float4 bv = *reinterpret_cast<const float4*>(&ws[e][kk][tx * 4]);
-        const float bb[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[e][i][j] = fmaf(aa[i], bb[j], acc[e][i][j]);
-      }
-    }
-  }
-  float* y = static_cast<float*>(p.y) + (p.offsets ? 0 : g * p.y_group);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t r = m0 + ty * 4 + i;
-    if (r >= count) break;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = n0 + tx * 4 + j;
-      if (c >= p.n) continue;
-      float v = acc[0][i][j] + (p.bias ? p.bias[c] : 0.f);
-      if (ACT) v = group_act(v, p.act) * (acc[NB - 1][i][j] + (p.bias ? p.bias[p.n + c] : 0.f));
-      y[(first + r) * p.y_stride + c] = v;
-    }
-  }
 }
 
 // ------------------------------------------------------------------------- few rows
@@ -1006,13 +935,14 @@ int fk_group_gemm(const void* x, int64_t x_stride, int64_t x_group, int64_t x_ro
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (is_f32) {
     FK_REQUIRE(y_f32, FK_ERR_INVALID_ARG, "fk_group_gemm: fp32 operands give an fp32 result");
-    const int64_t my = (rows + GA_M - 1) / GA_M;
-    FK_REQUIRE(my <= 65535, FK_ERR_UNSUPPORTED, "fk_group_gemm: too many rows");
-    const dim3 grid((unsigned)((n + GA_N - 1) / GA_N), (unsigned)my, (unsigned)groups);
-    FK_CUDA_OK(act >= 0 ? launch_kernel(group_any_kernel<true>, grid, dim3(256), 0, s, p)
-                        : launch_kernel(group_any_kernel<false>, grid, dim3(256), 0, s, p));
-    count_launch();
-    return FK_OK;
+    FK_REQUIRE((rows + 63) / 64 <= 65535, FK_ERR_UNSUPPORTED, "fk_group_gemm: too many rows");
+    F32Product f{};
+    f.x = static_cast<const float*>(x); f.x_stride = x_stride; f.x_group = x_group;
+    f.w = static_cast<const float*>(w); f.w_rows = p.w_rows; f.bias = bias;
+    f.y = static_cast<float*>(y); f.y_stride = y_stride; f.y_group = y_group;
+    f.offsets = offsets; f.gather = gather; f.rows = rows; f.x_rows = x_rows; f.groups = groups;
+    f.n = (int)n; f.k = (int)k; f.act = act; f.status = status;
+    return launch_f32_product(f, offsets ? rows / groups + 1 : rows, s);
   }
   FK_REQUIRE(act < 0 || !y_f32, FK_ERR_UNSUPPORTED,
              "fk_group_gemm: an activation gives a bf16 result");

@@ -224,6 +224,82 @@ def test_gemm_f32(m, n, k):
     close(ops.gemm(xd, wd), x @ w.T, F32, scale=np.sqrt(k))
 
 
+@pytest.mark.parametrize("m,n,k", [(2, 300, 4096), (33, 129, 36), (64, 128, 1024),
+                                   (65, 1000, 300), (127, 40, 2052), (257, 260, 640)])
+def test_gemm_f32_tiles_and_parts(m, n, k):
+    """Edges of the three row tiles, k in one part and in several."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(m)
+    x, xd = rnd(rs, m, k)
+    w, wd = rnd(rs, n, k)
+    want = x @ w.T
+    got = ops.gemm(xd, wd).double().cpu().numpy()
+    # sums of k products, each partial sum rounded once: k eps / 2 times the sum of magnitudes
+    # is the bound, a walk of k roundings what is seen
+    limit = 4 * np.sqrt(k) * 2.0 ** -24 * (np.abs(x) @ np.abs(w.T))
+    assert (np.abs(got - want) <= limit).all()
+
+
+@pytest.mark.parametrize("counts", [(0, 1, 0, 33), (64, 0, 129, 3, 65), (200, 257)])
+@pytest.mark.parametrize("act", [None, 0, 1])
+def test_group_f32_row_groups(counts, act):
+    """Row groups in fp32: empty groups, part-filled tiles, gathered rows, gate and up."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(len(counts))
+    rows, n, k = sum(counts), 77, 516
+    off = np.concatenate([[0], np.cumsum(counts)])
+    pick = rs.randint(0, 90, size=rows)
+    x, xd = rnd(rs, 90, k)
+    w, wd = rnd(rs, len(counts), n * (1 if act is None else 2), k)
+    bias, bd = rnd(rs, w.shape[1])
+    got = ops.group_gemm(xd, wd, bias=bd, offsets=i32(off), gather=i32(pick), act=act)
+    z = np.concatenate([x[pick[a:b]] @ wg.T + bias for a, b, wg in zip(off, off[1:], w)])
+    if act is not None:
+        gate, up = z[:, :n], z[:, n:]
+        z = (P.gelu_tanh(gate) if act else gate * P.sigmoid(gate)) * up
+    np.testing.assert_allclose(got.double().cpu().numpy(), z, rtol=2e-5,
+                               atol=2e-5 * np.abs(z).max())
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d,hq,hkv,portions", [
+    (4, 3, 1, [(0, 5), (40, 1)]), (68, 8, 2, [(0, 1), (70, 33), (3, 4)]),
+    (576, 16, 1, [(31, 1), (0, 1), (64, 2)]), (576, 5, 1, [(0, 70)]),
+    (1152, 2, 1, [(1, 9), (30, 1)])])
+def test_paged_attn_any_forms(d, hq, hkv, portions, dtype):
+    """Head sizes, shared heads, portions after a prefix and single tokens; the keys after a
+    row's own hold infinities, which must not reach it."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(d)
+    page, n = 16, sum(c for _, c in portions)
+    lens = [a + c for a, c in portions]
+    cols = max(-(-x // page) for x in lens)
+    order = rs.permutation(cols * len(lens))
+    bt = order.reshape(len(lens), cols)
+    k, kd = rnd(rs, len(order), page, hkv, d, dtype=dtype)
+    v, vd = rnd(rs, len(order), page, hkv, d, dtype=dtype)
+    q, qd = rnd(rs, n, hq, d, dtype=dtype)
+    cu = np.concatenate([[0], np.cumsum([c for _, c in portions])])
+    scale = d ** -0.5
+    for s, length in enumerate(lens):       # the last key of a portion is the future of its others
+        vd.view(-1, hkv, d)[bt[s, (length - 1) // page] * page + (length - 1) % page] = float("inf")
+    got = ops.paged_attn_any(qd, kd, vd, i32(cu), i32(lens), i32(bt), scale)
+    got = got.double().cpu().numpy()
+    for s, (a, c) in enumerate(portions):
+        ks, vs = (t[bt[s]].reshape(-1, hkv, d) for t in (k, v))
+        for i in range(c - 1):
+            seen = a + i + 1
+            for h in range(hq):
+                z = scale * ks[:seen, h * hkv // hq] @ q[cu[s] + i, h]
+                pr = np.exp(z - z.max())
+                want = pr @ vs[:seen, h * hkv // hq] / pr.sum()
+                # fp32 sums; a bf16 result is rounded once more
+                np.testing.assert_allclose(got[cu[s] + i, h], want, rtol=0,
+                                           atol=(1e-5 if dtype == F32 else 1e-2) *
+                                           max(1.0, np.abs(want).max()))
+        assert not np.isfinite(got[cu[s] + c - 1]).any()
+
+
 def test_embed_and_argmax_f32():
     from fastkernels_b200 import ops
     rs = np.random.RandomState(0)
