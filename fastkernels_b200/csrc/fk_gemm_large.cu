@@ -516,19 +516,18 @@ static int gl_map(const void* ptr, int64_t rows, int64_t cols, int64_t stride, i
   return FK_OK;
 }
 
-constexpr int GL_DEFAULT_PAIR_MODE = 0;
-
+// resident pairs: a property of the GPU model, asked once (0: no pair fits)
 template <int NH>
-static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmLargeParams& p,
-                       cudaStream_t stream) {
+static int resident_pairs() {
   using Cfg = G2Cfg<NH>;
   static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
   static int max_pairs = 0;
-  static PerDeviceOnce attr_once;
-  FK_CUDA_OK(set_max_dynamic_smem(attr_once, gemm_pair_kernel<NH>, Cfg::kAlloc));
-  // resident pairs: a property of the GPU model, asked once
   std::call_once(once, [] {
+    if (cudaFuncSetAttribute(gemm_pair_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             Cfg::kAlloc) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
     cudaLaunchConfig_t q{};
     q.gridDim = dim3(2 * (unsigned)sm_count());
     q.blockDim = dim3(GL_THREADS);
@@ -540,8 +539,19 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
     int n_cl = 0;
     if (cudaOccupancyMaxActiveClusters(&n_cl, gemm_pair_kernel<NH>, &q) == cudaSuccess)
       max_pairs = n_cl;
+    else
+      cudaGetLastError();
   });
-  FK_CUDA_OK(attr_err);
+  return max_pairs;
+}
+
+template <int NH>
+static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmLargeParams& p,
+                       cudaStream_t stream) {
+  using Cfg = G2Cfg<NH>;
+  static PerDeviceOnce attr_once;
+  FK_CUDA_OK(set_max_dynamic_smem(attr_once, gemm_pair_kernel<NH>, Cfg::kAlloc));
+  const int max_pairs = resident_pairs<NH>();
   FK_REQUIRE(max_pairs > 0, FK_ERR_CUDA, "fk_gemm_bf16: no CTA pair fits on this device");
   const int64_t tiles = (int64_t)p.m_tiles * ((p.n + Cfg::kTileN - 1) / Cfg::kTileN);
   const int pairs = (int)(tiles < max_pairs ? tiles : max_pairs);
@@ -567,6 +577,32 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
   return FK_OK;
 }
 
+// Which kernel: 0 = single CTAs, 1 = CTA pairs on 256 x 256, 2 = pairs on 256 x 512.
+//
+// All three multiply at about the same rate, so what decides is how the tiles fill their rounds.
+// A pair's round is shorter (half the work per SM), and its epilogue runs beside the next
+// tile's products, which the single CTA's does not.  Measured (us, k from 2048 to 12288): a
+// single CTA's round 12 + k / 100, a pair's 0.0072 k and 6 once.  k 2048, single -> pair:
+// 1000 x 3072 29.7 -> 21.0, 4096 x 3072 74.3 -> 55.8, 4096 x 12288 212 -> 173; k 4096:
+// 300 x 6144 49 -> 33, 2000 x 6144 96 -> 91, 2000 x 4096 (one full round) 51.7, pair 61.9.
+// The wide pair reads a quarter less: 2 to 4 % from k = 4096 on where it needs no more rounds
+// and there are several (8192 x 24576 x 4096 1286 -> 1242, 4096 x 4096 x 12288 294 -> 278).
+static int large_mode(const GemmLargeParams& p) {
+  auto rounds = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
+  const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
+  const int pairs = resident_pairs<1>();
+  if (pairs <= 0) return 0;
+  const double single = rounds(tiles, sm_count());
+  const double t_single = single * (12. + 0.01 * p.k);
+  const double t_pair = 6. + 0.0072 * p.k * rounds(tiles, pairs);
+  if (t_pair < t_single) return 1;
+  const int wide = resident_pairs<2>();
+  if (p.k >= 4096 && single >= 2. && wide > 0 &&
+      rounds((int64_t)p.m_tiles * ((p.n_tiles + 1) / 2), wide) <= single)
+    return 2;
+  return 0;
+}
+
 // Called by fk_gemm_bf16 for m > 256 after its argument checks.
 int gemm_large_launch(const void* x, int64_t x_stride, const void* w, const void* bias,
                       void* y, int64_t y_stride, int64_t m, int64_t n, int64_t k,
@@ -585,12 +621,12 @@ int gemm_large_launch(const void* x, int64_t x_stride, const void* w, const void
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   FK_REQUIRE(tiles <= 0x7fffffff, FK_ERR_UNSUPPORTED, "fk_gemm_bf16: too many tiles");
 
-  // FK_B200_GEMM_PAIR: 0 = single-CTA tiles, 1 = CTA pairs with 256 x 256 tiles,
-  // 2 = CTA pairs with 256 x 512 tiles
-  static const int pair_mode = [] {
+  // FK_B200_GEMM_PAIR: 0, 1 or 2 for one kernel at all sizes (see large_mode)
+  static const int forced = [] {
     const char* e = getenv("FK_B200_GEMM_PAIR");
-    return e != nullptr ? atoi(e) : GL_DEFAULT_PAIR_MODE;
+    return e != nullptr ? atoi(e) : -1;
   }();
+  const int pair_mode = forced >= 0 ? forced : large_mode(p);
   CUtensorMap mx, mw;
   if (pair_mode == 1 || pair_mode == 2) {
     int rc = gl_map(x, m, k, x_stride, 128, &mx);

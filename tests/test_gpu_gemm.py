@@ -192,6 +192,26 @@ print('pair ok')
     assert r.returncode == 0 and "pair ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("m,n,k", [(300, 1032, 4096),      # CTA pairs: few tiles, a short round
+                                   (2010, 4104, 2048),     # pairs over several rounds
+                                   (2010, 4096, 4096),     # single CTAs: one full round
+                                   (2048, 9472, 4096)])    # wide pairs: two full rounds
+def test_gemm_many_rows_kernel_choice(ops, m, n, k):
+    """Sizes on both sides of the rule that picks the many-row kernel; some rows of each tile
+    against the oracle, and nothing written past a row."""
+    rs = np.random.RandomState(m + n + k)
+    x = cases.randn_bf16(rs, (m, k))
+    w = cases.randn_bf16(rs, (n, k), 0.05)
+    out = torch.zeros((m, n + 8), dtype=torch.bfloat16, device="cuda")
+    st = ops.new_status("cuda")
+    ops.gemm_bf16(dev(x), dev(w), out=out[:, :n], status=st)
+    torch.cuda.synchronize()
+    assert int(st.item()) == 0
+    rows = np.unique(np.concatenate([np.arange(0, m, 97), np.arange(127, m, 128), [m - 1]]))
+    check(out[torch.from_numpy(rows).cuda()][:, :n], O.linear(x[rows], w), k)
+    assert float(out[:, n:].abs().max()) == 0.0
+
+
 # ---------------------------------------------------- gate/up projection + SiLU fused
 @pytest.mark.parametrize("m,n,k,bias", [
     (64, 24576, 4096, False),    # the 8B-shape MLP at batch 64
