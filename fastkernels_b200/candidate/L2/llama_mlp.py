@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from fastkernels_b200 import ops
+from fastkernels_b200 import _lib, ops
 from fastkernels_b200.candidate.L1.silu_and_mul import SiluAndMul
 from fastkernels_b200.candidate.L2.parallel_linear import (MergedColumnParallelLinear,
                                                             RowParallelLinear)
@@ -30,11 +30,13 @@ class LlamaMLP(nn.Module):
     def forward(self, x):
         gu = self.gate_up_proj
         if (self.fused_act and x.dim() == 2 and x.is_cuda and x.dtype == torch.bfloat16
-                and not torch.compiler.is_compiling()
-                and ops.gemm_silu_mul_fusable(x.shape[0], gu.weight.shape[0], x.shape[1])):
+                and not torch.compiler.is_compiling()):
             # gate/up projection and SiLU-and-multiply in one launch (same rounding
             # points as the two ops)
-            return self.down_proj(ops.gemm_silu_mul(x, gu.weight, gu.bias))
+            if ops.gemm_silu_mul_fusable(x.shape[0], gu.weight.shape[0], x.shape[1]):
+                return self.down_proj(ops.gemm_silu_mul(x, gu.weight, gu.bias))
+            if ops.gemm_act_mul_many_fits(x, gu.weight, gu.bias):
+                return self.down_proj(ops.gemm_act_mul_many(x, gu.weight, _lib.ACT_SILU, gu.bias))
         return self.down_proj(self.act_fn(gu(x)))
 
 

@@ -45,10 +45,11 @@ constexpr int GL_TMEM_COLS = 512;
 static_assert(GL_SMEM_ALLOC <= 232448, "shared memory budget");
 
 struct GemmLargeParams {
-  const uint16_t* bias;   // [n] or null
+  const uint16_t* bias;   // [n] ([2 n] with an activation) or null
   uint16_t* y; int64_t y_stride;
-  int m, n, k;
-  int m_tiles, n_tiles;
+  int m, n, k;            // n: outputs of a row
+  int m_tiles, n_tiles;   // tiles of 256 weight rows
+  int act;                // with an activation: FK_ACT_*
   int32_t* status;
 };
 
@@ -91,6 +92,43 @@ __device__ __forceinline__ void gl_bias(const GemmLargeParams& p, int col, float
   }
 }
 
+// With an activation W is [gate; up], and a 256-row weight tile is 128 gate rows and the 128 up
+// rows of the same outputs, so both meet in one accumulator and y = act(gate) * up leaves with
+// the tile: no [m, 2 n] result is written and read again.  Gate and up are rounded to bf16 first,
+// as the projection alone would leave them.
+//
+// 32 outputs of a row from column `col0` on: g (gate) and u (up) as they come out of tensor
+// memory.
+__device__ __forceinline__ void gl_store_act(const GemmLargeParams& p, uint16_t* y, int col0,
+                                             const uint32_t (&g)[32], const uint32_t (&u)[32]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int col = col0 + e * 8;
+    if (col >= p.n) break;                     // n is a multiple of 8
+    float bg[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float bu[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (p.bias) {
+      const uint4 a = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
+      const uint4 b = __ldg(reinterpret_cast<const uint4*>(p.bias + p.n + col));
+      bg[0] = bf16lo(a.x); bg[1] = bf16hi(a.x); bg[2] = bf16lo(a.y); bg[3] = bf16hi(a.y);
+      bg[4] = bf16lo(a.z); bg[5] = bf16hi(a.z); bg[6] = bf16lo(a.w); bg[7] = bf16hi(a.w);
+      bu[0] = bf16lo(b.x); bu[1] = bf16hi(b.x); bu[2] = bf16lo(b.y); bu[3] = bf16hi(b.y);
+      bu[4] = bf16lo(b.z); bu[5] = bf16hi(b.z); bu[6] = bf16lo(b.w); bu[7] = bf16hi(b.w);
+    }
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int a = e * 8 + 2 * i;
+      o[i] = act_mul2(pack_bf16(__uint_as_float(g[a]) + bg[2 * i],
+                                __uint_as_float(g[a + 1]) + bg[2 * i + 1]),
+                      pack_bf16(__uint_as_float(u[a]) + bu[2 * i],
+                                __uint_as_float(u[a + 1]) + bu[2 * i + 1]), p.act);
+    }
+    *reinterpret_cast<uint4*>(y + e * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+template <bool ACT>
 __global__ void __launch_bounds__(GL_THREADS, 1)
 gemm_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
                   const __grid_constant__ CUtensorMap tmap_w, const GemmLargeParams p) {
@@ -150,7 +188,13 @@ gemm_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
           uint8_t* dst = smem + stage * GL_STAGE_BYTES;
           mbar_arrive_expect_tx(&full[stage], (uint32_t)GL_STAGE_BYTES);
           tma_load_2d(dst, &tmap_x, &full[stage], kb * GL_BK, mt * GL_BM);
-          tma_load_2d(dst + GL_A_BYTES, &tmap_w, &full[stage], kb * GL_BK, nt * GL_BN);
+          if (ACT) {
+            tma_load_2d(dst + GL_A_BYTES, &tmap_w, &full[stage], kb * GL_BK, nt * (GL_BN / 2));
+            tma_load_2d(dst + GL_A_BYTES + GL_B_BYTES / 2, &tmap_w, &full[stage], kb * GL_BK,
+                        p.n + nt * (GL_BN / 2));
+          } else {
+            tma_load_2d(dst + GL_A_BYTES, &tmap_w, &full[stage], kb * GL_BK, nt * GL_BN);
+          }
           if (++stage == GL_STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -204,11 +248,22 @@ gemm_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int mt = ti % p.m_tiles, nt = ti / p.m_tiles;
       if (!gl_wait(acc_full, tiles_done & 1u, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
-      const int n0 = nt * GL_BN;
+      const int n0 = nt * (ACT ? GL_BN / 2 : GL_BN);
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         const int64_t tok = (int64_t)mt * GL_BM + h * 128 + row;
         uint16_t* yrow = p.y + tok * p.y_stride + n0;
+        if (ACT) {
+#pragma unroll 1
+          for (int c = 0; c < GL_BN / 64; ++c) {
+            uint32_t g[32], u[32];
+            tc_ld32(lane_addr + h * GL_BN + c * 32, g);
+            tc_ld32(lane_addr + h * GL_BN + GL_BN / 2 + c * 32, u);
+            tc_wait_ld();
+            if (tok < p.m) gl_store_act(p, yrow + c * 32, n0 + c * 32, g, u);
+          }
+          continue;
+        }
 #pragma unroll 1
         for (int c = 0; c < GL_BN / 32; ++c) {
           uint32_t v[32];
@@ -288,7 +343,7 @@ struct G2Cfg {
   static_assert(kAlloc <= 232448, "shared memory budget");
 };
 
-template <int NH>
+template <int NH, bool ACT>
 __global__ void __launch_bounds__(GL_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x,
                  const __grid_constant__ CUtensorMap tmap_w, const GemmLargeParams p) {
@@ -307,7 +362,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();       // 0 = even CTA (issues the MMAs)
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const int n_tiles = (p.n + Cfg::kTileN - 1) / Cfg::kTileN;
+  constexpr int kOutN = ACT ? Cfg::kTileN / 2 : Cfg::kTileN;     // outputs of a tile
+  const int n_tiles = (p.n + kOutN - 1) / kOutN;
   const int total_tiles = p.m_tiles * n_tiles;
   const int kb_total = p.k / GL_BK;
 
@@ -353,11 +409,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x,
           if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2u * Cfg::kStageBytes);
           const uint32_t bar = full0 + (uint32_t)stage * 8u;
           tma2_load_2d(dst, &tmap_x, bar, kb * GL_BK, mt * GL_BM + (int)rank * 128);
-          // N half h of the tile = [this CTA's 128 rows | the partner's 128 rows]
+          // N half h of the tile = [this CTA's 128 rows | the partner's 128 rows]; with an
+          // activation the even CTA's are gate rows, the odd one's the up rows beside them
 #pragma unroll
           for (int h = 0; h < NH; ++h)
             tma2_load_2d(dst + Cfg::kABytes + h * (128 * GL_BK * 2), &tmap_w, bar, kb * GL_BK,
-                         nt * Cfg::kTileN + h * 256 + (int)rank * 128);
+                         ACT ? nt * kOutN + h * 128 + (int)rank * p.n
+                             : nt * kOutN + h * 256 + (int)rank * 128);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -418,11 +476,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x,
         break;
       }
       tc_fence_after();
-      const int n0 = nt * Cfg::kTileN;
+      const int n0 = nt * kOutN;
       const int64_t tok = (int64_t)mt * GL_BM + (int)rank * 128 + row;
       uint16_t* yrow = p.y + tok * p.y_stride + n0;
+      if (ACT) {
 #pragma unroll 1
-      for (int c = 0; c < Cfg::kTileN / 32; ++c) {
+        for (int c = 0; c < kOutN / 32; ++c) {
+          uint32_t g[32], u[32];
+          const uint32_t at = lane_addr + buf * 256 + (c >> 2) * 256 + (c & 3) * 32;
+          tc_ld32(at, g);
+          tc_ld32(at + 128, u);
+          tc_wait_ld();
+          if (tok < p.m) gl_store_act(p, yrow + c * 32, n0 + c * 32, g, u);
+        }
+      }
+#pragma unroll 1
+      for (int c = 0; !ACT && c < Cfg::kTileN / 32; ++c) {
         uint32_t v[32];
         tc_ld32(lane_addr + buf * 256 + c * 32, v);
         tc_wait_ld();
@@ -517,13 +586,13 @@ static int gl_map(const void* ptr, int64_t rows, int64_t cols, int64_t stride, i
 }
 
 // resident pairs: a property of the GPU model, asked once (0: no pair fits)
-template <int NH>
+template <int NH, bool ACT>
 static int resident_pairs() {
   using Cfg = G2Cfg<NH>;
   static std::once_flag once;
   static int max_pairs = 0;
   std::call_once(once, [] {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(gemm_pair_kernel<NH, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg::kAlloc) != cudaSuccess) {
       cudaGetLastError();
       return;
@@ -537,7 +606,7 @@ static int resident_pairs() {
     a[0].val.clusterDim.x = 2; a[0].val.clusterDim.y = 1; a[0].val.clusterDim.z = 1;
     q.attrs = a; q.numAttrs = 1;
     int n_cl = 0;
-    if (cudaOccupancyMaxActiveClusters(&n_cl, gemm_pair_kernel<NH>, &q) == cudaSuccess)
+    if (cudaOccupancyMaxActiveClusters(&n_cl, gemm_pair_kernel<NH, ACT>, &q) == cudaSuccess)
       max_pairs = n_cl;
     else
       cudaGetLastError();
@@ -545,15 +614,16 @@ static int resident_pairs() {
   return max_pairs;
 }
 
-template <int NH>
+template <int NH, bool ACT>
 static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmLargeParams& p,
                        cudaStream_t stream) {
   using Cfg = G2Cfg<NH>;
   static PerDeviceOnce attr_once;
-  FK_CUDA_OK(set_max_dynamic_smem(attr_once, gemm_pair_kernel<NH>, Cfg::kAlloc));
-  const int max_pairs = resident_pairs<NH>();
+  FK_CUDA_OK(set_max_dynamic_smem(attr_once, gemm_pair_kernel<NH, ACT>, Cfg::kAlloc));
+  const int max_pairs = resident_pairs<NH, ACT>();
   FK_REQUIRE(max_pairs > 0, FK_ERR_CUDA, "fk_gemm_bf16: no CTA pair fits on this device");
-  const int64_t tiles = (int64_t)p.m_tiles * ((p.n + Cfg::kTileN - 1) / Cfg::kTileN);
+  constexpr int kOutN = ACT ? Cfg::kTileN / 2 : Cfg::kTileN;
+  const int64_t tiles = (int64_t)p.m_tiles * ((p.n + kOutN - 1) / kOutN);
   const int pairs = (int)(tiles < max_pairs ? tiles : max_pairs);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(2u * (unsigned)pairs);
@@ -572,7 +642,7 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
   ++na;
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  FK_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NH>, mx, mw, p));
+  FK_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<NH, ACT>, mx, mw, p));
   count_launch(1);
   return FK_OK;
 }
@@ -590,17 +660,50 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
 static int large_mode(const GemmLargeParams& p) {
   auto rounds = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
-  const int pairs = resident_pairs<1>();
+  const int pairs = resident_pairs<1, false>();
   if (pairs <= 0) return 0;
   const double single = rounds(tiles, sm_count());
   const double t_single = single * (12. + 0.01 * p.k);
   const double t_pair = 6. + 0.0072 * p.k * rounds(tiles, pairs);
   if (t_pair < t_single) return 1;
-  const int wide = resident_pairs<2>();
+  const int wide = resident_pairs<2, false>();
   if (p.k >= 4096 && single >= 2. && wide > 0 &&
       rounds((int64_t)p.m_tiles * ((p.n_tiles + 1) / 2), wide) <= single)
     return 2;
   return 0;
+}
+
+template <bool ACT>
+static int launch_large(const void* x, int64_t x_stride, const void* w, GemmLargeParams& p,
+                        cudaStream_t stream) {
+  p.m_tiles = (int)(((int64_t)p.m + GL_BM - 1) / GL_BM);
+  const int64_t w_rows = ACT ? 2ll * p.n : p.n;
+  p.n_tiles = (int)((w_rows + GL_BN - 1) / GL_BN);
+  const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
+  FK_REQUIRE(tiles <= 0x7fffffff, FK_ERR_UNSUPPORTED, "fk_gemm_bf16: too many tiles");
+
+  // FK_B200_GEMM_PAIR: 0, 1 or 2 for one kernel at all sizes (see large_mode)
+  static const int forced = [] {
+    const char* e = getenv("FK_B200_GEMM_PAIR");
+    return e != nullptr ? atoi(e) : -1;
+  }();
+  const int mode = forced >= 0 ? forced : large_mode(p);
+  const bool pair = mode == 1 || mode == 2;
+  CUtensorMap mx, mw;
+  int rc = gl_map(x, p.m, p.k, x_stride, pair ? 128 : 256, &mx);
+  if (rc != FK_OK) return rc;
+  rc = gl_map(w, w_rows, p.k, p.k, pair || ACT ? 128 : 256, &mw);
+  if (rc != FK_OK) return rc;
+  if (pair)
+    return mode == 2 ? launch_pair<2, ACT>(mx, mw, p, stream)
+                     : launch_pair<1, ACT>(mx, mw, p, stream);
+  static PerDeviceOnce attr_once;
+  FK_CUDA_OK(set_max_dynamic_smem(attr_once, gemm_large_kernel<ACT>, GL_SMEM_ALLOC));
+  const int ctas = (int)(tiles < sm_count() ? tiles : sm_count());
+  FK_CUDA_OK(launch_kernel(gemm_large_kernel<ACT>, dim3((unsigned)ctas), dim3(GL_THREADS),
+                           (size_t)GL_SMEM_ALLOC, stream, mx, mw, p));
+  count_launch(1);
+  return FK_OK;
 }
 
 // Called by fk_gemm_bf16 for m > 256 after its argument checks.
@@ -615,38 +718,40 @@ int gemm_large_launch(const void* x, int64_t x_stride, const void* w, const void
   p.y = static_cast<uint16_t*>(y);
   p.y_stride = y_stride;
   p.m = (int)m; p.n = (int)n; p.k = (int)k;
-  p.m_tiles = (int)((m + GL_BM - 1) / GL_BM);
-  p.n_tiles = (int)((n + GL_BN - 1) / GL_BN);
   p.status = status;
-  const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
-  FK_REQUIRE(tiles <= 0x7fffffff, FK_ERR_UNSUPPORTED, "fk_gemm_bf16: too many tiles");
-
-  // FK_B200_GEMM_PAIR: 0, 1 or 2 for one kernel at all sizes (see large_mode)
-  static const int forced = [] {
-    const char* e = getenv("FK_B200_GEMM_PAIR");
-    return e != nullptr ? atoi(e) : -1;
-  }();
-  const int pair_mode = forced >= 0 ? forced : large_mode(p);
-  CUtensorMap mx, mw;
-  if (pair_mode == 1 || pair_mode == 2) {
-    int rc = gl_map(x, m, k, x_stride, 128, &mx);
-    if (rc != FK_OK) return rc;
-    rc = gl_map(w, n, k, k, 128, &mw);
-    if (rc != FK_OK) return rc;
-    return pair_mode == 2 ? launch_pair<2>(mx, mw, p, stream) : launch_pair<1>(mx, mw, p, stream);
-  }
-
-  int rc = gl_map(x, m, k, x_stride, 256, &mx);
-  if (rc != FK_OK) return rc;
-  rc = gl_map(w, n, k, k, 256, &mw);
-  if (rc != FK_OK) return rc;
-  static PerDeviceOnce attr_once;
-  FK_CUDA_OK(set_max_dynamic_smem(attr_once, gemm_large_kernel, GL_SMEM_ALLOC));
-  const int ctas = (int)(tiles < sm_count() ? tiles : sm_count());
-  FK_CUDA_OK(launch_kernel(gemm_large_kernel, dim3((unsigned)ctas), dim3(GL_THREADS),
-                           (size_t)GL_SMEM_ALLOC, stream, mx, mw, p));
-  count_launch(1);
-  return FK_OK;
+  return launch_large<false>(x, x_stride, w, p, stream);
 }
 
 }  // namespace fk
+
+using namespace fk;
+
+extern "C" int fk_gemm_bf16_act_mul_many(const void* x, int64_t x_stride, const void* w,
+                                         const void* bias, void* y, int64_t y_stride, int64_t m,
+                                         int64_t n, int64_t k, int act, int32_t* status,
+                                         fk_stream_t stream) {
+  FK_REQUIRE(act == FK_ACT_SILU || act == FK_ACT_GELU_TANH, FK_ERR_INVALID_ARG,
+             "fk_gemm_bf16_act_mul_many: unknown activation %d", act);
+  FK_REQUIRE(m >= 0 && n >= 0 && k > 0 && n % 2 == 0, FK_ERR_INVALID_ARG,
+             "fk_gemm_bf16_act_mul_many: bad sizes");
+  if (m == 0 || n == 0) return FK_OK;
+  FK_REQUIRE(x && w && y, FK_ERR_INVALID_ARG, "fk_gemm_bf16_act_mul_many: null pointer");
+  const int64_t half = n / 2;
+  FK_REQUIRE(k % GL_BK == 0 && half % 8 == 0, FK_ERR_UNSUPPORTED,
+             "fk_gemm_bf16_act_mul_many: k must be a multiple of 64, n of 16");
+  FK_REQUIRE(m < (1ll << 31) && n < (1ll << 31) && k < (1ll << 31), FK_ERR_UNSUPPORTED,
+             "fk_gemm_bf16_act_mul_many: dimension too large");
+  FK_REQUIRE(x_stride >= k && y_stride >= half, FK_ERR_INVALID_ARG,
+             "fk_gemm_bf16_act_mul_many: row stride smaller than the row");
+  FK_REQUIRE(aligned16(x) && aligned16(w) && aligned16(y) && aligned16(bias) &&
+                 x_stride % 8 == 0 && y_stride % 8 == 0,
+             FK_ERR_ALIGNMENT, "fk_gemm_bf16_act_mul_many: rows need 16-byte alignment");
+  GemmLargeParams p{};
+  p.bias = static_cast<const uint16_t*>(bias);
+  p.y = static_cast<uint16_t*>(y);
+  p.y_stride = y_stride;
+  p.m = (int)m; p.n = (int)half; p.k = (int)k;
+  p.act = act;
+  p.status = status;
+  return launch_large<true>(x, x_stride, w, p, static_cast<cudaStream_t>(stream));
+}

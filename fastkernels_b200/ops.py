@@ -508,6 +508,37 @@ def gemm_silu_mul(x, w, bias=None, out=None, workspace=None, status=None):
     return out
 
 
+# rows from which fk_gemm_bf16 is the many-row kernel, which has a form with the activation in
+# its epilogue
+MANY_ROWS = 256
+
+
+def gemm_act_mul_many_fits(x, w, bias=None) -> bool:
+    """True when gemm_act_mul_many takes these operands."""
+    m, k = x.shape
+    return m > MANY_ROWS and x.dtype == BF16 and w.shape[0] % 16 == 0 and k % 64 == 0 and \
+        x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and \
+        (bias is None or bias.data_ptr() % 16 == 0)
+
+
+def gemm_act_mul_many(x, w, act, bias=None, out=None, status=None):
+    """act(x @ wg.T (+ bias)) * (x @ wu.T (+ bias)), w = [wg; wu] rows, for many rows in one
+    launch; gate and up are rounded to bf16 as the projection alone would leave them."""
+    _need(x, BF16, "x")
+    _need(w, BF16, "w")
+    if x.dim() != 2 or x.stride(1) != 1 or not w.is_contiguous():
+        raise _lib.FkError("gemm_act_mul_many needs row-dense x and contiguous w")
+    m, k = x.shape
+    n = w.shape[0]
+    if out is None:
+        out = torch.empty((m, n // 2), dtype=BF16, device=x.device)
+    check(lib.fk_gemm_bf16_act_mul_many(
+        _ptr(x), x.stride(0) if m else k, _ptr(w), _ptr(bias), _ptr(out),
+        out.stride(0) if m else n // 2, m, n, k, int(act), _status_ptr(status, x), _stream()),
+        "fk_gemm_bf16_act_mul_many")
+    return out
+
+
 def gemm_act_mul(x, w, act, bias=None, out=None, workspace=None, status=None):
     """act(x @ wg.T (+ bias)) * (x @ wu.T (+ bias)), w = [wg; wu] rows: one launch where
     the shape has one (see gemm_silu_mul_fusable), else the projection followed by
@@ -529,6 +560,11 @@ def gemm_act_mul(x, w, act, bias=None, out=None, workspace=None, status=None):
             workspace.numel() * workspace.element_size(), _status_ptr(status, x), _stream()),
             "fk_gemm_bf16_act_mul")
         return out
+    if out is None and x.is_cuda and x.dtype == w.dtype and x.stride(1) == 1 and \
+            w.is_contiguous() and w.shape[0] == 2 * half and \
+            (bias is None or (bias.dtype == BF16 and bias.is_contiguous())) and \
+            gemm_act_mul_many_fits(x, w, bias):
+        return gemm_act_mul_many(x, w, act, bias=bias, status=status)
     return act_and_mul(gemm(x, w, bias=bias, workspace=workspace, status=status), act, out=out)
 
 

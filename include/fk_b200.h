@@ -625,6 +625,11 @@ int fk_rope_rms_store(const void* q, const void* k, int64_t in_stride, int is_f3
 int fk_act_and_mul(const void* x, int64_t x_stride, void* out, int64_t out_stride, int is_f32,
                    int64_t rows, int64_t d, int act, fk_stream_t stream);
 
+/* The same for many rows (prompts; the kernels that fk_gemm_bf16 takes above 256 rows): any n
+ * that is a multiple of 16, no workspace; y and bias rows 16-byte aligned. */
+int fk_gemm_bf16_act_mul_many(const void* x, int64_t x_stride, const void* w, const void* bias,
+                              void* y, int64_t y_stride, int64_t m, int64_t n, int64_t k, int act,
+                              int32_t* status, fk_stream_t stream);
 /* fk_gemm_bf16_silu_mul with a choice of activation; same single-launch shapes. */
 int fk_gemm_bf16_act_mul(const void* x, int64_t x_stride, const void* w, const void* bias,
                          void* y, int64_t y_stride, int64_t m, int64_t n, int64_t k, int act,

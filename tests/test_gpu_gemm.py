@@ -264,3 +264,45 @@ def test_gemm_silu_mul_refuses_shapes_without_single_launch_form(ops):
     with pytest.raises(_lib.FkError, match="FK_ERR_UNSUPPORTED"):
         ops.gemm_silu_mul(x, w)
     assert _lib.lib.fk_launch_count() == before
+
+
+@pytest.mark.parametrize("mode", ["", "0", "1", "2"])
+def test_gemm_act_mul_many_rows(mode):
+    """Gate and up projection with the activation in the many-row kernels' epilogue: the bits of
+    the projection followed by the activation kernel, at part-filled tiles of every kernel."""
+    import os
+    import subprocess
+    import sys
+    code = r"""
+import sys
+import torch
+sys.path.insert(0, 'tests')
+from fastkernels_b200 import _lib, ops
+for (m, n, k, bias) in [(257, 16, 64, True), (300, 272, 192, False), (513, 2064, 128, True),
+                        (1000, 4096, 256, False), (2049, 1536, 64, True)]:
+    g = torch.Generator(device='cuda').manual_seed(m)
+    x = torch.empty((m, k + 8), dtype=torch.bfloat16, device='cuda').normal_(generator=g)[:, :k]
+    w = torch.empty((n, k), dtype=torch.bfloat16, device='cuda').normal_(0, 0.2, generator=g)
+    b = torch.empty(n, dtype=torch.bfloat16, device='cuda').normal_(generator=g) if bias else None
+    for act in (_lib.ACT_SILU, _lib.ACT_GELU_TANH):
+        out = torch.zeros((m, n // 2 + 8), dtype=torch.bfloat16, device='cuda')
+        st = ops.new_status('cuda')
+        c0 = _lib.lib.fk_launch_count()
+        ops.gemm_act_mul_many(x, w, act, bias=b, out=out[:, :n // 2], status=st)
+        assert _lib.lib.fk_launch_count() - c0 == 1
+        want = ops.act_and_mul(ops.gemm_bf16(x, w, b), act)
+        torch.cuda.synchronize()
+        assert int(st.item()) == 0
+        assert torch.equal(out[:, :n // 2], want), (m, n, k, act)
+        assert float(out[:, n // 2:].abs().max()) == 0.0
+        assert torch.equal(ops.gemm_act_mul(x, w, act, bias=b), want)
+print('act ok')
+"""
+    env = dict(os.environ)
+    env.pop("FK_B200_GEMM_PAIR", None)
+    if mode:
+        env["FK_B200_GEMM_PAIR"] = mode
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and "act ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
