@@ -295,7 +295,8 @@ class DecodeEngine:
         dev = self.device
         ids = np.concatenate([np.asarray(t, dtype=np.int64) for _, _, t in portions])
         pos = np.concatenate([np.arange(a, a + len(t), dtype=np.int64) for _, a, t in portions])
-        i32 = []                           # all int32 metadata travels in one copy
+        # token ids, positions and all int32 metadata travel in one copy
+        i32 = [ids.view(np.int32), pos.view(np.int32)]
 
         def put(a):
             a = np.ascontiguousarray(a, dtype=np.int32)
@@ -324,7 +325,8 @@ class DecodeEngine:
                                         [len(t) for _, _, t in portions]))
             cu_shape = put(np.concatenate([[0], np.cumsum([len(t) for _, _, t in portions])]))
         flat = torch.from_numpy(np.concatenate(i32)).to(dev)
-        at = 0
+        at = 4 * len(ids)
+        ids_dev, pos_dev = flat[:at].view(torch.int64).view(2, -1)
 
         def take(shape):
             nonlocal at
@@ -345,7 +347,7 @@ class DecodeEngine:
                     cu_portions=take(cu_shape) if cu_shape is not None else None,
                     longest_portion=max(len(t) for _, _, t in portions))
         try:
-            hidden = self.model(torch.from_numpy(ids).to(dev), torch.from_numpy(pos).to(dev))
+            hidden = self.model(ids_dev, pos_dev)
         finally:
             reset_context()
         for blocks in self.span_blocks:

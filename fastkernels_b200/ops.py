@@ -24,7 +24,9 @@ BF16 = torch.bfloat16
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the handle of torch.cuda.current_stream() without making a Stream object for it (about 5 us
+    # of each launch, a quarter of what a short prompt's launches cost the host)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:
@@ -49,6 +51,9 @@ _DEFAULT_STATUS: dict = {}
 def default_status(device=None) -> torch.Tensor:
     """The status word (one per device, made on first use) that wrappers called
     without `status=` hand to their kernels."""
+    st = _DEFAULT_STATUS.get(device)         # a device with its index
+    if st is not None:
+        return st
     key = torch.device("cuda", torch.cuda.current_device()) if device is None \
         else torch.device(device)
     if key.index is None:
@@ -431,6 +436,9 @@ def gemm_workspace(device) -> torch.Tensor:
     largest m, zero-initialised once.  The kernel leaves it zeroed, and GEMMs on
     one stream run one after the other, so a single buffer serves them all; a
     caller that runs GEMMs concurrently on several streams passes its own."""
+    ws = _GEMM_WS.get(device)                # a device with its index
+    if ws is not None:
+        return ws
     key = torch.device(device)
     if key.index is None and key.type == "cuda":
         key = torch.device("cuda", torch.cuda.current_device())
