@@ -10,6 +10,7 @@
 #include "fk_types.cuh"
 
 #include <cmath>
+#include <mutex>
 
 namespace fk {
 
@@ -240,6 +241,37 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 1 : 2)
   }
 }
 
+// CTAs that are resident at once as clusters of `parts` (GPC boundaries keep some SMs out of
+// large ones): a property of the GPU model, asked once.
+template <int WR, int WC, bool ACT>
+static int f32_slots(int parts) {
+  static std::once_flag once;
+  static int slots[4];
+  std::call_once(once, [] {
+    using Tile = F32Tile<WR, WC>;
+    for (int i = 0; i < 4; ++i) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(1024);
+      cfg.blockDim = dim3(Tile::kThreads);
+      cfg.dynamicSmemBytes = Tile::kSmem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 1u << i;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, f32_product_kernel<WR, WC, ACT>, &cfg) !=
+          cudaSuccess) {
+        cudaGetLastError();
+        n = 0;
+      }
+      slots[i] = n << i;
+    }
+  });
+  return slots[parts == 8 ? 3 : parts == 4 ? 2 : parts == 2 ? 1 : 0];
+}
+
 template <int WR, int WC, bool ACT>
 static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
   using Tile = F32Tile<WR, WC>;
@@ -250,17 +282,22 @@ static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
   const int64_t used = p.rows < p.groups ? p.rows : p.groups;
   const int64_t row_tiles = p.offsets ? upto + used : upto;
   const double tiles = (double)n_tiles * (p.offsets ? upto + used * 0.5 : (double)upto * p.groups);
-  // parts of k: those that fill the last round of CTAs best; each costs a reduction
-  const int slots = sm_count() * (WR * WC == 8 ? 1 : 2);
-  int parts = 1;
-  double best = 0.;
-  for (int c = 1; c <= 8 && p.k >= 128 * c && n_tiles * c < (1ll << 31); c *= 2) {
-    const double rounds = tiles * c / slots;
-    const double full = rounds / (double)(int64_t)(rounds + 0.999) * (c == 1 ? 1.0 : 0.97 - 0.01 * c);
-    if (full > best) { best = full; parts = c; }
-  }
+  // Parts of k: rounds of CTAs times what a round takes, 0.105 us a k (of a small tile
+  // that has its SM to itself 0.06) and 6.5 us around it.  k 2048, measured (us) in 1, 2, 4, 8 parts: 16 tiles
+  // 221 121 66 74, 64 tiles 221 123 128 172, 192 tiles 427 344 364 432, 384 tiles 657 692 737 885.
   static PerDeviceOnce once;
   FK_CUDA_OK(set_max_dynamic_smem(once, f32_product_kernel<WR, WC, ACT>, Tile::kSmem));
+  constexpr double kPerK = WR * WC == 8 ? 0.105 : WR * WC == 4 ? 0.11 : 0.08;
+  int parts = 1;
+  double best = 0.;
+  for (int c = 1; c <= 8 && p.k >= 64 * c && n_tiles * c < (1ll << 31); c *= 2) {
+    const int slots = f32_slots<WR, WC, ACT>(c);
+    if (slots == 0) continue;
+    const double rounds = ceil(tiles * c / slots);
+    const double per_k = WR * WC < 8 && tiles * c <= sm_count() ? 0.06 : kPerK;
+    const double t = rounds * (per_k * p.k / c + 6.5);
+    if (best == 0. || t < best) { best = t; parts = c; }
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(n_tiles * parts), (unsigned)(row_tiles < 65535 ? row_tiles : 65535),
                      p.offsets ? 1u : (unsigned)p.groups);
