@@ -71,13 +71,23 @@ struct Gate {
   }
 };
 
-// CTA = 16 tokens, some heads in turn.  VEC (blocks of bf16, rows of whole 16-byte pieces): a
-// thread takes 8 channels of a token, one 16-byte load per input, all requested before the decay
-// projection; the sum of k^2 stays within the lanes of the token.
+// CTA = 16 tokens, some heads in turn.  VEC (bf16, rows of whole 16-byte pieces): a thread takes
+// 8 channels of a token, one 16-byte load per input, all requested before the decay projection
+// (the first head's before the tanh too); the sum of k^2 stays within the lanes of the token.
 template <typename T, int DP, bool BLOCKED, bool VEC>
 __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPrepParams p) {
   extern __shared__ __align__(16) uint8_t dl_prep_smem[];
   pdl_launch_dependents();
+  if (VEC && !BLOCKED) {
+    // a decode step finds the decay projection's weights in HBM: towards L2 while the kernel
+    // in front still runs
+    const char* w2 = reinterpret_cast<const char*>(
+        static_cast<const T*>(p.w2) + (int64_t)blockIdx.y * p.heads_per_cta * p.d * p.w2_stride);
+    const int heads = min(p.heads_per_cta, p.heads - (int)blockIdx.y * p.heads_per_cta);
+    const int64_t bytes = (int64_t)heads * p.d * p.w2_stride * (int64_t)sizeof(T);
+    for (int64_t i = (int64_t)threadIdx.x * 128; i < bytes; i += DL_THREADS * 128)
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(w2 + i));
+  }
   pdl_wait();
   constexpr bool MMA = sizeof(T) == 2;
   constexpr int NW = DL_THREADS / 32;
@@ -104,6 +114,26 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
   float* vec = reinterpret_cast<float*>(dl_prep_smem) + DL_UNIT * ld;   // [6][16][DP]
   float* part = vec + DL_FIELDS * DL_UNIT * DP;                  // [16][DP / 32]
   float* unit = part + DL_UNIT * (DP / 32);                      // [16]
+  constexpr int TPT = DP / 8, TOKS = DL_THREADS / TPT;    // VEC: threads a token, tokens a pass
+  constexpr int NP8 = VEC ? (DL_UNIT + TOKS - 1) / TOKS : 1;
+  const int c8 = (int)(threadIdx.x % TPT) * 8;
+  uint4 k8[NP8], a8[NP8], r8[NP8], v8[NP8];
+  auto fetch8 = [&](int head) {
+#pragma unroll
+    for (int x = 0; x < NP8; ++x) {
+      const int t = (int)threadIdx.x / TPT + x * TOKS;
+      k8[x] = a8[x] = r8[x] = v8[x] = make_uint4(0u, 0u, 0u, 0u);
+      if (t < nt && c8 < p.d) {
+        const int64_t o = (t0 + t) * p.in_stride + (int64_t)head * p.d + c8;
+        k8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.k) + o));
+        a8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.a) + o));
+        r8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.r) + o));
+        v8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.v) + o));
+      }
+    }
+  };
+  const int h0 = blockIdx.y * p.heads_per_cta;
+  if (VEC) fetch8(h0);
   for (int i = threadIdx.x; i < DL_UNIT * rank_p; i += DL_THREADS) {
     const int t = i / rank_p, r = i - t * rank_p;
     float z = 0.f;
@@ -125,7 +155,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
     scal_off = 16 + f * 16 + row * 4 + (t - row * (row + 1) / 2);
   }
   const int h1 = min((int)(blockIdx.y + 1) * p.heads_per_cta, p.heads);
-  for (int h = blockIdx.y * p.heads_per_cta; h < h1; ++h) {
+  for (int h = h0; h < h1; ++h) {
     __syncthreads();       // tanh written; vec and unit of the last head consumed
     const int64_t ch0 = (int64_t)h * p.d;
     // this thread's elements of the head's [16][DP] tile.  Single tokens: requested before
@@ -157,24 +187,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
       w0c[x] = on ? __ldg(p.w0 + ch0 + chan(x)) : 0.f;
       abc[x] = on ? __ldg(p.a_bias + ch0 + chan(x)) : 0.f;
     }
-    constexpr int TPT = DP / 8, TOKS = DL_THREADS / TPT;  // VEC: threads a token, tokens a pass
-    constexpr int NP8 = VEC ? (DL_UNIT + TOKS - 1) / TOKS : 1;
-    const int c8 = (int)(threadIdx.x % TPT) * 8;
-    uint4 k8[NP8], a8[NP8], r8[NP8], v8[NP8];
-    if (VEC) {
-#pragma unroll
-      for (int x = 0; x < NP8; ++x) {
-        const int t = (int)threadIdx.x / TPT + x * TOKS;
-        k8[x] = a8[x] = r8[x] = v8[x] = make_uint4(0u, 0u, 0u, 0u);
-        if (t < nt && c8 < p.d) {
-          const int64_t o = (t0 + t) * p.in_stride + ch0 + c8;
-          k8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.k) + o));
-          a8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.a) + o));
-          r8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.r) + o));
-          v8[x] = __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.v) + o));
-        }
-      }
-    }
+    if (VEC && h != h0) fetch8(h);
     T kx[PASS], ax[PASS], rx[PASS], vx[PASS];
     auto fetch = [&](int x0) {
 #pragma unroll
@@ -189,7 +202,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
         }
       }
     };
-    if (!BLOCKED) fetch(0);
+    if (!BLOCKED && !VEC) fetch(0);
     // decay projection into field 0
     if (MMA) {
       const int kq = (lane & 3) * 2, r0 = lane >> 2;
@@ -288,12 +301,18 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
               b[e] = u[e] * Gate<T>::sigmoid(pick(aw) + abv[e]);
             }
           }
-          *reinterpret_cast<float4*>(vec + i) = make_float4(w[0], w[1], w[2], w[3]);
-          *reinterpret_cast<float4*>(vec + F + i) = make_float4(u[0], u[1], u[2], u[3]);
-          *reinterpret_cast<float4*>(vec + 2 * F + i) = make_float4(b[0], b[1], b[2], b[3]);
-          *reinterpret_cast<float4*>(vec + 3 * F + i) = make_float4(k[0], k[1], k[2], k[3]);
-          *reinterpret_cast<float4*>(vec + 4 * F + i) = make_float4(r[0], r[1], r[2], r[3]);
-          *reinterpret_cast<float4*>(vec + 5 * F + i) = make_float4(v[0], v[1], v[2], v[3]);
+          // blocks: into the tile; single tokens: straight to the token's fields
+          if (!BLOCKED && t >= nt) continue;
+          float* dst = BLOCKED ? vec + i
+                               : p.packed + (((int64_t)h * p.rows + t0 + t) * DL_FIELDS) * DP + c8 +
+                                     half * 4;
+          constexpr int S = BLOCKED ? F : DP;
+          *reinterpret_cast<float4*>(dst) = make_float4(w[0], w[1], w[2], w[3]);
+          *reinterpret_cast<float4*>(dst + S) = make_float4(u[0], u[1], u[2], u[3]);
+          *reinterpret_cast<float4*>(dst + 2 * S) = make_float4(b[0], b[1], b[2], b[3]);
+          *reinterpret_cast<float4*>(dst + 3 * S) = make_float4(k[0], k[1], k[2], k[3]);
+          *reinterpret_cast<float4*>(dst + 4 * S) = make_float4(r[0], r[1], r[2], r[3]);
+          *reinterpret_cast<float4*>(dst + 5 * S) = make_float4(v[0], v[1], v[2], v[3]);
         }
       }
     } else {
@@ -772,17 +791,18 @@ static int launch_prepare_one(const DeltaPrepParams& p, unsigned gx, cudaStream_
 }
 template <typename T, int DP>
 static int launch_prepare_dp(const DeltaPrepParams& p, bool blocked, cudaStream_t s) {
-  if (blocked) {
-    // rows of whole 16-byte pieces, where 2-byte loads waited for one another: five prompts of
-    // 700 to 2500 tokens, 64 heads of 64 687 -> 436 us, 24 heads of 128 765 -> 335
-    if constexpr (sizeof(T) == 2) {
-      if (p.d % 8 == 0 && p.in_stride % 8 == 0 && aligned16(p.r) && aligned16(p.k) &&
-          aligned16(p.v) && aligned16(p.a) && aligned16(p.w0) && aligned16(p.a_bias))
-        return launch_prepare_one<T, DP, true, true>(p, (unsigned)p.units, s);
-    }
-    return launch_prepare_one<T, DP, true, false>(p, (unsigned)p.units, s);
+  const unsigned single = (unsigned)((p.rows + DL_UNIT - 1) / DL_UNIT);
+  // rows of whole 16-byte pieces, where 2-byte loads waited for one another: five prompts of
+  // 700 to 2500 tokens, 64 heads of 64 687 -> 436 us, 24 heads of 128 765 -> 335;
+  // a decode step of 16 rows, 32 heads of 64, 10.9 -> 8.2
+  if constexpr (sizeof(T) == 2) {
+    if (p.d % 8 == 0 && p.in_stride % 8 == 0 && aligned16(p.r) && aligned16(p.k) &&
+        aligned16(p.v) && aligned16(p.a) && aligned16(p.w0) && aligned16(p.a_bias))
+      return blocked ? launch_prepare_one<T, DP, true, true>(p, (unsigned)p.units, s)
+                     : launch_prepare_one<T, DP, false, true>(p, single, s);
   }
-  return launch_prepare_one<T, DP, false, false>(p, (unsigned)((p.rows + DL_UNIT - 1) / DL_UNIT), s);
+  return blocked ? launch_prepare_one<T, DP, true, false>(p, (unsigned)p.units, s)
+                 : launch_prepare_one<T, DP, false, false>(p, single, s);
 }
 template <typename T>
 static int launch_prepare(const DeltaPrepParams& p, bool blocked, cudaStream_t s) {

@@ -455,8 +455,9 @@ def test_one_standing_out_key_at_every_edge(chunk, block, decode, dtype):
 
 
 # ------------------------------------------------------------------------- delta rule
+@pytest.mark.parametrize("blocked", [True, False])
 @pytest.mark.parametrize("heads,dim,rank", [(3, 24, 5), (2, 64, 40), (2, 128, 64), (1, 256, 17)])
-def test_delta_prepare_of_whole_pieces(heads, dim, rank):
+def test_delta_prepare_of_whole_pieces(heads, dim, rank, blocked):
     """Rows of 16-byte pieces take the wide loads: the same operands as from the same rows one
     element further on, which take the others.  Portions that end within a unit and a block."""
     from fastkernels_b200 import ops
@@ -468,13 +469,14 @@ def test_delta_prepare_of_whole_pieces(heads, dim, rank):
     further[:, 1:z.shape[1] + 1] = zd
     w2 = dev(rs.randn(hd, (rank + 3) // 4 * 4) / np.sqrt(rank), BF16)
     w0, ab = dev(rs.uniform(-4, 1, hd)), dev(rs.randn(hd))
-    n = int(ops.lib.fk_delta_packed_floats(rows, len(counts), heads, dim, 1))
+    n = int(ops.lib.fk_delta_packed_floats(rows, len(counts), heads, dim, int(blocked)))
     got = []
     for x, o in ((zd, 0), (further, 1)):
         cols = [x[:, o + i * hd:o + (i + 1) * hd] for i in range(4)]
         packed = torch.zeros(n, device="cuda")
         ops.delta_prepare(*cols, x[:, o + 4 * hd:o + 4 * hd + rank], w2, w0, ab, heads, dim,
-                          float(np.exp(-0.5)), 1e-6, cu_portions=i32(cu), packed=packed)
+                          float(np.exp(-0.5)), 1e-6, cu_portions=i32(cu) if blocked else None,
+                          packed=packed)
         got.append(packed.double().cpu().numpy())
     # only the sum of k^2 is taken in another order
     np.testing.assert_allclose(got[0], got[1], rtol=2e-6, atol=2e-6 * np.abs(got[1]).max())
