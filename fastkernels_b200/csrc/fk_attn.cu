@@ -706,18 +706,34 @@ __global__ void __launch_bounds__(256) attn_merge_kernel(const AttnParams p) {
     return;
   }
   const int64_t base = ((int64_t)seq * p.hq + head) * p.max_splits;
+  // Bound by the latency of what it reads: a lane has the (max, sum) of splits lane, lane + 32,
+  // ..., so all of them are one round of loads, and four partial rows are on the way at a time
+  // (in a decode step 3.4 -> 2.8 us for one sequence of 777 tokens, 8.9 -> 7.8 for 64 long ones).
   float M = -INFINITY;
-  for (int s = 0; s < n; ++s) M = fmaxf(M, p.part_ml[base + s].x);
+  for (int s = lane; s < n; s += 32) M = fmaxf(M, p.part_ml[base + s].x);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
   const float Mu = M == -INFINITY ? 0.f : M;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float lt = 0.f;
-  for (int s = 0; s < n; ++s) {
-    const float2 mlv = p.part_ml[base + s];
-    const float f = fast_exp2(mlv.x - Mu);
-    lt += mlv.y * f;
-    const float4 v =
-        reinterpret_cast<const float4*>(p.part_o + (base + s) * ATT_D)[lane];
-    acc.x += v.x * f; acc.y += v.y * f; acc.z += v.z * f; acc.w += v.w * f;
+  for (int s0 = 0; s0 < n; s0 += 32) {
+    const float2 mlv = s0 + lane < n ? p.part_ml[base + s0 + lane] : make_float2(-INFINITY, 0.f);
+    const float fl = fast_exp2(mlv.x - Mu), ll = mlv.y * fl;
+    const int cnt = min(32, n - s0);
+    const float4* src = reinterpret_cast<const float4*>(p.part_o + (base + s0) * ATT_D) + lane;
+    for (int s = 0; s < cnt; s += 4) {
+      float4 v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[i] = s + i < cnt ? src[(s + i) * (ATT_D / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float f = __shfl_sync(0xffffffffu, fl, s + i), l = __shfl_sync(0xffffffffu, ll, s + i);
+        if (s + i >= cnt) break;
+        lt += l;
+        acc.x += v[i].x * f; acc.y += v[i].y * f; acc.z += v[i].z * f; acc.w += v[i].w * f;
+      }
+    }
   }
   const float inv = lt > 0.f ? 1.0f / lt : 0.f;
   *dst = make_uint2(pack_bf16(acc.x * inv, acc.y * inv),
