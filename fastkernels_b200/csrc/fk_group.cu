@@ -71,8 +71,10 @@ __device__ __forceinline__ int64_t group_x_row(const GroupParams& p, int64_t row
 // A warp = 16 weight rows (of gate and of up with ACT) of one group, and every ks-th chunk
 // of 32 k's; the CTA's warps are ks parts of k by 16-row tiles.  Rows go 8 NT at a time,
 // blocks of them over grid.z.
-template <int NT, bool ACT, typename OUT>
-__global__ void __launch_bounds__(256) group_skinny_kernel(const GroupParams p, int ks) {
+// Column groups: the weights are asked towards L2 ahead of the wait for the kernel in front (their
+// place does not hang on it, and in a decode step they come from HBM); they are read after it.
+template <int NT, bool ACT, typename OUT, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) group_skinny_kernel(const GroupParams p, int ks) {
   extern __shared__ float gs_red[];            // [warps][TILES 16][8 NT + 1]
   pdl_launch_dependents();
   constexpr int TILES = ACT ? 2 : 1;
@@ -92,11 +94,19 @@ __global__ void __launch_bounds__(256) group_skinny_kernel(const GroupParams p, 
       if (r >= p.n) r = p.n - 1;               // computed, not stored
       wr[e][h] = w + ((int64_t)e * p.n + r) * p.k + tq * 8;
     }
+  const int chunks = (p.k + 31) >> 5;
+  constexpr int UN = TILES * 2 + NT <= 6 ? 4 : TILES * 2 + NT <= 8 ? 2 : 1;
+  if (!p.offsets && tq == 0)
+    for (int c = kpart; c < chunks; c += ks)
+#pragma unroll
+      for (int e = 0; e < TILES; ++e)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(wr[e][h] + c * 32));
   pdl_wait();
   int64_t first, count;
   group_range(p, g, &first, &count);
   const uint16_t* x = static_cast<const uint16_t*>(p.x) + (p.offsets ? 0 : g * p.x_group);
-  const int chunks = (p.k + 31) >> 5;
   constexpr int kUnit = 16 / (int)sizeof(OUT);
   const bool vec = p.y_stride % kUnit == 0 && p.y_group % kUnit == 0;
   for (int64_t t0 = (int64_t)blockIdx.z * COLS; t0 < count; t0 += (int64_t)gridDim.z * COLS) {
@@ -115,7 +125,6 @@ __global__ void __launch_bounds__(256) group_skinny_kernel(const GroupParams p, 
       for (int j = 0; j < NT; ++j)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[e][j][i] = 0.f;
-    constexpr int UN = TILES * 2 + NT <= 6 ? 4 : TILES * 2 + NT <= 8 ? 2 : 1;
     for (int c0 = kpart; c0 < chunks; c0 += ks * UN) {
       uint4 a[UN][TILES][2], b[UN][NT];
 #pragma unroll
@@ -793,15 +802,16 @@ static int gg_map(const void* ptr, int64_t rows, int64_t cols, int64_t stride, i
   return FK_OK;
 }
 
-template <int NT, bool ACT, typename OUT>
+template <int NT, bool ACT, typename OUT, int WARPS = 8>
 static int launch_skinny_one(const GroupParams& p, int ks, int fs, cudaStream_t s) {
   constexpr int kPerWarp = (ACT ? 2 : 1) * 16 * (8 * NT + 1) * 4;
   static PerDeviceOnce once;
-  FK_CUDA_OK(set_max_dynamic_smem(once, group_skinny_kernel<NT, ACT, OUT>, 8 * kPerWarp));
+  FK_CUDA_OK(set_max_dynamic_smem(once, group_skinny_kernel<NT, ACT, OUT, WARPS>,
+                                  WARPS * kPerWarp));
   const int64_t blocks = p.offsets ? 1 : (p.rows + 8 * NT - 1) / (8 * NT);
   const dim3 grid((unsigned)((p.n + 16 * fs - 1) / (16 * fs)), (unsigned)p.groups,
                   (unsigned)(blocks < 65535 ? blocks : 65535));
-  FK_CUDA_OK(launch_kernel(group_skinny_kernel<NT, ACT, OUT>, grid, dim3(32u * ks * fs),
+  FK_CUDA_OK(launch_kernel(group_skinny_kernel<NT, ACT, OUT, WARPS>, grid, dim3(32u * ks * fs),
                            (size_t)ks * fs * kPerWarp, s, p, ks));
   count_launch();
   return FK_OK;
@@ -816,6 +826,14 @@ static int launch_skinny(const GroupParams& p, int64_t expect, cudaStream_t s) {
   if (!p.offsets) {
     const int64_t tiles = (int64_t)((p.n + 16 * fs - 1) / (16 * fs)) * p.groups;
     while (nt > 1 && tiles * ((p.rows + 8 * nt - 1) / (8 * nt)) < sm_count()) nt /= 2;
+  }
+  // narrow products (a router, gates): few CTAs, so sixteen warps share k in each (9
+  // rows, n 32, k 2048 7.4 -> 4.1 us in a decode step, 64 rows, n 64, k 4096 12.9 -> 7.0; the
+  // weights asked for early are about half of it)
+  if constexpr (!ACT) {
+    const int64_t ctas = (int64_t)((p.n + 15) / 16) * p.groups * ((p.rows + 7) / 8);
+    if (nt == 1 && !p.offsets && chunks >= 32 && ctas <= sm_count())
+      return launch_skinny_one<1, ACT, OUT, 16>(p, 16, 1, s);
   }
   if (nt == 1) return launch_skinny_one<1, ACT, OUT>(p, ks, fs, s);
   if (nt == 2) return launch_skinny_one<2, ACT, OUT>(p, ks, fs, s);

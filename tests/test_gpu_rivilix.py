@@ -173,6 +173,25 @@ def test_column_groups(rows, groups, n, k, dtype):
         assert torch.all(got[:, :, n:] == 3.0)
 
 
+@pytest.mark.parametrize("rows", [1, 9, 40])
+@pytest.mark.parametrize("n,k", [(1, 1024), (31, 2056), (64, 1032)])
+def test_narrow_products(rows, n, k):
+    """Few outputs of a long row (routers, gates): sixteen warps share k, which may end inside
+    a turn of theirs; fp32 and bf16 results, two groups side by side."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(n)
+    x, w = values(rs, rows, 2 * k, dtype=BF16), values(rs, 2, n, k, dtype=BF16) / 8
+    bias = values(rs, n)
+    one = x[:, :k] @ w[0].T + bias
+    got = ops.group_gemm(dev(x, BF16)[:, :k], dev(w, BF16)[0], bias=dev(bias), out_f32=True)
+    close(got, one, F32, scale=np.abs(one).max())
+    pitch = (n + 7) // 8 * 8
+    two = ops.group_gemm(dev(x, BF16), dev(w, BF16), x_group=k, y_group=pitch)
+    for g in range(2):
+        want = x[:, g * k:(g + 1) * k] @ w[g].T
+        close(two[:, g * pitch:g * pitch + n], want, BF16, scale=np.abs(want).max())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("act", [None, 0, 1])
 @pytest.mark.parametrize("counts", [[3, 0, 1, 9], [0, 0, 0, 1], [70, 0, 129, 1, 128, 300],
