@@ -537,9 +537,18 @@ def gemm_act_mul_many(x, w, act, bias=None, out=None, status=None):
     if x.dim() != 2 or x.stride(1) != 1 or not w.is_contiguous():
         raise _lib.FkError("gemm_act_mul_many needs row-dense x and contiguous w")
     m, k = x.shape
+    if w.dim() != 2 or w.shape[1] != k:
+        raise _lib.FkError(f"gemm_act_mul_many: w of shape {tuple(w.shape)} for rows of {k}")
     n = w.shape[0]
+    if bias is not None:
+        _need(bias, BF16, "bias")
+        if bias.shape != (n,) or not bias.is_contiguous():
+            raise _lib.FkError("gemm_act_mul_many: bias must be contiguous, one entry per row of w")
     if out is None:
         out = torch.empty((m, n // 2), dtype=BF16, device=x.device)
+    _need(out, BF16, "out")
+    if out.dim() != 2 or out.shape[0] < m or out.shape[1] < n // 2 or out.stride(1) != 1:
+        raise _lib.FkError(f"gemm_act_mul_many: out must be row-dense, at least {m} x {n // 2}")
     check(lib.fk_gemm_bf16_act_mul_many(
         _ptr(x), x.stride(0) if m else k, _ptr(w), _ptr(bias), _ptr(out),
         out.stride(0) if m else n // 2, m, n, k, int(act), _status_ptr(status, x), _stream()),
@@ -569,9 +578,7 @@ def gemm_act_mul(x, w, act, bias=None, out=None, workspace=None, status=None):
             "fk_gemm_bf16_act_mul")
         return out
     if out is None and x.is_cuda and x.dtype == w.dtype and x.stride(1) == 1 and \
-            w.is_contiguous() and w.shape[0] == 2 * half and \
-            (bias is None or (bias.dtype == BF16 and bias.is_contiguous())) and \
-            gemm_act_mul_many_fits(x, w, bias):
+            w.is_contiguous() and w.shape[0] == 2 * half and gemm_act_mul_many_fits(x, w, bias):
         return gemm_act_mul_many(x, w, act, bias=bias, status=status)
     return act_and_mul(gemm(x, w, bias=bias, workspace=workspace, status=status), act, out=out)
 

@@ -306,3 +306,27 @@ print('act ok')
     r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and "act ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
+
+
+def test_gemm_act_mul_many_rows_refusals(ops):
+    """Operands that do not belong together raise, and nothing is launched."""
+    from fastkernels_b200 import _lib
+
+    def t(*shape, dtype=torch.bfloat16):
+        return torch.zeros(shape, dtype=dtype, device="cuda")
+    m, n, k = 300, 64, 128
+    x, w, act = t(m, k), t(n, k), _lib.ACT_SILU
+    before = _lib.lib.fk_launch_count()
+    for fn in (ops.gemm_act_mul_many, ops.gemm_act_mul):
+        for bias in (t(n // 2), t(n + 8), t(n, dtype=torch.float32), t(2 * n)[::2],
+                     torch.zeros(n, dtype=torch.bfloat16)):
+            with pytest.raises(_lib.FkError):
+                fn(x, w, act, bias=bias)
+    for bad_w in (t(n, k - 64), t(n, k + 64), t(1, n, k)):
+        with pytest.raises(_lib.FkError):
+            ops.gemm_act_mul_many(x, bad_w, act)
+    for out in (t(m - 1, n // 2), t(m, n // 2 - 8), t(m, n // 2, dtype=torch.float32),
+                t(n // 2, m).T, t(m * n // 2)):
+        with pytest.raises(_lib.FkError):
+            ops.gemm_act_mul_many(x, w, act, out=out)
+    assert _lib.lib.fk_launch_count() == before
