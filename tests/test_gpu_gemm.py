@@ -330,3 +330,50 @@ def test_gemm_act_mul_many_rows_refusals(ops):
         with pytest.raises(_lib.FkError):
             ops.gemm_act_mul_many(x, w, act, out=out)
     assert _lib.lib.fk_launch_count() == before
+
+
+@pytest.mark.parametrize("what", ["none", "hook", "pre_hook", "forward", "module", "global"])
+def test_llama_mlp_prompt_keeps_module_calls(ops, what):
+    """A prompt's gate/up projection runs as one launch only where nobody would notice: hooks on
+    the projection or the activation, and replaced ones, still run."""
+    from types import SimpleNamespace
+
+    from fastkernels_b200 import _lib
+    from fastkernels_b200.candidate.L1.silu_and_mul import SiluAndMul
+    from fastkernels_b200.candidate.L2.llama_mlp import LlamaMLP
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        mlp = LlamaMLP(SimpleNamespace(hidden_size=128, intermediate_size=192)).bfloat16()
+    for p in mlp.parameters():
+        p.requires_grad_(False).normal_(0, 0.1)
+    x = torch.randn(300, 128, dtype=torch.bfloat16, device="cuda")
+    want = mlp.down_proj(mlp.act_fn(mlp.gate_up_proj(x)))
+    calls, handle = [], None
+
+    def seen(*a, **k):
+        calls.append(1)
+    if what == "hook":
+        handle = mlp.gate_up_proj.register_forward_hook(seen)
+    elif what == "pre_hook":
+        handle = mlp.act_fn.register_forward_pre_hook(seen)
+    elif what == "forward":
+        plain = mlp.act_fn.forward
+        mlp.act_fn.forward = lambda z: (seen(), plain(z))[1]
+    elif what == "module":
+        class Other(SiluAndMul):
+            def forward(self, z):
+                seen()
+                return super().forward(z)
+        mlp.act_fn = Other()
+    elif what == "global":
+        handle = torch.nn.modules.module.register_module_forward_hook(
+            lambda m, i, o: seen() if m is mlp.act_fn else None)
+    try:
+        n = _lib.lib.fk_launch_count()
+        got = mlp(x)
+        launches = _lib.lib.fk_launch_count() - n
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert len(calls) == (what != "none") and launches == (2 if what == "none" else 3)
+    assert torch.equal(got, want)
