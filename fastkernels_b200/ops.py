@@ -23,10 +23,16 @@ from ._lib import check, lib
 BF16 = torch.bfloat16
 
 
+# the handle of a device's current stream without a Stream object made for it (about 5 us of each
+# launch, a quarter of what a short prompt's launches cost the host); torch does not promise it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream() -> int:
-    # the handle of torch.cuda.current_stream() without making a Stream object for it (about 5 us
-    # of each launch, a quarter of what a short prompt's launches cost the host)
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    device = torch.cuda.current_device()
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device)
 
 
 def _ptr(t: torch.Tensor | None) -> int | None:

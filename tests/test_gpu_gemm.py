@@ -377,3 +377,15 @@ def test_llama_mlp_prompt_keeps_module_calls(ops, what):
             handle.remove()
     assert len(calls) == (what != "none") and launches == (2 if what == "none" else 3)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("raw", [True, False])
+def test_launch_stream_is_the_current_one(ops, monkeypatch, raw):
+    """Also where torch has no call for the handle alone."""
+    if not raw:
+        monkeypatch.setattr(ops, "_raw_stream", None)
+    side = torch.cuda.Stream()
+    assert ops._stream() == torch.cuda.current_stream().cuda_stream
+    with torch.cuda.stream(side):
+        assert ops._stream() == side.cuda_stream != 0
+    assert ops._stream() == torch.cuda.current_stream().cuda_stream
