@@ -86,6 +86,7 @@ struct BlkCfg {
   static constexpr int kTmemCols = 2 * kAccCols;
   static_assert(kStages >= 3, "pipeline too shallow");
   static_assert(kAlloc <= 232448, "shared memory budget");
+  static_assert(tmem_alone(kAlloc), "two CTAs could wait for one another's tensor memory");
 };
 
 // Diagnostic build only (-DFK_BLOCK_TRACE): per CTA and phase, %globaltimer when the

@@ -60,6 +60,7 @@ struct GemmCfg {
   static_assert(kStages >= 3, "pipeline too shallow");
   static_assert(kAlloc <= 232448, "shared memory budget");
   static_assert(kTmemCols <= 512, "TMEM budget");
+  static_assert(tmem_alone(kAlloc), "two CTAs could wait for one another's tensor memory");
 };
 
 struct GemmParams {

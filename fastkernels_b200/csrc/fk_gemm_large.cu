@@ -43,6 +43,7 @@ constexpr int GL_SMEM_ALLOC = GL_SMEM + 1024;
 constexpr int GL_THREADS = 192;
 constexpr int GL_TMEM_COLS = 512;
 static_assert(GL_SMEM_ALLOC <= 232448, "shared memory budget");
+static_assert(tmem_alone(GL_SMEM_ALLOC), "two CTAs could wait for one another's tensor memory");
 
 struct GemmLargeParams {
   const uint16_t* bias;   // [n] ([2 n] with an activation) or null
@@ -341,6 +342,7 @@ struct G2Cfg {
   static constexpr int kSmem = kOffBar + 256;
   static constexpr int kAlloc = kSmem + 1024;
   static_assert(kAlloc <= 232448, "shared memory budget");
+  static_assert(tmem_alone(kAlloc), "two CTAs could wait for one another's tensor memory");
 };
 
 template <int NH, bool ACT>

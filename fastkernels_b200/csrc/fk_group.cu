@@ -232,6 +232,7 @@ struct GgCfg {
   static constexpr int kOffOut = kOffBar + 256;       // 4 warps x 32 rows x 128 bytes
   static constexpr int kSmem = kOffOut + 4 * 4096 + 1024;
   static_assert(kSmem <= 232448, "shared memory budget");
+  static_assert(tmem_alone(kSmem), "two CTAs could wait for one another's tensor memory");
 };
 
 __device__ __forceinline__ uint64_t gg_ns() {
@@ -566,6 +567,7 @@ struct GtCfg {
   static constexpr int kSmem = kOffUp + (ACT ? 2 * 16 * 64 * 4 : 0) + 1024;
   static constexpr int kTmemCols = 2 * NT;
   static_assert(kSmem <= 232448, "shared memory budget");
+  static_assert(tmem_alone(kSmem), "two CTAs could wait for one another's tensor memory");
   static_assert(kTmemCols >= 32 && (kTmemCols & (kTmemCols - 1)) == 0, "tensor memory");
 };
 
@@ -705,6 +707,7 @@ group_stream_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const uint32_t buf = done & 1u, use = done >> 1;
       // one answer for all four warps: with ACT they meet at barriers below
       if (!gt_all(gg_wait(&acc_full[buf], use & 1u, abort_flag, p.status))) break;
+      __syncwarp();                    // lanes left the wait one by one
       tc_fence_after();
       const int rows = (int)min((int64_t)NT, t.rows_left);
       const int col = t.nt * TN + (ACT ? (q & 1) : q) * 32 + lane;

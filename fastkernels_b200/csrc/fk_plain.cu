@@ -233,6 +233,7 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 1 : 2)
     }
     // peers may still read this CTA's sums; the next tile overwrites them
     if (parts > 1) {
+      __syncwarp();                    // lanes stored different numbers of outputs
       asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
                    "barrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else {

@@ -75,6 +75,7 @@ constexpr int PF_SMEM_ALLOC = PF_SMEM + 1024;
 constexpr int PF_TMEM_COLS = 512;
 constexpr float PF_RESCALE_LOG2 = 8.0f;
 static_assert(PF_SMEM_ALLOC <= 232448, "shared memory budget");
+static_assert(tmem_alone(PF_SMEM_ALLOC), "two CTAs could wait for one another's tensor memory");
 
 struct PrefillParams {
   uint16_t* out; int64_t out_stride;

@@ -5,6 +5,12 @@
 
 namespace fk {
 
+// tcgen05.alloc waits, without a limit, until its columns are free.  A kernel that allocates
+// therefore asks for more than half of an SM's 228 KiB of shared memory (1 KiB a CTA is the
+// system's): no two such CTAs are on one SM, whatever programmatic launch brings in early, and
+// the columns are there.
+constexpr bool tmem_alone(int dynamic_smem) { return dynamic_smem + 1024 > 228 * 1024 / 2; }
+
 #ifdef __CUDACC__
 
 __device__ __forceinline__ void tc_fence_before() {
