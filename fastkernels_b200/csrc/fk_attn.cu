@@ -718,7 +718,7 @@ __global__ void __launch_bounds__(256) attn_merge_kernel(const AttnParams p) {
   float lt = 0.f;
   for (int s0 = 0; s0 < n; s0 += 32) {
     const float2 mlv = s0 + lane < n ? p.part_ml[base + s0 + lane] : make_float2(-INFINITY, 0.f);
-    const float fl = fast_exp2(mlv.x - Mu), ll = mlv.y * fl;
+    const float fl = fast_exp2(mlv.x - Mu);
     const int cnt = min(32, n - s0);
     const float4* src = reinterpret_cast<const float4*>(p.part_o + (base + s0) * ATT_D) + lane;
     for (int s = 0; s < cnt; s += 4) {
@@ -728,9 +728,10 @@ __global__ void __launch_bounds__(256) attn_merge_kernel(const AttnParams p) {
         v[i] = s + i < cnt ? src[(s + i) * (ATT_D / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float f = __shfl_sync(0xffffffffu, fl, s + i), l = __shfl_sync(0xffffffffu, ll, s + i);
+        const float f = __shfl_sync(0xffffffffu, fl, s + i);
+        const float l = __shfl_sync(0xffffffffu, mlv.y, s + i);
         if (s + i >= cnt) break;
-        lt += l;
+        lt = fmaf(l, f, lt);           // one rounding a split
         acc.x += v[i].x * f; acc.y += v[i].y * f; acc.z += v[i].z * f; acc.w += v[i].w * f;
       }
     }

@@ -82,6 +82,17 @@ def test_split_bounds(ops, max_splits):
     check(run(ops, c, max_splits=max_splits), oracle(c))
 
 
+def test_more_than_32_splits(ops):
+    """The merge gives a lane splits lane and lane + 32: 33, 35, 63 and 64 splits of 128 tokens."""
+    c = cases.attention_case(9, 4, 4, 1, 128, 256, None, lens=[4200, 4480, 8064, 8192])
+    q, kc, vc = dev(c["q"]), dev(c["k_cache"]), dev(c["v_cache"])
+    ws = torch.empty(ops.attn_workspace_bytes(4, 4, 128, 64), dtype=torch.uint8, device="cuda")
+    out = ops.paged_decode_attn(q, kc, vc, dev(c["context_lens"]), dev(c["block_tables"]),
+                                c["scale"], ws, 64)
+    check(out, oracle(c))
+    assert ws[:8].view(torch.int32).tolist() == [33 + 35 + 63 + 64, 128]    # chunks, tokens each
+
+
 @pytest.mark.parametrize("layout,page", [("HND", 16), ("HND", 32), ("HND", 64),
                                          ("NHD", 16), ("NHD", 32)])
 def test_small_pages_and_hnd_layout(ops, layout, page):
