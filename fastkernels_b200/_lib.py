@@ -117,6 +117,7 @@ PROTOTYPES = {
     "fk_rope_rms_store": (_i32, [_vp, _vp, _i64, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i64,
                                  _i32, _i32, _i32, _i32, _i32, _i32, _f32, _i64, _vp, _vp]),
     "fk_act_and_mul": (_i32, [_vp, _i64, _vp, _i64, _i32, _i64, _i64, _i32, _vp]),
+    "fk_gemm_bf16_many_kernel": (_i32, [_i64, _i64, _i64]),
     "fk_gemm_bf16_act_mul_many": (_i32, [_vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32,
                                          _vp, _vp]),
     "fk_gemm_bf16_act_mul": (_i32, [_vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32, _vp,

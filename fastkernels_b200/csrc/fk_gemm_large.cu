@@ -649,30 +649,38 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
   return FK_OK;
 }
 
-// Which kernel: 0 = single CTAs, 1 = CTA pairs on 256 x 256, 2 = pairs on 256 x 512.
+// Which kernel: 0 = single CTAs, 1 = CTA pairs on 256 x 256 tiles.
 //
-// All three multiply at about the same rate, so what decides is how the tiles fill their rounds.
-// A pair's round is shorter (half the work per SM), and its epilogue runs beside the next
-// tile's products, which the single CTA's does not.  Measured (us, k from 2048 to 12288): a
-// single CTA's round 12 + k / 100, a pair's 0.0072 k and 6 once.  k 2048, single -> pair:
-// 1000 x 3072 29.7 -> 21.0, 4096 x 3072 74.3 -> 55.8, 4096 x 12288 212 -> 173; k 4096:
-// 300 x 6144 49 -> 33, 2000 x 6144 96 -> 91, 2000 x 4096 (one full round) 51.7, pair 61.9.
-// The wide pair reads a quarter less: 2 to 4 % from k = 4096 on where it needs no more rounds
-// and there are several (8192 x 24576 x 4096 1286 -> 1242, 4096 x 4096 x 12288 294 -> 278).
+// An SM gets about as much done in either, so what decides is how the tiles fill their rounds: a
+// pair's round is half as long, and its epilogue runs beside the next tile's products, which the
+// single CTA's does not; from k = 512 down a round is its epilogue, and the single CTAs' rounds,
+// which store twice as much, are the cheaper ones.  The times below (us, of rounds of tiles) are
+// fitted to 672 sizes, m 257 to 16384, n 1024 to 24576, k 64 to 12288, with and without an
+// activation, kernels in turn: the choice is 0.2 % from the faster one on average and 4 % at
+// worst.  Examples, single / pair: 537 x 2048 x 6144 67 / 48, 1000 x 3072 x 2048 30 / 21,
+// 2048 x 4608 x 3072 43 / 51, 1024 x 6144 x 4096 54 / 65, 4096 x 16384 x 64 54 / 68.
+// Pairs on 256 x 512 tiles read a quarter less and were never more than 2 % ahead
+// (16384 x 3072 x 8192 663 -> 651): by FK_B200_GEMM_PAIR only.
 static int large_mode(const GemmLargeParams& p) {
   auto rounds = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   const int pairs = resident_pairs<1, false>();
   if (pairs <= 0) return 0;
-  const double single = rounds(tiles, sm_count());
-  const double t_single = single * (12. + 0.01 * p.k);
-  const double t_pair = 6. + 0.0072 * p.k * rounds(tiles, pairs);
-  if (t_pair < t_single) return 1;
-  const int wide = resident_pairs<2, false>();
-  if (p.k >= 4096 && single >= 2. && wide > 0 &&
-      rounds((int64_t)p.m_tiles * ((p.n_tiles + 1) / 2), wide) <= single)
-    return 2;
-  return 0;
+  const double k = p.k, k1 = k < 3000. ? k : 3000.;
+  const double store = 5.8 + 0.002 * k, multiply = 0.0074 * k;
+  const double t_single = 2. + rounds(tiles, sm_count()) * (9.4 + 0.0117 * k);
+  const double t_pair =
+      3. + 0.0016 * k1 + rounds(tiles, pairs) * (store > multiply ? store : multiply);
+  return t_pair < t_single ? 1 : 0;
+}
+
+// FK_B200_GEMM_PAIR: 0, 1 or 2 for one kernel at all sizes
+static int kernel_for(const GemmLargeParams& p) {
+  static const int forced = [] {
+    const char* e = getenv("FK_B200_GEMM_PAIR");
+    return e != nullptr ? atoi(e) : -1;
+  }();
+  return forced >= 0 ? forced : large_mode(p);
 }
 
 template <bool ACT>
@@ -684,12 +692,7 @@ static int launch_large(const void* x, int64_t x_stride, const void* w, GemmLarg
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   FK_REQUIRE(tiles <= 0x7fffffff, FK_ERR_UNSUPPORTED, "fk_gemm_bf16: too many tiles");
 
-  // FK_B200_GEMM_PAIR: 0, 1 or 2 for one kernel at all sizes (see large_mode)
-  static const int forced = [] {
-    const char* e = getenv("FK_B200_GEMM_PAIR");
-    return e != nullptr ? atoi(e) : -1;
-  }();
-  const int mode = forced >= 0 ? forced : large_mode(p);
+  const int mode = kernel_for(p);
   const bool pair = mode == 1 || mode == 2;
   CUtensorMap mx, mw;
   int rc = gl_map(x, p.m, p.k, x_stride, pair ? 128 : 256, &mx);
@@ -727,6 +730,16 @@ int gemm_large_launch(const void* x, int64_t x_stride, const void* w, const void
 }  // namespace fk
 
 using namespace fk;
+
+extern "C" int fk_gemm_bf16_many_kernel(int64_t m, int64_t n, int64_t k) {
+  if (m <= 256 || n <= 0 || k <= 0 || m >= (1ll << 31) || n >= (1ll << 31) || k >= (1ll << 31))
+    return -1;
+  GemmLargeParams p{};
+  p.k = (int)k;
+  p.m_tiles = (int)((m + GL_BM - 1) / GL_BM);
+  p.n_tiles = (int)((n + GL_BN - 1) / GL_BN);
+  return kernel_for(p);
+}
 
 extern "C" int fk_gemm_bf16_act_mul_many(const void* x, int64_t x_stride, const void* w,
                                          const void* bias, void* y, int64_t y_stride, int64_t m,

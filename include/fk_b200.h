@@ -630,6 +630,9 @@ int fk_act_and_mul(const void* x, int64_t x_stride, void* out, int64_t out_strid
 int fk_gemm_bf16_act_mul_many(const void* x, int64_t x_stride, const void* w, const void* bias,
                               void* y, int64_t y_stride, int64_t m, int64_t n, int64_t k, int act,
                               int32_t* status, fk_stream_t stream);
+/* Kernel that a product of m > 256 rows with n weight rows takes, with an activation or without:
+ * 0 = single CTAs, 1 = CTA pairs, 2 = CTA pairs on wide tiles, -1 = not a many-row product. */
+int fk_gemm_bf16_many_kernel(int64_t m, int64_t n, int64_t k);
 /* fk_gemm_bf16_silu_mul with a choice of activation; same single-launch shapes. */
 int fk_gemm_bf16_act_mul(const void* x, int64_t x_stride, const void* w, const void* bias,
                          void* y, int64_t y_stride, int64_t m, int64_t n, int64_t k, int act,

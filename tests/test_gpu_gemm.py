@@ -192,13 +192,17 @@ print('pair ok')
     assert r.returncode == 0 and "pair ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
 
 
-@pytest.mark.parametrize("m,n,k", [(300, 1032, 4096),      # CTA pairs: few tiles, a short round
-                                   (2010, 4104, 2048),     # pairs over several rounds
-                                   (2010, 4096, 4096),     # single CTAs: one full round
-                                   (2048, 9472, 4096)])    # wide pairs: two full rounds
-def test_gemm_many_rows_kernel_choice(ops, m, n, k):
+@pytest.mark.parametrize("m,n,k,kernel", [(300, 1032, 4096, 1),    # few tiles, a short round
+                                          (2010, 6152, 2048, 1),   # pairs over several rounds
+                                          (2010, 4096, 4096, 0),   # single CTAs: one full round
+                                          (2048, 9472, 4096, 0),   # ... two full rounds
+                                          (300, 16384, 64, 0),     # a round is its epilogue
+                                          (257, 1000, 64, 1)])     # one tile row, one short round
+def test_gemm_many_rows_kernel_choice(ops, m, n, k, kernel):
     """Sizes on both sides of the rule that picks the many-row kernel; some rows of each tile
     against the oracle, and nothing written past a row."""
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert ops.lib.fk_gemm_bf16_many_kernel(m, n, k) == kernel
     rs = np.random.RandomState(m + n + k)
     x = cases.randn_bf16(rs, (m, k))
     w = cases.randn_bf16(rs, (n, k), 0.05)
@@ -279,7 +283,8 @@ import torch
 sys.path.insert(0, 'tests')
 from fastkernels_b200 import _lib, ops
 for (m, n, k, bias) in [(257, 16, 64, True), (300, 272, 192, False), (513, 2064, 128, True),
-                        (1000, 4096, 256, False), (2049, 1536, 64, True)]:
+                        (1000, 4096, 256, False), (2049, 1536, 64, True), (2010, 4096, 4096, True),
+                        (300, 16384, 64, False), (300, 1040, 4096, True)]:
     g = torch.Generator(device='cuda').manual_seed(m)
     x = torch.empty((m, k + 8), dtype=torch.bfloat16, device='cuda').normal_(generator=g)[:, :k]
     w = torch.empty((n, k), dtype=torch.bfloat16, device='cuda').normal_(0, 0.2, generator=g)
@@ -296,6 +301,11 @@ for (m, n, k, bias) in [(257, 16, 64, True), (300, 272, 192, False), (513, 2064,
         assert torch.equal(out[:, :n // 2], want), (m, n, k, act)
         assert float(out[:, n // 2:].abs().max()) == 0.0
         assert torch.equal(ops.gemm_act_mul(x, w, act, bias=b), want)
+if sys.argv[1]:
+    assert _lib.lib.fk_gemm_bf16_many_kernel(300, 16384, 64) == int(sys.argv[1])
+elif torch.cuda.get_device_properties(0).multi_processor_count == 148:
+    assert [_lib.lib.fk_gemm_bf16_many_kernel(*s) for s in
+            ((2010, 4096, 4096), (300, 16384, 64), (300, 1040, 4096))] == [0, 0, 1]
 print('act ok')
 """
     env = dict(os.environ)
@@ -303,7 +313,7 @@ print('act ok')
     if mode:
         env["FK_B200_GEMM_PAIR"] = mode
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-c", code], cwd=root, env=env, capture_output=True,
+    r = subprocess.run([sys.executable, "-c", code, mode], cwd=root, env=env, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0 and "act ok" in r.stdout, r.stdout[-2000:] + r.stderr[-2000:]
 
