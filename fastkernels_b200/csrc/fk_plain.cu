@@ -351,10 +351,8 @@ struct AnyAttnParams {
 // Bound by shared-memory reads and the fp32 rate.  A CTA takes 8 R queries of one sequence and
 // KV head (rows x the heads that share it) through runs of 32 keys, which it lays out in shared
 // memory once for all of them: lane j of a warp scores key j for its R queries, then the lanes
-// own the value channels lane, lane + 32, ...  R = 4 keeps two rows' worth of queries' sums in
-// registers; few queries per sequence (single tokens) are spread over all warps.  Three prompts
-// of up to 333 tokens, 16 heads of 576 channels on one KV head: 1627 -> 476 us against a warp
-// per query that reads its keys from L2.
+// own the value channels lane, lane + 32, ...; few queries per sequence (single tokens) are spread
+// over all warps.  R changes no sum's order.
 constexpr int AA_WARPS = 8, AA_THREADS = 32 * AA_WARPS, AA_KEYS = 32;
 constexpr int AA_MAX_SMEM = 227 * 1024 - 1024;
 
@@ -578,14 +576,21 @@ static int launch_any_r(const AnyAttnParams& p, cudaStream_t s) {
   count_launch();
   return FK_OK;
 }
-// Queries per warp: four, fewer where a sequence and KV head has too few of them for eight
-// warps, and one above 576 channels, where queries and keys share the memory.
+// Queries per warp: one while all CTAs are in the first round (or there are no more than eight
+// queries to share a run of keys), then two, which halve the CTAs for 5 to 10 % more time each.
+// Four, in keys of 576 channels, leave one CTA an SM and were behind at every size.  us, one / two /
+// four a warp (and a warp per query that reads its keys from L2): fp32, 576 channels, 4 heads on one
+// KV head, a portion of 5 tokens on 300 keys 131 / 135 / 252 (196); 16 heads, 40 portions of 5
+// 342 / 203 / 232 (1143); one of 900 tokens 1633 / 1031 / 1306 (5827); 128 channels, 16 heads on 4,
+// 64 single tokens on 500 keys 142 / 141 / 145 (346); 64 channels, 16 KV heads, 40 portions of two
+// tokens 72 / 134 / 204 (156).
 template <typename T, int CH>
 static int launch_any_ch(const AnyAttnParams& p, cudaStream_t s) {
-  const int64_t queries = p.rows * (p.hq / p.hkv) / p.num_seqs;
-  if (queries <= AA_WARPS) return launch_any_r<T, CH, 1>(p, s);
-  if (queries <= 2 * AA_WARPS) return launch_any_r<T, CH, 2>(p, s);
-  return launch_any_r<T, CH, 4>(p, s);
+  const int64_t queries = p.rows * (p.hq / p.hkv);
+  const int64_t ctas = ((queries + AA_WARPS - 1) / AA_WARPS) * p.hkv;
+  if (queries <= (int64_t)AA_WARPS * p.num_seqs || ctas <= sm_count())
+    return launch_any_r<T, CH, 1>(p, s);
+  return launch_any_r<T, CH, 2>(p, s);
 }
 template <typename T>
 static int launch_any(const AnyAttnParams& p, cudaStream_t s) {

@@ -265,10 +265,14 @@ def test_group_f32_row_groups(counts, act):
 @pytest.mark.parametrize("d,hq,hkv,portions", [
     (4, 3, 1, [(0, 5), (40, 1)]), (68, 8, 2, [(0, 1), (70, 33), (3, 4)]),
     (576, 16, 1, [(31, 1), (0, 1), (64, 2)]), (576, 5, 1, [(0, 70)]),
-    (1152, 2, 1, [(1, 9), (30, 1)])])
+    (1152, 2, 1, [(1, 9), (30, 1)]),
+    # single tokens: one, two and four queries a warp
+    (68, 3, 3, [(0, 1), (31, 1), (95, 1)]), (68, 16, 2, [(0, 1), (32, 1)]),
+    (68, 16, 1, [(70, 1), (5, 1)]), (68, 64, 1, [(70, 1)]), (576, 2, 2, [(33, 1), (4, 1)]),
+    (576, 8, 1, [(64, 1), (1, 1)]), (576, 16, 1, [(40, 1)]), (576, 40, 1, [(63, 1), (64, 1)])])
 def test_paged_attn_any_forms(d, hq, hkv, portions, dtype):
-    """Head sizes, shared heads, portions after a prefix and single tokens; the keys after a
-    row's own hold infinities, which must not reach it."""
+    """Head sizes, shared heads, portions after a prefix and single tokens, every row by value;
+    the key after a row's own may be an infinity, which must not reach it."""
     from fastkernels_b200 import ops
     rs = np.random.RandomState(d)
     page, n = 16, sum(c for _, c in portions)
@@ -281,23 +285,30 @@ def test_paged_attn_any_forms(d, hq, hkv, portions, dtype):
     q, qd = rnd(rs, n, hq, d, dtype=dtype)
     cu = np.concatenate([[0], np.cumsum([c for _, c in portions])])
     scale = d ** -0.5
+
+    def attend():
+        out = ops.paged_attn_any(qd, kd, vd, i32(cu), i32(lens), i32(bt), scale)
+        return out.double().cpu().numpy()
+
+    def compare(got, left_out):
+        for s, (a, c) in enumerate(portions):
+            ks, vs = (t[bt[s]].reshape(-1, hkv, d) for t in (k, v))
+            for i in range(c - left_out):
+                seen = a + i + 1
+                for h in range(hq):
+                    z = scale * ks[:seen, h * hkv // hq] @ q[cu[s] + i, h]
+                    pr = np.exp(z - z.max())
+                    want = pr @ vs[:seen, h * hkv // hq] / pr.sum()
+                    # fp32 sums; a bf16 result is rounded once more
+                    np.testing.assert_allclose(got[cu[s] + i, h], want, rtol=0,
+                                               atol=(1e-5 if dtype == F32 else 1e-2) *
+                                               max(1.0, np.abs(want).max()))
+    compare(attend(), 0)
     for s, length in enumerate(lens):       # the last key of a portion is the future of its others
         vd.view(-1, hkv, d)[bt[s, (length - 1) // page] * page + (length - 1) % page] = float("inf")
-    got = ops.paged_attn_any(qd, kd, vd, i32(cu), i32(lens), i32(bt), scale)
-    got = got.double().cpu().numpy()
-    for s, (a, c) in enumerate(portions):
-        ks, vs = (t[bt[s]].reshape(-1, hkv, d) for t in (k, v))
-        for i in range(c - 1):
-            seen = a + i + 1
-            for h in range(hq):
-                z = scale * ks[:seen, h * hkv // hq] @ q[cu[s] + i, h]
-                pr = np.exp(z - z.max())
-                want = pr @ vs[:seen, h * hkv // hq] / pr.sum()
-                # fp32 sums; a bf16 result is rounded once more
-                np.testing.assert_allclose(got[cu[s] + i, h], want, rtol=0,
-                                           atol=(1e-5 if dtype == F32 else 1e-2) *
-                                           max(1.0, np.abs(want).max()))
-        assert not np.isfinite(got[cu[s] + c - 1]).any()
+    got = attend()
+    compare(got, 1)
+    assert not np.isfinite(got[cu[1:] - 1]).any()
 
 
 def test_embed_and_argmax_f32():
