@@ -242,6 +242,112 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 1 : 2)
   }
 }
 
+// Short k: the tiles above spend their time filling the ring and handing sums on.  64 x 64
+// outputs, 4 x 4 a thread, k in one order.  us, 60 / 200 / 1000 rows, here and in the tiles above:
+// 16 heads of 96 -> 512 8 21 55 (18 21 80), 40 of 256 -> 64 15 35 50 (17 38 108 in one part),
+// 12288 x 256 34 58 196 (35 65 213; one row 31 and 21).
+constexpr int FS_M = 64, FS_N = 64, FS_K = 16, FS_MAX_K = 511;
+
+template <bool ACT>
+__global__ void __launch_bounds__(256) f32_short_kernel(const F32Product p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  constexpr int NB = ACT ? 2 : 1;
+  __shared__ float xs[FS_K][FS_M + 4], ws[NB][FS_K][FS_N + 4];
+  const int g = blockIdx.z;
+  int64_t first = 0, count = p.rows;
+  if (p.offsets) {
+    const int64_t a = p.offsets[g], b = p.offsets[g + 1];
+    if (a < 0 || b < a || b > p.rows) {
+      if (p.status && threadIdx.x == 0) atomicOr(p.status, FK_DEV_BAD_SLOT);
+      return;
+    }
+    first = a;
+    count = b - a;
+  }
+  const int n0 = blockIdx.x * FS_N;
+  const int64_t m0 = (int64_t)blockIdx.y * FS_M;
+  if (m0 >= count) return;
+  const float* x = p.x + (p.offsets ? 0 : g * p.x_group);
+  const float* w = p.w + (int64_t)g * p.w_rows * p.k;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int lr = threadIdx.x >> 2, lc = (threadIdx.x & 3) * 4;
+  const bool x_on = m0 + lr < count, w_on = n0 + lr < p.n;
+  int64_t row = 0;
+  if (x_on) {
+    row = first + m0 + lr;
+    if (p.gather) {
+      row = p.gather[row];
+      if (row < 0 || row >= p.x_rows) {
+        if (p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
+        row = 0;
+      }
+    }
+  }
+  const float* xr = x + row * p.x_stride;
+  float acc[NB][4][4] = {};
+  for (int k0 = 0; k0 < p.k; k0 += FS_K) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b[NB];
+#pragma unroll
+    for (int e = 0; e < NB; ++e) b[e] = a;
+    if (k0 + lc < p.k) {                        // k is a multiple of 4
+      if (x_on) a = *reinterpret_cast<const float4*>(xr + k0 + lc);
+#pragma unroll
+      for (int e = 0; e < NB; ++e)
+        if (w_on)
+          b[e] = *reinterpret_cast<const float4*>(w + ((int64_t)e * p.n + n0 + lr) * p.k + k0 + lc);
+    }
+    __syncthreads();
+    xs[lc][lr] = a.x; xs[lc + 1][lr] = a.y; xs[lc + 2][lr] = a.z; xs[lc + 3][lr] = a.w;
+#pragma unroll
+    for (int e = 0; e < NB; ++e) {
+      ws[e][lc][lr] = b[e].x; ws[e][lc + 1][lr] = b[e].y;
+      ws[e][lc + 2][lr] = b[e].z; ws[e][lc + 3][lr] = b[e].w;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < FS_K; ++kk) {
+      const float4 av = *reinterpret_cast<const float4*>(&xs[kk][ty * 4]);
+      const float aa[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+      for (int e = 0; e < NB; ++e) {
+        const float4 bv = *reinterpret_cast<const float4*>(&ws[e][kk][tx * 4]);
+        const float bb[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[e][i][j] = fmaf(aa[i], bb[j], acc[e][i][j]);
+      }
+    }
+  }
+  float* y = p.y + (p.offsets ? 0 : g * p.y_group);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int64_t r = m0 + ty * 4 + i;
+    if (r >= count) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = n0 + tx * 4 + j;
+      if (c >= p.n) continue;
+      float v = acc[0][i][j] + (p.bias ? p.bias[c] : 0.f);
+      if (ACT) {
+        const float up = acc[NB - 1][i][j] + (p.bias ? p.bias[p.n + c] : 0.f);
+        v = (p.act == FK_ACT_SILU ? v * sigmoid_f32(v) : gelu_tanh_f32(v)) * up;
+      }
+      y[(first + r) * p.y_stride + c] = v;
+    }
+  }
+}
+
+template <bool ACT>
+static int launch_f32_short(const F32Product& p, cudaStream_t s) {
+  const dim3 grid((unsigned)((p.n + FS_N - 1) / FS_N), (unsigned)((p.rows + FS_M - 1) / FS_M),
+                  (unsigned)p.groups);
+  FK_CUDA_OK(launch_kernel(f32_short_kernel<ACT>, grid, dim3(256), 0, s, p));
+  count_launch();
+  return FK_OK;
+}
+
 // CTAs that are resident at once as clusters of `parts` (GPC boundaries keep some SMs out of
 // large ones): a property of the GPU model, asked once.
 template <int WR, int WC, bool ACT>
@@ -328,6 +434,7 @@ static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
 // tiles on average, since their last tile is half empty.
 template <bool ACT>
 static int launch_f32(const F32Product& p, int64_t expect, cudaStream_t s) {
+  if (p.k <= FS_MAX_K) return launch_f32_short<ACT>(p, s);
   if (expect <= 32) return launch_f32_tile<1, 2, ACT>(p, s);
   if (expect <= 64 || (p.offsets && expect <= 192)) return launch_f32_tile<2, 2, ACT>(p, s);
   return launch_f32_tile<4, 2, ACT>(p, s);

@@ -225,9 +225,10 @@ def test_gemm_f32(m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k", [(2, 300, 4096), (33, 129, 36), (64, 128, 1024),
-                                   (65, 1000, 300), (127, 40, 2052), (257, 260, 640)])
+                                   (65, 1000, 300), (127, 40, 2052), (257, 260, 640),
+                                   (65, 65, 508), (65, 65, 512), (1, 1, 4)])
 def test_gemm_f32_tiles_and_parts(m, n, k):
-    """Edges of the three row tiles, k in one part and in several."""
+    """Edges of the three row tiles, k in one part and in several, short and long k."""
     from fastkernels_b200 import ops
     rs = np.random.RandomState(m)
     x, xd = rnd(rs, m, k)
@@ -242,11 +243,12 @@ def test_gemm_f32_tiles_and_parts(m, n, k):
 
 @pytest.mark.parametrize("counts", [(0, 1, 0, 33), (64, 0, 129, 3, 65), (200, 257)])
 @pytest.mark.parametrize("act", [None, 0, 1])
-def test_group_f32_row_groups(counts, act):
+@pytest.mark.parametrize("k", [516, 100])
+def test_group_f32_row_groups(counts, act, k):
     """Row groups in fp32: empty groups, part-filled tiles, gathered rows, gate and up."""
     from fastkernels_b200 import ops
     rs = np.random.RandomState(len(counts))
-    rows, n, k = sum(counts), 77, 516
+    rows, n = sum(counts), 77
     off = np.concatenate([[0], np.cumsum(counts)])
     pick = rs.randint(0, 90, size=rows)
     x, xd = rnd(rs, 90, k)
