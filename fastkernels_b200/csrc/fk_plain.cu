@@ -9,8 +9,6 @@
 #include "fk_f32_tile.cuh"
 #include "fk_types.cuh"
 
-#include <cmath>
-#include <mutex>
 
 namespace fk {
 
@@ -22,13 +20,9 @@ namespace fk {
 // padded to 36 floats, so the 8 rows that a quarter of a warp reads start in different banks.
 // WR x WC warps make the CTA's tile; loads run kStages - 1 blocks of 32 k's ahead (cp.async).
 //
-// Where the tiles alone leave SMs idle, a cluster of up to 8 CTAs shares one tile: each takes a
-// part of k, leaves its sums in its shared memory, and adds up its share of the rows over all
-// parts in their order.
-//
-// Measured on a prompt batch of about 500 rows (16 heads, width 2048, 32 experts): projections
-// 480 -> 311 us, gate and up of the experts 1021 -> 755 us against 64 x 64 tiles of scalar
-// multiply-adds.
+// A cluster of 2 to 8 CTAs shares one tile: each takes a part of k, leaves its sums in its shared
+// memory, and adds up its share of the rows over all parts in their order (f32_parts).
+// 1000 rows, 24576 x 4096: 44 TFLOP/s of 72 (scalar 64 x 64 tiles 33).
 template <int WR, int WC>
 struct F32Tile {
   static constexpr int kRows = 32 * WR, kCols = 64 * WC, kThreads = 32 * WR * WC;
@@ -200,18 +194,13 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 1 : 2)
       for (int j = 0; j < 8; ++j)
         f32_smem[(wr * 32 + i * 4 + ty) * Tile::kOutPitch + wc * 64 + j * 8 + tx] =
             acc[i][j].x + acc[i][j].y;
-    if (parts > 1) {
-      asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                   "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    } else {
-      __syncthreads();
-    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const int live = (int)(count - m0 < Tile::kRows ? count - m0 : Tile::kRows);
     const int r0 = live * part / parts, r1 = live * (part + 1) / parts;
     float* y = p.y + (p.offsets ? 0 : g * p.y_group);
     auto sum = [&](int r, int c) {
       const int at = r * Tile::kOutPitch + c;
-      if (parts == 1) return f32_smem[at];
       const uint32_t addr = smem_u32(f32_smem + at);
       float v = ld_cluster_f32(addr, 0);
       for (int q = 1; q < parts; ++q) v += ld_cluster_f32(addr, q);
@@ -232,13 +221,9 @@ __global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 1 : 2)
       y[(first + m0 + r) * p.y_stride + n0 + c] = v;
     }
     // peers may still read this CTA's sums; the next tile overwrites them
-    if (parts > 1) {
-      __syncwarp();                    // lanes stored different numbers of outputs
-      asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                   "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    } else {
-      __syncthreads();
-    }
+    __syncwarp();                      // lanes stored different numbers of outputs
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 }
 
@@ -348,35 +333,20 @@ static int launch_f32_short(const F32Product& p, cudaStream_t s) {
   return FK_OK;
 }
 
-// CTAs that are resident at once as clusters of `parts` (GPC boundaries keep some SMs out of
-// large ones): a property of the GPU model, asked once.
-template <int WR, int WC, bool ACT>
-static int f32_slots(int parts) {
-  static std::once_flag once;
-  static int slots[4];
-  std::call_once(once, [] {
-    using Tile = F32Tile<WR, WC>;
-    for (int i = 0; i < 4; ++i) {
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(1024);
-      cfg.blockDim = dim3(Tile::kThreads);
-      cfg.dynamicSmemBytes = Tile::kSmem;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 1u << i;
-      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, f32_product_kernel<WR, WC, ACT>, &cfg) !=
-          cudaSuccess) {
-        cudaGetLastError();
-        n = 0;
-      }
-      slots[i] = n << i;
-    }
-  });
-  return slots[parts == 8 ? 3 : parts == 4 ? 2 : parts == 2 ? 1 : 0];
+// Parts of k, by the weights' sizes alone: a row's sums are taken in the same order whatever other
+// rows are in the call (tiles of every height add up k alike).  Few weight tiles get more parts, so
+// that few rows find SMs; many rows would have them anyway and pay for the exchange.  us, rows 1 /
+// 100 / 500 / 1000, k 2048 unless said, in 2, 4 and 8 parts (scalar 64 x 64 tiles):
+//   n 544            67 115 118 120     36 61 64 123       21 34 68 102       (94 98 99 193)
+//   n 2048           67 113 118 231     36 61 123 244      21 66 168 302      (94 99 278 297)
+//   n 4096, k 4096   131 216 436 869    93 112 451 898     58 175 534 1063    (213 353 604 1043)
+//   n 6144           78 116 347 685     54 120 366 729     32 131 437 871     (126 198 441 797)
+//   n 4352           68 114 230 458     40 119 303 544     32 99 333 633      (95 199 297 580)
+// 32 experts, 2 x 1024 x 2048, 4 / 60 / 400 / 3100 rows in all: 70 201 239 753, 59 207 257 808,
+// 51 234 299 936 (243 364 632 999).
+static int f32_parts(const F32Product& p) {
+  const int64_t tiles = (p.w_rows + 127) / 128 * p.groups;
+  return tiles <= 12 && p.k >= 2048 ? 8 : tiles <= 32 && p.k >= 1024 ? 4 : 2;
 }
 
 template <int WR, int WC, bool ACT>
@@ -385,26 +355,12 @@ static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
   constexpr int kOut = ACT ? Tile::kCols / 2 : Tile::kCols;
   const int64_t n_tiles = (p.n + kOut - 1) / kOut;
   const int64_t upto = (p.rows + Tile::kRows - 1) / Tile::kRows;
-  // row groups: at most one part-filled tile a group; about half of them are expected
+  // row groups: at most one part-filled tile a group
   const int64_t used = p.rows < p.groups ? p.rows : p.groups;
   const int64_t row_tiles = p.offsets ? upto + used : upto;
-  const double tiles = (double)n_tiles * (p.offsets ? upto + used * 0.5 : (double)upto * p.groups);
-  // Parts of k: rounds of CTAs times what a round takes, 0.105 us a k (of a small tile
-  // that has its SM to itself 0.06) and 6.5 us around it.  k 2048, measured (us) in 1, 2, 4, 8 parts: 16 tiles
-  // 221 121 66 74, 64 tiles 221 123 128 172, 192 tiles 427 344 364 432, 384 tiles 657 692 737 885.
+  const int parts = f32_parts(p);
   static PerDeviceOnce once;
   FK_CUDA_OK(set_max_dynamic_smem(once, f32_product_kernel<WR, WC, ACT>, Tile::kSmem));
-  constexpr double kPerK = WR * WC == 8 ? 0.105 : WR * WC == 4 ? 0.11 : 0.08;
-  int parts = 1;
-  double best = 0.;
-  for (int c = 1; c <= 8 && p.k >= 64 * c && n_tiles * c < (1ll << 31); c *= 2) {
-    const int slots = f32_slots<WR, WC, ACT>(c);
-    if (slots == 0) continue;
-    const double rounds = ceil(tiles * c / slots);
-    const double per_k = WR * WC < 8 && tiles * c <= sm_count() ? 0.06 : kPerK;
-    const double t = rounds * (per_k * p.k / c + 6.5);
-    if (best == 0. || t < best) { best = t; parts = c; }
-  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(n_tiles * parts), (unsigned)(row_tiles < 65535 ? row_tiles : 65535),
                      p.offsets ? 1u : (unsigned)p.groups);
@@ -417,12 +373,10 @@ static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
     attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[na++].val.programmaticStreamSerializationAllowed = 1;
   }
-  if (parts > 1) {
-    attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = (unsigned)parts;
-    attr[na].val.clusterDim.y = 1;
-    attr[na++].val.clusterDim.z = 1;
-  }
+  attr[na].id = cudaLaunchAttributeClusterDimension;
+  attr[na].val.clusterDim.x = (unsigned)parts;
+  attr[na].val.clusterDim.y = 1;
+  attr[na++].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = na;
   FK_CUDA_OK(cudaLaunchKernelEx(&cfg, f32_product_kernel<WR, WC, ACT>, p, parts, row_tiles));

@@ -263,6 +263,24 @@ def test_group_f32_row_groups(counts, act, k):
                                atol=2e-5 * np.abs(z).max())
 
 
+@pytest.mark.parametrize("n,k", [(2048, 2048), (300, 4096), (6144, 1024), (129, 512), (1000, 300)])
+def test_f32_rows_do_not_hang_on_the_call(n, k):
+    """A row's bits are the same alone, in batches that take other tiles, and, in row groups,
+    beside other numbers of rows."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(n)
+    x, w, bias = (dev(rs.randn(*s)) for s in ((300, k), (n, k), (n,)))
+    all_rows = ops.gemm(x, w, bias=bias)
+    for a, b in ((0, 1), (7, 40), (100, 165), (171, 300)):
+        assert torch.equal(ops.gemm(x[a:b], w, bias=bias), all_rows[a:b])
+    groups = dev(rs.randn(3, n, k))
+    whole = ops.group_gemm(x, groups, offsets=i32([0, 10, 10, 300]))
+    for a, b in ((0, 1), (10, 80), (250, 300)):
+        g = 0 if b <= 10 else 2
+        off = [0] * (g + 1) + [b - a] * (3 - g)
+        assert torch.equal(ops.group_gemm(x[a:b], groups, offsets=i32(off)), whole[a:b])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("d,hq,hkv,portions", [
     (4, 3, 1, [(0, 5), (40, 1)]), (68, 8, 2, [(0, 1), (70, 33), (3, 4)]),
