@@ -78,9 +78,9 @@ template <typename T, int DP, bool BLOCKED, bool VEC>
 __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPrepParams p) {
   extern __shared__ __align__(16) uint8_t dl_prep_smem[];
   pdl_launch_dependents();
-  if (VEC && !BLOCKED && blockIdx.x == 0) {
+  if (VEC && !BLOCKED) {
     // a decode step finds the decay projection's weights in HBM: towards L2 while the kernel
-    // in front still runs; the first unit of tokens asks for all units
+    // in front still runs
     const char* w2 = reinterpret_cast<const char*>(
         static_cast<const T*>(p.w2) + (int64_t)blockIdx.y * p.heads_per_cta * p.d * p.w2_stride);
     const int heads = min(p.heads_per_cta, p.heads - (int)blockIdx.y * p.heads_per_cta);

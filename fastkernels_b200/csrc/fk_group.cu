@@ -72,8 +72,7 @@ __device__ __forceinline__ int64_t group_x_row(const GroupParams& p, int64_t row
 // of 32 k's; the CTA's warps are ks parts of k by 16-row tiles.  Rows go 8 NT at a time,
 // blocks of them over grid.z.
 // Column groups: the weights are asked towards L2 ahead of the wait for the kernel in front (their
-// place does not hang on it, and in a decode step they come from HBM), by the first block of rows
-// for all of them; they are read after it.
+// place does not hang on it, and in a decode step they come from HBM); they are read after it.
 template <int NT, bool ACT, typename OUT, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) group_skinny_kernel(const GroupParams p, int ks) {
   extern __shared__ float gs_red[];            // [warps][TILES 16][8 NT + 1]
@@ -97,7 +96,7 @@ __global__ void __launch_bounds__(32 * WARPS) group_skinny_kernel(const GroupPar
     }
   const int chunks = (p.k + 31) >> 5;
   constexpr int UN = TILES * 2 + NT <= 6 ? 4 : TILES * 2 + NT <= 8 ? 2 : 1;
-  if (!p.offsets && blockIdx.z == 0 && tq == 0)
+  if (!p.offsets && tq == 0)
     for (int c = kpart; c < chunks; c += ks)
 #pragma unroll
       for (int e = 0; e < TILES; ++e)
