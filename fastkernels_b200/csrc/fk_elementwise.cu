@@ -499,6 +499,26 @@ static inline int grid_for(int64_t threads, int block) {
   return (int)g;
 }
 
+// What a decode step brings back and hands on: status words, then the token ids, side by side so
+// that one copy takes them to the host; the ids also into the next step's input.
+__global__ void __launch_bounds__(256) step_result_kernel(
+    const int64_t* ids, int64_t n, int64_t* next_ids, int32_t* result, const int32_t* w0,
+    const int32_t* w1, const int32_t* w2, int words) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = threadIdx.x;
+  if (t < words) {
+    const int32_t* w = t == 0 ? w0 : t == 1 ? w1 : t == 2 ? w2 : nullptr;
+    result[t] = w ? *w : 0;
+  }
+  int64_t* out = reinterpret_cast<int64_t*>(result + words);
+  for (int64_t i = t; i < n; i += 256) {
+    const int64_t id = ids[i];
+    out[i] = id;
+    if (next_ids) next_ids[i] = id;
+  }
+}
+
 }  // namespace fk
 
 using namespace fk;
@@ -865,6 +885,22 @@ int fk_argmax_f32(const float* x, int64_t x_stride, int64_t rows, int64_t cols,
              "fk_argmax_f32: bad stride or row count");
   FK_LAUNCH((argmax_rows_kernel<float>), dim3((int)rows), dim3(1024), 0,
             static_cast<cudaStream_t>(stream), x, x_stride, cols, out_val, out_idx);
+  count_launch();
+  FK_CUDA_OK(cudaGetLastError());
+  return FK_OK;
+}
+
+int fk_step_result(const int64_t* ids, int64_t n, int64_t* next_ids, int32_t* result,
+                   const int32_t* word0, const int32_t* word1, const int32_t* word2, int words,
+                   fk_stream_t stream) {
+  FK_REQUIRE(n >= 0 && words >= 0 && words <= 4 && words % 2 == 0, FK_ERR_INVALID_ARG,
+             "fk_step_result: bad sizes");
+  FK_REQUIRE(result && (ids || n == 0), FK_ERR_INVALID_ARG, "fk_step_result: null pointer");
+  FK_REQUIRE((reinterpret_cast<uintptr_t>(result) & 7u) == 0, FK_ERR_ALIGNMENT,
+             "fk_step_result: result must be 8-byte aligned");
+  if (n == 0 && words == 0) return FK_OK;
+  FK_LAUNCH((step_result_kernel), dim3(1), dim3(256), 0, static_cast<cudaStream_t>(stream), ids, n,
+            next_ids, result, word0, word1, word2, words);
   count_launch();
   FK_CUDA_OK(cudaGetLastError());
   return FK_OK;

@@ -190,6 +190,13 @@ class DecodeEngine:
             if "state_slots" in v:
                 v["state_slots"].fill_(-1)
 
+        # what a step brings back, in one copy: the device status words, then the token ids
+        words = self._num_words = 2 if self.comm is None else 4
+
+        def result_views(buf):
+            return dict(result=buf, words=buf[:words].view(torch.int64),
+                        token_ids=buf[words:].view(torch.int64))
+
         self._packed_dev = torch.zeros(self._packed_bytes, dtype=torch.uint8, device=dev)
         tables = [torch.full((n, cols), -1, dtype=torch.int32, device=dev)
                   for cols in self.max_num_blocks]
@@ -200,7 +207,7 @@ class DecodeEngine:
             lm_logits=torch.zeros((n, self.model.logit_columns), dtype=c.dtype, device=dev),
             lm_max_vals=torch.zeros(n, dtype=torch.float32, device=dev),
             lm_max_idxs=torch.zeros(n, dtype=torch.int64, device=dev),
-            token_ids=torch.zeros(n, dtype=torch.int64, device=dev),
+            **result_views(torch.zeros(words + 2 * n, dtype=torch.int32, device=dev)),
             cu_rows=torch.arange(n + 1, dtype=torch.int32, device=dev),
         )
         clear(self.graph_vars)
@@ -219,7 +226,7 @@ class DecodeEngine:
             packed = pinned(self._packed_bytes, torch.uint8)
             tables = [pinned((n, cols), torch.int32) for cols in self.max_num_blocks]
             slot = dict(**packed_views(packed), packed=packed, block_tables=tables[0],
-                        span_tables=tables, token_ids=pinned(n, torch.int64))
+                        span_tables=tables, **result_views(pinned(words + 2 * n, torch.int32)))
             clear(slot)
             self._ring.append(slot)
         self._ring_np = [{k: [t.numpy() for t in v] if isinstance(v, list) else v.numpy()
@@ -232,6 +239,33 @@ class DecodeEngine:
         self.host, self.host_np = self._ring[0], self._ring_np[0]
         self.status = self.model.preallocate(n, self.max_model_len, dev, self._attn_max_splits)
         self.attn_workspace = getattr(self.model, "attn_workspace", None)
+        self._status_host = pinned(words, torch.int32)
+        self._status_np = self._status_host.numpy()
+        self._status_host_words = self._status_host.split(1)
+
+    def _status_words(self) -> list[torch.Tensor]:
+        """The device status words that this engine's kernels write."""
+        w = [self.status]
+        if self.device.type == "cuda":
+            w.append(ops.default_status(self.device))
+        return w if self.comm is None else w + [self.comm.status]
+
+    def _raise_on(self, words) -> None:
+        """Raises on status words (int32, copied to the host) that are not all zero.  The
+        device's are cleared, so that what comes next is not taken for it."""
+        st = 0
+        for w in words:
+            st |= int(w)
+        if not st:
+            return
+        for w in self._status_words():
+            w.zero_()
+        if st & 4 and self.device.type == "cuda":
+            # a wait ran out: a late stream-K contributor may have left its flag
+            # raised, so the shared GEMM workspace starts the next call zeroed again
+            ops.gemm_workspace(self.device)[:1024].zero_()
+        raise RuntimeError(f"device status word {st} (fk_device_status bits): a slot, page or "
+                           "position was out of range or a wait ran out; results are not valid")
 
     # ---------------------------------------------------------------- sequences
     def _new_sequence(self, num_tokens: int, last_token: int = 0) -> Sequence:
@@ -286,17 +320,19 @@ class DecodeEngine:
             self.state_slots.release(seq)
 
     @torch.no_grad()
-    def _forward_portions(self, portions, use_block_tables: bool = True):
+    def _forward_portions(self, portions, use_block_tables: bool = True, rows=()):
         """Run portions [(sequence, first position, token ids)], at most one per
-        sequence, through the model; hidden rows in the order of the tokens.  Metadata
+        sequence, through the model; hidden rows in the order of the tokens, `rows` of them
+        where the caller names some.  Metadata
         as in prepare_prefill (fastkernels/infra/engine.py:4902-4990): cu_seqlens,
         per-token slots and block tables, so attention reads the pages the store has
         just written.  In a chunked span a portion falls into one segment per chunk."""
         dev = self.device
         ids = np.concatenate([np.asarray(t, dtype=np.int64) for _, _, t in portions])
         pos = np.concatenate([np.arange(a, a + len(t), dtype=np.int64) for _, a, t in portions])
-        # token ids, positions and all int32 metadata travel in one copy
-        i32 = [ids.view(np.int32), pos.view(np.int32)]
+        # token ids, positions, wanted rows and all int32 metadata travel in one copy
+        i32 = [ids.view(np.int32), pos.view(np.int32),
+               np.asarray(rows, dtype=np.int64).view(np.int32)]
 
         def put(a):
             a = np.ascontiguousarray(a, dtype=np.int32)
@@ -325,8 +361,9 @@ class DecodeEngine:
                                         [len(t) for _, _, t in portions]))
             cu_shape = put(np.concatenate([[0], np.cumsum([len(t) for _, _, t in portions])]))
         flat = torch.from_numpy(np.concatenate(i32)).to(dev)
-        at = 4 * len(ids)
-        ids_dev, pos_dev = flat[:at].view(torch.int64).view(2, -1)
+        at = 4 * len(ids) + 2 * len(rows)
+        ids_dev, pos_dev, rows_dev = flat[:at].view(torch.int64).split(
+            [len(ids), len(ids), len(rows)])
 
         def take(shape):
             nonlocal at
@@ -354,7 +391,7 @@ class DecodeEngine:
             blocks.flush()
         self._bt_dirty = True          # the page tables have grown
         self._ahead = None
-        return hidden
+        return hidden.index_select(0, rows_dev) if len(rows) else hidden
 
     @torch.no_grad()
     def prefill(self, prompts, chunk_tokens: int | None = None,
@@ -410,7 +447,9 @@ class DecodeEngine:
                 rows = torch.from_numpy(row_end[[j for j, _ in ends]].astype(np.int64) - 1)
                 logits = self.model.project(hidden.index_select(0, rows.to(self.device)))
                 vals, idxs = ops.argmax_rows(logits)
+                self._copy_status()
                 tok = self.model.greedy(vals, idxs).cpu().numpy()
+                self._raise_on(self._status_np)
                 for (j, i), t in zip(ends, tok):
                     first[i] = int(t)
             for i, a, c in part:
@@ -438,16 +477,21 @@ class DecodeEngine:
         empty = torch.empty((0, self.model.logit_columns))
         out = [empty] * len(entries)
         if rest:
-            hidden = self._forward_portions([(entries[i][0], entries[i][0].num_tokens,
-                                              entries[i][1]) for i in rest])
             rows, o = [], 0
             for i in rest:
                 rows += [o + int(w) for w in want[i]]
                 o += len(entries[i][1])
+            if rows and not 0 <= min(rows) <= max(rows) < o:
+                raise ValueError("want names places outside the tokens")
+            hidden = self._forward_portions([(entries[i][0], entries[i][0].num_tokens,
+                                              entries[i][1]) for i in rest], rows=rows)
+            for i in rest:
                 entries[i][0].num_tokens += len(entries[i][1])
             if rows:
-                idx = torch.tensor(rows, dtype=torch.int64, device=self.device)
-                logits = self.model.project(hidden.index_select(0, idx)).float().cpu()
+                logits = self.model.project(hidden).float()
+                self._copy_status()
+                logits = logits.cpu()
+                self._raise_on(self._status_np)
                 o = 0
                 for i in rest:
                     out[i] = logits[o:o + len(want[i])]
@@ -465,10 +509,17 @@ class DecodeEngine:
             self.run_step_device(bs)
             self._mark_slot_in_flight()
             if any(len(want[i]) for i in single):
+                self._copy_status()
                 logits = self.graph_vars["lm_logits"][:n].float().cpu()
+                self._raise_on(self._status_np)
                 for j, i in enumerate(single):
                     out[i] = logits[j:j + 1].expand(len(want[i]), -1)
         return out
+
+    def _copy_status(self) -> None:
+        """Status words so far to the host, ahead of a copy that is waited for."""
+        for at, w in zip(self._status_host_words, self._status_words()):
+            at.copy_(w, non_blocking=True)
 
     def graph_batch_size(self, n: int) -> int:
         for bs in sorted(self.graphs):
@@ -580,9 +631,10 @@ class DecodeEngine:
         gv["lm_logits"][:bs] = logits
         ops.argmax_rows(gv["lm_logits"][:bs], gv["lm_max_vals"][:bs], gv["lm_max_idxs"][:bs])
         ids = self.model.greedy(gv["lm_max_vals"][:bs], gv["lm_max_idxs"][:bs])
-        gv["token_ids"][:bs] = ids
-        # hand the sampled ids to the next step on the device (engine.py:5689-5705)
-        gv["input_ids"][:bs] = ids
+        # for the host with the status words; the sampled ids also go to the next step on the
+        # device (engine.py:5689-5705)
+        ops.step_result(ids.contiguous(), gv["input_ids"], gv["result"], self._status_words(),
+                        self._num_words)
 
     def _set_context(self, bs: int, max_ctx: int) -> None:
         gv = self.graph_vars
@@ -646,26 +698,31 @@ class DecodeEngine:
         """One decode step for all running sequences through the public path:
         host prep -> pinned H2D staging -> graph replay -> D2H of the token ids.
         With sync=True the sampled ids come back to the host before returning
-        and feed the next step from the host; with sync=False the next step
-        reads them from the device buffer and the host copy is deferred."""
+        and feed the next step from the host (a device-side anomaly up to here
+        raises); with sync=False the next step reads them from the device buffer
+        and the host copy is deferred."""
         n = self.prepare_decode(use_host_ids=sync)
         bs = self.graph_batch_size(n)
         self.stage_inputs(n, bs, use_host_ids=sync)
         self.run_step_device(bs)
-        self.host["token_ids"][:n].copy_(self.graph_vars["token_ids"][:n], non_blocking=True)
+        back = self._num_words + 2 * n          # status words and token ids
+        self.host["result"][:back].copy_(self.graph_vars["result"][:back], non_blocking=True)
         self._mark_slot_in_flight()
-        self.d2h_bytes += n * 8
+        self.d2h_bytes += 4 * back
         for s in self.seqs:
             s.num_tokens += 1
         if not sync:
             return None
         landing = self.host_np["token_ids"]     # this step's slot (the next call moves on)
+        words = self.host_np["words"]
         self._prepare_ahead()
         torch.cuda.current_stream().synchronize()
         ids = landing[:n].copy()
         for s, t in zip(self.seqs, ids.tolist()):
             s.last_token = t
             s.output.append(t)
+        if words[0] or words[-1]:
+            self._raise_on(words.view(np.int32))
         return ids
 
     def device_status(self) -> int:
@@ -673,20 +730,13 @@ class DecodeEngine:
         workspace word, the per-device default word of the row kernels and GEMMs,
         the tensor-parallel communicator's): 0 = no slot / page / position out of
         range and no wait ran out.  Synchronises; call between steps."""
-        st = int(self.status.item()) | int(ops.default_status(self.device).item())
-        if self.comm is not None:
-            st |= int(self.comm.status.item())
+        st = 0
+        for w in self._status_words():
+            st |= int(w.item())
         return st
 
     def decode(self, steps: int) -> np.ndarray:
         """Greedy-decode `steps` tokens for every running sequence; [steps, n].
         Raises if a kernel reported a device-side anomaly on the way."""
         toks = np.stack([self.step(sync=True) for _ in range(steps)])
-        st = self.device_status()
-        if st:
-            if st & 4:
-                # a wait ran out: a late stream-K contributor may have left its flag
-                # raised, so the shared GEMM workspace starts the next call zeroed again
-                ops.gemm_workspace(self.device)[:1024].zero_()
-            raise RuntimeError(f"device status word {st} after decoding (fk_device_status bits)")
         return toks

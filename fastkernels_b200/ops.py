@@ -429,6 +429,25 @@ def argmax_rows(x, out_val=None, out_idx=None):
     return out_val, out_idx
 
 
+def step_result(ids, next_ids, result, words, num_words) -> None:
+    """result [num_words + 2 n] int32 = the status words `words` (zeros behind them up to
+    num_words), then ids [n] int64 in their bits; next_ids[:n] = ids too unless None."""
+    for name, t, dtype in (("ids", ids, torch.int64), ("result", result, torch.int32),
+                           *((f"words[{i}]", w, torch.int32) for i, w in enumerate(words))):
+        _need(t, dtype, name)
+        if not t.is_contiguous():
+            raise _lib.FkError(f"step_result: {name} must be contiguous")
+    n = ids.numel()
+    if next_ids is not None:
+        _need(next_ids, torch.int64, "next_ids")
+    if len(words) > 3 or result.numel() < num_words + 2 * n or num_words < len(words) or \
+            (next_ids is not None and (next_ids.numel() < n or not next_ids.is_contiguous())):
+        raise _lib.FkError("step_result: shape mismatch")
+    w = [_ptr(t) for t in words] + [None] * (3 - len(words))
+    check(lib.fk_step_result(_ptr(ids), n, _ptr(next_ids), _ptr(result), *w, num_words, _stream()),
+          "fk_step_result")
+
+
 # ---------------------------------------------------------------------------- gemm
 def gemm_workspace_bytes(m, n, k) -> int:
     return int(lib.fk_gemm_bf16_workspace_bytes(m, n, k))

@@ -505,6 +505,15 @@ int fk_allreduce_add_rmsnorm_group(void* const* bases, int nranks,
                                    int32_t* status, fk_stream_t stream);
 
 /* ------------------------------------------------------------------------
+ * End of a decode step: result[0 .. words) = the status words behind word0 .. word2 (null: 0;
+ * words is 0, 2 or 4), behind them the n token ids as int64; the ids also to next_ids unless
+ * null.  result is 8-byte aligned; one device-to-host copy then brings both.
+ * ---------------------------------------------------------------------- */
+int fk_step_result(const int64_t* ids, int64_t n, int64_t* next_ids, int32_t* result,
+                   const int32_t* word0, const int32_t* word1, const int32_t* word2, int words,
+                   fk_stream_t stream);
+
+/* ------------------------------------------------------------------------
  * Fill `count` 32-bit words at dst (16-byte aligned) with `value`: zeroing of
  * workspaces and KV pools on the caller's stream, and the L2 flush of the
  * micro-benchmarks.  No counterpart in the reference (torch.zeros there).

@@ -173,3 +173,12 @@ def test_row_kernel_refusals():
                                None) == INVALID and "pair table" in err()
     assert L.fk_softcap(P, 8, 0, 2, 16, 5.0, None) == INVALID
     assert L.fk_softcap(P, 16, 0, 2, 16, 0.0, None) == INVALID
+
+
+def test_step_result_refusals():
+    def call(ids=P, n=4, result=P, words=2):
+        return L.fk_step_result(ids, n, None, result, P, None, None, words, None)
+    assert call(n=0, words=0) == 0
+    assert call(n=-1) == INVALID and call(words=3) == INVALID and call(words=6) == INVALID
+    assert call(ids=None) == INVALID and call(result=None) == INVALID and "null" in err()
+    assert call(result=P + 4) == ALIGNMENT

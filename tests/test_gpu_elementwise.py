@@ -333,3 +333,22 @@ def test_xor_checksum_matches_numpy():
         acc ^= ref
         assert int(single.item()) & 0xffffffff == ref
         assert int(out.item()) & 0xffffffff == acc
+
+
+@pytest.mark.parametrize("n", [0, 1, 255, 256, 257, 600])
+@pytest.mark.parametrize("words,room", [(0, 0), (1, 2), (2, 2), (3, 4)])
+def test_step_result(n, words, room):
+    """Status words, zeros up to their room, then the ids; what lies behind stays."""
+    from fastkernels_b200 import _lib, ops
+    g = torch.Generator(device="cuda").manual_seed(n)
+    ids = torch.randint(-2**62, 2**62, (n,), generator=g, device="cuda")
+    w = [torch.tensor([5 + i], dtype=torch.int32, device="cuda") for i in range(words)]
+    result = torch.full((room + 2 * n + 2,), 77, dtype=torch.int32, device="cuda")
+    nxt = torch.full((n + 1,), -9, device="cuda")
+    ops.step_result(ids, nxt, result, w, room)
+    assert result[:room].tolist() == [5 + i for i in range(words)] + [0] * (room - words)
+    assert torch.equal(result[room:room + 2 * n].view(torch.int64), ids)
+    assert result[room + 2 * n:].tolist() == [77, 77]
+    assert torch.equal(nxt[:n], ids) and int(nxt[n]) == -9
+    with pytest.raises(_lib.FkError):
+        ops.step_result(ids, nxt, result[:room + 2 * n - 1] if n or room else ids, w, room)

@@ -208,3 +208,28 @@ def test_prefill_then_decode_matches_oracle(mode):
     # hand-over to decode: the engine continues from its own first tokens
     equal, near, _ = lockstep(cfg_d, w, eng, got, kcs, vcs, 8)
     assert equal + near == 8 * len(plens) and equal >= 0.9 * 8 * len(plens)
+
+
+@pytest.mark.parametrize("graphs", [(), (3,)])
+def test_step_and_feed_raise_on_device_status(graphs):
+    """A status bit that a kernel left makes the step whose tokens come back raise, also from a
+    replayed graph; it is cleared, and the engine goes on."""
+    from fastkernels_b200 import ops
+    cfg_d = cases.TINY_QWEN3
+    w = cases.decoder_weights(5, cfg_d, scale=0.05)
+    lens = [30, 64, 127]
+    eng = make_engine(cfg_d, w, lens, graphs=graphs)
+    seed_context(eng, lens, 17)
+    eng.step()
+    for word in (eng.status, ops.default_status("cuda")):
+        word.fill_(4)
+        with pytest.raises(RuntimeError, match="device status word 4"):
+            eng.step()
+        assert len(eng.step()) == 3 and eng.device_status() == 0
+    eng.finish(eng.seqs[-1])
+    s = eng.open_sequence()
+    for tokens in ([1, 2, 3], [4]):
+        eng.status.fill_(1)
+        with pytest.raises(RuntimeError, match="device status word 1"):
+            eng.feed([(s, tokens)])
+        assert eng.feed([(s, tokens)])[0].shape[0] == 1 and eng.device_status() == 0

@@ -253,6 +253,32 @@ def test_feeding_a_portion_invalidates_the_staged_tables(tmp_path, monkeypatch):
         eng.feed([(s, [1] * 400)])
 
 
+def test_device_status_raises_with_the_logits(tmp_path, monkeypatch):
+    """A kernel that reports a wait that ran out (or a bad slot) makes the call whose results it
+    spoilt raise; the next call starts clean."""
+    small(tmp_path)
+    config, source = registry.load_folder(tmp_path, torch.float32)
+    config.kv_block_size = 8
+    eng = DecodeEngine(config, max_num_seqs=2, max_model_len=200, num_kv_blocks=40, device="cpu",
+                       init_scale=None)
+    eng.load_weights(source)
+    bad = []
+
+    def forward(self, ids, pos):
+        eng.status.bitwise_or_(bad.pop() if bad else 0)
+        return torch.zeros(len(ids), self.stride)
+    monkeypatch.setattr(type(eng.model), "forward", forward)
+    monkeypatch.setattr(type(eng.model), "project", lambda self, h: torch.zeros(h.shape[0], 51))
+    monkeypatch.setattr(eng, "run_step_device",
+                        lambda bs: eng.status.bitwise_or_(bad.pop() if bad else 0))
+    s = eng.open_sequence()
+    for tokens in ([1, 2, 3], [4]):
+        bad.append(4)
+        with pytest.raises(RuntimeError, match="device status word 4"):
+            eng.feed([(s, tokens)])
+        assert len(eng.feed([(s, tokens)])) == 1 and eng.device_status() == 0
+
+
 def test_trace_runner_protocol(tmp_path, monkeypatch):
     """Ids become sequences, wanted rows go to files in order, ended requests are given
     back, one 'done' line per step."""
