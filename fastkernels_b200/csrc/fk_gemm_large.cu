@@ -79,17 +79,19 @@ __device__ __forceinline__ bool gl_wait_warp(uint64_t* bar, uint32_t parity,
   return __all_sync(0xffffffffu, gl_wait(bar, parity, abort_flag, status) ? 1 : 0) != 0;
 }
 
-// bias of the 8 columns from `col` on
-__device__ __forceinline__ void gl_bias(const GemmLargeParams& p, int col, float (&b)[8]) {
+// bias of the 8 columns from `col` on; `from`: where the columns' own begins
+__device__ __forceinline__ void gl_bias(const GemmLargeParams& p, int col, float (&b)[8],
+                                        int from = 0) {
   if (!p.bias) return;
+  const uint16_t* bias = p.bias + from;
   if (col + 8 <= p.n) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(bias + col));
     b[0] = bf16lo(v.x); b[1] = bf16hi(v.x); b[2] = bf16lo(v.y); b[3] = bf16hi(v.y);
     b[4] = bf16lo(v.z); b[5] = bf16hi(v.z); b[6] = bf16lo(v.w); b[7] = bf16hi(v.w);
   } else {
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (col + i < p.n) b[i] = bf16_bits_to_float(p.bias[col + i]);
+      if (col + i < p.n) b[i] = bf16_bits_to_float(bias[col + i]);
   }
 }
 
@@ -108,14 +110,8 @@ __device__ __forceinline__ void gl_store_act(const GemmLargeParams& p, uint16_t*
     if (col >= p.n) break;                     // n is a multiple of 8
     float bg[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float bu[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (p.bias) {
-      const uint4 a = __ldg(reinterpret_cast<const uint4*>(p.bias + col));
-      const uint4 b = __ldg(reinterpret_cast<const uint4*>(p.bias + p.n + col));
-      bg[0] = bf16lo(a.x); bg[1] = bf16hi(a.x); bg[2] = bf16lo(a.y); bg[3] = bf16hi(a.y);
-      bg[4] = bf16lo(a.z); bg[5] = bf16hi(a.z); bg[6] = bf16lo(a.w); bg[7] = bf16hi(a.w);
-      bu[0] = bf16lo(b.x); bu[1] = bf16hi(b.x); bu[2] = bf16lo(b.y); bu[3] = bf16hi(b.y);
-      bu[4] = bf16lo(b.z); bu[5] = bf16hi(b.z); bu[6] = bf16lo(b.w); bu[7] = bf16hi(b.w);
-    }
+    gl_bias(p, col, bg);
+    gl_bias(p, col, bu, p.n);
     uint32_t o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -649,7 +645,7 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
   return FK_OK;
 }
 
-// Which kernel: 0 = single CTAs, 1 = CTA pairs on 256 x 256 tiles.
+// Which kernel: 0 = single CTAs, 1 = CTA pairs on 256 x 256 tiles, 2 = pairs on 256 x 512.
 //
 // An SM gets about as much done in either, so what decides is how the tiles fill their rounds: a
 // pair's round is half as long, and its epilogue runs beside the next tile's products, which the
@@ -659,8 +655,10 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
 // activation, kernels in turn: the choice is 0.2 % from the faster one on average and 4 % at
 // worst.  Examples, single / pair: 537 x 2048 x 6144 67 / 48, 1000 x 3072 x 2048 30 / 21,
 // 2048 x 4608 x 3072 43 / 51, 1024 x 6144 x 4096 54 / 65, 4096 x 16384 x 64 54 / 68.
-// Pairs on 256 x 512 tiles read a quarter less and were never more than 2 % ahead
-// (16384 x 3072 x 8192 663 -> 651): by FK_B200_GEMM_PAIR only.
+// Pairs on 256 x 512 tiles read a quarter less.  One product at a time they are level with single
+// CTAs at best, but in a prompt, where the power limit sets the clock, they are ahead on long k
+// over several rounds: 8192 tokens of the 8b Llama sizes 14.46 -> 14.30 ms, five prompts of the 8b
+// Pinuvik sizes 24.17 -> 23.58.
 static int large_mode(const GemmLargeParams& p) {
   auto rounds = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
@@ -671,6 +669,9 @@ static int large_mode(const GemmLargeParams& p) {
   const double t_single = 2. + rounds(tiles, sm_count()) * (9.4 + 0.0117 * k);
   const double t_pair =
       3. + 0.0016 * k1 + rounds(tiles, pairs) * (store > multiply ? store : multiply);
+  if (p.k >= 4096 && rounds(tiles, sm_count()) >= 2. && t_pair > 0.95 * t_single &&
+      rounds((int64_t)p.m_tiles * ((p.n_tiles + 1) / 2), pairs) <= rounds(tiles, sm_count()))
+    return 2;
   return t_pair < t_single ? 1 : 0;
 }
 

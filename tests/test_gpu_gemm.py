@@ -196,6 +196,7 @@ print('pair ok')
                                           (2010, 6152, 2048, 1),   # pairs over several rounds
                                           (2010, 4096, 4096, 0),   # single CTAs: one full round
                                           (2048, 9472, 4096, 0),   # ... two full rounds
+                                          (2048, 9216, 4096, 2),   # wide pairs: no more rounds
                                           (300, 16384, 64, 0),     # a round is its epilogue
                                           (257, 1000, 64, 1)])     # one tile row, one short round
 def test_gemm_many_rows_kernel_choice(ops, m, n, k, kernel):
@@ -284,7 +285,8 @@ sys.path.insert(0, 'tests')
 from fastkernels_b200 import _lib, ops
 for (m, n, k, bias) in [(257, 16, 64, True), (300, 272, 192, False), (513, 2064, 128, True),
                         (1000, 4096, 256, False), (2049, 1536, 64, True), (2010, 4096, 4096, True),
-                        (300, 16384, 64, False), (300, 1040, 4096, True)]:
+                        (300, 16384, 64, False), (300, 1040, 4096, True),
+                        (2048, 9216, 4096, False)]:
     g = torch.Generator(device='cuda').manual_seed(m)
     x = torch.empty((m, k + 8), dtype=torch.bfloat16, device='cuda').normal_(generator=g)[:, :k]
     w = torch.empty((n, k), dtype=torch.bfloat16, device='cuda').normal_(0, 0.2, generator=g)
@@ -305,7 +307,8 @@ if sys.argv[1]:
     assert _lib.lib.fk_gemm_bf16_many_kernel(300, 16384, 64) == int(sys.argv[1])
 elif torch.cuda.get_device_properties(0).multi_processor_count == 148:
     assert [_lib.lib.fk_gemm_bf16_many_kernel(*s) for s in
-            ((2010, 4096, 4096), (300, 16384, 64), (300, 1040, 4096))] == [0, 0, 1]
+            ((2010, 4096, 4096), (300, 16384, 64), (300, 1040, 4096),
+             (2048, 9216, 4096))] == [0, 0, 1, 2]
 print('act ok')
 """
     env = dict(os.environ)
