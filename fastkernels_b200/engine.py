@@ -449,7 +449,7 @@ class DecodeEngine:
                 vals, idxs = ops.argmax_rows(logits)
                 self._copy_status()
                 tok = self.model.greedy(vals, idxs).cpu().numpy()
-                self._raise_on(self._status_np)
+                self._raise_on_copied()
                 for (j, i), t in zip(ends, tok):
                     first[i] = int(t)
             for i, a, c in part:
@@ -491,7 +491,7 @@ class DecodeEngine:
                 logits = self.model.project(hidden).float()
                 self._copy_status()
                 logits = logits.cpu()
-                self._raise_on(self._status_np)
+                self._raise_on_copied()
                 o = 0
                 for i in rest:
                     out[i] = logits[o:o + len(want[i])]
@@ -511,7 +511,7 @@ class DecodeEngine:
             if any(len(want[i]) for i in single):
                 self._copy_status()
                 logits = self.graph_vars["lm_logits"][:n].float().cpu()
-                self._raise_on(self._status_np)
+                self._raise_on_copied()
                 for j, i in enumerate(single):
                     out[i] = logits[j:j + 1].expand(len(want[i]), -1)
         return out
@@ -520,6 +520,12 @@ class DecodeEngine:
         """Status words so far to the host, ahead of a copy that is waited for."""
         for at, w in zip(self._status_host_words, self._status_words()):
             at.copy_(w, non_blocking=True)
+
+    def _raise_on_copied(self) -> None:
+        """Several ranks go on together: a rank that raised alone would leave the others waiting
+        for it, so theirs is seen by decode() and device_status()."""
+        if self.tp == 1:
+            self._raise_on(self._status_np)
 
     def graph_batch_size(self, n: int) -> int:
         for bs in sorted(self.graphs):
@@ -698,9 +704,9 @@ class DecodeEngine:
         """One decode step for all running sequences through the public path:
         host prep -> pinned H2D staging -> graph replay -> D2H of the token ids.
         With sync=True the sampled ids come back to the host before returning
-        and feed the next step from the host (a device-side anomaly up to here
-        raises); with sync=False the next step reads them from the device buffer
-        and the host copy is deferred."""
+        and feed the next step from the host (on one GPU, a device-side anomaly up
+        to here raises); with sync=False the next step reads them from the device
+        buffer and the host copy is deferred."""
         n = self.prepare_decode(use_host_ids=sync)
         bs = self.graph_batch_size(n)
         self.stage_inputs(n, bs, use_host_ids=sync)
@@ -721,7 +727,7 @@ class DecodeEngine:
         for s, t in zip(self.seqs, ids.tolist()):
             s.last_token = t
             s.output.append(t)
-        if words[0] or words[-1]:
+        if (words[0] or words[-1]) and self.tp == 1:
             self._raise_on(words.view(np.int32))
         return ids
 
@@ -739,4 +745,5 @@ class DecodeEngine:
         """Greedy-decode `steps` tokens for every running sequence; [steps, n].
         Raises if a kernel reported a device-side anomaly on the way."""
         toks = np.stack([self.step(sync=True) for _ in range(steps)])
+        self._raise_on([self.device_status()])
         return toks
