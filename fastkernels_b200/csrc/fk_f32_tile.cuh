@@ -1,4 +1,4 @@
-// True fp32 products on the FMA pipes: fk_gemm_f32 and the fp32 form of fk_group_gemm.
+// True fp32 products: fk_gemm_f32 and the fp32 form of fk_group_gemm.
 #pragma once
 
 #include "fk_common.cuh"
@@ -16,8 +16,8 @@ struct F32Product {
   int32_t* status;
 };
 
-// expect: rows of a group (row groups: on average).  Rows of x and w are 16-byte aligned, k a
-// multiple of 4, sizes within 31 bits and at most 65535 groups.
-int launch_f32_product(const F32Product& p, int64_t expect, cudaStream_t stream);
+// Rows of x and w are 16-byte aligned, k a multiple of 4, sizes within 31 bits and at most 65535
+// groups.
+int launch_f32_product(const F32Product& p, cudaStream_t stream);
 
 }  // namespace fk

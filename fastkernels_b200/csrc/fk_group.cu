@@ -10,7 +10,7 @@
 // each with its part of the bias.
 // bf16 operands with fp32 accumulation and bf16 or fp32 results, or true fp32.
 //
-//   f32_product_kernel   fp32 FMA, any sizes (fp32 operands; fk_plain.cu)
+//   f32_product_kernel   fp32 operands, any sizes (fk_plain.cu)
 //   group_skinny_kernel  few rows: streams the weights straight into mma.sync fragments.
 //                        A product may take its k in any order as long as both operands
 //                        do, so a lane's 16 contiguous bytes of a row serve as the k's of
@@ -963,7 +963,7 @@ int fk_group_gemm(const void* x, int64_t x_stride, int64_t x_group, int64_t x_ro
     f.y = static_cast<float*>(y); f.y_stride = y_stride; f.y_group = y_group;
     f.offsets = offsets; f.gather = gather; f.rows = rows; f.x_rows = x_rows; f.groups = groups;
     f.n = (int)n; f.k = (int)k; f.act = act; f.status = status;
-    return launch_f32_product(f, offsets ? rows / groups + 1 : rows, s);
+    return launch_f32_product(f, s);
   }
   FK_REQUIRE(act < 0 || !y_f32, FK_ERR_UNSUPPORTED,
              "fk_group_gemm: an activation gives a bf16 result");

@@ -1,44 +1,85 @@
 // Kernels without shape restrictions, for the number format and the head sizes the
 // tensor-core kernels do not take:
 //
-//   fk_gemm_f32         y = x w^T (+ bias) in true fp32 (no tensor cores, so no reduced
-//                       precision), any m, n
+//   fk_gemm_f32         y = x w^T (+ bias) in true fp32, any m, n
 //   fk_paged_attn_any   causal attention over the paged NHD pool, bf16 or fp32, any
 //                       head size up to 1152 and any query / KV head ratio; prompt
 //                       portions and single decoded tokens alike
 #include "fk_f32_tile.cuh"
+#include "fk_gemm_shared.cuh"
 #include "fk_types.cuh"
-
 
 namespace fk {
 
 // ------------------------------------------------------------------- fp32 products
-// Bound by the fp32 rate.  A warp computes 32 rows x 64 weight rows, a lane 8 x 8 of them, with
-// the packed fma.rn.f32x2: both halves of an accumulator are the same output, over the even and
-// over the odd k's, so operands come as they lie in memory (k runs along both rows) and nothing
-// is packed or transposed.  Per 4 k's a lane reads 16 float4 for 256 multiply-adds; rows are
-// padded to 36 floats, so the 8 rows that a quarter of a warp reads start in different banks.
-// WR x WC warps make the CTA's tile; loads run kStages - 1 blocks of 32 k's ahead (cp.async).
+// True fp32 products on the tensor cores.  An fp32 number is the sum of three bf16 numbers (each
+// the rest rounded to 8 bits, so nothing is left over), and a product of two of them is six
+// products of parts; the three that are left out are below 2^-26 of it.  Products of parts are
+// exact in fp32, and sums are kept in fp32: 32 k's in tensor memory (whose adder cuts off instead
+// of rounding, so chains there are kept short), smallest parts first, and the blocks of 32 in
+// registers, rounded to nearest.  Off from 64 bits by 1.2 to 1.9e-7 (2-norm; k 2048 to 12288,
+// normal operands), where chains of fp32 multiply-adds are by 2.1 to 5.0e-7.  Numbers below 2^-110
+// are kept to 2^-134, which is as far as bf16 goes.
 //
-// A cluster of 2 to 8 CTAs shares one tile: each takes a part of k, leaves its sums in its shared
-// memory, and adds up its share of the rows over all parts in their order (f32_parts).
-// 1000 rows, 24576 x 4096: 44 TFLOP/s of 72 (scalar 64 x 64 tiles 33).
-template <int WR, int WC>
+// A CTA computes 128 weight rows (the M operand) x up to 128 rows of x.  Two teams of eight warps
+// take every other block of k each: they read it ahead, take the numbers apart, and lay the parts
+// out, the weights' in tensor memory, x's in shared memory, in a ring of four blocks.  One warp
+// issues the 12 instructions of a block, four add up its sums.  Two teams, because the stretches of
+// a block (waits, conversions, loads) follow one another in a warp: sixteen warps on one block go
+// through them in step and take 1800 cycles for it, the teams 1350, the tensor cores alone 770.
+//
+// us, 1 / 100 / 1000 rows (fp32 multiply-adds in register tiles): 24576 x 4096 135 184 1270 (217 644
+// 4542), 2048 x 2048 14 23 96 (36 60 243), 4096 x 12288 68 89 683 (267 317 2540): 160 TFLOP/s.
+//
+// A cluster of CTAs shares one tile: each takes a part of k, leaves its sums in its shared
+// memory, and adds up its share of the rows over all parts in their order (f32_parts).  Where a
+// sum is not finite, an operand may not have been either (the parts of an infinity are no
+// numbers), or one too large for bf16: that output is computed again from the operands.
 struct F32Tile {
-  static constexpr int kRows = 32 * WR, kCols = 64 * WC, kThreads = 32 * WR * WC;
-  static constexpr int kBK = 32, kPitch = kBK + 4;
-  static constexpr int kStages = 3;
-  static constexpr int kStageFloats = (kRows + kCols) * kPitch;
-  static constexpr int kOutPitch = kCols + 8;  // lanes of a store: 4 rows x 8 columns
-  static constexpr int kSmem = kStages * kStageFloats * 4;
-  static_assert(kSmem % 8 == 0 && kRows * kOutPitch * 4 <= kSmem, "sums take the place of the operands");
+  static constexpr int kRows = 128, kCols = 128;       // rows of x, weight rows
+  static constexpr int kBK = 32, kStages = 4, kSums = 2;
+  // two teams of warps that lay out operands, every other block each; warps that add up sums; a
+  // warpgroup of which one issues the products
+  static constexpr int kTeams = 2, kTeam = 8, kWarps = kTeams * kTeam, kAdders = 4;
+  static constexpr int kIssuer = kWarps + kAdders;
+  static constexpr int kThreads = 32 * (kIssuer + 4);
+  static constexpr int kPlane = kRows * kBK * 2;       // one part of the rows of x
+  static constexpr int kStageBytes = 3 * kPlane;
+  // tensor memory: two blocks' sums, then the weights' parts, two numbers a cell
+  static constexpr int kSumCols = kSums * kRows, kPartCols = kBK / 2, kTmemCols = 512;
+  static constexpr int kOutPitch = kCols + 8;
+  static constexpr int kSmem = 128 * 1024;
+  static_assert(kSumCols + kStages * 3 * kPartCols <= kTmemCols, "tensor memory");
+  static_assert(kStages * kStageBytes + 1024 <= kSmem && kRows * kOutPitch * 4 + 1024 <= kSmem,
+                "operands, and the sums in their place");
+  static_assert(tmem_alone(kSmem), "two CTAs could wait for one another's tensor memory");
 };
 
-__device__ __forceinline__ void fma_f32x2(float2& c, float ax, float ay, float bx, float by) {
+// 16 rows x 8 cells: lane l has cells 2 (l & 3), + 1 of rows l / 4 and l / 4 + 8
+__device__ __forceinline__ void tc_st_16x256(uint32_t taddr, uint2 a, uint2 b) {
+  asm volatile("tcgen05.st.sync.aligned.16x256b.x1.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr),
+               "r"(a.x), "r"(a.y), "r"(b.x), "r"(b.y)
+               : "memory");
+}
+// K-major operand in rows of 64 bytes, 64-byte swizzle: 16-byte piece c of row r lies at
+// c ^ (r >> 1 & 3); groups of 8 rows 512 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3fff) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 |
+         (uint64_t)1 << 46 | (uint64_t)4 << 61;
+}
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
+  float2 c;
   asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-      "mov.b64 c, {%0, %1};\n\tfma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
-      : "+f"(c.x), "+f"(c.y)
-      : "f"(ax), "f"(ay), "f"(bx), "f"(by));
+      "add.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(c.x), "=f"(c.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return c;
+}
+// One part of two numbers, and what is left of them
+__device__ __forceinline__ uint32_t f32_part(float2& a) {
+  const uint32_t p = pack_bf16(a.x, a.y);
+  const uint32_t n = p ^ 0x80008000u;
+  a = add_f32x2(a, make_float2(bf16lo(n), bf16hi(n)));
+  return p;
 }
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int rank) {
   uint32_t remote;
@@ -46,6 +87,19 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
+}
+// One output from the operands
+__device__ __noinline__ float f32_dot(const float* x, const float* w, int k) {
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int i = 0; i < k; i += 4) {
+    const float4 a = *reinterpret_cast<const float4*>(x + i);
+    const float4 b = *reinterpret_cast<const float4*>(w + i);
+    s[0] = fmaf(a.x, b.x, s[0]);
+    s[1] = fmaf(a.y, b.y, s[1]);
+    s[2] = fmaf(a.z, b.z, s[2]);
+    s[3] = fmaf(a.w, b.w, s[3]);
+  }
+  return (s[0] + s[1]) + (s[2] + s[3]);
 }
 
 // Row tile `t` of a product with row groups: its group and first row (of the group).
@@ -82,155 +136,253 @@ __device__ __forceinline__ bool f32_row_tile(const F32Product& p, int tile_rows,
   return false;
 }
 
-template <int WR, int WC, bool ACT>
-__global__ void __launch_bounds__(32 * WR * WC, WR * WC == 8 ? 1 : 2)
+template <bool ACT>
+__global__ void __launch_bounds__(F32Tile::kThreads, 1)
     f32_product_kernel(const F32Product p, int parts, int64_t row_tiles) {
-  using Tile = F32Tile<WR, WC>;
-  extern __shared__ __align__(16) float f32_smem[];
-  constexpr int kLoads = (Tile::kRows + Tile::kCols) * (Tile::kBK / 4) / Tile::kThreads;
-  __shared__ const float* f32_rows[Tile::kRows + Tile::kCols];
+  using Tile = F32Tile;
+  extern __shared__ uint8_t f32_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(f32_raw) + 1023) &
+                                             ~uintptr_t(1023));
+  __shared__ const float* f32_rows[Tile::kCols + Tile::kRows];   // weight rows, rows of x
+  __shared__ uint64_t full[Tile::kStages], done[Tile::kStages],
+      taken[Tile::kSums];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+  volatile int* abort_flag = &abort_word;
   constexpr int kOut = ACT ? Tile::kCols / 2 : Tile::kCols;     // outputs a row
-  pdl_launch_dependents();
-  pdl_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ty = lane >> 3, tx = lane & 7, wr = warp / WC, wc = warp % WC;
+  pdl_launch_dependents();
+  if (tid == 0) {
+    for (int i = 0; i < Tile::kStages; ++i) {
+      mbar_init(&full[i], Tile::kTeam);
+      mbar_init(&done[i], 1);
+    }
+    for (int i = 0; i < Tile::kSums; ++i) mbar_init(&taken[i], Tile::kAdders);
+    abort_word = 0;
+    mbar_fence_init();
+  }
+  if (warp == Tile::kIssuer) tmem_alloc(&tmem_slot, Tile::kTmemCols);
+  pdl_wait();
   const int part = (int)(blockIdx.x % parts);
-  const int n0 = (int)(blockIdx.x / parts) * kOut;
+  const int64_t tile = blockIdx.x / parts, t = tile % row_tiles;
+  const int n0 = (int)(tile / row_tiles) * kOut;
   const int blocks_all = (p.k + Tile::kBK - 1) / Tile::kBK;
   const int first_block = (int)((int64_t)blocks_all * part / parts);
   const int blocks = (int)((int64_t)blocks_all * (part + 1) / parts) - first_block;
-  const int c4 = (tid & 7) * 4;                 // 8 threads a row of a block
-  for (int64_t t = blockIdx.y; t < row_tiles; t += gridDim.y) {
-    int g = blockIdx.z;
-    int64_t m0 = t * Tile::kRows, first = 0, count = p.rows;
-    if (p.offsets) {
-      if (!f32_row_tile(p, Tile::kRows, t, &g, &m0)) return;    // uniform over the cluster
+  int g = blockIdx.z;
+  int64_t m0 = t * Tile::kRows, first = 0, count = p.rows;
+  bool there = true;                               // uniform over the cluster
+  if (p.offsets) {
+    there = f32_row_tile(p, Tile::kRows, t, &g, &m0);
+    if (there) {
       first = p.offsets[g];
       count = p.offsets[g + 1] - first;
     }
-    const float* x = p.x + (p.offsets ? 0 : g * p.x_group);
-    const float* w = p.w + (int64_t)g * p.w_rows * p.k;
-    // addresses of the tile's rows, null where there is none (in registers they would spill)
-    for (int r = tid; r < Tile::kRows + Tile::kCols; r += Tile::kThreads) {
-      const float* src = nullptr;
-      if (r < Tile::kRows) {
-        if (m0 + r < count) {
-          int64_t xr = first + m0 + r;
-          if (p.gather) {
-            xr = p.gather[xr];
-            if (xr < 0 || xr >= p.x_rows) {
-              if (p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
-              xr = 0;
-            }
-          }
-          src = x + xr * p.x_stride;
+  }
+  const int live = there ? (int)(count - m0 < Tile::kRows ? count - m0 : Tile::kRows) : 0;
+  const int width = (live + 15) & ~15;             // rows of x that are multiplied
+  // addresses of the tile's rows; where there is none the last one, whose products are not kept
+  if (there && tid < Tile::kCols + Tile::kRows) {
+    const float* src;
+    if (tid < Tile::kCols) {
+      // with an activation 64 gate rows and the 64 up rows of the same outputs
+      const int wrow = min(n0 + (ACT ? tid & 63 : tid), p.n - 1);
+      src = p.w + ((int64_t)g * p.w_rows + wrow + (ACT && tid >= 64 ? p.n : 0)) * p.k;
+    } else {
+      int64_t xr = first + m0 + min(tid - Tile::kCols, live - 1);
+      if (p.gather) {
+        xr = p.gather[xr];
+        if (xr < 0 || xr >= p.x_rows) {
+          if (p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
+          xr = 0;
         }
-      } else {
-        // with an activation 32 of a warp's 64 columns are gate rows, 32 the up rows of the
-        // same outputs
-        const int c = r - Tile::kRows;
-        const int wrow = n0 + (ACT ? (c >> 6) * 32 + (c & 31) : c);
-        if (wrow < p.n) src = w + (int64_t)(wrow + (ACT && (c & 32) ? p.n : 0)) * p.k;
       }
-      f32_rows[r] = src;
+      src = p.x + (p.offsets ? 0 : g * p.x_group) + xr * p.x_stride;
     }
-    __syncthreads();
-    auto load = [&](int stage, int block) {
-      const int k0 = (first_block + block) * Tile::kBK + c4;
-      float* dst = f32_smem + stage * Tile::kStageFloats + (tid >> 3) * Tile::kPitch + c4;
+    f32_rows[tid] = src;
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  auto cluster_sync = [] {
+    __syncwarp();                      // lanes may have stored different numbers of outputs
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  };
+  // a wait of all of the warp's lanes; false in all of them when it ran out
+  auto wait = [&](uint64_t* bar, int use) {
+    const bool ok = gemm_wait(bar, (uint32_t)use & 1u, abort_flag, p.status);
+    return __all_sync(0xffffffffu, ok) != 0;
+  };
+  float* const out = reinterpret_cast<float*>(smem);
+  // registers: 768 threads x 80 = 512 x 72 + 128 x 152 + 128 x 40
+  if (warp >= Tile::kIssuer) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width >> 3) << 17) |
+                           ((uint32_t)(Tile::kCols >> 4) << 24);
+    // the products of a block, smallest first, when all of its parts are laid out and the sums
+    // that were in their place are taken
+    for (int b = 0; there && warp == Tile::kIssuer && b < blocks; ++b) {
+      const int stage = b % Tile::kStages, sum = b % Tile::kSums;
+      if (b >= Tile::kSums && !wait(&taken[sum], b / Tile::kSums - 1)) break;
+      if (!wait(&full[stage], b / Tile::kStages)) break;
+      tc_fence_after();
+      const uint32_t w = tmem + Tile::kSumCols + stage * 3 * Tile::kPartCols;
+      constexpr int kW[6] = {2, 0, 1, 1, 0, 0}, kX[6] = {0, 2, 1, 0, 1, 0};
+      // one branch for all: an instruction every 64 cycles, 130 where each has its own
+      if (elect_one()) {
+        const uint64_t x = smem_desc_sw64(smem_u32(smem + stage * Tile::kStageBytes));
 #pragma unroll
-      for (int i = 0; i < kLoads; ++i) {
-        const float* src = f32_rows[(tid >> 3) + i * (Tile::kThreads / 8)];
-        const bool ok = src != nullptr && k0 < p.k;
-        const uint32_t bytes = ok ? 16u : 0u;   // the rest is filled with zeros
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                         smem_u32(dst + i * (Tile::kThreads / 8) * Tile::kPitch)),
-                     "l"(ok ? src + k0 : p.w), "r"(bytes)
-                     : "memory");
+        for (int i = 0; i < 6; ++i)
+#pragma unroll
+          for (int kk = 0; kk < Tile::kBK / 16; ++kk)
+            tc_mma_bf16_ts(tmem + sum * Tile::kRows, w + kW[i] * Tile::kPartCols + kk * 8,
+                           x + ((kX[i] * Tile::kPlane + kk * 32) >> 4), idesc,
+                           i > 0 || kk > 0 ? 1u : 0u);
+        tc_commit(&done[stage]);
       }
-    };
-    float2 acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int s = 0; s < Tile::kStages - 1; ++s) {
-      if (s < blocks) load(s, s);
-      asm volatile("cp.async.commit_group;" ::: "memory");
+      __syncwarp();
     }
-    int stage = 0;
-    for (int b = 0; b < blocks; ++b) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(Tile::kStages - 2) : "memory");
-      __syncthreads();
-      const int ahead = b + Tile::kStages - 1;
-      if (ahead < blocks) load(stage == 0 ? Tile::kStages - 1 : stage - 1, ahead);
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      const float* xs = f32_smem + stage * Tile::kStageFloats + (wr * 32 + ty) * Tile::kPitch;
-      const float* ws = f32_smem + stage * Tile::kStageFloats +
-                        (Tile::kRows + wc * 64 + tx) * Tile::kPitch;
+    cluster_sync();                    // sums are laid out
+    cluster_sync();                    // and read
+    if (warp == Tile::kIssuer) tmem_dealloc(tmem, Tile::kTmemCols);
+    return;
+  }
+  if (warp >= Tile::kWarps) {
+    // a lane has one weight row and all rows of x
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+    const int q = warp & 3;
+    float2 acc[Tile::kRows / 2];
 #pragma unroll
-      for (int kk = 0; kk < Tile::kBK; kk += 4) {
-        float4 a[8];
+    for (int i = 0; i < Tile::kRows / 2; ++i) acc[i] = make_float2(0.f, 0.f);
+    bool ok = true;
+    for (int b = 0; there && b < blocks; ++b) {
+      const int sum = b % Tile::kSums;
+      ok = wait(&done[b % Tile::kStages], b / Tile::kStages);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int h = 0; h < Tile::kRows; h += 16) {
+        if (h >= width) break;
+        uint32_t v[16];
+        tc_ld16(tmem + sum * Tile::kRows + h + ((uint32_t)(q * 32) << 16), v);
+        tc_wait_ld();
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-          a[i] = *reinterpret_cast<const float4*>(xs + i * 4 * Tile::kPitch + kk);
+          acc[h / 2 + i] = add_f32x2(acc[h / 2 + i], make_float2(__uint_as_float(v[2 * i]),
+                                                                 __uint_as_float(v[2 * i + 1])));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&taken[sum]);
+    }
+    // a wait ran out: no number, so that the outputs are computed from the operands
+    float* to = out + q * 32 + lane;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float4 v = *reinterpret_cast<const float4*>(ws + j * 8 * Tile::kPitch + kk);
+    for (int i = 0; i < Tile::kRows; ++i)
+      if (i < live)
+        to[i * Tile::kOutPitch] = ok ? (i & 1 ? acc[i / 2].y : acc[i / 2].x) : __int_as_float(0x7fffffff);
+    cluster_sync();
+    cluster_sync();
+    return;
+  }
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  if (there) {
+    const int team = warp / Tile::kTeam, half = warp >> 2 & 1;
+    // weights: 16-byte pieces lane & 3 and 4 further of rows w0 and w0 + 8, as tc_st_16x256 wants
+    // them; x: piece `c` of rows r, r + 32, ...
+    const int w0 = (warp & 3) * 32 + half * 16;
+    const uint32_t wdst = tmem + Tile::kSumCols + ((uint32_t)w0 << 16);
+    const float* ws[2] = {f32_rows[w0 + (lane >> 2)], f32_rows[w0 + (lane >> 2) + 8]};
+    const int c = tid & 7, r = (tid & 255) >> 3;
+    const int xdst = r * 64 + (((c >> 1) ^ ((r >> 1) & 3)) << 4) + (c & 1) * 8;   // rows + 32 too
+    const float* const* xs = f32_rows + Tile::kCols + r;
+    float4 wv[4], xv[4];
+    auto load = [&](int b) {
+      if (b >= blocks) return;
+      const int k0 = (first_block + b) * Tile::kBK;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) fma_f32x2(acc[i][j], a[i].x, a[i].y, v.x, v.y);
+      for (int i = 0; i < 4; ++i) {
+        const int k1 = k0 + (i >> 1) * 16 + (lane & 3) * 4;
+        wv[i] = k1 < p.k ? __ldg(reinterpret_cast<const float4*>(ws[i & 1] + k1)) : zero;
+      }
+      const bool in = k0 + c * 4 < p.k;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) fma_f32x2(acc[i][j], a[i].z, a[i].w, v.z, v.w);
+      for (int i = 0; i < 4; ++i)
+        if (r + 32 * i < width)
+          xv[i] = in ? __ldg(reinterpret_cast<const float4*>(xs[32 * i] + k0 + c * 4)) : zero;
+    };
+    load(team);
+    for (int b = team; b < blocks; b += Tile::kTeams) {
+      const int stage = b % Tile::kStages;
+      if (b >= Tile::kStages && !wait(&done[stage], b / Tile::kStages - 1)) break;
+      tc_fence_after();
+      const uint32_t wto = wdst + stage * 3 * Tile::kPartCols;
+#pragma unroll
+      for (int i = 0; i < 4; i += 2) {
+        float2 lo0 = make_float2(wv[i].x, wv[i].y), hi0 = make_float2(wv[i].z, wv[i].w);
+        float2 lo1 = make_float2(wv[i + 1].x, wv[i + 1].y), hi1 = make_float2(wv[i + 1].z, wv[i + 1].w);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const uint2 a = make_uint2(f32_part(lo0), f32_part(hi0));
+          const uint2 e = make_uint2(f32_part(lo1), f32_part(hi1));
+          tc_st_16x256(wto + j * Tile::kPartCols + i * 4, a, e);
         }
       }
-      if (++stage == Tile::kStages) stage = 0;
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+      uint8_t* xto = smem + stage * Tile::kStageBytes + xdst;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < 4; ++i) {
+        if (r + 32 * i >= width) continue;
+        float2 lo = make_float2(xv[i].x, xv[i].y), hi = make_float2(xv[i].z, xv[i].w);
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        f32_smem[(wr * 32 + i * 4 + ty) * Tile::kOutPitch + wc * 64 + j * 8 + tx] =
-            acc[i][j].x + acc[i][j].y;
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    const int live = (int)(count - m0 < Tile::kRows ? count - m0 : Tile::kRows);
-    const int r0 = live * part / parts, r1 = live * (part + 1) / parts;
-    float* y = p.y + (p.offsets ? 0 : g * p.y_group);
-    auto sum = [&](int r, int c) {
-      const int at = r * Tile::kOutPitch + c;
-      const uint32_t addr = smem_u32(f32_smem + at);
-      float v = ld_cluster_f32(addr, 0);
-      for (int q = 1; q < parts; ++q) v += ld_cluster_f32(addr, q);
-      return v;
-    };
-    for (int i = r0 * kOut + tid; i < r1 * kOut; i += Tile::kThreads) {
-      const int r = i / kOut, c = i % kOut;
-      if (n0 + c >= p.n) continue;
-      float v;
-      if (ACT) {
-        const int col = (c >> 5) * 64 + (c & 31);
-        const float gate = sum(r, col) + (p.bias ? p.bias[n0 + c] : 0.f);
-        const float up = sum(r, col + 32) + (p.bias ? p.bias[p.n + n0 + c] : 0.f);
-        v = (p.act == FK_ACT_SILU ? gate * sigmoid_f32(gate) : gelu_tanh_f32(gate)) * up;
-      } else {
-        v = sum(r, c) + (p.bias ? p.bias[n0 + c] : 0.f);
+        for (int j = 0; j < 3; ++j) {
+          const uint32_t pl = f32_part(lo), ph = f32_part(hi);
+          *reinterpret_cast<uint2*>(xto + j * Tile::kPlane + i * 32 * 64) = make_uint2(pl, ph);
+        }
       }
-      y[(first + m0 + r) * p.y_stride + n0 + c] = v;
+      load(b + Tile::kTeams);
+      tc_wait_st();
+      tc_fence_before();
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[stage]);
     }
-    // peers may still read this CTA's sums; the next tile overwrites them
-    __syncwarp();                      // lanes stored different numbers of outputs
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
+  cluster_sync();
+  const int r0 = live * part / parts, r1 = live * (part + 1) / parts;
+  float* y = p.y + (p.offsets ? 0 : g * p.y_group);
+  auto sum = [&](int r, int c) {
+    const uint32_t addr = smem_u32(out + r * Tile::kOutPitch + c);
+    float v = ld_cluster_f32(addr, 0);
+    for (int q = 1; q < parts; ++q) v += ld_cluster_f32(addr, q);
+    if (!(fabsf(v) <= 3.402823466e38f)) v = f32_dot(f32_rows[Tile::kCols + r], f32_rows[c], p.k);
+    return v;
+  };
+  for (int i = r0 * kOut + tid; i < r1 * kOut; i += 32 * Tile::kWarps) {
+    const int r = i / kOut, c = i % kOut;
+    if (n0 + c >= p.n) continue;
+    float v;
+    if (ACT) {
+      const float gate = sum(r, c) + (p.bias ? p.bias[n0 + c] : 0.f);
+      const float up = sum(r, c + 64) + (p.bias ? p.bias[p.n + n0 + c] : 0.f);
+      v = (p.act == FK_ACT_SILU ? gate * sigmoid_f32(gate) : gelu_tanh_f32(gate)) * up;
+    } else {
+      v = sum(r, c) + (p.bias ? p.bias[n0 + c] : 0.f);
+    }
+    y[(first + m0 + r) * p.y_stride + n0 + c] = v;
+  }
+  cluster_sync();                      // peers may still read this CTA's sums
 }
 
-// Short k: the tiles above spend their time filling the ring and handing sums on.  64 x 64
+// Short k: the tiles above spend their time filling the ring and handing sums on, and half of a
+// tile's weight rows may be missing.  fp32 multiply-adds, 64 x 64
 // outputs, 4 x 4 a thread, k in one order.  us, 60 / 200 / 1000 rows, here and in the tiles above:
-// 16 heads of 96 -> 512 8 21 55 (18 21 80), 40 of 256 -> 64 15 35 50 (17 38 108 in one part),
-// 12288 x 256 34 58 196 (35 65 213; one row 31 and 21).
+// 16 heads of 96 -> 512 7 21 54 (11 28 98), 40 of 256 -> 64 15 35 50 (13 28 76), 40 of 64 -> 256
+// 10 15 48 (20 34 116).
 constexpr int FS_M = 64, FS_N = 64, FS_K = 16, FS_MAX_K = 511;
 
 template <bool ACT>
@@ -334,24 +486,24 @@ static int launch_f32_short(const F32Product& p, cudaStream_t s) {
 }
 
 // Parts of k, by the weights' sizes alone: a row's sums are taken in the same order whatever other
-// rows are in the call (tiles of every height add up k alike).  Few weight tiles get more parts, so
-// that few rows find SMs; many rows would have them anyway and pay for the exchange.  us, rows 1 /
-// 100 / 500 / 1000, k 2048 unless said, in 2, 4 and 8 parts (scalar 64 x 64 tiles):
-//   n 544            67 115 118 120     36 61 64 123       21 34 68 102       (94 98 99 193)
-//   n 2048           67 113 118 231     36 61 123 244      21 66 168 302      (94 99 278 297)
-//   n 4096, k 4096   131 216 436 869    93 112 451 898     58 175 534 1063    (213 353 604 1043)
-//   n 6144           78 116 347 685     54 120 366 729     32 131 437 871     (126 198 441 797)
-//   n 4352           68 114 230 458     40 119 303 544     32 99 333 633      (95 199 297 580)
-// 32 experts, 2 x 1024 x 2048, 4 / 60 / 400 / 3100 rows in all: 70 201 239 753, 59 207 257 808,
-// 51 234 299 936 (243 364 632 999).
+// rows are in the call.  Few weight tiles get more parts, so that few rows find SMs; many rows
+// would have them anyway and pay for the exchange.  us, rows 1 / 100 / 500 / 1000 in 1, 2, 4, 8 parts:
+//   n 544, k 2048     36 55 60 61     21 34 38 38     14 22 25 46      11 17 35 51
+//   n 2048, k 2048    36 55 61 64     21 34 39 75     14 23 49 95      20 32 86 152
+//   n 4096, k 4096    70 101 117 223  39 58 124 243   23 35 145 288    41 65 211 416
+//   n 7680, k 2560    48 71 149 292   28 43 173 300   33 51 216 402    47 72 308 607
+//   n 24576, k 4096   163 222 682 1231  135 184 677 1279  154 215 858 1662  210 303 1213 2382
+//   n 32768, k 2048   91 125 438 853  101 146 526 1032  126 188 754 1458  198 303 1189 2332
+// 32 experts, 2 x 1024 x 2048, 4 / 60 / 400 / 3100 rows in all: 38 180 187 264, 26 185 199 297,
+// 34 256 283 437, 52 424 473 743; 64 of 4096 x 1408: 37 285 485 595, 43 354 573 751.
 static int f32_parts(const F32Product& p) {
   const int64_t tiles = (p.w_rows + 127) / 128 * p.groups;
-  return tiles <= 12 && p.k >= 2048 ? 8 : tiles <= 32 && p.k >= 1024 ? 4 : 2;
+  return tiles <= 12 && p.k >= 2048 ? 8 : tiles <= 32 && p.k >= 1024 ? 4 : tiles < 256 ? 2 : 1;
 }
 
-template <int WR, int WC, bool ACT>
+template <bool ACT>
 static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
-  using Tile = F32Tile<WR, WC>;
+  using Tile = F32Tile;
   constexpr int kOut = ACT ? Tile::kCols / 2 : Tile::kCols;
   const int64_t n_tiles = (p.n + kOut - 1) / kOut;
   const int64_t upto = (p.rows + Tile::kRows - 1) / Tile::kRows;
@@ -359,10 +511,13 @@ static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
   const int64_t used = p.rows < p.groups ? p.rows : p.groups;
   const int64_t row_tiles = p.offsets ? upto + used : upto;
   const int parts = f32_parts(p);
+  FK_REQUIRE(n_tiles * row_tiles * parts <= 0x7fffffff, FK_ERR_UNSUPPORTED,
+             "fp32 product: too many tiles");
   static PerDeviceOnce once;
-  FK_CUDA_OK(set_max_dynamic_smem(once, f32_product_kernel<WR, WC, ACT>, Tile::kSmem));
+  FK_CUDA_OK(set_max_dynamic_smem(once, f32_product_kernel<ACT>, Tile::kSmem));
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(n_tiles * parts), (unsigned)(row_tiles < 65535 ? row_tiles : 65535),
+  // rows fastest: the tiles of a weight tile find it in L2
+  cfg.gridDim = dim3((unsigned)(n_tiles * row_tiles * parts), 1u,
                      p.offsets ? 1u : (unsigned)p.groups);
   cfg.blockDim = dim3(Tile::kThreads);
   cfg.dynamicSmemBytes = Tile::kSmem;
@@ -379,22 +534,17 @@ static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
   attr[na++].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  FK_CUDA_OK(cudaLaunchKernelEx(&cfg, f32_product_kernel<WR, WC, ACT>, p, parts, row_tiles));
+  FK_CUDA_OK(cudaLaunchKernelEx(&cfg, f32_product_kernel<ACT>, p, parts, row_tiles));
   count_launch();
   return FK_OK;
 }
 
-// Row tiles of 32, 64 or 128: the smallest that holds the rows; row groups take 64 up to three
-// tiles on average, since their last tile is half empty.
 template <bool ACT>
-static int launch_f32(const F32Product& p, int64_t expect, cudaStream_t s) {
-  if (p.k <= FS_MAX_K) return launch_f32_short<ACT>(p, s);
-  if (expect <= 32) return launch_f32_tile<1, 2, ACT>(p, s);
-  if (expect <= 64 || (p.offsets && expect <= 192)) return launch_f32_tile<2, 2, ACT>(p, s);
-  return launch_f32_tile<4, 2, ACT>(p, s);
+static int launch_f32(const F32Product& p, cudaStream_t s) {
+  return p.k <= FS_MAX_K ? launch_f32_short<ACT>(p, s) : launch_f32_tile<ACT>(p, s);
 }
-int launch_f32_product(const F32Product& p, int64_t expect, cudaStream_t s) {
-  return p.act >= 0 ? launch_f32<true>(p, expect, s) : launch_f32<false>(p, expect, s);
+int launch_f32_product(const F32Product& p, cudaStream_t s) {
+  return p.act >= 0 ? launch_f32<true>(p, s) : launch_f32<false>(p, s);
 }
 
 // ----------------------------------------------------------------------- attention
@@ -682,7 +832,7 @@ int fk_gemm_f32(const float* x, int64_t x_stride, const float* w, const float* b
   p.x = x; p.x_stride = x_stride; p.w = w; p.w_rows = n; p.bias = bias; p.y = y;
   p.y_stride = y_stride; p.rows = p.x_rows = m; p.groups = 1; p.n = (int)n; p.k = (int)k;
   p.act = -1;
-  return launch_f32_product(p, m, static_cast<cudaStream_t>(stream));
+  return launch_f32_product(p, static_cast<cudaStream_t>(stream));
 }
 
 int fk_paged_attn_any(const void* q, int64_t q_stride, void* out, int64_t out_stride,

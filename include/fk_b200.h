@@ -679,7 +679,7 @@ int fk_head_norm_gate(const float* o, const void* gate, int64_t gate_stride, con
                     void* out, int64_t out_stride, int is_f32, int64_t rows, int heads, int dim,
                     float eps, fk_stream_t stream);
 
-/* y[m, n] = x[m, k] w[n, k]^T (+ bias) in fp32 (no tensor cores); k % 4 == 0.  A row comes out
+/* y[m, n] = x[m, k] w[n, k]^T (+ bias) in fp32; k % 4 == 0.  A row comes out
  * with the same bits whatever other rows are in the call: the order of its sums hangs on the sizes
  * of w alone (here and in the fp32 form of fk_group_gemm). */
 int fk_gemm_f32(const float* x, int64_t x_stride, const float* w, const float* bias, float* y,

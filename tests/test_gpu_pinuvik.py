@@ -281,6 +281,55 @@ def test_f32_rows_do_not_hang_on_the_call(n, k):
         assert torch.equal(ops.group_gemm(x[a:b], groups, offsets=i32(off)), whole[a:b])
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 128, 129])
+@pytest.mark.parametrize("n,k,act", [(128, 2048, None), (129, 2044, None), (2048, 1028, None),
+                                     (5000, 544, None), (33000, 512, None), (64, 2076, 0),
+                                     (200, 1056, 1)])
+def test_f32_tile_edges(m, n, k, act):
+    """Edges of the tiles in rows, weight rows and blocks of k, in 8, 4, 2 and 1 parts."""
+    from fastkernels_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(m * n + k)
+    x = torch.randn(m, k, generator=gen, device="cuda")
+    w = torch.randn(1, n * (1 if act is None else 2), k, generator=gen, device="cuda")
+    z, size = x.double() @ w[0].double().T, x.double().abs() @ w[0].double().abs().T
+    # a block of 32 products: 12 additions in tensor memory of up to 2^-23 of it each; the blocks'
+    # sums, rounded once each; the products of parts left out
+    limit = (12 + k / 32) * 2.0 ** -23 * size
+    if act is None:
+        assert ((ops.gemm(x, w[0]).double() - z).abs() <= limit).all()
+        return
+    got = ops.group_gemm(x, w, offsets=i32([0, m]), act=act).double().cpu().numpy()
+    z = z.cpu().numpy()
+    gate, up = z[:, :n], z[:, n:]
+    want = (P.gelu_tanh(gate) if act else gate * P.sigmoid(gate)) * up
+    # |act'| <= 1.13
+    off = limit.cpu().numpy()
+    limit = 1.13 * off[:, :n] * np.abs(up) + np.abs(gate) * off[:, n:] + 2e-6 * (np.abs(want) + 1)
+    assert (np.abs(got - want) <= limit).all()
+
+
+@pytest.mark.parametrize("k", [300, 2048])
+def test_f32_products_of_what_is_not_finite(k):
+    """Infinities, numbers beyond bf16's largest and sums that overflow come out as fp32
+    arithmetic has them, and touch no other row or column."""
+    from fastkernels_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(20, k, generator=gen, device="cuda")
+    w = torch.randn(150, k, generator=gen, device="cuda")
+    clean = ops.gemm(x, w)
+    x[3, 7], x[4, 9], x[6, 0], x[7] = np.inf, np.nan, 3.4e38, 0.0
+    w[5, 11], w[8, 0], w[9] = -np.inf, 0.5, 0.0
+    got, want = ops.gemm(x, w), x.double() @ w.double().T
+    want = want.float().double()                  # an overflow of the sum
+    assert torch.equal(got.isnan(), want.isnan())
+    inf = want.isinf()
+    assert torch.equal(got.isinf(), inf) and torch.equal(got[inf].double(), want[inf])
+    assert (got[6, 8].double() - want[6, 8]).abs() <= 1e-6 * want[6, 8].abs()
+    rows = [i for i in range(20) if i not in (3, 4, 6, 7)]
+    cols = [i for i in range(150) if i not in (5, 8, 9)]
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("d,hq,hkv,portions", [
     (4, 3, 1, [(0, 5), (40, 1)]), (68, 8, 2, [(0, 1), (70, 33), (3, 4)]),
