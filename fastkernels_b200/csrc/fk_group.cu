@@ -430,11 +430,14 @@ group_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
         tc_fence_after();
         const uint32_t a = smem_u32(smem + stage * Cfg::kStageBytes);
         const uint32_t b = a + GG_A_BYTES;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < GG_BK / 16; ++kk)
-          tc_mma_bf16_elect(buf * BN, smem_desc_sw128(a + kk * 32),
-                            smem_desc_sw128(b + kk * 32), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-        tc_commit_elect(&empty[stage]);
+          for (int kk = 0; kk < GG_BK / 16; ++kk)
+            tc_mma_bf16(buf * BN, smem_desc_sw128(a + kk * 32), smem_desc_sw128(b + kk * 32), idesc,
+                        (kb > 0 || kk > 0) ? 1u : 0u);
+          tc_commit(&empty[stage]);
+        }
+        __syncwarp();
         if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
       if (!ok) break;
@@ -685,11 +688,14 @@ group_stream_kernel(const __grid_constant__ CUtensorMap tmap_x,
         tc_fence_after();
         const uint32_t a = smem_u32(smem + stage * Cfg::kStageBytes);
         const uint32_t b = a + Cfg::kABytes;
+        if (elect_one()) {
 #pragma unroll
-        for (int kk = 0; kk < GG_BK / 16; ++kk)
-          tc_mma_bf16_elect(tmem + buf * NT, smem_desc_sw128(a + kk * 32),
-                            smem_desc_sw128(b + kk * 32), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-        tc_commit_elect(&empty[stage]);
+          for (int kk = 0; kk < GG_BK / 16; ++kk)
+            tc_mma_bf16(tmem + buf * NT, smem_desc_sw128(a + kk * 32),
+                        smem_desc_sw128(b + kk * 32), idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+          tc_commit(&empty[stage]);
+        }
+        __syncwarp();
         if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
       if (!ok) break;

@@ -324,7 +324,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
     }
   } else if (warp == PF_WARP_MMA) {
     // ============================= MMA issuer =============================
-    // The whole warp walks the schedule converged; one elected lane issues.
+    // The whole warp walks the schedule converged; one elected lane issues a product's instructions.
     constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) |
                                  ((uint32_t)(PF_BN >> 3) << 17) |
                                  ((uint32_t)(PF_BM >> 4) << 24);
@@ -334,28 +334,32 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
     auto issue_s = [&](int t, int slot) {
       const uint32_t a = q_addr + t * PF_TILE_BYTES;
       const uint32_t b = kv_addr + slot * PF_TILE_BYTES;
+      if (elect_one()) {
 #pragma unroll
-      for (int kk = 0; kk < PF_D / 16; ++kk) {
-        const uint32_t o = (kk >> 2) * PF_HALF_BYTES + (kk & 3) * 32;
-        tc_mma_bf16_elect(tmem_base + t * PF_BN, smem_desc_sw128(a + o),
-                          smem_desc_sw128(b + o), idesc_s, kk > 0 ? 1u : 0u);
+        for (int kk = 0; kk < PF_D / 16; ++kk) {
+          const uint32_t o = (kk >> 2) * PF_HALF_BYTES + (kk & 3) * 32;
+          tc_mma_bf16(tmem_base + t * PF_BN, smem_desc_sw128(a + o), smem_desc_sw128(b + o), idesc_s,
+                      kk > 0 ? 1u : 0u);
+        }
       }
+      __syncwarp();
     };
     auto issue_pv = [&](int t, int slot, bool acc) {
       // P_t sits in the first 64 columns of S_t (two bf16 per cell): 16 keys
       // = 8 columns per instruction
       const uint32_t a = tmem_base + t * PF_BN;
       const uint32_t b = kv_addr + slot * PF_TILE_BYTES;
+      if (elect_one()) {
 #pragma unroll
-      for (int kk = 0; kk < PF_BN / 16; ++kk) {
-        tc_mma_bf16_ts_elect(tmem_base + 2 * PF_BN + t * PF_D, a + kk * 8,
-                             smem_desc_sw128_mn(b + kk * 2048, PF_HALF_BYTES, 1024),
-                             idesc_pv, (acc || kk > 0) ? 1u : 0u);
-        if (SPLIT)
-          tc_mma_bf16_ts_elect(tmem_base + 2 * PF_BN + t * PF_D, a + 64 + kk * 8,
-                               smem_desc_sw128_mn(b + kk * 2048, PF_HALF_BYTES, 1024),
-                               idesc_pv, 1u);
+        for (int kk = 0; kk < PF_BN / 16; ++kk) {
+          const uint64_t v = smem_desc_sw128_mn(b + kk * 2048, PF_HALF_BYTES, 1024);
+          tc_mma_bf16_ts(tmem_base + 2 * PF_BN + t * PF_D, a + kk * 8, v, idesc_pv,
+                         (acc || kk > 0) ? 1u : 0u);
+          if (SPLIT)
+            tc_mma_bf16_ts(tmem_base + 2 * PF_BN + t * PF_D, a + 64 + kk * 8, v, idesc_pv, 1u);
+        }
       }
+      __syncwarp();
     };
     int kv_base = 0;               // slot uses before this item
     int items = 0;                 // items with work so far

@@ -72,9 +72,9 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   return d;
 }
 
-// Issue by one elected lane of a CONVERGED warp.  The operands are computed by
-// all lanes outside the branch, so warp-uniform descriptors stay in the uniform
-// datapath and the issue rate is not bound by per-instruction register moves.
+// One lane of a CONVERGED warp.  All instructions of a pipeline stage go into one branch: an
+// instruction of 128 rows x up to 128 columns x 16 k's then goes out every 64 cycles, and every 130
+// where each has a branch of its own.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t pred;
   asm volatile(
@@ -84,16 +84,6 @@ __device__ __forceinline__ uint32_t elect_one() {
       : "=r"(pred));
   return pred;
 }
-__device__ __forceinline__ void tc_mma_bf16_elect(uint32_t tmem_d, uint64_t desc_a,
-                                                  uint64_t desc_b, uint32_t idesc,
-                                                  uint32_t accumulate) {
-  if (elect_one()) tc_mma_bf16(tmem_d, desc_a, desc_b, idesc, accumulate);
-}
-__device__ __forceinline__ void tc_mma_bf16_ts_elect(uint32_t tmem_d, uint32_t tmem_a,
-                                                     uint64_t desc_b, uint32_t idesc,
-                                                     uint32_t accumulate) {
-  if (elect_one()) tc_mma_bf16_ts(tmem_d, tmem_a, desc_b, idesc, accumulate);
-}
 __device__ __forceinline__ void tc_commit_elect(uint64_t* bar) {
   if (elect_one()) tc_commit(bar);
 }
@@ -102,28 +92,26 @@ __device__ __forceinline__ void tc_commit_elect(uint64_t* bar) {
 // Issued by the even CTA of a 2-CTA cluster.  The descriptors hold shared-memory
 // offsets that are valid in both CTAs: A = 128 rows per CTA (M = 256 in all), B =
 // one half of the N rows per CTA; D = 128 TMEM lanes x N columns in each CTA.
-__device__ __forceinline__ void tc2_mma_bf16_elect(uint32_t tmem_d, uint64_t desc_a,
-                                                   uint64_t desc_b, uint32_t idesc,
-                                                   uint32_t accumulate) {
-  if (elect_one()) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-  }
+__device__ __forceinline__ void tc2_mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
+                                             uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in BOTH CTAs of the pair
 // once all MMAs issued so far have completed.
+__device__ __forceinline__ void tc2_commit(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster."
+      "multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
 __device__ __forceinline__ void tc2_commit_elect(uint64_t* bar) {
-  if (elect_one()) {
-    asm volatile(
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster."
-        "multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-        "h"((uint16_t)3)
-        : "memory");
-  }
+  if (elect_one()) tc2_commit(bar);
 }
 __device__ __forceinline__ void tmem_alloc2(uint32_t* slot, uint32_t cols) {
   asm volatile(
