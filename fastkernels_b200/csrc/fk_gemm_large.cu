@@ -651,30 +651,32 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
 
 // Which kernel: 0 = single CTAs, 1 = CTA pairs on 256 x 256 tiles, 2 = pairs on 256 x 512.
 //
-// An SM gets about as much done in either, so what decides is how the tiles fill their rounds: a
-// pair's round is half as long, and its epilogue runs beside the next tile's products, which the
-// single CTA's does not; from k = 512 down a round is its epilogue, and the single CTAs' rounds,
-// which store twice as much, are the cheaper ones.  The times below (us, of rounds of tiles) are
-// fitted to 672 sizes, m 257 to 16384, n 1024 to 24576, k 64 to 12288, with and without an
-// activation, kernels in turn: the choice is 0.2 % from the faster one on average and 4 % at
-// worst.  Examples, single / pair: 537 x 2048 x 6144 67 / 48, 1000 x 3072 x 2048 30 / 21,
-// 2048 x 4608 x 3072 43 / 51, 1024 x 6144 x 4096 54 / 65, 4096 x 16384 x 64 54 / 68.
-// Pairs on 256 x 512 tiles read a quarter less.  One product at a time they are level with single
-// CTAs at best, but in a prompt, where the power limit sets the clock, they are ahead on long k
-// over several rounds: 8192 tokens of the 8b Llama sizes 14.46 -> 14.30 ms, five prompts of the 8b
-// Pinuvik sizes 24.17 -> 23.58.
+// A pair's round is half as long, and its epilogue runs beside the next tile's products, which that
+// of the other two does not: above k = 256 the pairs are ahead or level at all 450 sizes measured (m
+// 257 to 16384, n 1024 to 24576).  us, single / pair / wide: 537 x 2048 x 6144 66 / 37 / 66, 4096 x 3072
+// x 2048 58 / 39 / 60, 8192 x 4096 x 4096 218 / 187 / 219, 8192 x 9472 x 4096 489 / 428 / 547, 16384 x
+// 24576 x 4096 with an activation 3139 / 2555 / 3070; and in prompts, where the power limit sets the
+// clock: 8192 tokens of the 8b Llama sizes 14.1 -> 13.7 ms, five prompts of the 8b Pinuvik sizes 23.5
+// -> 23.1.  Where long k's fill one or two rounds of single CTAs, the estimate below decides as it does
+// for short k (2048 x 4096 x 4096 48 / 47; two full rounds are behind, 2048 x 9472 x 4096 120 / 105).
+//
+// From k = 256 down a round is its epilogue, and the single CTAs' rounds, which store twice as
+// much, are the cheaper ones: 300 x 16384 x 64 9.0 / 10.4, 8192 x 8192 x 256 69 / 80.
 static int large_mode(const GemmLargeParams& p) {
   auto rounds = [](int64_t tiles, int64_t slots) { return (double)((tiles + slots - 1) / slots); };
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
   const int pairs = resident_pairs<1, false>();
   if (pairs <= 0) return 0;
+  const double single = rounds(tiles, sm_count()), filled = (double)tiles / (single * sm_count());
+  const bool full = (single == 1. && filled > 0.86) || (single == 2. && filled > 0.97);
+  if (p.k > 256 && !(full && p.k >= 4096)) return 1;
   const double k = p.k, k1 = k < 3000. ? k : 3000.;
   const double store = 5.8 + 0.002 * k, multiply = 0.0074 * k;
-  const double t_single = 2. + rounds(tiles, sm_count()) * (9.4 + 0.0117 * k);
+  const double t_single = 2. + single * (9.4 + 0.0117 * k);
   const double t_pair =
       3. + 0.0016 * k1 + rounds(tiles, pairs) * (store > multiply ? store : multiply);
-  if (p.k >= 4096 && rounds(tiles, sm_count()) >= 2. && t_pair > 0.95 * t_single &&
-      rounds((int64_t)p.m_tiles * ((p.n_tiles + 1) / 2), pairs) <= rounds(tiles, sm_count()))
+  if (p.k >= 4096 && single >= 2. && t_pair > 0.95 * t_single &&
+      rounds((int64_t)p.m_tiles * ((p.n_tiles + 1) / 2), pairs) <= single)
     return 2;
   return t_pair < t_single ? 1 : 0;
 }
