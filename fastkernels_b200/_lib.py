@@ -102,6 +102,7 @@ PROTOTYPES = {
     "fk_prefill_attn": (_i32, [_vp, _i64, _vp, _i64, _vp, _vp, _vp, _i64, _i64, _i32, _i32,
                                _vp, _vp, _vp, _i64, _i32, _i64, _i64, _i32, _i32, _i32, _i32,
                                _f32, _i32, _vp, _vp]),
+    "fk_llama_prompt_layers": (_i32, [_vp, _i32, _i32, _vp, _vp]),
     "fk_merge_attn_states": (_i32, [_vp, _i64, _i64, _vp, _vp, _i64, _i64, _vp, _vp, _i64,
                                     _i64, _vp, _i64, _i32, _i32, _i64, _vp]),
     "fk_gemm_bf16_workspace_bytes": (_sz, [_i64, _i64, _i64]),

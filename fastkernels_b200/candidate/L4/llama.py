@@ -22,6 +22,7 @@ from fastkernels_b200.candidate.L2.parallel_embedding import (ParallelLMHead,
                                                                VocabParallelEmbedding)
 from fastkernels_b200.candidate.L3.llama_decoder import LlamaDecoderLayer
 from fastkernels_b200.candidate import share_classes
+from fastkernels_b200.prompt_layers import PromptRun
 
 __targets__ = ["LlamaForCausalLM"]
 
@@ -149,8 +150,12 @@ class LlamaModel(nn.Module):
         if self._block_path(hidden_states):
             return self._forward_blocks(hidden_states, positions)
         residual = None
+        # a prompt portion's layers are launched from one native call each where that is the same
+        run = PromptRun.begin(self.rotary_emb, hidden_states, positions)
         for layer in self.layers:
-            hidden_states, residual = layer(positions, hidden_states, residual)
+            done = run.layer(layer, hidden_states, residual) if run is not None else None
+            hidden_states, residual = done if done is not None else \
+                layer(positions, hidden_states, residual)
         hidden_states, _ = LlamaDecoderLayer.add_norm(self.norm, hidden_states, residual, 1)
         return hidden_states
 

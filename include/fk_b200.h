@@ -563,6 +563,38 @@ int fk_prefill_attn(const void* q, int64_t q_stride_token, void* out,
                     int32_t* status, fk_stream_t stream);
 
 /* ------------------------------------------------------------------------
+ * The decoder layers of a Llama / Qwen3 prompt portion, launched from one call: per layer
+ *   (add +) input norm, qkv projection, split + q/k norm + RoPE + store, attention over the
+ *   pages, output projection, add + norm, gate/up projection + SiLU, down projection
+ * (fastkernels/tasks/baseline/L3/llama_decoder.py:33-42 over L2/attention.py and llama_mlp.py),
+ * by the entry points above with the arguments that they would get one by one.
+ * Rows are dense, [tokens, hidden].  With `first` residual holds the embeddings and x is written;
+ * else x is what the layer before has left to be added to the residual.  The residual is updated,
+ * and the last layer's down projection is left in x.
+ * qkv, attn and act are scratch of [tokens, (Hq + 2 Hkv) * D], [tokens, Hq * D], [tokens, ff].
+ * ---------------------------------------------------------------------- */
+struct fk_llama_layer {
+  const void *input_norm, *qkv, *qkv_bias, *q_norm, *k_norm, *o, *o_bias, *post_norm, *gate_up,
+      *gate_up_bias, *down, *down_bias;   /* biases and q/k norms may be null */
+  void *k_cache, *v_cache;
+  int32_t* attn_status;
+  double input_eps, qk_eps, post_eps, softmax_scale;
+};
+struct fk_llama_prompt {
+  void *residual, *x, *qkv, *attn, *act;
+  const int64_t* positions;
+  const void* cos_sin_cache;              /* bf16 */
+  const int32_t *slots, *cu_seqlens_q, *cu_seqlens_k, *block_table;
+  void* workspace;                        /* of fk_gemm_bf16 */
+  int32_t* status;
+  int64_t workspace_bytes, tokens, hidden, ff, max_position, num_blocks, block_size,
+      kv_block_stride, kv_layout, block_table_stride, num_seqs, max_seqlen_q, num_q_heads,
+      num_kv_heads, head_dim;
+};
+int fk_llama_prompt_layers(const struct fk_llama_layer* layers, int num_layers, int first,
+                           const struct fk_llama_prompt* prompt, fk_stream_t stream);
+
+/* ------------------------------------------------------------------------
  * Merge of two partial attention results over disjoint key ranges.
  * Replaces merge_attn_states / MergeAttnStates.forward
  *   (fastkernels/tasks/baseline/L1/merge_attn_states.py:32-122, kernel
