@@ -111,13 +111,16 @@ class BlockManager:
             b = end if self.chunk is None else min(end, base + self.chunk)
             self._grow(seq, a)
             self._grow(seq, b - 1)
-            pages = np.asarray(seq.table(self.span), dtype=np.int64)
-            off = np.arange(a - base, b - base)
-            slots.append(pages[off // self.block_size] * self.block_size
-                         + off % self.block_size)
+            pages = np.array(seq.table(self.span), dtype=np.int32)
+            # the slots of all pages from the first token's on
+            skip = (a - base) // self.block_size
+            of_page = np.arange(self.block_size, dtype=np.int32)
+            every = (pages[skip:, None] * np.int32(self.block_size) + of_page).reshape(-1)
+            at = a - base - skip * self.block_size
+            slots.append(every[at:at + b - a])
             segments.append((b - a, b - base, pages))
             a = b
-        return segments, np.concatenate(slots).astype(np.int32)
+        return segments, slots[0] if len(slots) == 1 else np.concatenate(slots)
 
     def flush(self) -> None:
         """Give back the pages of finished chunks: nothing launched from here on

@@ -25,6 +25,8 @@ all captured in the CUDA graph.
 from __future__ import annotations
 
 import os
+import struct
+from itertools import accumulate
 
 import numpy as np
 import torch
@@ -38,6 +40,18 @@ from .models.registry import load_folder, model_class
 # FK_B200_PREPARE_AHEAD=0: stage every step's host arrays only when the step is
 # called (for A/B timing of the look-ahead in DecodeEngine.step)
 _NO_PREPARE_AHEAD = os.environ.get("FK_B200_PREPARE_AHEAD", "1") == "0"
+
+
+def _write_ids(out: np.ndarray, tokens) -> None:
+    """Token ids into an int64 array; a list of ints goes through struct, which takes a third
+    of numpy's time (4096 tokens: 57 us, 173)."""
+    if type(tokens) is list:
+        try:
+            struct.pack_into(f"{len(tokens)}q", out, 0, *tokens)
+            return
+        except struct.error:             # not ints: as numpy converts them
+            pass
+    out[:] = np.asarray(tokens, dtype=np.int64)
 
 
 class DecodeEngine:
@@ -233,8 +247,12 @@ class DecodeEngine:
                           for k, v in slot.items()} for slot in self._ring]
         self._ring_events = [None] * self.RING
         self._ring_pos = 0
-        # (sequence-set version, count) the staging slot was prepared ahead for, or None
+        # (sequence-set version, count) the staging slot was prepared ahead for, or None; the
+        # batch size and stream for which it is on the device already, but for the token ids,
+        # and the ids that the step before has left there
         self._ahead = None
+        self._staged_ahead = None
+        self._sampled: list[int] = []
         self._seq_epoch = 0
         self.host, self.host_np = self._ring[0], self._ring_np[0]
         self.status = self.model.preallocate(n, self.max_model_len, dev, self._attn_max_splits)
@@ -308,7 +326,12 @@ class DecodeEngine:
 
     def finish(self, seq: Sequence) -> None:
         """End a sequence: its pages and its state slot go back."""
-        self.seqs.remove(seq)
+        for i, s in enumerate(self.seqs):
+            if s is seq:                 # comparing by value takes longer than all the rest
+                del self.seqs[i]
+                break
+        else:
+            self.seqs.remove(seq)
         self._release(seq)
         self._running_set_changed()
 
@@ -327,62 +350,65 @@ class DecodeEngine:
         as in prepare_prefill (fastkernels/infra/engine.py:4902-4990): cu_seqlens,
         per-token slots and block tables, so attention reads the pages the store has
         just written.  In a chunked span a portion falls into one segment per chunk."""
-        dev = self.device
-        ids = np.concatenate([np.asarray(t, dtype=np.int64) for _, _, t in portions])
-        pos = np.concatenate([np.arange(a, a + len(t), dtype=np.int64) for _, a, t in portions])
-        # token ids, positions, wanted rows and all int32 metadata travel in one copy
-        i32 = [ids.view(np.int32), pos.view(np.int32),
-               np.asarray(rows, dtype=np.int64).view(np.int32)]
+        counts = [len(t) for _, _, t in portions]
+        total = sum(counts)
+        # token ids, positions, wanted rows and all int32 metadata travel in one copy from
+        # pinned memory
+        i32, sizes, layout = [], [2 * total, 2 * total, 2 * len(rows)], []
 
         def put(a):
-            a = np.ascontiguousarray(a, dtype=np.int32)
-            i32.append(a.reshape(-1))
-            return a.shape
+            i32.append(a)
+            sizes.append(a.size)
 
-        layout = []
         for blocks in self.span_blocks:
             segs, slots = [], []
-            for s, a, t in portions:
-                seg, sl = blocks.extend(s, a, len(t))
+            for (s, a, _), n in zip(portions, counts):
+                seg, sl = blocks.extend(s, a, n)
                 segs += seg
                 slots.append(sl)
-            q = np.array([c for c, _, _ in segs])
-            kv = np.array([k for _, k, _ in segs])
-            bt = np.full((len(segs), max(len(pg) for _, _, pg in segs)), -1, dtype=np.int32)
-            for j, (_, _, pg) in enumerate(segs):
-                bt[j, :len(pg)] = pg
-            layout.append((put(np.concatenate(slots)), put(bt), put(kv),
-                           put(np.concatenate([[0], np.cumsum(q)])),
-                           put(np.concatenate([[0], np.cumsum(kv)])), int(q.max()),
-                           int(kv.max()), int(kv.sum())))
-        state_shape = cu_shape = None
+            q, kv = [c for c, _, _ in segs], [k for _, k, _ in segs]
+            cols = max(len(pg) for _, _, pg in segs)
+            bt = np.full((len(segs), cols), -1, dtype=np.int32)
+            for row, (_, _, pg) in zip(bt, segs):
+                row[:len(pg)] = pg
+            for a in (slots[0] if len(slots) == 1 else np.concatenate(slots), bt.reshape(-1),
+                      np.array(kv, dtype=np.int32),
+                      np.fromiter(accumulate(q, initial=0), np.int32, len(q) + 1),
+                      np.fromiter(accumulate(kv, initial=0), np.int32, len(kv) + 1)):
+                put(a)
+            layout.append((cols, max(q), max(kv), sum(kv)))
         if self.state_slots is not None:
-            state_shape = put(np.repeat([s.state_slot for s, _, _ in portions],
-                                        [len(t) for _, _, t in portions]))
-            cu_shape = put(np.concatenate([[0], np.cumsum([len(t) for _, _, t in portions])]))
-        flat = torch.from_numpy(np.concatenate(i32)).to(dev)
-        at = 4 * len(ids) + 2 * len(rows)
-        ids_dev, pos_dev, rows_dev = flat[:at].view(torch.int64).split(
-            [len(ids), len(ids), len(rows)])
+            put(np.repeat(np.array([s.state_slot for s, _, _ in portions], dtype=np.int32), counts))
+            put(np.fromiter(accumulate(counts, initial=0), np.int32, len(counts) + 1))
 
-        def take(shape):
-            nonlocal at
-            n = int(np.prod(shape))
-            v = flat[at:at + n].view(*shape)
-            at += n
-            return v
-
+        flat = torch.empty(sum(sizes), dtype=torch.int32, pin_memory=self.device.type == "cuda")
+        host = flat.numpy()
+        ids, pos = host[:2 * total].view(np.int64), host[2 * total:4 * total].view(np.int64)
+        o = 0
+        for (_, a, t), n in zip(portions, counts):
+            _write_ids(ids[o:o + n], t)
+            pos[o:o + n] = np.arange(a, a + n)
+            o += n
+        at = 4 * total
+        host[at:at + 2 * len(rows)].view(np.int64)[:] = rows
+        at += 2 * len(rows)
+        for a in i32:
+            host[at:at + a.size] = a
+            at += a.size
+        ids_dev, pos_dev, rows_dev, *parts = flat.to(self.device, non_blocking=True).split(sizes)
+        ids_dev, pos_dev, rows_dev = (t.view(torch.int64) for t in (ids_dev, pos_dev, rows_dev))
+        parts = iter(parts)
         spans = []
-        for slots, bt, kv, cq, ck, *sizes in layout:
-            spans.append(SpanBatch(take(slots), take(bt), take(kv), take(cq), take(ck), *sizes))
+        for cols, *extent in layout:
+            slots, bt, kv, cq, ck = (next(parts) for _ in range(5))
+            spans.append(SpanBatch(slots, bt.view(-1, cols), kv, cq, ck, *extent))
         first = spans[0]
         set_context(True, cu_seqlens_q=first.cu_seqlens_q, cu_seqlens_k=first.cu_seqlens_k,
                     max_seqlen_q=first.max_seqlen_q, max_seqlen_k=first.max_seqlen_k,
                     slot_mapping=first.slot_mapping,
                     block_tables=first.block_tables if use_block_tables else None, spans=spans,
-                    state_slots=take(state_shape) if state_shape is not None else None,
-                    cu_portions=take(cu_shape) if cu_shape is not None else None,
-                    longest_portion=max(len(t) for _, _, t in portions))
+                    state_slots=next(parts, None), cu_portions=next(parts, None),
+                    longest_portion=max(counts))
         try:
             hidden = self.model(ids_dev, pos_dev)
         finally:
@@ -545,18 +571,19 @@ class DecodeEngine:
             n = len(self.seqs)
         else:
             n = self._prepare_layout(seqs)
+            self._staged_ahead = None
         self._ahead = None
         if use_host_ids:
-            ids = self.host_np["input_ids"]
-            for i, s in enumerate(self.seqs if seqs is None else seqs):
-                ids[i] = s.last_token
+            self.host_np["input_ids"][:n] = [s.last_token
+                                             for s in (self.seqs if seqs is None else seqs)]
         return n
 
     def _prepare_ahead(self) -> None:
         """Called between the launch of a step and the wait for its tokens: the next
         step's positions, lengths, slots and block-table changes depend on no token
         value, so they are written into the next staging slot while the device is
-        busy.  Skipped when the next step could fail (length limit, pool nearly
+        busy, and copied to the device behind the running step, on its stream.
+        Skipped when the next step could fail (length limit, pool nearly
         empty), so that such errors are still raised by the step they belong to."""
         if not self.seqs or _NO_PREPARE_AHEAD:
             return
@@ -565,8 +592,13 @@ class DecodeEngine:
         for blocks in self.span_blocks:
             if sum(blocks.pages_missing(s) for s in self.seqs) > len(blocks.free):
                 return
-        self._prepare_layout()
+        n = self._prepare_layout()
         self._ahead = (self._seq_epoch, len(self.seqs))
+        if self.device.type == "cuda":
+            bs = self.graph_batch_size(n)
+            self.stage_inputs(n, bs, False)
+            self._mark_slot_in_flight()
+            self._staged_ahead = bs, ops.current_stream()
 
     def _prepare_layout(self, seqs=None) -> int:
         seqs = self.seqs if seqs is None else seqs
@@ -610,14 +642,14 @@ class DecodeEngine:
     def stage_inputs(self, n: int, bs: int, use_host_ids: bool) -> None:
         """H2D copies from pinned memory into the graph's input buffers; padded
         rows get slot -1 / context_len 0 (engine.py:5404-5406)."""
-        gv, h = self.graph_vars, self.host
+        gv, h, hn = self.graph_vars, self.host, self.host_np
         if bs > n:
-            for slots, lens in zip(h["span_slots"], h["span_lens"]):
+            for slots, lens in zip(hn["span_slots"], hn["span_lens"]):
                 slots[n:bs] = -1
                 lens[n:bs] = 0
             if self.state_slots is not None:
-                h["state_slots"][n:bs] = -1
-            h["positions"][n:bs] = 0
+                hn["state_slots"][n:bs] = -1
+            hn["positions"][n:bs] = 0
         first = 0 if use_host_ids else 8 * self.max_num_seqs
         self._packed_dev[first:].copy_(h["packed"][first:], non_blocking=True)
         self.h2d_bytes += h["packed"].numel() - first
@@ -691,6 +723,7 @@ class DecodeEngine:
     def run_step_device(self, bs: int) -> None:
         """Replay (or eagerly run) the step for batch size `bs` on inputs that
         are already in the graph buffers."""
+        self._staged_ahead = None       # the step leaves its own tokens on the device
         g = self.graphs.get(bs)
         if g is not None and not self.enforce_eager:
             g.replay()
@@ -709,7 +742,10 @@ class DecodeEngine:
         buffer and the host copy is deferred."""
         n = self.prepare_decode(use_host_ids=sync)
         bs = self.graph_batch_size(n)
-        self.stage_inputs(n, bs, use_host_ids=sync)
+        # staged behind the step before, which has also left its tokens on the device
+        if self._staged_ahead is None or self._staged_ahead != (bs, ops.current_stream()) or \
+                (sync and self._sampled != [s.last_token for s in self.seqs]):
+            self.stage_inputs(n, bs, use_host_ids=sync)
         self.run_step_device(bs)
         back = self._num_words + 2 * n          # status words and token ids
         self.host["result"][:back].copy_(self.graph_vars["result"][:back], non_blocking=True)
@@ -721,10 +757,15 @@ class DecodeEngine:
             return None
         landing = self.host_np["token_ids"]     # this step's slot (the next call moves on)
         words = self.host_np["words"]
+        landed = self._ring_events[self._ring_pos]
         self._prepare_ahead()
-        torch.cuda.current_stream().synchronize()
+        if landed is None:
+            torch.cuda.current_stream().synchronize()
+        else:
+            landed.synchronize()                # not for the next step's inputs
         ids = landing[:n].copy()
-        for s, t in zip(self.seqs, ids.tolist()):
+        self._sampled = ids.tolist()
+        for s, t in zip(self.seqs, self._sampled):
             s.last_token = t
             s.output.append(t)
         if (words[0] or words[-1]) and self.tp == 1:

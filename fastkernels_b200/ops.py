@@ -35,6 +35,9 @@ def _stream() -> int:
     return _raw_stream(device)
 
 
+current_stream = _stream           # handle of the stream that a wrapper's kernels go to
+
+
 def _ptr(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 

@@ -1,5 +1,6 @@
 """Prompt portions of the Llama / Qwen3 decoders through the native call against the loop over
-the layers' modules: the same bits, and every module that a program has changed is called."""
+the layers' modules: the same bits, and every module that a program has changed is called.  Steps
+whose inputs were staged behind the step before against steps that stage their own."""
 import numpy as np
 import pytest
 import torch
@@ -101,3 +102,48 @@ def test_what_a_program_changed_is_called(change, monkeypatch):
     # the op-by-op chain rounds between norm and rotation
     torch.testing.assert_close(got, want, atol=3e-2 * float(want.std()), rtol=3e-2) \
         if change is _forward else torch.testing.assert_close(got, want, atol=0.0, rtol=0.0)
+
+
+@pytest.mark.parametrize("graphs", [[], [4]])
+def test_steps_staged_ahead(graphs, monkeypatch):
+    """Tokens that the program replaces, sequences that come and go, another stream, steps that
+    do not wait, and prompts in between: the same tokens as without staging ahead."""
+    from fastkernels_b200 import engine as E
+
+    def run(ahead):
+        monkeypatch.setattr(E, "_NO_PREPARE_AHEAD", not ahead)
+        eng, rs, out = engine("HND", True, False, ff=9600), np.random.RandomState(2), []
+        if graphs:
+            eng.capture_cudagraph(graphs)
+        eng.prefill([rs.randint(0, VOCAB, n).tolist() for n in (15, 33, 7)])
+        staged = 0
+        for i in range(24):
+            if i == 5:
+                eng.seqs[1].last_token = 11
+            if i == 8:
+                eng.finish(eng.seqs[0])
+            if i == 10:
+                eng.prefill([rs.randint(0, VOCAB, 20).tolist()])
+            if i == 16:
+                s = eng.open_sequence()
+                eng.feed([(s, [1, 2, 3])])
+                out.append(eng.feed([(s, [4])])[0])
+                eng.finish(s)
+            staged += eng._staged_ahead is not None and eng._ahead is not None
+            if i == 13:
+                with torch.cuda.stream(torch.cuda.Stream()):
+                    out.append(torch.from_numpy(eng.step()))
+                    torch.cuda.current_stream().synchronize()
+            elif i == 19:
+                eng.step(sync=False)
+                torch.cuda.synchronize()
+                for q, t in zip(eng.seqs, eng.host_np["token_ids"]):
+                    q.last_token = int(t)
+            else:
+                out.append(torch.from_numpy(eng.step()))
+        assert eng.device_status() == 0
+        return out, staged
+    got, staged = run(True)
+    want, none = run(False)
+    assert staged >= 16 and none == 0
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
