@@ -15,7 +15,7 @@
 // Prefill attention is the one compute-bound kernel of the engine, so it runs on
 // the 5th-generation tensor cores.  A work item is 256 query rows of one head as
 // two 128-row tiles that take turns on the tensor pipe; one persistent CTA per SM
-// walks a static list of items (heaviest first), so the Q / K fetch of the next
+// walks its part of the items (heaviest first), so the Q / K fetch of the next
 // item and the output write of the previous one overlap the matrix work:
 //
 //   warp 8        TMA producer: the two Q tiles once, then K_0 V_0 K_1 V_1 ...
@@ -70,7 +70,9 @@ static_assert(PF_REGS_NEEDED <= 168 * PF_THREADS, "register split exceeds the CT
 constexpr int PF_OFF_Q = 0;
 constexpr int PF_OFF_KV = PF_OFF_Q + PF_QT * PF_TILE_BYTES;
 constexpr int PF_OFF_BAR = PF_OFF_KV + PF_SLOTS * PF_TILE_BYTES;
-constexpr int PF_SMEM = PF_OFF_BAR + 256;
+constexpr int PF_OFF_LIST = PF_OFF_BAR + 256;
+constexpr int PF_LIST = PF_THREADS;             // blocks of 256 query rows that are put in order
+constexpr int PF_SMEM = PF_OFF_LIST + PF_LIST * 4;
 constexpr int PF_SMEM_ALLOC = PF_SMEM + 1024;
 constexpr int PF_TMEM_COLS = 512;
 constexpr float PF_RESCALE_LOG2 = 8.0f;
@@ -87,7 +89,7 @@ struct PrefillParams {
   int paged, hnd, block_size, bs_shift, sub_tokens, num_blocks;
   float scale_log2;                 // softmax_scale * log2(e)
   int causal;
-  int num_seqs, q_blocks;           // work items: q_blocks x num_seqs x hq
+  int num_seqs, q_blocks;           // work items: up to q_blocks x num_seqs x hq
   int32_t* status;
 };
 
@@ -153,17 +155,86 @@ __device__ __forceinline__ bool pf_wait_warp(uint64_t* bar, uint32_t parity,
   return __all_sync(0xffffffffu, pf_wait(bar, parity, abort_flag, status) ? 1 : 0) != 0;
 }
 
-// Items are numbered heaviest first (last query block first: causal rows see the
-// most keys), sequences and heads inside a block adjacent so that CTAs running at
-// the same time share K/V in L2.  CTA c of G takes items c, c + G, c + 2G, ...
-// (a boustrophedon order measured no better).
-__device__ __forceinline__ PfItem pf_load_item(const PrefillParams& p, int idx) {
+// K/V tiles of 128 query rows from m0 on.
+__device__ __forceinline__ int pf_tiles(const PrefillParams& p, int q_len, int k_len, int m0) {
+  if (m0 >= q_len) return 0;
+  const int last_row = min(m0 + PF_BM - 1, q_len - 1);
+  const int hi = p.causal ? min(k_len - q_len + last_row, k_len - 1) : k_len - 1;
+  return hi >= 0 ? hi / PF_BN + 1 : 0;
+}
+
+// Blocks of 256 query rows of all sequences in order of their K/V tiles, most first, as
+// (sequence << 16 | block); all threads.  At most PF_LIST sequences and blocks, which the host sees
+// to.  Returns the number of blocks.
+__device__ __forceinline__ int pf_order_blocks(const PrefillParams& p, uint32_t* list,
+                                               int* scratch) {
+  int* first = scratch;                        // [num_seqs + 1]
+  int* tiles = scratch + PF_LIST + 1;          // [blocks]
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < p.num_seqs)
+    first[tid] = max(0, (p.cu_q[tid + 1] - p.cu_q[tid] + PF_QT * PF_BM - 1) / (PF_QT * PF_BM));
+  __syncthreads();
+  if (tid < 32) {
+    int base = 0;
+    for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
+      const int mine = s0 + lane < p.num_seqs ? first[s0 + lane] : 0;
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      if (s0 + lane < p.num_seqs) first[s0 + lane] = base + upto - mine;
+      base += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (lane == 0) first[p.num_seqs] = base;
+  }
+  __syncthreads();
+  const int blocks = min(first[p.num_seqs], PF_LIST);
+  int mine = 0, n = 0;
+  if (tid < blocks) {
+    int lo = 0, hi = p.num_seqs;               // the last sequence that starts at or before tid
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (first[mid] <= tid) lo = mid; else hi = mid;
+    }
+    const int qb = tid - first[lo], m0 = qb * PF_QT * PF_BM;
+    const int q_len = p.cu_q[lo + 1] - p.cu_q[lo], k_len = p.cu_k[lo + 1] - p.cu_k[lo];
+    n = max(pf_tiles(p, q_len, k_len, m0), pf_tiles(p, q_len, k_len, m0 + PF_BM));
+    mine = lo << 16 | qb;
+    tiles[tid] = n;
+  }
+  __syncthreads();
+  if (tid < blocks) {
+    int rank = 0;
+    for (int u = 0; u < blocks; ++u) rank += tiles[u] > n || (tiles[u] == n && u < tid) ? 1 : 0;
+    list[rank] = (uint32_t)mine;
+  }
+  fence_proxy_async_smem();                    // the scratch becomes K/V tiles
+  __syncthreads();
+  return blocks;
+}
+
+// Items are numbered heaviest first, heads inside a block adjacent so that CTAs running at
+// the same time share K/V in L2: from the list, or by the last query block (causal rows see the
+// most keys), sequences inside it.
+template <bool ORDER>
+__device__ __forceinline__ PfItem pf_load_item(const PrefillParams& p, const uint32_t* list,
+                                               int idx) {
   PfItem it;
-  const int per_block = p.num_seqs * p.hq;
-  const int qb = p.q_blocks - 1 - idx / per_block;
-  const int rem = idx % per_block;
-  it.seq = rem / p.hq;
-  it.head = rem % p.hq;
+  int qb;
+  if (ORDER) {
+    const uint32_t e = list[idx / p.hq];
+    it.seq = (int)(e >> 16);
+    it.head = idx % p.hq;
+    qb = (int)(e & 0xffffu);
+  } else {
+    const int per_block = p.num_seqs * p.hq;
+    qb = p.q_blocks - 1 - idx / per_block;
+    const int rem = idx % per_block;
+    it.seq = rem / p.hq;
+    it.head = rem % p.hq;
+  }
   it.m0 = qb * (PF_QT * PF_BM);
   it.qs = p.cu_q[it.seq];
   it.q_len = p.cu_q[it.seq + 1] - it.qs;
@@ -172,22 +243,16 @@ __device__ __forceinline__ PfItem pf_load_item(const PrefillParams& p, int idx) 
   it.nkv = 0;
 #pragma unroll
   for (int t = 0; t < PF_QT; ++t) {
-    const int m0t = it.m0 + t * PF_BM;
-    int n = 0;
-    if (m0t < it.q_len) {
-      const int last_row = min(m0t + PF_BM - 1, it.q_len - 1);
-      const int hi = p.causal ? min(it.k_len - it.q_len + last_row, it.k_len - 1) : it.k_len - 1;
-      if (hi >= 0) n = hi / PF_BN + 1;
-    }
-    it.n_t[t] = n;
-    it.nkv = max(it.nkv, n);
+    it.n_t[t] = pf_tiles(p, it.q_len, it.k_len, it.m0 + t * PF_BM);
+    it.nkv = max(it.nkv, it.n_t[t]);
   }
   return it;
 }
 
 // SPLIT: P enters P V as two bf16 parts (16 significant bits): the high parts in the
 // first 64 columns of S_t, the low parts in the other 64, two products per K/V tile.
-template <bool SPLIT>
+// ORDER: the items come from a list of the blocks in order.
+template <bool SPLIT, bool ORDER>
 __global__ void __launch_bounds__(PF_THREADS, 1)
 prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
                     const __grid_constant__ CUtensorMap tmap_k,
@@ -209,9 +274,6 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
   volatile int* abort_flag = reinterpret_cast<volatile int*>(o_empty + PF_QT + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int total_items = p.q_blocks * p.num_seqs * p.hq;
-  const int stride = gridDim.x;
-
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -250,6 +312,16 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
     return;
   }
   pdl_wait();     // q, K/V, cu_seqlens and block tables may come from earlier kernels
+  const uint32_t* list = reinterpret_cast<const uint32_t*>(smem + PF_OFF_LIST);
+  int total_items = p.q_blocks * p.num_seqs * p.hq;
+  if (ORDER)
+    total_items = p.hq * pf_order_blocks(p, reinterpret_cast<uint32_t*>(smem + PF_OFF_LIST),
+                                         reinterpret_cast<int*>(smem + PF_OFF_KV));
+  // rounds of items, every other one backwards: who takes the first of one takes the last of the next
+  const int ctas = gridDim.x;
+  auto item_of = [&](int round) {
+    return round * ctas + (round & 1 ? ctas - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  };
 
   if (warp >= PF_WARP_TMA) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PF_REGS_OTHER));
@@ -263,8 +335,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
     int kv_idx = 0;          // running slot-use count over all items
     int q_loads = 0;         // items whose Q has been requested
     bool ok = true;
-    for (int idx = blockIdx.x; idx < total_items && ok; idx += stride) {
-      const PfItem it = pf_load_item(p, idx);
+    for (int round = 0, idx; ok && (idx = item_of(round)) < total_items; ++round) {
+      const PfItem it = pf_load_item<ORDER>(p, list, idx);
       if (it.nkv == 0) continue;
       const int kvh = it.head / p.g;
       int pass = 1;
@@ -366,8 +438,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
     uint32_t n_sp[PF_QT] = {0, 0}; // S / P hand-overs per tile so far
     uint32_t n_o[PF_QT] = {0, 0};  // items per tile so far
     bool ok = true;
-    for (int idx = blockIdx.x; idx < total_items && ok; idx += stride) {
-      const PfItem it = pf_load_item(p, idx);
+    for (int round = 0, idx; ok && (idx = item_of(round)) < total_items; ++round) {
+      const PfItem it = pf_load_item<ORDER>(p, list, idx);
       if (it.nkv == 0) continue;
       const int k0i = kv_base;     // K_0 of this item
       ok = pf_wait_warp(q_full, (uint32_t)items & 1u, abort_flag, p.status) &&
@@ -447,12 +519,12 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
     int kv_base = 0;
     uint32_t n_sp = 0, n_o = 0;
     bool ok = true;
-    for (int idx = blockIdx.x; idx < total_items && ok; idx += stride) {
+    for (int round = 0, idx; ok && (idx = item_of(round)) < total_items; ++round) {
       // Only what the tile loop needs stays live across it; the output pointers are
       // recomputed for the epilogue (the score row takes most of the registers).
       int my_n, nkv_item, k_len, lim;
       {
-        const PfItem it = pf_load_item(p, idx);
+        const PfItem it = pf_load_item<ORDER>(p, list, idx);
         const int m0t = it.m0 + t * PF_BM;
         my_n = t ? it.n_t[1] : it.n_t[0];
         nkv_item = it.nkv;
@@ -590,7 +662,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
       }
       tc_fence_after();
       const float inv = l > 0.f ? 1.0f / l : 0.f;
-      const PfItem it = pf_load_item(p, idx);
+      const PfItem it = pf_load_item<ORDER>(p, list, idx);
       const bool row_valid = it.m0 + t * PF_BM + row < it.q_len;
       const int64_t tok = (int64_t)it.qs + it.m0 + t * PF_BM + row;
       uint4* dst = reinterpret_cast<uint4*>(p.out + tok * p.out_stride +
@@ -872,33 +944,40 @@ static int prefill_impl(bool split, int out_head, const void* q, int64_t q_strid
   p.causal = causal ? 1 : 0;
   p.status = status;
 
-  static std::once_flag once;
-  static cudaError_t attr_err = cudaSuccess;
-  static int launch_regs = 0;
-  static PerDeviceOnce smem_once;
-  static PerDeviceOnce smem_once2;
-  FK_CUDA_OK(set_max_dynamic_smem(smem_once, prefill_attn_kernel<false>, PF_SMEM_ALLOC));
-  FK_CUDA_OK(set_max_dynamic_smem(smem_once2, prefill_attn_kernel<true>, PF_SMEM_ALLOC));
-  // registers per thread of the compiled kernel: the same on every device
-  std::call_once(once, [] {
-    cudaFuncAttributes fa, fb;
-    attr_err = cudaFuncGetAttributes(&fa, prefill_attn_kernel<false>);
-    if (attr_err == cudaSuccess) attr_err = cudaFuncGetAttributes(&fb, prefill_attn_kernel<true>);
-    if (attr_err == cudaSuccess) launch_regs = fa.numRegs < fb.numRegs ? fa.numRegs : fb.numRegs;
-  });
-  FK_CUDA_OK(attr_err);
-  FK_REQUIRE(launch_regs * PF_THREADS >= PF_REGS_NEEDED, FK_ERR_UNSUPPORTED,
-             "fk_prefill_attn: this build of the kernel holds %d registers per thread, "
-             "fewer than its warpgroup register split needs", launch_regs);
   const int q_blocks = (max_seqlen_q + PF_QT * PF_BM - 1) / (PF_QT * PF_BM);
   const int64_t items = (int64_t)q_blocks * num_q_heads * num_seqs;
   FK_REQUIRE(items <= 0x7fffffff, FK_ERR_UNSUPPORTED, "fk_prefill_attn: too many work items");
   p.num_seqs = num_seqs;
   p.q_blocks = q_blocks;
+  // Blocks in order where several sequences' items do not fit one round.  Without it the items of
+  // short sequences are holes in the numbering, and what is left falls on the CTAs unevenly: 4096
+  // tokens of 3 to 7 prompts, 16 heads, 63 -> 54 us; 7800 of 5 prompts, 32 heads, weights in two
+  // parts, 355 -> 258.  The list takes 2 us to make.
+  const bool order = num_seqs > 1 && items > sm_count() &&
+                     total_q / (PF_QT * PF_BM) + num_seqs <= PF_LIST;
+  auto kernel = split ? (order ? prefill_attn_kernel<true, true> : prefill_attn_kernel<true, false>)
+                      : (order ? prefill_attn_kernel<false, true> : prefill_attn_kernel<false, false>);
+  static PerDeviceOnce smem_once[4];
+  FK_CUDA_OK(set_max_dynamic_smem(smem_once[split * 2 + order], kernel, PF_SMEM_ALLOC));
+  // registers per thread of the compiled kernels: the same on every device
+  static std::once_flag once;
+  static cudaError_t attr_err = cudaSuccess;
+  static int launch_regs = 1 << 20;
+  std::call_once(once, [] {
+    for (auto k : {prefill_attn_kernel<true, true>, prefill_attn_kernel<true, false>,
+                   prefill_attn_kernel<false, true>, prefill_attn_kernel<false, false>}) {
+      cudaFuncAttributes f;
+      if (attr_err == cudaSuccess) attr_err = cudaFuncGetAttributes(&f, k);
+      if (attr_err == cudaSuccess && f.numRegs < launch_regs) launch_regs = f.numRegs;
+    }
+  });
+  FK_CUDA_OK(attr_err);
+  FK_REQUIRE(launch_regs * PF_THREADS >= PF_REGS_NEEDED, FK_ERR_UNSUPPORTED,
+             "fk_prefill_attn: this build of the kernel holds %d registers per thread, "
+             "fewer than its warpgroup register split needs", launch_regs);
   const int ctas = (int)(items < sm_count() ? items : sm_count());
   dim3 grid((unsigned)ctas);
-  FK_CUDA_OK(launch_kernel(split ? prefill_attn_kernel<true> : prefill_attn_kernel<false>, grid,
-                           dim3(PF_THREADS), (size_t)PF_SMEM_ALLOC,
+  FK_CUDA_OK(launch_kernel(kernel, grid, dim3(PF_THREADS), (size_t)PF_SMEM_ALLOC,
                            static_cast<cudaStream_t>(stream), mq, mk, mv, p));
   count_launch(1);
   return FK_OK;

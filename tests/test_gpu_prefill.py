@@ -233,3 +233,38 @@ def test_prefill_random_shapes(seed):
     got_lse = lse.cpu().numpy()
     assert (np.isfinite(got_lse) == fin).all(), what
     assert np.abs(got_lse[fin] - want_lse[fin]).max() < 2e-2, what
+
+
+@pytest.mark.parametrize("heads,kv", [(16, 4), (32, 32)])
+@pytest.mark.parametrize("causal,split", [(True, False), (True, True), (False, False)])
+@pytest.mark.parametrize("lens,more", [
+    ([300, 1, 700, 256, 0, 257, 513], [0, 40, 0, 300, 5, 0, 1]),   # heavy ones anywhere, an empty one
+    ([40] * 380, [0] * 380),                                       # the longest list
+    ([30] * 390, [0] * 390)])                                      # one too long for it
+def test_batches_in_order_equal_their_sequences(heads, kv, causal, split, lens, more):
+    """Blocks of query rows go to the CTAs in order of their keys: every sequence of a batch
+    gets the bits that it gets alone."""
+    from fastkernels_b200 import ops
+    if len(lens) > 100 and (heads != 16 or split):
+        pytest.skip("one form is enough")
+    g = torch.Generator(device="cuda").manual_seed(len(lens))
+    keys = [a + b for a, b in zip(lens, more)]
+
+    def rows(n, h):
+        return torch.randn((n, h, 128), generator=g, device="cuda").bfloat16()
+    q, k, v = rows(sum(lens), heads), rows(sum(keys), kv), rows(sum(keys), kv)
+
+    def cu(a):
+        return torch.tensor([0] + list(a), device="cuda").cumsum(0).int()
+    st = ops.new_status("cuda")
+    out = torch.full_like(q, 7.0)
+    ops.prefill_attn(q, k, v, cu(lens), cu(keys), max(lens), 0.1, causal=causal, out=out,
+                     split_weights=split, status=st)
+    a = b = 0
+    for i, (n, m) in enumerate(zip(lens, keys)):
+        if n and (len(lens) < 100 or i % 37 == 0):
+            alone = ops.prefill_attn(q[a:a + n], k[b:b + m], v[b:b + m], cu([n]), cu([m]), n, 0.1,
+                                     causal=causal, split_weights=split)
+            assert torch.equal(alone, out[a:a + n])
+        a, b = a + n, b + m
+    assert int(st.item()) == 0
