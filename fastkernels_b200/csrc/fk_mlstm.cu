@@ -157,109 +157,252 @@ __global__ void __launch_bounds__(MS_THREADS) mlstm_step_kernel(const MlstmParam
 }
 
 // ----------------------------------------------------------------- portions, any size
-constexpr int MC_COLS = 32, MC_GROUPS = 4;
-template <typename T>
-__global__ void __launch_bounds__(MC_COLS * MC_GROUPS) mlstm_scan_kernel(const MlstmParams p) {
-  extern __shared__ float mc_smem[];    // S [dim][32] | n [dim] | q [2][dim] | k [2][dim]
+// Token by token, but what does not hang on the state goes 16 tokens at a time: their loads, asked
+// for a block ahead, their gates (by a warp of its own a block ahead, a lane each; only the running
+// maximum goes from one to the next), q and k into shared memory, the normalizer's sums (16 at once),
+// the outputs.  A thread keeps every fourth row of one column of S in registers; a token is a pass
+// over them, without a barrier.  Bound by the latency of a block's steps.  fp32, portions of up to
+// 333 tokens, 8 heads of 128 x 256: 134 us, the normalizer's kernel 36 (token by token with S in
+// shared memory 874 and 246).
+constexpr int MC_COLS = 32, MC_GROUPS = 4, MC_TOKENS = 16;
+constexpr int MC_THREADS = MC_COLS * MC_GROUPS;   // and a warp for the gates
+
+struct McGates {
+  float keep[MC_TOKENS], add[MC_TOKENS], low[MC_TOKENS];   // low: e^{-m}
+};
+// Gates of tokens t .. t + count - 1, by one warp; returns m after them.
+__device__ __forceinline__ float mc_gates(const MlstmParams& p, int64_t t, int count, int h, float m,
+                                          McGates& out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t at = t + min(lane, count - 1);
+  const float gi = ml_input_gate(p.z[at * p.z_stride + h], p.cap);
+  const float gf = ml_forget_gate(p.z[at * p.z_stride + p.heads + h], p.cap);
+  float before = m;                            // the maximum ahead of and after this lane's token
+  float after = m;
+  for (int i = 0; i < count; ++i) {
+    const float next = fmaxf(__shfl_sync(0xffffffffu, gf, i) + m, __shfl_sync(0xffffffffu, gi, i));
+    if (lane == i) { before = m; after = next; }
+    m = next;
+  }
+  if (lane < count) {
+    out.keep[lane] = expf(gf + before - after);
+    out.add[lane] = expf(gi - after);
+    out.low[lane] = expf(-after);
+  }
+  return m;
+}
+
+// RP: rows of S a thread (dim up to 4 RP)
+template <typename T, int RP>
+__global__ void __launch_bounds__(MC_THREADS + 32) mlstm_scan_kernel(const MlstmParams p) {
+  constexpr int NR = (RP * MC_GROUPS + MC_THREADS - 1) / MC_THREADS;   // rows of n a thread
+  constexpr int GP = RP + 8, TP = MC_GROUPS * GP;    // row r of a token lies at r % 4 * GP + r / 4
+  extern __shared__ __align__(16) float mc_smem[];   // q [16][TP] | k [16][TP]
+  __shared__ McGates gates[2];
+  __shared__ float part[MC_TOKENS][MC_GROUPS][MC_COLS], sums[MC_TOKENS][MC_THREADS / 32];
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float red[64], part[2][MC_GROUPS][MC_COLS];
-  int flip = 0;
-  const int h = blockIdx.y, pi = blockIdx.z, tid = threadIdx.x;
+  const int h = blockIdx.y, pi = blockIdx.z, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t t0 = p.cu[pi], t1 = min((int64_t)p.cu[pi + 1], p.rows);
   if (t0 < 0 || t0 >= t1) return;
   const int slot = p.slots[t0];
   const bool keep_state = ml_slot_ok(p, slot);
-  const int col = tid % MC_COLS, rg = tid / MC_COLS;
-  const int c = blockIdx.x * MC_COLS + col;
-  const bool on = c < p.vdim;
-  float* S = mc_smem;
-  float* n = S + p.dim * MC_COLS;
-  float* qs = n + p.dim;
-  float* ks = qs + 2 * p.dim;
+  const int rg = warp, c = blockIdx.x * MC_COLS + lane;
+  const bool worker = warp < MC_GROUPS, on = c < p.vdim && worker;
+  float* qs = mc_smem;
+  float* ks = qs + MC_TOKENS * TP;
   const int64_t at = keep_state ? slot : 0;
   float* gS = p.s_state + (at * p.heads + h) * p.dim * p.vp;
-  float* gN = p.n_state + (at * p.heads + h) * p.np;
+  const float* gN = p.n_state + (at * p.heads + h) * p.np;
   const bool load = keep_state && p.positions[t0] > 0;
-  for (int r = rg; r < p.dim; r += MC_GROUPS)
-    S[r * MC_COLS + col] = load && on ? gS[(int64_t)r * p.vp + c] : 0.f;
-  for (int r = tid; r < p.dim; r += blockDim.x) n[r] = load ? gN[r] : 0.f;
-  float m = load ? gN[p.dim] : 0.f;
-  for (int64_t t = t0; t < t1; ++t) {
-    const int b = (int)(t & 1);
-    const float gi = ml_input_gate(p.z[t * p.z_stride + h], p.cap);
-    const float gf = ml_forget_gate(p.z[t * p.z_stride + p.heads + h], p.cap);
-    const float m2 = fmaxf(gf + m, gi);
-    const float keep = expf(gf + m - m2), add = expf(gi - m2);
-    m = m2;
-    const T* q = static_cast<const T*>(p.q) + t * p.in_stride + h * p.dim;
-    const T* k = static_cast<const T*>(p.k) + t * p.in_stride + h * p.dim;
-    float nq[1] = {0.f};
-    for (int r = tid; r < p.dim; r += blockDim.x) {
-      const float kc = Elem<T>::load(k + r), qc = Elem<T>::load(q + r) * p.q_scale;
-      qs[b * p.dim + r] = qc;
-      ks[b * p.dim + r] = kc * add;
-      n[r] = keep * n[r] + add * kc;
-      nq[0] += n[r] * qc;
-    }
-    block_sums<1>(nq, red, flip);
-    const float vv = on ? Elem<T>::load(static_cast<const T*>(p.v) + t * p.in_stride +
-                                        h * p.vdim + c) : 0.f;
-    float acc = 0.f;
-    for (int r = rg; r < p.dim; r += MC_GROUPS) {
-      const float s = keep * S[r * MC_COLS + col] + ks[b * p.dim + r] * vv;
-      S[r * MC_COLS + col] = s;
-      acc = fmaf(s, qs[b * p.dim + r], acc);
-    }
-    part[b][rg][col] = acc;
-    __syncthreads();
-    if (rg == 0 && on) {
-      float o = 0.f;
+  float S[RP], n[NR];
 #pragma unroll
-      for (int g = 0; g < MC_GROUPS; ++g) o += part[b][g][col];
-      p.o[t * ((int64_t)p.heads * p.vdim) + h * p.vdim + c] =
-          o / (fmaxf(fabsf(nq[0]), expf(-m)) + ML_EPS);
-    }
+  for (int i = 0; i < RP; ++i) {
+    const int r = i * MC_GROUPS + rg;
+    S[i] = load && on && r < p.dim ? gS[(int64_t)r * p.vp + c] : 0.f;
   }
-  if (!keep_state) return;
-  for (int r = rg; r < p.dim; r += MC_GROUPS)
-    if (on) gS[(int64_t)r * p.vp + c] = S[r * MC_COLS + col];
+#pragma unroll
+  for (int j = 0; j < NR; ++j) {
+    const int r = tid + j * MC_THREADS;
+    n[j] = load && worker && r < p.dim ? gN[r] : 0.f;
+  }
+  float m = load ? gN[p.dim] : 0.f;                  // the gates' warp
+  // q, k and v of a block, requested while the block before is worked on
+  float qx[MC_TOKENS], kx[MC_TOKENS], vx[MC_TOKENS], vn[MC_TOKENS];
+  auto count_at = [&](int64_t tb) { return (int)min((int64_t)MC_TOKENS, t1 - tb); };
+  auto row = [&](const void* x, int64_t tb, int t, int width) {
+    return static_cast<const T*>(x) + (tb + t) * p.in_stride + h * width;
+  };
+  auto request = [&](int64_t tb) {
+    const int count = count_at(tb);
+#pragma unroll
+    for (int t = 0; t < MC_TOKENS; ++t) {
+      const bool there = t < count && tid < p.dim;
+      qx[t] = there ? Elem<T>::load(row(p.q, tb, t, p.dim) + tid) : 0.f;
+      kx[t] = there ? Elem<T>::load(row(p.k, tb, t, p.dim) + tid) : 0.f;
+      vn[t] = t < count && on ? Elem<T>::load(row(p.v, tb, t, p.vdim) + c) : 0.f;
+    }
+  };
+  // rows beyond dim stay zero
+  for (int i = tid; i < 2 * MC_TOKENS * TP; i += MC_THREADS + 32) mc_smem[i] = 0.f;
+  if (worker)
+    request(t0);
+  else
+    m = mc_gates(p, t0, count_at(t0), h, m, gates[0]);
+  __syncthreads();
+  int b = 0;
+  for (int64_t tb = t0; tb < t1; tb += MC_TOKENS, b ^= 1) {
+    const int count = count_at(tb);
+    const int64_t next = tb + MC_TOKENS;
+    const McGates& gate = gates[b];
+    if (!worker) {
+      if (next < t1) m = mc_gates(p, next, count_at(next), h, m, gates[b ^ 1]);
+    } else {
+      float nq[MC_TOKENS];
+#pragma unroll
+      for (int t = 0; t < MC_TOKENS; ++t) {
+        nq[t] = 0.f;
+        vx[t] = vn[t];
+      }
+#pragma unroll
+      for (int j = 0; j < NR; ++j) {
+        const int r = tid + j * MC_THREADS;
+        if (j > 0) {
+#pragma unroll
+          for (int t = 0; t < MC_TOKENS; ++t) {
+            const bool there = t < count && r < p.dim;
+            qx[t] = there ? Elem<T>::load(row(p.q, tb, t, p.dim) + r) : 0.f;
+            kx[t] = there ? Elem<T>::load(row(p.k, tb, t, p.dim) + r) : 0.f;
+          }
+        }
+        if (r < p.dim) {
+          float* to = qs + (r & 3) * GP + (r >> 2);
+#pragma unroll
+          for (int t = 0; t < MC_TOKENS; ++t) {
+            if (t >= count) break;
+            const float qc = qx[t] * p.q_scale, ka = kx[t] * gate.add[t];
+            to[t * TP] = qc;
+            to[(MC_TOKENS + t) * TP] = ka;
+            n[j] = fmaf(gate.keep[t], n[j], ka);
+            nq[t] = fmaf(n[j], qc, nq[t]);
+          }
+        }
+      }
+      if (next < t1) request(next);
+      // 16 sums over the warp in halving exchanges: lane l ends with that of token l / 2
+#pragma unroll
+      for (int w = 16; w >= 2; w >>= 1) {
+        const bool up = (lane & w) != 0;
+#pragma unroll
+        for (int i = 0; i < w / 2; ++i) {
+          const float mine = up ? nq[i + w / 2] : nq[i], give = up ? nq[i] : nq[i + w / 2];
+          nq[i] = mine + __shfl_xor_sync(0xffffffffu, give, w);
+        }
+      }
+      nq[0] += __shfl_xor_sync(0xffffffffu, nq[0], 1);
+      if ((lane & 1) == 0) sums[lane >> 1][warp] = nq[0];
+    }
+    __syncthreads();
+    if (worker) {
+#pragma unroll
+      for (int t = 0; t < MC_TOKENS; ++t) {
+        if (t >= count) break;
+        const float keep = gate.keep[t];
+        const float* qr = qs + t * TP + rg * GP;
+        const float* kr = ks + t * TP + rg * GP;
+        float acc[2] = {0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < RP; i += 4) {
+          const float4 kv = *reinterpret_cast<const float4*>(kr + i);
+          const float4 qv = *reinterpret_cast<const float4*>(qr + i);
+          S[i] = fmaf(kv.x, vx[t], keep * S[i]);
+          S[i + 1] = fmaf(kv.y, vx[t], keep * S[i + 1]);
+          S[i + 2] = fmaf(kv.z, vx[t], keep * S[i + 2]);
+          S[i + 3] = fmaf(kv.w, vx[t], keep * S[i + 3]);
+          acc[0] = fmaf(S[i], qv.x, acc[0]);
+          acc[1] = fmaf(S[i + 1], qv.y, acc[1]);
+          acc[0] = fmaf(S[i + 2], qv.z, acc[0]);
+          acc[1] = fmaf(S[i + 3], qv.w, acc[1]);
+        }
+        part[t][rg][lane] = acc[0] + acc[1];
+      }
+    }
+    __syncthreads();
+    if (on)
+      for (int t = warp; t < count; t += MC_GROUPS) {
+        float o = 0.f, all = 0.f;
+#pragma unroll
+        for (int g = 0; g < MC_GROUPS; ++g) {
+          o += part[t][g][lane];
+          all += sums[t][g];
+        }
+        p.o[(tb + t) * ((int64_t)p.heads * p.vdim) + h * p.vdim + c] =
+            o / (fmaxf(fabsf(all), gate.low[t]) + ML_EPS);
+      }
+    __syncthreads();                 // this block's gates, q, k and sums are free
+  }
+  if (!keep_state || !on) return;
+#pragma unroll
+  for (int i = 0; i < RP; ++i) {
+    const int r = i * MC_GROUPS + rg;
+    if (r < p.dim) gS[(int64_t)r * p.vp + c] = S[i];
+  }
 }
 
 // n and m after the portions, for the scan: several CTAs of a head read the old values, so
 // they are written by a launch of their own.
 template <typename T>
-__global__ void __launch_bounds__(128) mlstm_scan_norm_kernel(const MlstmParams p) {
+__global__ void __launch_bounds__(512) mlstm_scan_norm_kernel(const MlstmParams p) {
+  __shared__ McGates gate;
   pdl_launch_dependents();
   pdl_wait();
-  const int h = blockIdx.x, pi = blockIdx.y;
+  const int h = blockIdx.x, pi = blockIdx.y, r = threadIdx.x;      // a thread a row
   const int64_t t0 = p.cu[pi], t1 = min((int64_t)p.cu[pi + 1], p.rows);
   if (t0 < 0 || t0 >= t1) return;
   const int slot = p.slots[t0];
   if (!ml_slot_ok(p, slot)) return;
   float* gN = p.n_state + ((int64_t)slot * p.heads + h) * p.np;
-  const bool load = p.positions[t0] > 0;
-  const float m0 = load ? gN[p.dim] : 0.f;
-  __syncthreads();
-  float m = m0;
-  for (int r0 = 0; r0 < p.dim; r0 += blockDim.x) {
-    const int r = r0 + threadIdx.x;
-    const bool on = r < p.dim;
-    float n = load && on ? gN[r] : 0.f;
-    m = m0;
-    for (int64_t t = t0; t < t1; ++t) {
-      const float gi = ml_input_gate(p.z[t * p.z_stride + h], p.cap);
-      const float gf = ml_forget_gate(p.z[t * p.z_stride + p.heads + h], p.cap);
-      const float m2 = fmaxf(gf + m, gi);
-      const float keep = expf(gf + m - m2), add = expf(gi - m2);
-      m = m2;
-      if (on)
-        n = keep * n + add * Elem<T>::load(static_cast<const T*>(p.k) + t * p.in_stride +
-                                           h * p.dim + r);
-    }
-    if (on) gN[r] = n;
+  const bool load = p.positions[t0] > 0, on = r < p.dim;
+  float n = load && on ? gN[r] : 0.f;
+  float m = load ? gN[p.dim] : 0.f;
+  for (int64_t tb = t0; tb < t1; tb += MC_TOKENS) {
+    const int count = (int)min((int64_t)MC_TOKENS, t1 - tb);
+    const T* k = static_cast<const T*>(p.k) + tb * p.in_stride + h * p.dim + r;
+    float kx[MC_TOKENS];
+#pragma unroll
+    for (int t = 0; t < MC_TOKENS; ++t)
+      kx[t] = t < count && on ? Elem<T>::load(k + t * p.in_stride) : 0.f;
+    __syncthreads();                 // the block before has been read
+    if (r < 32) m = mc_gates(p, tb, count, h, m, gate);
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < MC_TOKENS; ++t)
+      if (t < count) n = fmaf(gate.keep[t], n, kx[t] * gate.add[t]);
   }
-  if (threadIdx.x == 0) gN[p.dim] = m;
+  if (on) gN[r] = n;
+  if (r == 0) gN[p.dim] = m;
+}
+
+template <typename T, int RP>
+static int launch_scan_rows(const MlstmParams& p, cudaStream_t s) {
+  constexpr size_t kSmem = 2ull * MC_TOKENS * MC_GROUPS * (RP + 8) * sizeof(float);
+  static PerDeviceOnce once;
+  FK_CUDA_OK(set_max_dynamic_smem(once, mlstm_scan_kernel<T, RP>, (int)kSmem));
+  const dim3 grid((unsigned)((p.vdim + MC_COLS - 1) / MC_COLS), (unsigned)p.heads,
+                  (unsigned)p.num_portions);
+  FK_CUDA_OK(launch_kernel(mlstm_scan_kernel<T, RP>, grid, dim3(MC_THREADS + 32), kSmem, s, p));
+  const dim3 ngrid((unsigned)p.heads, (unsigned)p.num_portions);
+  FK_CUDA_OK(launch_kernel(mlstm_scan_norm_kernel<T>, ngrid,
+                           dim3((unsigned)((p.dim + 31) / 32 * 32)), 0, s, p));
+  count_launch(2);
+  return FK_OK;
+}
+template <typename T>
+static int launch_scan(const MlstmParams& p, cudaStream_t s) {
+  if (p.dim <= 64) return launch_scan_rows<T, 16>(p, s);
+  if (p.dim <= 128) return launch_scan_rows<T, 32>(p, s);
+  if (p.dim <= 256) return launch_scan_rows<T, 64>(p, s);
+  return launch_scan_rows<T, 128>(p, s);
 }
 
 // ------------------------------------------------------------------------ chunked form
@@ -829,26 +972,7 @@ int fk_mlstm_portions(const void* q, const void* k, const void* v, int64_t in_st
   const int64_t units = ml_units(rows, num_portions);
   const bool chunked = !is_f32 && workspace != nullptr && dim <= 256 && units <= 65535 &&
                        longest <= (int64_t)MG_MAX_UNITS * ML_UNIT;
-  if (!chunked) {
-    const size_t smem = (size_t)dim * (MC_COLS + 5) * 4;
-    const dim3 grid((unsigned)((vdim + MC_COLS - 1) / MC_COLS), (unsigned)heads,
-                    (unsigned)num_portions);
-    const dim3 ngrid((unsigned)heads, (unsigned)num_portions);
-    static PerDeviceOnce once_f, once_h;
-    FK_CUDA_OK(set_max_dynamic_smem(once_f, mlstm_scan_kernel<float>, 512 * (MC_COLS + 5) * 4));
-    FK_CUDA_OK(set_max_dynamic_smem(once_h, mlstm_scan_kernel<uint16_t>, 512 * (MC_COLS + 5) * 4));
-    if (is_f32) {
-      FK_CUDA_OK(launch_kernel(mlstm_scan_kernel<float>, grid, dim3(MC_COLS * MC_GROUPS), smem, s,
-                               p));
-      FK_CUDA_OK(launch_kernel(mlstm_scan_norm_kernel<float>, ngrid, dim3(128), 0, s, p));
-    } else {
-      FK_CUDA_OK(launch_kernel(mlstm_scan_kernel<uint16_t>, grid, dim3(MC_COLS * MC_GROUPS), smem,
-                               s, p));
-      FK_CUDA_OK(launch_kernel(mlstm_scan_norm_kernel<uint16_t>, ngrid, dim3(128), 0, s, p));
-    }
-    count_launch(2);
-    return FK_OK;
-  }
+  if (!chunked) return is_f32 ? launch_scan<float>(p, s) : launch_scan<uint16_t>(p, s);
   FK_REQUIRE(aligned16(workspace) && workspace_floats >= fk_mlstm_workspace_floats(
                  rows, num_portions, heads, dim, vdim),
              FK_ERR_WORKSPACE, "fk_mlstm_portions: workspace too small");
