@@ -9,11 +9,13 @@
 // Kernels:
 //   delta_prepare_kernel        everything of a token that does not depend on the state:
 //                               w, u, b = a * u, k, r, v as fp32, packed per (head, token);
-//                               for portions in blocks of 4 tokens, with what the tokens
-//                               of a block do to one another worked out (below)
+//                               for portions in blocks of 4 or chunks of 16 tokens, with
+//                               what their tokens do to one another worked out (below)
 //   delta_scan_kernel           the recurrence, token by token: single tokens, bound by
 //                               the state's bytes
 //   delta_scan_blocked_kernel   the recurrence over blocks, for portions
+//   delta_scan_chunk_kernel     the recurrence over chunks, for portions in bf16 with heads
+//                               of 33 to 128 channels
 //
 // The columns of S (value channels) are independent, so a column lives in the registers
 // of LANES threads; a CTA owns some columns of one head of one sequence.  The state comes
@@ -34,6 +36,15 @@
 //   u_i w_{1..i-1} [4][dp] | k_j w_{j+1..4} | -b_j w_{j+1..4} | r_i w_{1..i} | v_i |
 //   w_{1..4} [dp] | A (6) C (6) pad (4) | E [4][4] | F [4][4]
 // Blocks come in units of 16 tokens; portion i owns the units from cu[i] / 16 + i on.
+//
+// Chunks.  The same over 16 tokens, where every sum over channels or tokens is a 16 x 16 x n
+// product for mma; that leaves the state's multiply-adds (four a channel, value channel and token)
+// to the tensor cores.  Five portions of 700 to 2400 tokens, us of prepare / scan, blocks and then
+// chunks: 64 heads of 64 370 / 1174 and 538 / 388, 24 heads of 128 275 / 1311 and 470 / 520; one of
+// 1500, 32 heads of 64 59 / 280 and 79 / 167; 60 of 24 77 / 73 and 101 / 68, of 3 46 / 27 and
+// 60 / 51, so that portions below 32 tokens on average stay with blocks.  Error of o against 64
+// bits, of the norm: 2.0 to 2.6e-7 (5.4e-7 with decays that forget nothing in 1500 tokens), blocks
+// 2.7e-7 to 1.6e-6, most of it the decays' (decay_of).
 #include "fk_types.cuh"
 
 #include <cmath>
@@ -49,6 +60,54 @@ constexpr int DL_MAX_DIM = 256;
 constexpr int DL_THREADS = 128;
 constexpr uint32_t DL_WAIT_LIMIT = 1u << 20;
 __host__ __device__ constexpr int dl_block_floats(int dp) { return 21 * dp + 48; }
+
+// A chunk's record, in bytes: four operands of [16 tokens][dp], four of [16][16], each in three
+// bf16 parts and the order of mma fragments; v in one part; w_{1..16} in fp32; a flag.
+constexpr int DL_FRAG = 512;      // a 16 x 16 piece of one part: 16 bytes a lane
+__host__ __device__ constexpr int dl_chunk_mats(int dp) { return 4 * (dp / 16) * 3 * DL_FRAG; }
+__host__ __device__ constexpr int dl_chunk_v(int dp) { return dl_chunk_mats(dp) + 4 * 3 * DL_FRAG; }
+__host__ __device__ constexpr int dl_chunk_decay(int dp) { return dl_chunk_v(dp) + dp / 16 * DL_FRAG; }
+__host__ __device__ constexpr int dl_chunk_flag(int dp) { return dl_chunk_decay(dp) + dp * 4; }
+__host__ __device__ constexpr int dl_chunk_bytes(int dp) { return dl_chunk_flag(dp) + 16; }
+__host__ __device__ constexpr int dl_chunk_stages(int dp) { return dp == 64 ? 3 : 2; }
+static_assert(dl_chunk_flag(64) >= DL_FIELDS * DL_UNIT * 64 * 4 &&
+              dl_chunk_flag(128) >= DL_FIELDS * DL_UNIT * 128 * 4, "a plain record fits");
+
+// Packed pairs of fp32: one instruction, two IEEE multiply-adds.
+__device__ __forceinline__ uint64_t dl_pack(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void dl_unpack(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ uint64_t dl_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t dl_mul(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// Two fp32 as three packed bf16 pairs: x = hi + mid + lo up to 2^-25 |x|.
+__device__ __forceinline__ void dl_split(float a, float b, uint32_t& hi, uint32_t& mid,
+                                         uint32_t& lo) {
+  auto pack = [](float x, float y) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
+  };
+  const uint64_t minus = dl_pack(-1.f, -1.f);
+  hi = pack(a, b);
+  dl_unpack(dl_fma(dl_pack(bf16lo(hi), bf16hi(hi)), minus, dl_pack(a, b)), a, b);
+  mid = pack(a, b);
+  dl_unpack(dl_fma(dl_pack(bf16lo(mid), bf16hi(mid)), minus, dl_pack(a, b)), a, b);
+  lo = pack(a, b);
+}
 
 struct DeltaPrepParams {
   const void* r; const void* k; const void* v; const void* a; const void* y1;
@@ -71,11 +130,252 @@ struct Gate {
   }
 };
 
+// A decay's error is that of every later token.  Chunks: e^x as 1 + x (1 + x/2 (1 + x/3 ...)),
+// Taylor's series up to x^10, rounded once at the end (0.7^11 / 11! < 2^-30), where the hardware's
+// approximation is off by 2 units in the last place.
+template <typename T, bool CHUNK>
+__device__ __forceinline__ float decay_of(float x) {
+  if (!CHUNK) return Gate<T>::exp(x);
+  if (!(fabsf(x) <= 0.7f)) return expf(x);
+  float y = fmaf(x, 1.f / 10, 1.f);
+#pragma unroll
+  for (int i = 9; i > 1; --i) y = fmaf(x * (1.f / i), y, 1.f);
+  return fmaf(x, y, 1.f);
+}
+
+// The record of one chunk from its operands vec [6][16][DP + 4] (w, u, b, k, r, v; overwritten),
+// by all threads of a CTA.  mats [4][16][16] is zero on entry.
+//
+// A warp first takes the 4 tokens of a block as for blocks (the sums over the channels of what its
+// tokens do to one another); then a thread takes the four sums of one pair of tokens of different
+// blocks, whose operands carry the decays inside their blocks and are a product of whole blocks'
+// decays apart.  (I + C)^-1 is a product of contractions: no entry exceeds 1.
+template <int DP>
+__device__ void delta_chunk_record(float* vec, float* mats, uint8_t* rec) {
+  constexpr int VP = DP + 4, F = DL_UNIT * VP, KT = DP / 16;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* ma = mats;              // A [i][j]
+  float* mc = mats + 256;        // C [j][i], then (I + C)^-1 [i][j]
+  float* me = mats + 512;        // E [i][j]
+  float* mf = mats + 768;        // F [i][j]
+  {
+    float acc[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+#pragma unroll
+    for (int c0 = 0; c0 < DP; c0 += 32) {
+      float* src = vec + warp * DL_BLK * VP + c0 + lane;
+      float kk[DL_BLK], bb[DL_BLK], gam = 1.f;
+#pragma unroll
+      for (int i = 0; i < DL_BLK; ++i) {
+        const int ia = i * (i - 1) / 2, ie = 12 + i * (i + 1) / 2;
+        float* s = src + i * VP;
+        const float w = s[0], u = s[F], r = s[4 * F];
+#pragma unroll
+        for (int j = 0; j < i; ++j) {
+          acc[ia + j] = fmaf(u, kk[j], acc[ia + j]);
+          acc[6 + ia + j] = fmaf(u, bb[j], acc[6 + ia + j]);
+          kk[j] *= w;
+          bb[j] *= w;
+        }
+        bb[i] = s[2 * F];
+        kk[i] = s[3 * F];
+#pragma unroll
+        for (int j = 0; j <= i; ++j) {
+          acc[ie + j] = fmaf(r, kk[j], acc[ie + j]);
+          acc[10 + ie + j] = fmaf(r, bb[j], acc[10 + ie + j]);
+        }
+        s[F] = u * gam;
+        gam *= w;
+        s[4 * F] = r * gam;
+      }
+      src[0] = gam;              // of the whole block; the row behind it: one
+      src[VP] = 1.f;
+#pragma unroll
+      for (int j = 0; j < DL_BLK; ++j) {
+        src[j * VP + 3 * F] = kk[j];
+        src[j * VP + 2 * F] = bb[j];
+      }
+    }
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      const bool up = (lane & w) != 0;
+#pragma unroll
+      for (int i = 0; i < w; ++i) {
+        const float keep = up ? acc[i + w] : acc[i];
+        const float give = up ? acc[i] : acc[i + w];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+      }
+    }
+    const int t = lane < 12 ? lane % 6 : (lane - 12) % 10;
+    const int tri = t < 1 ? 0 : t < 3 ? 1 : t < 6 ? 2 : 3;
+    const int j = t - tri * (tri + 1) / 2 + warp * DL_BLK;
+    const int i = warp * DL_BLK + tri + (lane < 12 ? 1 : 0);
+    if (lane < 6) ma[i * 16 + j] = acc[0];
+    else if (lane < 12) mc[j * 16 + i] = acc[0];
+    else if (lane < 22) me[i * 16 + j] = acc[0];
+    else mf[i * 16 + j] = -acc[0];
+  }
+  __syncthreads();
+  if (threadIdx.x < 96) {
+    const int pair = threadIdx.x >> 4;                 // (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+    const int bi = pair < 1 ? 1 : pair < 3 ? 2 : 3, bj = pair - bi * (bi - 1) / 2;
+    const int i = bi * DL_BLK + ((threadIdx.x >> 2) & 3), j = bj * DL_BLK + (threadIdx.x & 3);
+    const float* g1 = vec + (bi > 1 && bj < 1 ? DL_BLK : 1) * VP;        // blocks between
+    const float* g2 = vec + (bi > 2 && bj < 2 ? 2 * DL_BLK : 1) * VP;
+    const float* u = vec + F + i * VP;
+    const float* r = vec + 4 * F + i * VP;
+    const float* k = vec + 3 * F + j * VP;
+    const float* b = vec + 2 * F + j * VP;
+    uint64_t sum[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll 4
+    for (int x = 0; x < DP / 4; ++x) {
+      const int at = x * 4;
+      const ulonglong2 uu = *reinterpret_cast<const ulonglong2*>(u + at);
+      const ulonglong2 rr = *reinterpret_cast<const ulonglong2*>(r + at);
+      ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(k + at);
+      ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(b + at);
+      ulonglong2 gg = *reinterpret_cast<const ulonglong2*>(g1 + at);
+      const ulonglong2 x2 = *reinterpret_cast<const ulonglong2*>(g2 + at);
+      gg.x = dl_mul(gg.x, x2.x);
+      gg.y = dl_mul(gg.y, x2.y);
+      kk.x = dl_mul(kk.x, gg.x);
+      kk.y = dl_mul(kk.y, gg.y);
+      bb.x = dl_mul(bb.x, gg.x);
+      bb.y = dl_mul(bb.y, gg.y);
+      sum[0] = dl_fma(uu.y, kk.y, dl_fma(uu.x, kk.x, sum[0]));
+      sum[1] = dl_fma(uu.y, bb.y, dl_fma(uu.x, bb.x, sum[1]));
+      sum[2] = dl_fma(rr.y, kk.y, dl_fma(rr.x, kk.x, sum[2]));
+      sum[3] = dl_fma(rr.y, bb.y, dl_fma(rr.x, bb.x, sum[3]));
+    }
+    auto both = [](uint64_t v) {
+      float x, y;
+      dl_unpack(v, x, y);
+      return x + y;
+    };
+    ma[i * 16 + j] = both(sum[0]);
+    mc[j * 16 + i] = both(sum[1]);
+    me[i * 16 + j] = both(sum[2]);
+    mf[i * 16 + j] = -both(sum[3]);
+  }
+  __syncthreads();
+  const int g = lane >> 2, q2 = (lane & 3) * 2;
+  auto put = [&](int at, float2 x0, float2 x1, float2 x2, float2 x3, float sign) {
+    uint4 hi, mid, lo;
+    dl_split(x0.x * sign, x0.y * sign, hi.x, mid.x, lo.x);
+    dl_split(x1.x * sign, x1.y * sign, hi.y, mid.y, lo.y);
+    dl_split(x2.x * sign, x2.y * sign, hi.z, mid.z, lo.z);
+    dl_split(x3.x * sign, x3.y * sign, hi.w, mid.w, lo.w);
+    uint4* dst = reinterpret_cast<uint4*>(rec + at) + lane;
+    dst[0] = hi;
+    dst[DL_FRAG / 16] = mid;
+    dst[2 * (DL_FRAG / 16)] = lo;
+  };
+  auto decay = [&](int blk, int c) { return vec[blk * DL_BLK * VP + c]; };
+  // u and r: a lane's channels of tokens g and g + 8, decayed from the chunk's start
+  for (int kt = warp; kt < KT; kt += DL_THREADS / 32) {
+    float2 f0[2], f1[2];
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      float lo[2], hi[2];
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int c = kt * 16 + hf * 8 + q2 + y;
+        const float d0 = decay(0, c), d1 = decay(1, c), d2 = decay(2, c);
+        lo[y] = g < DL_BLK ? 1.f : d0;
+        hi[y] = g < DL_BLK ? d0 * d1 : d0 * d1 * d2;
+      }
+      f0[hf] = make_float2(lo[0], lo[1]);
+      f1[hf] = make_float2(hi[0], hi[1]);
+    }
+#pragma unroll
+    for (int op = 0; op < 2; ++op) {
+      const float* src = vec + (op == 0 ? 1 : 4) * F + kt * 16 + q2;
+      float2 x[4];
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const float2 z = *reinterpret_cast<const float2*>(src + (g + y / 2 * 8) * VP + y % 2 * 8);
+        const float2 f = y < 2 ? f0[y] : f1[y - 2];
+        x[y] = make_float2(z.x * f.x, z.y * f.y);
+      }
+      put((op * KT + kt) * 3 * DL_FRAG, x[0], x[1], x[2], x[3], 1.f);
+    }
+  }
+  // k and -b: a lane's tokens of channels g and g + 8, decayed to the chunk's end; v as it is
+  for (int kt = warp; kt < KT; kt += DL_THREADS / 32) {
+    const int c = kt * 16 + g;
+    float f[2][2];                       // [channel][tokens 2 q2 .. / 8 + 2 q2 ..]
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const float d1 = decay(1, c + y * 8), d2 = decay(2, c + y * 8), d3 = decay(3, c + y * 8);
+      f[y][0] = q2 < DL_BLK ? d1 * d2 * d3 : d2 * d3;
+      f[y][1] = q2 < DL_BLK ? d3 : 1.f;
+    }
+#pragma unroll
+    for (int op = 0; op < 2; ++op) {
+      const float* src = vec + (op == 0 ? 3 : 2) * F + c;
+      float2 x[4];
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {      // channel y / 2, token half y % 2
+        const float* at = src + (q2 + y % 2 * 8) * VP + y / 2 * 8;
+        x[y] = make_float2(at[0] * f[y / 2][y % 2], at[VP] * f[y / 2][y % 2]);
+      }
+      put(((2 + op) * KT + kt) * 3 * DL_FRAG, x[0], x[1], x[2], x[3], op == 0 ? 1.f : -1.f);
+    }
+    const float* sv = vec + 5 * F + c;
+    uint32_t vv[4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {        // rows g, g + 8; then tokens from 8 on
+      const float* at = sv + (q2 + y / 2 * 8) * VP + y % 2 * 8;
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(vv[y]) : "f"(at[VP]), "f"(at[0]));
+    }
+    reinterpret_cast<uint4*>(rec + dl_chunk_v(DP))[kt * 32 + lane] =
+        make_uint4(vv[0], vv[1], vv[2], vv[3]);
+  }
+  for (int c = threadIdx.x; c < DP; c += DL_THREADS)
+    reinterpret_cast<float*>(rec + dl_chunk_decay(DP))[c] =
+        decay(0, c) * decay(1, c) * (decay(2, c) * decay(3, c));
+  if (warp == 3) {
+    // (I + C)^-1, a column a lane: what is known of it goes into all rows below at once
+    float x[16];
+    const int col = lane & 15;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = i == col ? 1.f : 0.f;
+#pragma unroll
+    for (int k = 0; k < 15; ++k) {
+      float row[16];
+#pragma unroll
+      for (int y = k / 4 * 4; y < 16; y += 4) {
+        const float4 z = *reinterpret_cast<const float4*>(mc + k * 16 + y);
+        row[y] = z.x;
+        row[y + 1] = z.y;
+        row[y + 2] = z.z;
+        row[y + 3] = z.w;
+      }
+#pragma unroll
+      for (int i = k + 1; i < 16; ++i) x[i] = fmaf(-row[i], x[k], x[i]);
+    }
+    __syncwarp();
+    if (lane < 16)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) mc[i * 16 + col] = x[i];
+  }
+  __syncthreads();
+  {
+    const float* m = mats + warp * 256;
+    float2 x[4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+      x[y] = *reinterpret_cast<const float2*>(m + (g + y / 2 * 8) * 16 + q2 + y % 2 * 8);
+    put(dl_chunk_mats(DP) + warp * 3 * DL_FRAG, x[0], x[1], x[2], x[3], 1.f);
+  }
+}
+
 // CTA = 16 tokens, some heads in turn.  VEC (bf16, rows of whole 16-byte pieces): a thread takes
 // 8 channels of a token, one 16-byte load per input, all requested before the decay projection
 // (the first head's before the tanh too); the sum of k^2 stays within the lanes of the token.
-template <typename T, int DP, bool BLOCKED, bool VEC>
-__global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPrepParams p) {
+template <typename T, int DP, bool BLOCKED, bool VEC, bool CHUNK>
+__global__ void __launch_bounds__(DL_THREADS, !CHUNK ? 0 : DP == 64 ? 6 : 4) delta_prepare_kernel(const DeltaPrepParams p) {
   extern __shared__ __align__(16) uint8_t dl_prep_smem[];
   pdl_launch_dependents();
   if (VEC && !BLOCKED) {
@@ -90,6 +390,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
   }
   pdl_wait();
   constexpr bool MMA = sizeof(T) == 2;
+  constexpr int VP = CHUNK ? DP + 4 : DP;      // fragments read 8 rows at a time
   constexpr int NW = DL_THREADS / 32;
   int64_t t0 = (int64_t)blockIdx.x * DL_UNIT;
   int nt = (int)min((int64_t)DL_UNIT, p.rows - t0);
@@ -111,9 +412,10 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
   uint16_t* hi = reinterpret_cast<uint16_t*>(dl_prep_smem);      // [16][ld] each
   uint16_t* lo = hi + DL_UNIT * ld;
   float* th = reinterpret_cast<float*>(dl_prep_smem);            // fp32: [16][rank_p]
-  float* vec = reinterpret_cast<float*>(dl_prep_smem) + DL_UNIT * ld;   // [6][16][DP]
-  float* part = vec + DL_FIELDS * DL_UNIT * DP;                  // [16][DP / 32]
+  float* vec = reinterpret_cast<float*>(dl_prep_smem) + DL_UNIT * ld;   // [6][16][VP]
+  float* part = vec + DL_FIELDS * DL_UNIT * VP;                  // [16][DP / 32]
   float* unit = part + DL_UNIT * (DP / 32);                      // [16]
+  float* mats = unit + DL_UNIT;                                  // chunks: [4][16][16]
   constexpr int TPT = DP / 8, TOKS = DL_THREADS / TPT;    // VEC: threads a token, tokens a pass
   constexpr int NP8 = VEC ? (DL_UNIT + TOKS - 1) / TOKS : 1;
   const int c8 = (int)(threadIdx.x % TPT) * 8;
@@ -158,11 +460,12 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
   for (int h = h0; h < h1; ++h) {
     __syncthreads();       // tanh written; vec and unit of the last head consumed
     const int64_t ch0 = (int64_t)h * p.d;
+    float seen = 0.f;      // becomes NaN where anything is not finite
     // this thread's elements of the head's [16][DP] tile.  Single tokens: requested before
     // the decay projection so that their latency passes behind it; blocks: as they are
     // needed, many CTAs share an SM
-    constexpr int F = DL_UNIT * DP;                      // floats of one field
-    constexpr int NIT = F / DL_THREADS;
+    constexpr int F = DL_UNIT * VP;                      // floats of one field
+    constexpr int NIT = DL_UNIT * DP / DL_THREADS;
     constexpr int PASS = BLOCKED ? 4 : NIT < 16 ? NIT : 16;
     constexpr int SL = DP / 32;                          // warps that hold one token
     // element x: token tok(x), channel chan(x); one channel per thread up to DP = 128
@@ -239,8 +542,8 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
             mma_bf16_16816(c, fh, b0[x], b1[x]);
           }
         }
-        *reinterpret_cast<float2*>(vec + r0 * DP + n0 + kq) = make_float2(c[0], c[1]);
-        *reinterpret_cast<float2*>(vec + (r0 + 8) * DP + n0 + kq) = make_float2(c[2], c[3]);
+        *reinterpret_cast<float2*>(vec + r0 * VP + n0 + kq) = make_float2(c[0], c[1]);
+        *reinterpret_cast<float2*>(vec + (r0 + 8) * VP + n0 + kq) = make_float2(c[2], c[3]);
       }
     } else {
       for (int i = threadIdx.x; i < nt * DP; i += DL_THREADS) {
@@ -274,7 +577,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
         const bool on = t < nt && c8 < p.d;
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-          const int half = hh ^ swap, i = t * DP + c8 + half * 4;
+          const int half = hh ^ swap, i = t * VP + c8 + half * 4;
           float w[4], u[4], b[4], k[4], r[4], v[4];
           const float4 z = *reinterpret_cast<const float4*>(vec + i);
           const float zz[4] = {z.x, z.y, z.z, z.w};
@@ -296,10 +599,11 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
             w[e] = 1.f;
             u[e] = b[e] = 0.f;
             if (on) {
-              w[e] = Gate<T>::exp(-p.decay_scale * Gate<T>::sigmoid(zz[e] + w0v[e]));
+              w[e] = decay_of<T, CHUNK>(-p.decay_scale * Gate<T>::sigmoid(zz[e] + w0v[e]));
               u[e] = k[e] * un;
               b[e] = u[e] * Gate<T>::sigmoid(pick(aw) + abv[e]);
             }
+            if (CHUNK) seen = fmaf(w[e] + u[e] + b[e] + k[e] + r[e] + v[e], 0.f, seen);
           }
           // blocks: into the tile; single tokens: straight to the token's fields
           if (!BLOCKED && t >= nt) continue;
@@ -340,16 +644,17 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
       if (BLOCKED || x0 > 0) fetch(x0);
 #pragma unroll
       for (int x = 0; x < PASS; ++x) {
-        const int t = tok(x0 + x), c = chan(x0 + x), i = t * DP + c;
+        const int t = tok(x0 + x), c = chan(x0 + x), i = t * VP + c;
         const bool on = t < nt && c < p.d;
         float w = 1.f, u = 0.f, b = 0.f;
         const float k = Elem<T>::load(&kx[x]), r = Elem<T>::load(&rx[x]);
         const float v = Elem<T>::load(&vx[x]);
         if (on) {
-          w = Gate<T>::exp(-p.decay_scale * Gate<T>::sigmoid(vec[i] + w0c[x % CPT]));
+          w = decay_of<T, CHUNK>(-p.decay_scale * Gate<T>::sigmoid(vec[i] + w0c[x % CPT]));
           u = k * unit[t];
           b = u * Gate<T>::sigmoid(Elem<T>::load(&ax[x]) + abc[x % CPT]);
         }
+        if (CHUNK) seen = fmaf(w + u + b + k + r + v, 0.f, seen);
         if (BLOCKED) {
           vec[i] = w;
           vec[F + i] = u;
@@ -370,6 +675,20 @@ __global__ void __launch_bounds__(DL_THREADS) delta_prepare_kernel(const DeltaPr
     }
     }
     if (!BLOCKED) continue;
+    if constexpr (CHUNK) {
+      uint8_t* rec = reinterpret_cast<uint8_t*>(p.packed) +
+                     ((int64_t)h * p.units + blockIdx.x) * dl_chunk_bytes(DP);
+      for (int i = threadIdx.x; i < 1024; i += DL_THREADS) mats[i] = 0.f;
+      const bool plain = __syncthreads_or(seen != 0.f);
+      if (threadIdx.x == 0) *reinterpret_cast<int*>(rec + dl_chunk_flag(DP)) = plain;
+      if (plain) {
+        for (int i = threadIdx.x; i < DL_FIELDS * DL_UNIT * DP; i += DL_THREADS)
+          reinterpret_cast<float*>(rec)[i] = vec[i / DP * VP + i % DP];
+      } else {
+        delta_chunk_record<DP>(vec, mats, rec);
+      }
+      continue;
+    }
     __syncthreads();
     // a warp per block, lane = channel
     for (int blk = warp; blk * DL_BLK < nt; blk += NW) {
@@ -442,25 +761,6 @@ struct DeltaScanParams {
   int32_t* status;
 };
 
-// Packed pairs of fp32: one instruction, two IEEE multiply-adds.
-__device__ __forceinline__ uint64_t dl_pack(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void dl_unpack(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ uint64_t dl_fma(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t dl_mul(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 // The CPL key channels of lane q: 4 q .., 4 (LANES + q) .., ...
 template <int LANES, int CPL>
 __device__ __forceinline__ void dl_load(const float* row, int q, uint64_t (&x)[CPL / 2]) {
@@ -773,31 +1073,331 @@ __global__ void __launch_bounds__(DL_THREADS) delta_scan_blocked_kernel(const De
     if (col_on[j]) dl_store<LANES, CPL>(st[j], q, s[j]);
 }
 
+// Chunks of a portion, on the tensor cores: S^T, 16 value channels a warp, stays in the registers
+// of its mma accumulators, which are also the layout of an A operand.  With S ahead of a chunk
+// (operands as in its record, tokens 1..16)
+//
+//   P = (I + C)^-1 (U S + A V)      O = R S + E V - F P      S' = diag(w_{1..16}) S + K^T V - B^T P
+//
+// Bound by the tensor cores where the SMs have two CTAs (8 cycles an mma, 204 a chunk and warp at 64
+// channels), else by a chunk's chain of products: 3500 cycles, 6000 at 128 channels.
+//
+// Every product is of three bf16 parts a number (v has one), the six of them that reach 2^-24.
+// The largest of them, hi hi, has an accumulator of its own for each 16 k's, which it fills almost
+// exactly, and those are added in fp32; the others share one, whose rounding is 2^-8 of that.
+struct DlParts { uint32_t hi[4], mid[4], lo[4]; };
+struct DlFrag { uint4 hi, mid, lo; };
+__device__ __forceinline__ void dl_mma1(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
+                                        uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
+      "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// c[0], c[1] += a times the two halves of b
+__device__ __forceinline__ void dl_mma(float (&c)[2][4], const uint32_t (&a)[4], const uint4& b) {
+  dl_mma1(c[0], a, b.x, b.y);
+  dl_mma1(c[1], a, b.z, b.w);
+}
+__device__ __forceinline__ void dl_add(float (&c)[2][4], const float (&t)[2][4]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[i][e] += t[i][e];
+}
+// two 16 x 8 accumulator tiles as one 16 x 16 A operand
+__device__ __forceinline__ void dl_parts(const float (&x)[4], const float (&y)[4], DlParts& a) {
+  dl_split(x[0], x[1], a.hi[0], a.mid[0], a.lo[0]);
+  dl_split(x[2], x[3], a.hi[1], a.mid[1], a.lo[1]);
+  dl_split(y[0], y[1], a.hi[2], a.mid[2], a.lo[2]);
+  dl_split(y[2], y[3], a.hi[3], a.mid[3], a.lo[3]);
+}
+__device__ __forceinline__ DlFrag dl_frag(const uint8_t* at, int lane) {
+  const uint4* x = reinterpret_cast<const uint4*>(at) + lane;
+  return {x[0], x[DL_FRAG / 16], x[2 * (DL_FRAG / 16)]};
+}
+// the five smaller products of two operands at once, so that four chains run side by side
+__device__ __forceinline__ void dl_five(float (&c)[2][4], const DlParts& a, const DlFrag& x,
+                                        float (&d)[2][4], const DlParts& b, const DlFrag& y) {
+  dl_mma(c, a.lo, x.hi);
+  dl_mma(d, b.lo, y.hi);
+  dl_mma(c, a.hi, x.lo);
+  dl_mma(d, b.hi, y.lo);
+  dl_mma(c, a.mid, x.mid);
+  dl_mma(d, b.mid, y.mid);
+  dl_mma(c, a.mid, x.hi);
+  dl_mma(d, b.mid, y.hi);
+  dl_mma(c, a.hi, x.mid);
+  dl_mma(d, b.hi, y.mid);
+}
+
+// The longest portions come first, so that their CTAs start one an SM; two CTAs an SM, as a third
+// one slows those that the kernel waits for (five portions of 700 to 2400 tokens, 64 heads: 577 us
+// in the order of the batch, 448 longest first, 388 and no more than two an SM).
+constexpr int DL_RANKED = 128;    // portions that are put in order; more even themselves out
+template <int DP, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, DP == 64 ? 2 : 1)
+delta_scan_chunk_kernel(const DeltaScanParams p) {
+  extern __shared__ __align__(128) uint8_t dl_smem[];
+  constexpr int KT = DP / 16, BYTES = dl_chunk_bytes(DP), ST = dl_chunk_stages(DP);
+  uint64_t* full = reinterpret_cast<uint64_t*>(dl_smem + ST * BYTES);
+  __shared__ int failed;
+  __shared__ int ranked;
+  const int h = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = (int)(blockIdx.z * WARPS + (threadIdx.x >> 5));
+  const int g = lane >> 2, q2 = (lane & 3) * 2;
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < ST; ++i) mbar_init(&full[i], 1);
+    mbar_fence_init();
+    failed = 0;
+    ranked = blockIdx.y;
+  }
+  pdl_wait();
+  __syncthreads();
+  for (int j = threadIdx.x; j < p.num_portions && p.num_portions <= DL_RANKED; j += 32 * WARPS) {
+    // portion j is this CTA's, if blockIdx.y are ahead of it
+    const int len = p.cu[j + 1] - p.cu[j];
+    int ahead = 0;
+    for (int i = 0; i < p.num_portions; ++i) {
+      const int other = p.cu[i + 1] - p.cu[i];
+      ahead += other > len || (other == len && i < j) ? 1 : 0;
+    }
+    if (ahead == (int)blockIdx.y) ranked = j;
+  }
+  __syncthreads();
+  const int seq = ranked;
+  const int64_t begin = p.cu[seq], end = p.cu[seq + 1];
+  const int slot = begin < end ? p.slots[begin] : -1;
+  if (slot >= p.num_slots) {
+    if (threadIdx.x == 0 && p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
+    return;
+  }
+  if (slot < 0) return;
+  const int chunks = (int)((end - begin + DL_UNIT - 1) / DL_UNIT);
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(p.packed) +
+                       ((int64_t)h * p.units + begin / DL_UNIT + seq) * BYTES;
+  auto issue = [&](int n) {
+    mbar_arrive_expect_tx(&full[n % ST], BYTES);
+    bulk_load(dl_smem + n % ST * BYTES, src + (int64_t)n * BYTES, BYTES, &full[n % ST]);
+  };
+  if (threadIdx.x == 0)
+    for (int n = 0; n < ST && n < chunks; ++n) issue(n);
+
+  // rows (value channels) v0 and v0 + 8 of S^T; columns 8 n + q2, + 1
+  const int v0 = warp * 16 + g;
+  const bool on0 = v0 < p.d, on1 = v0 + 8 < p.d;
+  float s[2 * KT][4];
+  float* st = p.state + ((int64_t)slot * p.heads + h) * p.d * DP + q2;
+  const bool fresh = p.positions[begin] == 0;
+#pragma unroll
+  for (int n = 0; n < 2 * KT; ++n) {
+    float2 a = make_float2(0.f, 0.f), b = a;
+    if (on0 && !fresh) a = *reinterpret_cast<const float2*>(st + (int64_t)v0 * DP + n * 8);
+    if (on1 && !fresh) b = *reinterpret_cast<const float2*>(st + (int64_t)(v0 + 8) * DP + n * 8);
+    s[n][0] = a.x;
+    s[n][1] = a.y;
+    s[n][2] = b.x;
+    s[n][3] = b.y;
+  }
+  const bool live = warp * 16 < p.d;
+  float* out = p.o + (int64_t)h * p.d + v0;
+  const int64_t o_stride = (int64_t)p.heads * p.d;
+  int n = 0;
+  for (; n < chunks; ++n) {
+    if (!mbar_wait(&full[n % ST], (uint32_t)(n / ST) & 1u, DL_WAIT_LIMIT)) {
+      if (p.status) atomicOr(p.status, FK_DEV_WAIT_TIMEOUT);
+      failed = 1;
+    }
+    const uint8_t* rec = dl_smem + n % ST * BYTES;
+    const int64_t row0 = begin + (int64_t)n * DL_UNIT;
+    const int cnt = (int)min((int64_t)DL_UNIT, end - row0);
+    if (live && *reinterpret_cast<const int*>(rec + dl_chunk_flag(DP)) != 0) {
+      // something is not finite: token by token, so that no token before it sees it
+      const float* f = reinterpret_cast<const float*>(rec);
+      constexpr int F = DL_UNIT * DP;
+      for (int t = 0; t < cnt; ++t) {
+        const float* x = f + t * DP + q2;
+        float d0 = 0.f, d1 = 0.f, o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int i = 0; i < 2 * KT; ++i) {
+          const float2 u = *reinterpret_cast<const float2*>(x + F + i * 8);
+          d0 = fmaf(u.y, s[i][1], fmaf(u.x, s[i][0], d0));
+          d1 = fmaf(u.y, s[i][3], fmaf(u.x, s[i][2], d1));
+        }
+#pragma unroll
+        for (int w = 1; w < 4; w <<= 1) {
+          d0 += __shfl_xor_sync(0xffffffffu, d0, w);
+          d1 += __shfl_xor_sync(0xffffffffu, d1, w);
+        }
+        const float va = f[5 * F + t * DP + v0], vb = f[5 * F + t * DP + v0 + 8];
+#pragma unroll
+        for (int i = 0; i < 2 * KT; ++i) {
+          const float2 w = *reinterpret_cast<const float2*>(x + i * 8);
+          const float2 b = *reinterpret_cast<const float2*>(x + 2 * F + i * 8);
+          const float2 k = *reinterpret_cast<const float2*>(x + 3 * F + i * 8);
+          const float2 r = *reinterpret_cast<const float2*>(x + 4 * F + i * 8);
+          s[i][0] = fmaf(b.x, -d0, fmaf(k.x, va, w.x * s[i][0]));
+          s[i][1] = fmaf(b.y, -d0, fmaf(k.y, va, w.y * s[i][1]));
+          s[i][2] = fmaf(b.x, -d1, fmaf(k.x, vb, w.x * s[i][2]));
+          s[i][3] = fmaf(b.y, -d1, fmaf(k.y, vb, w.y * s[i][3]));
+          o0 = fmaf(r.y, s[i][1], fmaf(r.x, s[i][0], o0));
+          o1 = fmaf(r.y, s[i][3], fmaf(r.x, s[i][2], o1));
+        }
+#pragma unroll
+        for (int w = 1; w < 4; w <<= 1) {
+          o0 += __shfl_xor_sync(0xffffffffu, o0, w);
+          o1 += __shfl_xor_sync(0xffffffffu, o1, w);
+        }
+        if (q2 == 0) {
+          if (on0) out[(row0 + t) * o_stride] = o0;
+          if (on1) out[(row0 + t) * o_stride + 8] = o1;
+        }
+      }
+    } else if (live) {
+      float pp[2][4] = {}, oo[2][4] = {}, ps[2][4] = {}, os[2][4] = {};
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt) {
+        DlParts a;
+        dl_parts(s[2 * kt], s[2 * kt + 1], a);
+        const DlFrag u = dl_frag(rec + kt * 3 * DL_FRAG, lane);
+        const DlFrag r = dl_frag(rec + (KT + kt) * 3 * DL_FRAG, lane);
+        float t[2][4] = {}, z[2][4] = {};
+        dl_mma(t, a.hi, u.hi);
+        dl_mma(z, a.hi, r.hi);
+        dl_five(ps, a, u, os, a, r);
+        dl_add(pp, t);
+        dl_add(oo, z);
+      }
+      const uint4 v4 = reinterpret_cast<const uint4*>(rec + dl_chunk_v(DP))[warp * 32 + lane];
+      const uint32_t v[4] = {v4.x, v4.y, v4.z, v4.w};
+      const uint8_t* mats = rec + dl_chunk_mats(DP);
+      DlParts a;
+      {
+        const DlFrag x = dl_frag(mats, lane);
+        float t[2][4] = {};
+        dl_mma(t, v, x.hi);
+        dl_mma(ps, v, x.lo);
+        dl_mma(ps, v, x.mid);
+        dl_add(pp, t);
+        dl_add(pp, ps);
+        dl_parts(pp[0], pp[1], a);
+        const DlFrag m = dl_frag(mats + 3 * DL_FRAG, lane);
+        float z[2][4] = {}, y0[2][4] = {}, y1[2][4] = {};
+        dl_mma(z, a.hi, m.hi);
+        dl_mma(y0, a.lo, m.hi);
+        dl_mma(y1, a.mid, m.hi);
+        dl_mma(y0, a.hi, m.lo);
+        dl_mma(y1, a.hi, m.mid);
+        dl_mma(y0, a.mid, m.mid);
+        dl_add(y1, y0);
+        dl_add(z, y1);
+        dl_parts(z[0], z[1], a);
+      }
+      const float* gam = reinterpret_cast<const float*>(rec + dl_chunk_decay(DP)) + q2;
+#pragma unroll
+      for (int kt = 0; kt < KT; ++kt) {
+        const DlFrag x = dl_frag(rec + (2 * KT + kt) * 3 * DL_FRAG, lane);
+        const DlFrag y = dl_frag(rec + (3 * KT + kt) * 3 * DL_FRAG, lane);
+        float t[2][4] = {}, z[2][4] = {}, y0[2][4] = {}, y1[2][4] = {};
+        dl_mma(t, v, x.hi);
+        dl_mma(z, a.hi, y.hi);
+        dl_mma(y0, v, x.lo);
+        dl_mma(y1, a.lo, y.hi);
+        dl_mma(y0, v, x.mid);
+        dl_mma(y1, a.hi, y.lo);
+        dl_mma(y0, a.mid, y.hi);
+        dl_mma(y1, a.mid, y.mid);
+        dl_mma(y0, a.hi, y.mid);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float2 w = *reinterpret_cast<const float2*>(gam + (2 * kt + i) * 8);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float& x1 = s[2 * kt + i][e];
+            x1 = fmaf(e & 1 ? w.y : w.x, x1, t[i][e] + z[i][e]) + (y0[i][e] + y1[i][e]);
+          }
+        }
+      }
+      {
+        const DlFrag x = dl_frag(mats + 6 * DL_FRAG, lane), y = dl_frag(mats + 9 * DL_FRAG, lane);
+        float t[2][4] = {}, z[2][4] = {}, y1[2][4] = {};
+        dl_mma(t, v, x.hi);
+        dl_mma(z, a.hi, y.hi);
+        dl_mma(os, v, x.lo);
+        dl_mma(y1, a.lo, y.hi);
+        dl_mma(os, v, x.mid);
+        dl_mma(y1, a.hi, y.lo);
+        dl_mma(os, a.mid, y.hi);
+        dl_mma(y1, a.mid, y.mid);
+        dl_mma(os, a.hi, y.mid);
+        dl_add(os, y1);
+        dl_add(oo, t);
+        dl_add(oo, z);
+        dl_add(oo, os);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int tok = i * 8 + q2 + (e & 1);
+            if (tok < cnt && (e < 2 ? on0 : on1))
+              out[(row0 + tok) * o_stride + (e < 2 ? 0 : 8)] = oo[i][e];
+          }
+      }
+    }
+    __syncthreads();             // the record has been read
+    if (failed) break;
+    if (threadIdx.x == 0 && n + ST < chunks) issue(n + ST);
+  }
+  if (failed) {
+    // copies that were requested must land before the shared memory goes away
+    for (int i = n; i < chunks && i < n + ST; ++i)
+      (void)mbar_wait(&full[i % ST], (uint32_t)(i / ST) & 1u, DL_WAIT_LIMIT);
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 2 * KT; ++i) {
+    if (on0)
+      *reinterpret_cast<float2*>(st + (int64_t)v0 * DP + i * 8) = make_float2(s[i][0], s[i][1]);
+    if (on1)
+      *reinterpret_cast<float2*>(st + (int64_t)(v0 + 8) * DP + i * 8) =
+          make_float2(s[i][2], s[i][3]);
+  }
+}
+
 static int delta_padded(int d) { return d <= 32 ? 32 : d <= 64 ? 64 : d <= 128 ? 128 : 256; }
 
-template <typename T, int DP, bool BLOCKED, bool VEC>
+template <typename T, int DP, bool BLOCKED, bool VEC, bool CHUNK = false>
 static int launch_prepare_one(const DeltaPrepParams& p, unsigned gx, cudaStream_t s) {
-  const size_t smem = (size_t)DL_UNIT * (p.rank_p + 8) * 4 +
-                      (size_t)DL_FIELDS * DL_UNIT * DP * 4 + DL_UNIT * (DP / 32 + 1) * 4;
+  constexpr int kFixed = DL_FIELDS * DL_UNIT * (CHUNK ? DP + 4 : DP) * 4 +
+                         DL_UNIT * (DP / 32 + 1) * 4 + (CHUNK ? 4 * 256 * 4 : 0);
+  const size_t smem = (size_t)DL_UNIT * (p.rank_p + 8) * 4 + kFixed;
   static PerDeviceOnce once;
-  constexpr int kMaxSmem = DL_UNIT * 520 * 4 + DL_FIELDS * DL_UNIT * DP * 4 +
-                           DL_UNIT * (DP / 32 + 1) * 4;
-  FK_CUDA_OK(set_max_dynamic_smem(once, delta_prepare_kernel<T, DP, BLOCKED, VEC>, kMaxSmem));
+  constexpr int kMaxSmem = DL_UNIT * 520 * 4 + kFixed;
+  FK_CUDA_OK(set_max_dynamic_smem(once, delta_prepare_kernel<T, DP, BLOCKED, VEC, CHUNK>,
+                                  kMaxSmem));
   const dim3 grid(gx, (unsigned)((p.heads + p.heads_per_cta - 1) / p.heads_per_cta));
-  FK_CUDA_OK(launch_kernel(delta_prepare_kernel<T, DP, BLOCKED, VEC>, grid, dim3(DL_THREADS), smem, s,
-                           p));
+  FK_CUDA_OK(launch_kernel(delta_prepare_kernel<T, DP, BLOCKED, VEC, CHUNK>, grid,
+                           dim3(DL_THREADS), smem, s, p));
   count_launch();
   return FK_OK;
 }
 template <typename T, int DP>
-static int launch_prepare_dp(const DeltaPrepParams& p, bool blocked, cudaStream_t s) {
+static int launch_prepare_dp(const DeltaPrepParams& p, int blocked, cudaStream_t s) {
   const unsigned single = (unsigned)((p.rows + DL_UNIT - 1) / DL_UNIT);
   // rows of whole 16-byte pieces, where 2-byte loads waited for one another: five prompts of
   // 700 to 2500 tokens, 64 heads of 64 687 -> 436 us, 24 heads of 128 765 -> 335;
   // a decode step of 16 rows, 32 heads of 64, 10.9 -> 8.2
   if constexpr (sizeof(T) == 2) {
-    if (p.d % 8 == 0 && p.in_stride % 8 == 0 && aligned16(p.r) && aligned16(p.k) &&
-        aligned16(p.v) && aligned16(p.a) && aligned16(p.w0) && aligned16(p.a_bias))
+    const bool pieces = p.d % 8 == 0 && p.in_stride % 8 == 0 && aligned16(p.r) &&
+                        aligned16(p.k) && aligned16(p.v) && aligned16(p.a) && aligned16(p.w0) &&
+                        aligned16(p.a_bias);
+    if constexpr (DP == 64 || DP == 128) {
+      if (blocked == 2)
+        return pieces ? launch_prepare_one<T, DP, true, true, true>(p, (unsigned)p.units, s)
+                      : launch_prepare_one<T, DP, true, false, true>(p, (unsigned)p.units, s);
+    }
+    if (pieces)
       return blocked ? launch_prepare_one<T, DP, true, true>(p, (unsigned)p.units, s)
                      : launch_prepare_one<T, DP, false, true>(p, single, s);
   }
@@ -805,7 +1405,7 @@ static int launch_prepare_dp(const DeltaPrepParams& p, bool blocked, cudaStream_
                  : launch_prepare_one<T, DP, false, false>(p, single, s);
 }
 template <typename T>
-static int launch_prepare(const DeltaPrepParams& p, bool blocked, cudaStream_t s) {
+static int launch_prepare(const DeltaPrepParams& p, int blocked, cudaStream_t s) {
   switch (delta_padded(p.d)) {
     case 32: return launch_prepare_dp<T, 32>(p, blocked, s);
     case 64: return launch_prepare_dp<T, 64>(p, blocked, s);
@@ -831,9 +1431,32 @@ static int launch_scan_blocked(DeltaScanParams& p, cudaStream_t s) {
   count_launch();
   return FK_OK;
 }
+template <int DP, int WARPS>
+static int launch_scan_chunks(const DeltaScanParams& p, cudaStream_t s) {
+  constexpr int kSmem = dl_chunk_stages(DP) * (dl_chunk_bytes(DP) + (int)sizeof(uint64_t));
+  static PerDeviceOnce once;
+  FK_CUDA_OK(set_max_dynamic_smem(once, delta_scan_chunk_kernel<DP, WARPS>, kSmem));
+  const dim3 grid((unsigned)p.heads, (unsigned)p.num_portions,
+                  (unsigned)((p.d + 16 * WARPS - 1) / (16 * WARPS)));
+  FK_CUDA_OK(launch_kernel_after(delta_scan_chunk_kernel<DP, WARPS>, grid, dim3(32 * WARPS), kSmem,
+                                 s, p));
+  count_launch();
+  return FK_OK;
+}
+static int launch_scan_chunks(const DeltaScanParams& p, int dp, cudaStream_t s) {
+  // heads of 128 channels: as two CTAs while every head of every portion has an SM to itself (24
+  // heads: one portion of 1500 tokens 471 -> 290 us, five of 700 to 2400 749 -> 520); more of them
+  // share a record's copy between all columns
+  if (dp == 64) return launch_scan_chunks<64, 4>(p, s);
+  return p.heads * (int64_t)p.num_portions <= sm_count() ? launch_scan_chunks<128, 4>(p, s)
+                                                             : launch_scan_chunks<128, 8>(p, s);
+}
 // LANES x CPL for single tokens, BL x BC for blocks
 template <int LANES, int CPL, int BL, int BC>
-static int launch_scan(DeltaScanParams& p, bool blocked, cudaStream_t s) {
+static int launch_scan(DeltaScanParams& p, int blocked, cudaStream_t s) {
+  if constexpr (LANES * CPL == 64 || LANES * CPL == 128) {
+    if (blocked == 2) return launch_scan_chunks(p, LANES * CPL, s);
+  }
   if (!blocked) {
     constexpr int COLS = DL_THREADS / LANES * 2;
     const dim3 grid((unsigned)((p.d + COLS - 1) / COLS), (unsigned)p.heads,
@@ -861,9 +1484,17 @@ int fk_delta_padded_dim(int dim) {
   return dim <= 0 || dim > DL_MAX_DIM ? 0 : delta_padded(dim);
 }
 
+int fk_delta_chunked(int dim) {
+  const int dp = fk_delta_padded_dim(dim);
+  return dp == 64 || dp == 128;
+}
+
 int64_t fk_delta_packed_floats(int64_t rows, int num_portions, int heads, int dim, int blocked) {
   const int dp = fk_delta_padded_dim(dim);
   if (dp == 0 || rows < 0 || num_portions < 0 || heads <= 0) return 0;
+  if (blocked == 2)
+    return fk_delta_chunked(dim) ? heads * (rows / DL_UNIT + num_portions) *
+                                       (int64_t)(dl_chunk_bytes(dp) / 4) : 0;
   return blocked ? heads * (rows / DL_UNIT + num_portions) * (DL_UNIT / DL_BLK) *
                        (int64_t)dl_block_floats(dp)
                  : heads * rows * (int64_t)DL_FIELDS * dp;
@@ -882,6 +1513,8 @@ int fk_delta_prepare(const void* r, const void* k, const void* v, const void* a,
              "fk_delta_prepare: null pointer");
   FK_REQUIRE(!blocked || (cu_portions && num_portions > 0), FK_ERR_INVALID_ARG,
              "fk_delta_prepare: blocks need the portions");
+  FK_REQUIRE(blocked != 2 || (fk_delta_chunked(dim) && !is_f32), FK_ERR_UNSUPPORTED,
+             "fk_delta_prepare: chunks need bf16 and heads of 33 to 128 channels");
   FK_REQUIRE(dim <= DL_MAX_DIM && rank <= 512 && heads <= 65535 && rows < (1ll << 31),
              FK_ERR_UNSUPPORTED, "fk_delta_prepare: head size %d or rank %d too large", dim, rank);
   FK_REQUIRE(w2_stride % 4 == 0 && w2_stride >= rank && aligned16(w2) && aligned16(packed),
@@ -895,11 +1528,12 @@ int fk_delta_prepare(const void* r, const void* k, const void* v, const void* a,
   p.decay_scale = decay_scale; p.unit_eps = unit_eps;
   // heads per CTA: the tanh tile is shared by them, as long as the SMs stay busy
   int hpc = 1;
-  while (hpc < 8 && (rows / DL_UNIT + 1) * heads / (hpc * 2) >= 16 * sm_count()) hpc *= 2;
+  // (chunks, at most six CTAs an SM: more of them leave a shorter last wave)
+  const int least = (blocked == 2 ? 32 : 16) * sm_count();
+  while (hpc < 8 && (rows / DL_UNIT + 1) * heads / (hpc * 2) >= least) hpc *= 2;
   p.heads_per_cta = hpc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return is_f32 ? launch_prepare<float>(p, blocked != 0, s)
-                : launch_prepare<uint16_t>(p, blocked != 0, s);
+  return is_f32 ? launch_prepare<float>(p, blocked, s) : launch_prepare<uint16_t>(p, blocked, s);
 }
 
 int fk_delta_scan(const float* packed, int blocked, float* o, float* state, int num_slots,
@@ -913,6 +1547,8 @@ int fk_delta_scan(const float* packed, int blocked, float* o, float* state, int 
              FK_ERR_INVALID_ARG, "fk_delta_scan: null pointer");
   FK_REQUIRE(dim <= DL_MAX_DIM && heads <= 65535 && num_portions <= 65535, FK_ERR_UNSUPPORTED,
              "fk_delta_scan: head size %d or counts too large", dim);
+  FK_REQUIRE(blocked != 2 || fk_delta_chunked(dim), FK_ERR_UNSUPPORTED,
+             "fk_delta_scan: chunks need heads of 33 to 128 channels");
   FK_REQUIRE(aligned16(packed) && aligned16(state), FK_ERR_ALIGNMENT,
              "fk_delta_scan: 16-byte alignment required");
   DeltaScanParams p{};
@@ -922,10 +1558,10 @@ int fk_delta_scan(const float* packed, int blocked, float* o, float* state, int 
   p.status = status;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (delta_padded(dim)) {
-    case 32: return launch_scan<4, 8, 4, 8>(p, blocked != 0, s);
-    case 64: return launch_scan<8, 8, 8, 8>(p, blocked != 0, s);
-    case 128: return launch_scan<16, 8, 16, 8>(p, blocked != 0, s);
-    default: return launch_scan<32, 8, 32, 8>(p, blocked != 0, s);
+    case 32: return launch_scan<4, 8, 4, 8>(p, blocked, s);
+    case 64: return launch_scan<8, 8, 8, 8>(p, blocked, s);
+    case 128: return launch_scan<16, 8, 16, 8>(p, blocked, s);
+    default: return launch_scan<32, 8, 32, 8>(p, blocked, s);
   }
 }
 

@@ -762,9 +762,9 @@ def delta_padded_dim(dim: int) -> int:
 
 
 def delta_prepare(r, k, v, a, y1, w2, w0, a_bias, heads, dim, decay_scale, unit_eps,
-                  cu_portions=None, packed=None):
-    """Operands of the delta rule (fp32, opaque): in blocks of 8 tokens of the portions
-    when cu_portions is given, else token by token.  r, k, v, a [T, heads * dim] and
+                  cu_portions=None, packed=None, chunks=False):
+    """Operands of the delta rule (fp32, opaque): in blocks of 4 tokens of the portions
+    when cu_portions is given (16 with `chunks`, see delta_chunks), else token by token.  r, k, v, a [T, heads * dim] and
     y1 [T, rank] are column ranges of the same rows; w2 [heads * dim, padded rank]."""
     f32 = _is_f32(k, "k")
     rows, rank = y1.shape
@@ -781,19 +781,28 @@ def delta_prepare(r, k, v, a, y1, w2, w0, a_bias, heads, dim, decay_scale, unit_
         _need(cu_portions, torch.int32, "cu_portions")
         n_port = cu_portions.numel() - 1
     delta_padded_dim(dim)
+    blocked = (2 if chunks else 1) if n_port > 0 else 0
     if packed is None:
-        n = int(lib.fk_delta_packed_floats(rows, n_port, heads, dim, int(n_port > 0)))
+        n = int(lib.fk_delta_packed_floats(rows, n_port, heads, dim, blocked))
         packed = torch.empty(n, dtype=torch.float32, device=k.device)
     check(lib.fk_delta_prepare(
         _ptr(r), _ptr(k), _ptr(v), _ptr(a), _ptr(y1), k.stride(0) if rows else 0, f32, _ptr(w2),
-        w2.shape[1], _ptr(w0), _ptr(a_bias), _ptr(packed), int(n_port > 0), _ptr(cu_portions),
+        w2.shape[1], _ptr(w0), _ptr(a_bias), _ptr(packed), blocked, _ptr(cu_portions),
         n_port, rows, heads, dim, rank, float(decay_scale), float(unit_eps), _stream()),
         "fk_delta_prepare")
     return packed
 
 
-def delta_scan(packed, state, cu_portions, slots, positions, blocked, out=None, status=None):
-    """The recurrence over prepared operands (`blocked`: prepared with cu_portions);
+def delta_chunks(dim: int, dtype, rows: int, portions: int) -> bool:
+    """Whether portions of `rows` tokens in all go 16 tokens at a time (prepare and scan with
+    chunks=True): bf16, 33 to 128 channels a head, not mostly padding."""
+    return dtype == BF16 and rows >= 32 * portions and bool(lib.fk_delta_chunked(int(dim)))
+
+
+def delta_scan(packed, state, cu_portions, slots, positions, blocked, out=None, status=None,
+               chunks=False):
+    """The recurrence over prepared operands (`blocked`: prepared with cu_portions, and as there
+    with `chunks`);
     state [slots, heads, dim, padded_dim] fp32 is read and replaced.  Returns
     o [T, heads * dim] fp32."""
     _need(packed, torch.float32, "packed")
@@ -803,14 +812,15 @@ def delta_scan(packed, state, cu_portions, slots, positions, blocked, out=None, 
     _need(positions, torch.int64, "positions")
     rows, heads, dim = positions.shape[0], state.shape[1], state.shape[2]
     n_port = cu_portions.numel() - 1
+    form = (2 if chunks else 1) if blocked else 0
     if not packed.is_contiguous() or not state.is_contiguous() or \
             state.shape[3] != delta_padded_dim(dim) or packed.numel() < \
-            int(lib.fk_delta_packed_floats(rows, n_port, heads, dim, int(bool(blocked)))):
+            int(lib.fk_delta_packed_floats(rows, n_port, heads, dim, form)):
         raise _lib.FkError("delta_scan: packed or state has the wrong shape")
     if out is None:
         out = torch.empty((rows, heads * dim), dtype=torch.float32, device=packed.device)
     check(lib.fk_delta_scan(
-        _ptr(packed), int(bool(blocked)), _ptr(out), _ptr(state), state.shape[0],
+        _ptr(packed), form, _ptr(out), _ptr(state), state.shape[0],
         _ptr(cu_portions), n_port, _ptr(slots), _ptr(positions), rows, heads, dim,
         _status_ptr(status, packed), _stream()), "fk_delta_scan")
     return out

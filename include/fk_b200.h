@@ -689,13 +689,16 @@ int fk_gemm_bf16_act_mul(const void* x, int64_t x_stride, const void* w, const v
  * projection rows; w2 [heads * dim, w2_stride] in the activation type, rows zero-padded
  * to a multiple of 4 (rank <= 512).  blocked 0: per token, packed
  * [heads][rows][6][padded_dim] fp32 (w, u, a * u, k, r, v), for single tokens;
- * blocked 1: blocks of 8 tokens of a portion (layout: csrc/fk_delta.cu), for portions.
+ * blocked 1: blocks of 4 tokens of a portion (layout: csrc/fk_delta.cu), for portions;
+ * blocked 2: chunks of 16 tokens, bf16 and head sizes where fk_delta_chunked is 1 (33 to 128).
+ * `packed` is scanned with the `blocked` that it was prepared with.
  * fk_delta_packed_floats: size of `packed` in floats.
  * fk_delta_scan runs the recurrence for every portion from and to
  * state [num_slots][heads][dim (value)][padded_dim (key)] fp32 and writes
  * o [rows, heads * dim] fp32.  fk_head_norm_gate: out = rms(o per head) * weight *
  * sigmoid(gate), columns beyond heads * dim zeroed. */
 int fk_delta_padded_dim(int dim);
+int fk_delta_chunked(int dim);
 int64_t fk_delta_packed_floats(int64_t rows, int num_portions, int heads, int dim, int blocked);
 int fk_delta_prepare(const void* r, const void* k, const void* v, const void* a, const void* y1,
                      int64_t in_stride, int is_f32, const void* w2, int64_t w2_stride,

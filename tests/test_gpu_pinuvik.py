@@ -636,6 +636,72 @@ def test_delta_rule_in_portions(heads, dim, rank, dtype):
     assert torch.all(state[1] == 3.0) and torch.all(state[3] == 3.0)
 
 
+@pytest.mark.parametrize("heads,dim,rank", [(2, 36, 5), (3, 64, 33), (2, 100, 64), (9, 128, 16)])
+def test_delta_rule_in_chunks(heads, dim, rank):
+    """16 tokens at a time on the tensor cores against the plain recurrence: portions that end
+    at, before and behind a chunk's end, one that goes on from the carried state, a padded row,
+    enough of them for whole and for split heads; and a token that is not finite changes no
+    token ahead of it."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(dim)
+    hd, counts = heads * dim, [33, 1, 16, 15, 17, 48, 3] + [2] * 10
+    total = sum(counts) + 1
+    cu = np.concatenate([[0], np.cumsum(counts + [1])])
+    z, _ = rnd(rs, total, 4 * hd + rank, dtype=BF16)
+    w2 = P.bf16(rs.randn(hd, rank) / np.sqrt(rank))
+    w2p = np.zeros((hd, (rank + 3) // 4 * 4))
+    w2p[:, :rank] = w2
+    w0, ab = rs.uniform(-6, 1, hd), rs.randn(hd)
+    dp = ops.delta_padded_dim(dim)
+    n = len(counts)
+    first = rs.randn(n, heads, dim, dim)                   # [.., key, value]
+    state0 = torch.full((n + 2, heads, dim, dp), 3.0, device="cuda")
+    state0[:n] = 0
+    state0[:n, :, :, :dim] = dev(first.transpose(0, 1, 3, 2))
+    st = ops.new_status("cuda")
+
+    def run(z):
+        x = torch.zeros((total, (4 * hd + rank + 7) // 8 * 8), dtype=BF16, device="cuda")
+        x[:, :4 * hd + rank] = dev(z, BF16)
+        state, o = state0.clone(), torch.full((total, hd), 9.0, device="cuda")
+        cols = [x[:, i * hd:(i + 1) * hd] for i in range(4)] + [x[:, 4 * hd:4 * hd + rank]]
+        packed = ops.delta_prepare(*cols, dev(w2p, BF16), dev(w0), dev(ab), heads, dim,
+                                   float(np.exp(-0.5)), 1e-6, cu_portions=i32(cu), chunks=True)
+        slots = np.repeat(np.arange(n + 1), counts + [1])
+        slots[-1] = -1
+        pos = np.concatenate([np.arange(c) + (5 if i % 2 else 0) for i, c in enumerate(counts)] +
+                             [[0]])
+        ops.delta_scan(packed, state, i32(cu), i32(slots), i64(pos), True, out=o, status=st,
+                       chunks=True)
+        return o, state
+
+    o, state = run(z)
+    r, k, v, a = (z[:, i * hd:(i + 1) * hd].reshape(total, heads, dim) for i in range(4))
+    decay = P.delta_decay(z[:, 4 * hd:], w2, w0).reshape(total, heads, dim)
+    rate = P.sigmoid(a + ab.reshape(heads, dim))
+    for i, c in enumerate(counts):
+        t = slice(cu[i], cu[i] + c)
+        want, s = P.delta_rule(r[t], k[t], v[t], decay[t], rate[t], first[i] if i % 2 else None)
+        close(o[t], want.reshape(c, -1), F32, scale=10)
+        close(state[i, :, :, :dim].permute(0, 2, 1), s, F32, scale=10)
+    assert torch.all(o[-1] == 9.0) and torch.all(state[n:] == 3.0) and int(st.item()) == 0
+
+    # the gate of token 20, v of token 10 of the sequence behind 33 + 1 + 16, k of its second chunk
+    for row, col, value, lost in ((20, 3 * hd, np.nan, slice(0, dim)),
+                                  (cu[3] + 10, 2 * hd + 1, np.inf, slice(1, 2)),
+                                  (cu[5] + 30, hd + dim, -np.inf, slice(dim, 2 * dim))):
+        bad = z.copy()
+        bad[row, col] = value
+        got, _ = run(bad)
+        seq = np.searchsorted(cu, row, side="right") - 1
+        ahead = torch.ones(total, dtype=torch.bool, device="cuda")
+        ahead[row:cu[seq + 1]] = False
+        # the chunk in question goes token by token: not the same bits
+        torch.testing.assert_close(got[ahead], o[ahead], rtol=1e-4, atol=2e-4)
+        assert not torch.any(torch.isfinite(got[row + 1:cu[seq + 1], lost]))
+        assert int(torch.count_nonzero(~torch.isfinite(got))) >= lost.stop - lost.start
+
+
 def test_delta_rule_long_run_does_not_drift():
     """1500 tokens with slow decay in one portion, in portions of 7 and of 64, and token
     by token give the same state, close to the plain recurrence; many heads and
