@@ -569,6 +569,86 @@ constexpr int AA_MAX_SMEM = 227 * 1024 - 1024;
 
 __host__ __device__ inline int aa_pitch(int d) { return (d + 31) / 32 * 32 + 4; }
 
+// The sequence whose queries blk (then within it) QB at a time are, its rows, -1: none; every warp
+// finds it by itself.
+template <int QB>
+__device__ __forceinline__ int aa_find(const AnyAttnParams& p, int grp, int64_t& blk, int64_t& row0,
+                                       int64_t& row1) {
+  const int lane = threadIdx.x & 31;
+  int seq = -1;
+  row0 = row1 = 0;
+  for (int s0 = 0; s0 < p.num_seqs && seq < 0; s0 += 32) {
+    const int sq = s0 + lane;
+    int64_t a = 0, b = 0;
+    if (sq < p.num_seqs) {
+      a = sq == 0 ? 0 : p.cu_q[sq];
+      b = sq == p.num_seqs - 1 ? p.rows : p.cu_q[sq + 1];
+      a = a < 0 ? 0 : a;
+      b = b > p.rows ? p.rows : b;
+    }
+    const int64_t mine = b > a ? ((b - a) * grp + QB - 1) / QB : 0;
+    int64_t upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const uint32_t hit = __ballot_sync(0xffffffffu, blk < upto);
+    if (hit) {
+      const int l = __ffs(hit) - 1;
+      seq = s0 + l;
+      blk -= __shfl_sync(0xffffffffu, upto - mine, l);
+      row0 = __shfl_sync(0xffffffffu, a, l);
+      row1 = __shfl_sync(0xffffffffu, b, l);
+    } else {
+      blk -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+  }
+  return seq;
+}
+
+// Rows of one run of keys to shared memory; keys that are not there are rows of zeros.  All pieces
+// of a thread are under way at once: in a loop, each waited for the one before it (fp32, 576
+// channels, 16 heads on one KV head, 20 tokens on 700 keys 313 -> 231 us, 4 heads, 5 on 300
+// 151 -> 116; 128 channels, 16 heads on 4, 900 tokens 371 -> 313; bf16 368 -> 328).
+template <typename T, int CH, int WARPS>
+__device__ __forceinline__ void aa_stage(const AnyAttnParams& p, const void* cache,
+                                         const int64_t* key_off, float* ks, int pitch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quads = p.d >> 2;
+  if constexpr (sizeof(T) == 4) {
+    for (int j = warp; j < AA_KEYS; j += WARPS) {
+      const int64_t off = key_off[j];
+      const float* src = static_cast<const float*>(cache) + (off < 0 ? 0 : off);
+      const uint32_t dst = smem_u32(ks + j * pitch), bytes = off < 0 ? 0 : 16;
+#pragma unroll
+      for (int i = 0; i < (CH + 3) / 4; ++i) {
+        const int c = lane + i * 32;
+        if (c < quads)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + c * 16),
+                       "l"(src + c * 4), "r"(bytes) : "memory");
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else {
+    for (int j = warp; j < AA_KEYS; j += WARPS) {
+      const int64_t off = key_off[j];
+      const T* src = static_cast<const T*>(cache) + off;
+      float4 v[(CH + 3) / 4];
+#pragma unroll
+      for (int i = 0; i < (CH + 3) / 4; ++i) {
+        const int c = lane + i * 32;
+        v[i] = off < 0 || c >= quads ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                     : Elem<T>::load4(src + c * 4);
+      }
+#pragma unroll
+      for (int i = 0; i < (CH + 3) / 4; ++i) {
+        const int c = lane + i * 32;
+        if (c < quads) *reinterpret_cast<float4*>(ks + j * pitch + c * 4) = v[i];
+      }
+    }
+  }
+}
+
 template <typename T, int CH, int R>
 __global__ void __launch_bounds__(AA_THREADS) paged_attn_any_kernel(const AnyAttnParams p,
                                                                     int64_t blocks) {
@@ -585,36 +665,8 @@ __global__ void __launch_bounds__(AA_THREADS) paged_attn_any_kernel(const AnyAtt
   for (int64_t it = blockIdx.x; it < blocks * p.hkv; it += gridDim.x) {
     const int kvh = (int)(it % p.hkv);
     int64_t blk = it / p.hkv;
-    // the sequence of block `blk`; every warp finds it by itself
-    int seq = -1;
-    int64_t row0 = 0, row1 = 0;
-    for (int s0 = 0; s0 < p.num_seqs && seq < 0; s0 += 32) {
-      const int sq = s0 + lane;
-      int64_t a = 0, b = 0;
-      if (sq < p.num_seqs) {
-        a = sq == 0 ? 0 : p.cu_q[sq];
-        b = sq == p.num_seqs - 1 ? p.rows : p.cu_q[sq + 1];
-        a = a < 0 ? 0 : a;
-        b = b > p.rows ? p.rows : b;
-      }
-      const int64_t mine = b > a ? ((b - a) * grp + QB - 1) / QB : 0;
-      int64_t upto = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int64_t v = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += v;
-      }
-      const uint32_t hit = __ballot_sync(0xffffffffu, blk < upto);
-      if (hit) {
-        const int l = __ffs(hit) - 1;
-        seq = s0 + l;
-        blk -= __shfl_sync(0xffffffffu, upto - mine, l);
-        row0 = __shfl_sync(0xffffffffu, a, l);
-        row1 = __shfl_sync(0xffffffffu, b, l);
-      } else {
-        blk -= __shfl_sync(0xffffffffu, upto, 31);
-      }
-    }
+    int64_t row0, row1;
+    const int seq = aa_find<QB>(p, grp, blk, row0, row1);
     if (seq < 0) continue;                      // uniform over the block
     const int64_t queries = (row1 - row0) * grp, q0 = blk * QB;
     const int live = (int)(queries - q0 < QB ? queries - q0 : QB);
@@ -652,17 +704,7 @@ __global__ void __launch_bounds__(AA_THREADS) paged_attn_any_kernel(const AnyAtt
     }
     const bool idle = warp >= live;
     const int32_t* bt = p.block_tables + (int64_t)seq * p.bt_stride;
-    // rows of one run of keys; keys that are not there are rows of zeros
-    auto stage = [&](const void* cache) {
-      const int quads = p.d >> 2;
-      for (int j = warp; j < AA_KEYS; j += AA_WARPS) {
-        const int64_t off = key_off[j];
-        const T* src = static_cast<const T*>(cache) + off;
-        for (int c = lane; c < quads; c += 32)
-          *reinterpret_cast<float4*>(ks + j * pitch + c * 4) =
-              off < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : Elem<T>::load4(src + c * 4);
-      }
-    };
+    auto stage = [&](const void* cache) { aa_stage<T, CH, AA_WARPS>(p, cache, key_off, ks, pitch); };
     for (int k0 = 0; k0 < keys; k0 += AA_KEYS) {
       __syncthreads();
       if (tid < AA_KEYS) {
@@ -773,6 +815,264 @@ __global__ void __launch_bounds__(AA_THREADS) paged_attn_any_kernel(const AnyAtt
   }
 }
 
+// Many queries a sequence: 32 of them (rows x the heads that share a KV head) through runs of 32
+// keys.  What bounds it is the latency and the bytes of shared-memory reads, so that both products
+// are tiles in registers: a warp makes the scores of 16 queries from an eighth of the channels, a
+// thread 4 x 4 of them, and the parts are added; then a warp has 8 queries and a quarter of the
+// channels.  16 warps an SM are what fits (8, with twice the tile each: 864 us where these take
+// 680, one portion of 900 tokens, 16 heads of 576 channels).  The longest queries come first.
+constexpr int AT_WARPS = 16, AT_THREADS = 32 * AT_WARPS, AT_SLICES = 8;
+constexpr int AT_QUERIES = 32, AT_PPITCH = AT_QUERIES + 4, AT_SPITCH = AA_KEYS + 8;
+__host__ __device__ inline int at_smem(int d) {
+  return ((AT_QUERIES + AA_KEYS) * aa_pitch(d) + AT_SLICES * AT_QUERIES * AT_SPITCH +
+          AA_KEYS * AT_PPITCH) * 4;
+}
+__device__ __forceinline__ uint64_t at_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t at_pack(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 at_unpack(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+template <typename T, int CH>
+__global__ void __launch_bounds__(AT_THREADS, 1)
+paged_attn_tile_kernel(const AnyAttnParams p, int64_t blocks) {
+  extern __shared__ __align__(16) float aa_smem[];
+  __shared__ int64_t key_off[AA_KEYS];
+  __shared__ int vis_s[AT_QUERIES];
+  __shared__ __align__(16) float alpha_s[AT_QUERIES], inv_s[AT_QUERIES];
+  constexpr int HC = (CH + 3) / 4;              // chunks of 32 channels a warp owns
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int grp = p.hq / p.hkv, pitch = aa_pitch(p.d);
+  float* qs = aa_smem;                          // [32][pitch], scaled
+  float* ks = qs + AT_QUERIES * pitch;          // [32][pitch]
+  float* part = ks + AA_KEYS * pitch;           // [8 slices][32 queries][40]: scores
+  float* pt = part + AT_SLICES * AT_QUERIES * AT_SPITCH;    // [32 keys][36]: weights
+  const bool shared_rows = p.k_cache == p.v_cache;
+  const int quads = p.d >> 2, per = (quads + AT_SLICES - 1) / AT_SLICES * 4;
+  const int slice = warp & 7, half = warp >> 3;
+  const int c_begin = min(p.d, slice * per), c_end = min(p.d, c_begin + per);
+  const int hc = ((p.d + 31) / 32 + 3) / 4;     // of them in use
+  const int group = warp >> 2, ch0 = (warp & 3) * hc * 32 + lane;
+  const int ch1 = min(p.d, ch0 - lane + hc * 32);
+  const bool wide_q = sizeof(T) == 4 && ((uintptr_t)p.q | (uintptr_t)(p.q_stride * 4)) % 16 == 0;
+  for (int64_t it = blocks * p.hkv - 1 - blockIdx.x; it >= 0; it -= gridDim.x) {
+    const int kvh = (int)(it % p.hkv);
+    int64_t blk = it / p.hkv, row0, row1;
+    const int seq = aa_find<AT_QUERIES>(p, grp, blk, row0, row1);
+    if (seq < 0) continue;                      // uniform over the block
+    const int64_t queries = (row1 - row0) * grp, q0 = blk * AT_QUERIES;
+    const int live = (int)(queries - q0 < AT_QUERIES ? queries - q0 : AT_QUERIES);
+    const int kv_len = p.kv_lens[seq];
+    const int64_t seen0 = (int64_t)kv_len - (p.cu_q[seq + 1] - p.cu_q[seq]) + 1 - p.cu_q[seq];
+    auto visible = [&](int64_t row) {
+      const int64_t v = seen0 + row;
+      return (int)(v < kv_len ? v : kv_len);
+    };
+    const int keys = visible(row0 + (q0 + live - 1) / grp);
+    __syncthreads();                            // the queries before are done with
+    for (int j = warp; j < AT_QUERIES; j += AT_WARPS) {
+      const int64_t row = row0 + (q0 + j) / grp;
+      const T* src = static_cast<const T*>(p.q) + row * p.q_stride +
+                     (int64_t)(kvh * grp + (int)((q0 + j) % grp)) * p.d;
+      if (lane == 0) vis_s[j] = j < live ? visible(row) : 0;
+      for (int c = lane * 4; c < p.d; c += 128) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < live) {
+          if (wide_q) v = Elem<T>::load4(src + c);
+          else v = make_float4(Elem<T>::load(src + c), Elem<T>::load(src + c + 1),
+                               Elem<T>::load(src + c + 2), Elem<T>::load(src + c + 3));
+        }
+        *reinterpret_cast<float4*>(qs + j * pitch + c) = v * p.scale;
+      }
+    }
+    float m[2], l[2];                           // of queries 2 warp, 2 warp + 1
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      m[r] = -INFINITY;
+      l[r] = 0.f;
+    }
+    uint64_t acc[4][HC];                        // pairs of queries 8 group ..
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int i = 0; i < HC; ++i) acc[r][i] = 0ull;
+    const int32_t* bt = p.block_tables + (int64_t)seq * p.bt_stride;
+    auto stage = [&](const void* cache) { aa_stage<T, CH, AT_WARPS>(p, cache, key_off, ks, pitch); };
+    for (int k0 = 0; k0 < keys; k0 += AA_KEYS) {
+      __syncthreads();
+      if (tid < AA_KEYS) {
+        const int kk = k0 + tid;
+        int64_t off = -1;
+        if (kk < keys) {
+          const int page = bt[kk / p.block_size];
+          if (page < 0 || page >= p.num_blocks) {
+            if (p.status) atomicOr(p.status, FK_DEV_BAD_PAGE);
+          } else {
+            off = (((int64_t)page * p.block_size + kk % p.block_size) * p.hkv + kvh) * p.d;
+          }
+        }
+        key_off[tid] = off;
+      }
+      __syncthreads();
+      stage(p.k_cache);
+      __syncthreads();
+      {
+        // queries qg, qg + 4, ..; keys kg, kg + 8, ..
+        const int qg = half * 16 + (lane >> 3), kg = lane & 7;
+        uint64_t s2[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) s2[q][k] = 0ull;
+        const float* kr = ks + kg * pitch;
+        const float* qr = qs + qg * pitch;
+        for (int c = c_begin; c < c_end; c += 4) {
+          ulonglong2 kv[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            kv[k] = *reinterpret_cast<const ulonglong2*>(kr + k * 8 * pitch + c);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qr + q * 4 * pitch + c);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              s2[q][k] = at_fma(kv[k].y, qv.y, at_fma(kv[k].x, qv.x, s2[q][k]));
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float2 v = at_unpack(s2[q][k]);
+            part[(slice * AT_QUERIES + qg + q * 4) * AT_SPITCH + kg + k * 8] = v.x + v.y;
+          }
+      }
+      __syncthreads();
+      if (!shared_rows) stage(p.v_cache);
+      {
+        const bool there = key_off[lane] >= 0;
+        float pr[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int q = warp * 2 + r;
+          float s = 0.f;
+#pragma unroll
+          for (int w = 0; w < AT_SLICES; ++w) s += part[(w * AT_QUERIES + q) * AT_SPITCH + lane];
+          if (!there || k0 + lane >= vis_s[q]) s = -INFINITY;
+          float mx = s;
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+          const float m_new = fmaxf(m[r], mx);
+          float alpha = 1.f;
+          pr[r] = 0.f;
+          if (m_new != -INFINITY) {             // uniform over the warp
+            alpha = expf(m[r] - m_new);
+            m[r] = m_new;
+            pr[r] = expf(s - m_new);
+            l[r] = l[r] * alpha + warp_sum(pr[r]);
+          }
+          if (lane == 0) alpha_s[q] = alpha;
+        }
+        *reinterpret_cast<float2*>(pt + lane * AT_PPITCH + warp * 2) = make_float2(pr[0], pr[1]);
+      }
+      __syncthreads();
+      const int first = group * 8;
+      if (first >= live) continue;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float2 a = *reinterpret_cast<const float2*>(alpha_s + first + r * 2);
+        if (a.x != 1.f || a.y != 1.f) {
+#pragma unroll
+          for (int i = 0; i < HC; ++i) {
+            const float2 v = at_unpack(acc[r][i]);
+            acc[r][i] = at_pack(v.x * a.x, v.y * a.y);
+          }
+        }
+      }
+      const int cnt = min(AA_KEYS, keys - k0);
+      const int all = max(0, min(cnt, vis_s[first] - k0));      // keys that all eight see
+#pragma unroll 4
+      for (int j = 0; j < all; ++j) {
+        const ulonglong2 pa = *reinterpret_cast<const ulonglong2*>(pt + j * AT_PPITCH + first);
+        const ulonglong2 pb = *reinterpret_cast<const ulonglong2*>(pt + j * AT_PPITCH + first + 4);
+#pragma unroll
+        for (int i = 0; i < HC; ++i) {
+          if (ch0 + i * 32 < ch1) {
+            const float v = ks[j * pitch + ch0 + i * 32];
+            const uint64_t vv = at_pack(v, v);
+            acc[0][i] = at_fma(pa.x, vv, acc[0][i]);
+            acc[1][i] = at_fma(pa.y, vv, acc[1][i]);
+            acc[2][i] = at_fma(pb.x, vv, acc[2][i]);
+            acc[3][i] = at_fma(pb.y, vv, acc[3][i]);
+          }
+        }
+      }
+      // what a query does not see is not multiplied by a weight of zero, it may be anything
+      if (all < cnt) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const int n = min(cnt, vis_s[first + r] - k0);
+          for (int j = all; j < n; ++j) {
+            const float pj = pt[j * AT_PPITCH + first + r];
+#pragma unroll
+            for (int i = 0; i < HC; ++i)
+              if (ch0 + i * 32 < ch1) {
+                float2 v = at_unpack(acc[r / 2][i]);
+                float& x = r % 2 ? v.y : v.x;
+                x = fmaf(pj, ks[j * pitch + ch0 + i * 32], x);
+                acc[r / 2][i] = at_pack(v.x, v.y);
+              }
+          }
+        }
+      }
+    }
+    if (lane < 2) {
+      const float s = lane == 0 ? l[0] : l[1];
+      inv_s[warp * 2 + lane] = s > 0.f ? 1.0f / s : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int j = group * 8 + r;
+      if (j >= live) break;
+      const float inv = inv_s[j];
+      T* o = static_cast<T*>(p.out) + (row0 + (q0 + j) / grp) * p.out_stride +
+             (kvh * grp + (q0 + j) % grp) * p.d;
+#pragma unroll
+      for (int i = 0; i < HC; ++i) {
+        const int c = ch0 + i * 32;
+        const float2 v = at_unpack(acc[r / 2][i]);
+        if (c < ch1) Elem<T>::store(o + c, (r % 2 ? v.y : v.x) * inv);
+      }
+    }
+  }
+}
+
+template <typename T, int CH>
+static int launch_attn_tile(const AnyAttnParams& p, cudaStream_t s) {
+  const int64_t queries = p.rows * (p.hq / p.hkv);
+  const int64_t blocks = (queries + AT_QUERIES - 1) / AT_QUERIES + p.num_seqs;
+  const int64_t cap = (int64_t)sm_count() * 32, want = blocks * p.hkv;
+  static PerDeviceOnce once;
+  FK_CUDA_OK(set_max_dynamic_smem(once, paged_attn_tile_kernel<T, CH>, AA_MAX_SMEM));
+  FK_CUDA_OK(launch_kernel(paged_attn_tile_kernel<T, CH>,
+                           dim3((unsigned)(want < cap ? want : cap)), dim3(AT_THREADS),
+                           (size_t)at_smem(p.d), s, p, blocks));
+  count_launch();
+  return FK_OK;
+}
 template <typename T, int CH, int R>
 static int launch_any_r(const AnyAttnParams& p, cudaStream_t s) {
   const int64_t queries = p.rows * (p.hq / p.hkv);
@@ -794,11 +1094,21 @@ static int launch_any_r(const AnyAttnParams& p, cudaStream_t s) {
 // KV head, a portion of 5 tokens on 300 keys 131 / 135 / 252 (196); 16 heads, 40 portions of 5
 // 342 / 203 / 232 (1143); one of 900 tokens 1633 / 1031 / 1306 (5827); 128 channels, 16 heads on 4,
 // 64 single tokens on 500 keys 142 / 141 / 145 (346); 64 channels, 16 KV heads, 40 portions of two
-// tokens 72 / 134 / 204 (156).
+// tokens 72 / 134 / 204 (156) - all before a run's rows came at once.
 template <typename T, int CH>
 static int launch_any_ch(const AnyAttnParams& p, cudaStream_t s) {
   const int64_t queries = p.rows * (p.hq / p.hkv);
   const int64_t ctas = ((queries + AA_WARPS - 1) / AA_WARPS) * p.hkv;
+  if constexpr (CH == 18) {
+    // Tiles where they are full enough and give the SMs enough to do (us, these / tiles): fp32, 576
+    // channels, 16 heads on one KV head, portions of 40, 120 and 333 tokens 288 / 176, 40 of 5 on 200
+    // keys 162 / 118, one of 20 on 700 233 / 331; 256 channels, 8 heads on 2, 900 tokens 440 / 332,
+    // 20 portions of 9 on 300 111 / 130.  Up to 128 channels the two are too close for a second form.
+    const int64_t tiles = queries / AT_QUERIES * p.hkv;
+    if (queries >= 2 * (int64_t)AT_QUERIES * p.num_seqs &&
+        tiles * p.d >= (int64_t)sm_count() * 288)
+      return launch_attn_tile<T, CH>(p, s);
+  }
   if (queries <= (int64_t)AA_WARPS * p.num_seqs || ctas <= sm_count())
     return launch_any_r<T, CH, 1>(p, s);
   return launch_any_r<T, CH, 2>(p, s);

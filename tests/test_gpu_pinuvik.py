@@ -380,6 +380,16 @@ def test_paged_attn_any_forms(d, hq, hkv, portions, dtype):
     assert not np.isfinite(got[cu[1:] - 1]).any()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d,hq,hkv,portions", [
+    (576, 40, 1, [(30, 45), (0, 17)]), (300, 48, 3, [(1, 64), (33, 33)]),
+    (132, 64, 8, [(0, 31), (32, 97), (20, 36)])])
+def test_paged_attn_any_of_many_queries(d, hq, hkv, portions, dtype):
+    """The same of enough queries for tiles of 32, whose rows end inside a tile and a run of
+    keys."""
+    test_paged_attn_any_forms(d, hq, hkv, portions, dtype)
+
+
 def test_embed_and_argmax_f32():
     from fastkernels_b200 import ops
     rs = np.random.RandomState(0)
