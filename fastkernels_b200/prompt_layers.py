@@ -8,7 +8,6 @@ between calls.
 """
 from __future__ import annotations
 
-import ctypes
 import struct
 
 import torch
@@ -213,8 +212,10 @@ class PromptRun:
         first = residual is None
         if first:
             hidden, residual = torch.empty_like(hidden), hidden
-        _lib.check(_lib.lib.fk_llama_prompt_layers(
-            ctypes.cast(struct.pack("15Q4d", *fields), ctypes.c_void_p), 1, int(first),
-            ctypes.cast(struct.pack("2Q", residual.data_ptr(), hidden.data_ptr()) + self.tail,
-                        ctypes.c_void_p), ops._stream()), "fk_llama_prompt_layers")
+        # objects that live until the call returns: it reads both structs between its launches, with
+        # the interpreter's lock released, and a pointer made of a temporary holds nothing
+        fields = struct.pack("15Q4d", *fields)
+        prompt = struct.pack("2Q", residual.data_ptr(), hidden.data_ptr()) + self.tail
+        _lib.check(_lib.lib.fk_llama_prompt_layers(fields, 1, int(first), prompt, ops._stream()),
+                   "fk_llama_prompt_layers")
         return hidden, residual
