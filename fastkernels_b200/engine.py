@@ -51,7 +51,10 @@ def _write_ids(out: np.ndarray, tokens) -> None:
             return
         except struct.error:             # not ints: as numpy converts them
             pass
-    out[:] = np.asarray(tokens, dtype=np.int64)
+    ids = np.asarray(tokens, dtype=np.int64)
+    if ids.shape != out.shape:
+        raise ValueError("token ids must be a list of numbers")
+    out[:] = ids
 
 
 class DecodeEngine:
@@ -352,14 +355,24 @@ class DecodeEngine:
         just written.  In a chunked span a portion falls into one segment per chunk."""
         counts = [len(t) for _, _, t in portions]
         total = sum(counts)
+        # before any page is taken: a list that is refused leaves the sequences as they were
+        ids, pos = np.empty(total, dtype=np.int64), np.empty(total, dtype=np.int64)
+        o = 0
+        for (_, a, t), n in zip(portions, counts):
+            _write_ids(ids[o:o + n], t)
+            pos[o:o + n] = np.arange(a, a + n)
+            o += n
+        wanted = np.array(rows, dtype=np.int64)
         # token ids, positions, wanted rows and all int32 metadata travel in one copy from
         # pinned memory
-        i32, sizes, layout = [], [2 * total, 2 * total, 2 * len(rows)], []
+        i32, sizes, layout = [], [], []
 
         def put(a):
             i32.append(a)
             sizes.append(a.size)
 
+        for a in (ids, pos, wanted):
+            put(a.view(np.int32))
         for blocks in self.span_blocks:
             segs, slots = [], []
             for (s, a, _), n in zip(portions, counts):
@@ -383,15 +396,7 @@ class DecodeEngine:
 
         flat = torch.empty(sum(sizes), dtype=torch.int32, pin_memory=self.device.type == "cuda")
         host = flat.numpy()
-        ids, pos = host[:2 * total].view(np.int64), host[2 * total:4 * total].view(np.int64)
-        o = 0
-        for (_, a, t), n in zip(portions, counts):
-            _write_ids(ids[o:o + n], t)
-            pos[o:o + n] = np.arange(a, a + n)
-            o += n
-        at = 4 * total
-        host[at:at + 2 * len(rows)].view(np.int64)[:] = rows
-        at += 2 * len(rows)
+        at = 0
         for a in i32:
             host[at:at + a.size] = a
             at += a.size

@@ -383,3 +383,55 @@ def test_a_prefill_that_does_not_fit_gives_everything_back(tmp_path, monkeypatch
         bm = BlockManager(n, 8, 0, chunk)
         for i, t in enumerate((50, 40)):
             bm.extend(Sequence(i, 0), 0, t)
+
+
+class _Fits:
+    """As long as it says, but nothing that becomes token ids."""
+
+    def __len__(self):
+        return 30
+
+    def __getitem__(self, i):
+        raise TypeError("no token ids")
+
+
+@pytest.mark.parametrize("bad", [["7"] * 29 + ["x"], [1.5] * 29 + [None], [1] * 29 + [1 << 70],
+                                 [[1, 2]] * 30, _Fits()])
+def test_refused_tokens_leave_the_sequences_as_they_were(bad, tmp_path, monkeypatch):
+    """A portion that would cross a chunk's end, whose ids cannot be converted: no page is taken or
+    given back, and the next portion goes on where the sequence was."""
+    small(tmp_path)
+    config, source = registry.load_folder(tmp_path, torch.float32)
+    config.kv_block_size = 8
+    eng = DecodeEngine(config, max_num_seqs=3, max_model_len=200, num_kv_blocks=40, device="cpu",
+                       init_scale=None)
+    eng.load_weights(source)
+    seen = []
+
+    def forward(self, ids, pos):
+        from fastkernels_b200.infra.context import get_context
+        seen.append((ids.tolist(), pos.tolist(), [
+            [t.tolist() for t in (s.slot_mapping, s.block_tables, s.cu_seqlens_q)]
+            for s in get_context().spans]))
+        return torch.zeros(len(ids), self.stride)
+    monkeypatch.setattr(type(eng.model), "forward", forward)
+    monkeypatch.setattr(type(eng.model), "project", lambda self, h: torch.zeros(h.shape[0], 51))
+    a, b = eng.open_sequence(), eng.open_sequence()
+    eng.feed([(a, list(range(20))), (b, [3, 4])])
+
+    def state():
+        return [(s.num_tokens, {k: list(v) for k, v in s.tables.items()}, dict(s.bases))
+                for s in (a, b)], [(list(g.free), list(g._retired)) for g in eng.span_blocks]
+    before = state()
+    with pytest.raises((TypeError, ValueError, OverflowError)):
+        eng.feed([(b, [5, 6]), (a, bad)])
+    with pytest.raises(ValueError):
+        eng.feed([(eng.open_sequence(), [[5]])])
+    assert state() == before and len(seen) == 1
+    eng.feed([(b, [5, 6]), (a, [9] * 30)])
+    ids, pos, spans = seen[1]
+    assert ids == [5, 6] + [9] * 30 and pos == [2, 3, *range(20, 50)]
+    # chunk of 24: the four tokens of a that are left of it go to pages it began with
+    slots, tables, cu = spans[0]
+    assert cu[:3] == [0, 2, 6] and tables[1][:3] == before[0][0][1][0]
+    assert slots[2:6] == [tables[1][2] * 8 + i for i in range(4, 8)]
