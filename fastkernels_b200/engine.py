@@ -255,6 +255,9 @@ class DecodeEngine:
         # and the ids that the step before has left there
         self._ahead = None
         self._staged_ahead = None
+        # the event behind the copies that _prepare_ahead has queued last, and their stream:
+        # step() returns without waiting for them
+        self._staging = None
         self._sampled: list[int] = []
         self._seq_epoch = 0
         self.host, self.host_np = self._ring[0], self._ring_np[0]
@@ -603,7 +606,21 @@ class DecodeEngine:
             bs = self.graph_batch_size(n)
             self.stage_inputs(n, bs, False)
             self._mark_slot_in_flight()
-            self._staged_ahead = bs, ops.current_stream()
+            stream = ops.current_stream()
+            if self._staging is None or self._staging[1] != stream:
+                # an engine that goes away keeps these until the copies have landed
+                for t in (self._packed_dev, *self.graph_vars["span_tables"]):
+                    t.record_stream(torch.cuda.current_stream())
+            self._staged_ahead = bs, stream
+            self._staging = self._ring_events[self._ring_pos], stream
+
+    def _after_staging(self) -> None:
+        """What the current stream does from here on comes after the copies that were staged
+        ahead: on their own stream it does anyway.  (A capture begins with the device idle, and
+        may not wait for what was queued before it.)"""
+        if self._staging is not None and self._staging[1] != ops.current_stream() and \
+                not torch.cuda.is_current_stream_capturing():
+            torch.cuda.current_stream().wait_event(self._staging[0])
 
     def _prepare_layout(self, seqs=None) -> int:
         seqs = self.seqs if seqs is None else seqs
@@ -648,6 +665,7 @@ class DecodeEngine:
         """H2D copies from pinned memory into the graph's input buffers; padded
         rows get slot -1 / context_len 0 (engine.py:5404-5406)."""
         gv, h, hn = self.graph_vars, self.host, self.host_np
+        self._after_staging()
         if bs > n:
             for slots, lens in zip(hn["span_slots"], hn["span_lens"]):
                 slots[n:bs] = -1
@@ -697,6 +715,7 @@ class DecodeEngine:
         inputs; max_context_len is max_model_len at capture (engine.py:6832-6836)
         and the real lengths are read on the device at replay."""
         gv = self.graph_vars
+        self._after_staging()
         inputs = [self._packed_dev, *gv["span_tables"]]
         saved = [t.clone() for t in inputs]
         for slots, lens, tables in zip(gv["span_slots"], gv["span_lens"], gv["span_tables"]):
@@ -729,6 +748,7 @@ class DecodeEngine:
         """Replay (or eagerly run) the step for batch size `bs` on inputs that
         are already in the graph buffers."""
         self._staged_ahead = None       # the step leaves its own tokens on the device
+        self._after_staging()
         g = self.graphs.get(bs)
         if g is not None and not self.enforce_eager:
             g.replay()

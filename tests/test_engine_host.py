@@ -165,3 +165,129 @@ def test_prefill_chunk_packing_covers_every_token_once():
         assert all(s_ == list(range(n)) for s_, n in zip(seen, lens))
         if budget is None:
             assert rounds == 1
+
+
+class _Device:
+    """Streams and events by name: what has been queued where, and what comes after what."""
+
+    def __init__(self):
+        self.at, self.clock, self.known = "a", {}, {}
+
+    def tick(self, what):
+        """Something is queued on the current stream."""
+        self.clock[self.at] = self.clock.get(self.at, 0) + 1
+        what(self.at, self.clock[self.at])
+
+    def seen(self, stream):
+        """How far into each stream the current end of `stream` is certain to come after."""
+        return dict(self.known.get(stream, {}), **{stream: self.clock.get(stream, 0)})
+
+    def join(self, stream, upto):
+        mine = self.known.setdefault(stream, {})
+        for s, n in upto.items():
+            mine[s] = max(mine.get(s, 0), n)
+
+
+@pytest.mark.parametrize("between", ["nothing", "finish", "open", "portion", "single", "capture",
+                                     "replace", "direct"])
+def test_staged_copies_come_before_what_other_streams_do(between, monkeypatch):
+    """step() returns while the next step's inputs are on their way on its stream.  Whatever the
+    engine does next on another stream, with the same sequences or others, at a page's end, waits
+    for them before it writes or reads the same buffers."""
+    dev = _Device()
+
+    class Event:
+        def record(self):
+            self.upto = dev.seen(dev.at)
+
+        def synchronize(self):
+            for s in "ab":
+                dev.join(s, self.upto)
+
+    class Stream:
+        def wait_event(self, ev):
+            dev.join(dev.at, ev.upto)
+
+        def synchronize(self):
+            for s in "ab":
+                dev.join(s, dev.seen(dev.at))
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "current_stream", Stream)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda: None)
+    monkeypatch.setattr("fastkernels_b200.ops.current_stream", lambda: "ab".index(dev.at))
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda *a: None)
+    eng = DecodeEngine(tiny_cfg(64), max_num_seqs=3, max_model_len=256, num_kv_blocks=16,
+                       device="cpu")
+    last, late, kept = {}, [], []
+
+    def touch(stream, n):
+        for s, m in last.items():
+            if s != stream and dev.known.get(stream, {}).get(s, 0) < m:
+                late.append((s, stream))
+        last[stream] = n
+
+    class Staged:
+        """_packed_dev: copies into it are what is queued."""
+
+        def __getitem__(self, i):
+            return self
+
+        def copy_(self, *a, **k):
+            dev.tick(touch)
+
+        def clone(self):
+            dev.tick(touch)
+            return self
+
+        def record_stream(self, stream):
+            kept.append(dev.at)
+    eng._packed_dev = Staged()
+    run, tables = eng.run_step_device, eng.graph_vars["span_tables"][0]
+
+    def step(bs):
+        monkeypatch.setattr(eng, "_forward", lambda bs: dev.tick(touch))
+        run(bs)
+    monkeypatch.setattr(eng, "run_step_device", step)
+    monkeypatch.setattr(eng.model, "forward", lambda *a: torch.zeros(len(a[0]), 128))
+    monkeypatch.setattr(eng.model, "project", lambda h: torch.zeros(h.shape[0], 256))
+    eng.add_sequences([63, 20], [1, 2])
+    # host buffers and status words stay on the CPU
+    monkeypatch.setattr(eng, "device", type("Cuda", (), {"type": "cuda"})())
+    monkeypatch.setattr(eng, "_copy_status", lambda: None)
+    portion = eng._forward_portions
+
+    def on_host(*a, **k):
+        with monkeypatch.context() as m:
+            m.setattr(eng, "device", torch.device("cpu"))
+            return portion(*a, **k)
+    monkeypatch.setattr(eng, "_forward_portions", on_host)
+    for i in range(3):                          # 64 tokens, then 65: the tables change
+        eng.step()
+    assert eng._staged_ahead is not None and kept == ["a"]
+    dev.at = "b"
+    if between == "finish":
+        eng.finish(eng.seqs[0])
+    elif between in ("open", "portion", "single"):
+        s = eng.open_sequence()
+        eng.feed([(s, [1, 2, 3])])
+        if between == "single":
+            eng.feed([(s, [4])])
+        if between != "open":
+            eng.finish(s)
+        else:
+            s.num_tokens += 1
+    elif between == "replace":
+        eng.seqs[0].last_token = 9
+    elif between == "direct":
+        bs = eng.prepare_decode(True)
+        eng.stage_inputs(bs, bs, True)
+        eng.run_step_device(bs)
+    elif between == "capture":
+        eng.capture_cudagraph([])
+    eng.step()
+    eng.step(sync=False)
+    dev.at = "a"
+    Stream().synchronize()
+    assert not late and set(last) == {"a", "b"}
+    assert tables[0, :1].tolist() == eng.seqs[0].block_table[:1]
