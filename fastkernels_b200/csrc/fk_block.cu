@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) decode_block_kernel(
   uint64_t* acc_empty = acc_full + 2;          // [2] epilogue -> MMA
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* stop = abort_flag + 1;         // row phases: the epilogue leaves
   float* red = reinterpret_cast<float*>(smem + Cfg::kRed);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -341,17 +342,17 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) decode_block_kernel(
     const int t128 = threadIdx.x - 64;
     int seg = 0, out_it = 0;
     uint16_t* out_stage = reinterpret_cast<uint16_t*>(smem + Cfg::kOut);
-    bool ok = true;
-    for (int pi = 0; pi < p.num_phases && ok; ++pi) {
+    for (int pi = 0; pi < p.num_phases; ++pi) {
       const BlkPhase& ph = p.ph[pi];
       if (ph.kind == PH_ADD_RMSNORM || ph.kind == PH_ROPE_STORE) {
         // needs everything the earlier phases of every CTA wrote
-        int pass = 1;
-        if (pi > 0 && t128 == 0)
-          pass = blk_wait_phases(counters + pi - 1, G, abort_flag, p.status) ? 1 : 0;
+        // one thread decides for all, who have read the last decision by the barriers between
+        if (t128 == 0)
+          *stop = (pi > 0 && !blk_wait_phases(counters + pi - 1, G, abort_flag, p.status)) ||
+                  *abort_flag;
         named_bar_sync(1, 128);
         if (t128 == 0) BLK_TRACE(pi, 3);
-        if (*abort_flag || !pass) { ok = false; break; }
+        if (*stop) break;
         if (ph.kind == PH_ADD_RMSNORM) {
           for (int row = cta; row < p.m; row += G) {
             if (ph.cols_vec <= 128) blk_norm_row<1>(ph, row, t128, red);
@@ -379,7 +380,7 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) decode_block_kernel(
         const long long u0 = cta < Gp ? unit_begin(cta, units, Gp) : 0;
         const long long u1 = cta < Gp ? unit_begin(cta + 1, units, Gp) : 0;
         long long u = u0;
-        while (u < u1 && ok) {
+        while (u < u1) {
           const int tile = (int)(u / ph.kb_total);
           const long long tile_begin = (long long)tile * ph.kb_total;
           const long long tile_end = tile_begin + ph.kb_total;
@@ -417,10 +418,10 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) decode_block_kernel(
                 pre[j] = __ldcg(src + (size_t)j * GEMM_BN);
             }
           }
-          if (!gemm_wait(&acc_full[buf], (seg >> 1) & 1, abort_flag, p.status)) {
-            ok = false;
-            break;
-          }
+          // Where it ran out no thread leaves by itself, the others would stay at the barriers
+          // below: they go on with what is there and announce nothing (as fk_gemm.cu).
+          (void)gemm_wait(&acc_full[buf], (seg >> 1) & 1, abort_flag, p.status);
+          __syncwarp();
           tc_fence_after();
           const uint32_t taddr =
               tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * Cfg::kAccCols);
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) decode_block_kernel(
             }
             __threadfence();
             named_bar_sync(1, 128);
-            if (t128 == 0) st_release_gpu(p.flags + cta, pi + 1);
+            if (t128 == 0 && !*abort_flag) st_release_gpu(p.flags + cta, pi + 1);
           } else {
             const float bias = (ph.bias && n < ph.n) ? bf16_bits_to_float(ph.bias[n]) : 0.f;
             const int n0 = SILU ? tile * 64 : tile * GEMM_BN;
@@ -530,10 +531,9 @@ __global__ void __launch_bounds__(BLK_THREADS, 1) decode_block_kernel(
           ++seg;
         }
       }
-      if (!ok) break;
       // this CTA's share of the phase is written: tell the grid
       named_bar_sync(1, 128);
-      if (t128 == 0) {
+      if (t128 == 0 && !*abort_flag) {
         BLK_TRACE(pi, 4);
         __threadfence();
         const int old = atomicAdd(counters + pi, 1);

@@ -314,8 +314,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(
     int seg = 0, out_it = 0;
     uint16_t* out_stage = reinterpret_cast<uint16_t*>(smem + Cfg::kOut);
     long long u = u0;
-    bool ok = true;
-    while (u < u1 && ok) {
+    while (u < u1) {
       const int tile = (int)(u / p.kb_total);
       const long long tile_begin = (long long)tile * p.kb_total;
       const long long tile_end = tile_begin + p.kb_total;
@@ -358,10 +357,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(
           for (int j = 0; j < (PRE ? MPAD : 1); ++j) pre[j] = __ldcg(src + (size_t)j * GEMM_BN);
         }
       }
-      if (!gemm_wait(&acc_full[buf], (seg >> 1) & 1, abort_flag, p.status)) {
-        ok = false;
-        break;
-      }
+      // Where it ran out no thread leaves: one that did would leave the others at the barriers
+      // below for good, and a barrier to agree on it would cost every segment.  They go on with
+      // what is there, fail their next waits at once, and the status says that nothing is valid;
+      // neither a partial tile nor a row for another rank is announced.
+      (void)gemm_wait(&acc_full[buf], (seg >> 1) & 1, abort_flag, p.status);
+      __syncwarp();
       tc_fence_after();
       if (threadIdx.x == 64) FK_TRACE(5);     // accumulator of the segment complete
       const uint32_t taddr =
@@ -414,7 +415,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(
         }
         __threadfence();
         named_bar_sync(1, 128);
-        if (threadIdx.x == 64) st_release_gpu(p.flags + cta, 1);
+        if (threadIdx.x == 64 && !*abort_flag) st_release_gpu(p.flags + cta, 1);
       } else {
         const float bias = (p.bias && n < p.n) ? bf16_bits_to_float(p.bias[n]) : 0.f;  // p.n = all W rows
         // first output column of the tile and how many it has
@@ -491,7 +492,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_bf16_kernel(
                 uint16_t* yrow = p.y + (int64_t)(c + r) * p.y_stride + n0 + ch * 8;
                 const uint16_t* srow = st + r * GEMM_BN + ch * 8;
                 if (p.push.nranks > 0) {
-                  if (n0 + ch * 8 < p.n) {       // n % 8 == 0: the eight columns exist
+                  if (n0 + ch * 8 < p.n && !*abort_flag) {   // n % 8 == 0: eight columns exist
                     const uint4 o = *reinterpret_cast<const uint4*>(srow);
                     const uint32_t call = p.push.epoch[c + r] + 1;
                     push_out4(p, c + r, n0 + ch * 8, o.x, o.y, call);

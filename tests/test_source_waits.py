@@ -1,0 +1,47 @@
+"""Read from the kernels' source: how threads that share barriers leave when a wait runs out."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "fastkernels_b200" / "csrc"
+
+
+def _branch(text, start):
+    """The text of the braces that open after `start`."""
+    i = text.index("{", start)
+    depth, j = 0, i
+    while True:
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        j += 1
+        if depth == 0:
+            return text[i:j]
+
+
+def _code(name):
+    return re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+
+
+@pytest.mark.parametrize("name,mark", [("fk_gemm.cu", "} else if (warp >= 2) {"),
+                                       ("fk_block.cu", "    const int t128 = threadIdx.x - 64;")])
+def test_epilogue_threads_of_few_row_products_leave_together(name, mark):
+    """128 threads meet at named barriers, and each waits for the accumulators by itself: one that
+    left alone when its wait ran out would leave the others there without end.  So no thread's own
+    wait, nor what it reads of the abort flag, decides about a loop or a barrier."""
+    text = _code(name)
+    start = text.index(mark) if mark.startswith("}") else text.rindex("{", 0, text.index(mark))
+    body = _branch(text, start)
+    assert "named_bar_sync(1, 128)" in body
+    assert len(re.findall(r"\(void\)gemm_wait\(&acc_full", body)) == 1
+    assert "gemm_wait(" not in body.replace("(void)gemm_wait(&acc_full", "")
+    # who leaves, and by what: a chunk that is not there, one thread's wait for flags, and a
+    # decision that one thread wrote ahead of a barrier
+    leaves = re.findall(r"([^;{}]*)\b(?:break|return)\b", body)
+    allowed = {"if (c >= p.m)", "if (*stop)"} | \
+        {x for x in leaves if "atomicOr(p.status" in x}
+    assert {x.strip() for x in leaves if x.strip()} <= allowed
+    for cond in re.findall(r"(?:while|for) \(([^{}]*)\) \{", body):
+        assert "ok" not in re.findall(r"\w+", cond)
+    for m in re.finditer(r"if \(([^{};]*abort_flag[^{};]*)\)\s*(\{)?", body):
+        after = _branch(body, m.end() - 1) if m.group(2) else body[m.end():body.index(";", m.end())]
+        assert "bar_sync" not in after
