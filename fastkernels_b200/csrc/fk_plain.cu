@@ -9,6 +9,8 @@
 #include "fk_gemm_shared.cuh"
 #include "fk_types.cuh"
 
+#include <mutex>
+
 namespace fk {
 
 // ------------------------------------------------------------------- fp32 products
@@ -43,6 +45,12 @@ struct F32Tile {
   static constexpr int kTeams = 2, kTeam = 8, kWarps = kTeams * kTeam, kAdders = 4;
   static constexpr int kIssuer = kWarps + kAdders;
   static constexpr int kThreads = 32 * (kIssuer + 4);
+  // registers a thread of the three (setmaxnreg); what the warpgroup that adds up takes must come
+  // from what the CTA was launched with: the host refuses a build that has fewer
+  static constexpr int kRegsTeam = 72, kRegsAdder = 152, kRegsIssuer = 40;
+  static constexpr int kRegsNeeded =
+      32 * (kWarps * kRegsTeam + kAdders * kRegsAdder + 4 * kRegsIssuer);
+  static_assert(kRegsNeeded <= 80 * kThreads, "register split exceeds the CTA's pool");
   static constexpr int kPlane = kRows * kBK * 2;       // one part of the rows of x
   static constexpr int kStageBytes = 3 * kPlane;
   // tensor memory: two blocks' sums, then the weights' parts, two numbers a cell
@@ -218,9 +226,8 @@ __global__ void __launch_bounds__(F32Tile::kThreads, 1)
     return __all_sync(0xffffffffu, ok) != 0;
   };
   float* const out = reinterpret_cast<float*>(smem);
-  // registers: 768 threads x 80 = 512 x 72 + 128 x 152 + 128 x 40
   if (warp >= Tile::kIssuer) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Tile::kRegsIssuer));
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(width >> 3) << 17) |
                            ((uint32_t)(Tile::kCols >> 4) << 24);
     // the products of a block, smallest first, when all of its parts are laid out and the sums
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(F32Tile::kThreads, 1)
   }
   if (warp >= Tile::kWarps) {
     // a lane has one weight row and all rows of x
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Tile::kRegsAdder));
     const int q = warp & 3;
     float2 acc[Tile::kRows / 2];
 #pragma unroll
@@ -289,7 +296,7 @@ __global__ void __launch_bounds__(F32Tile::kThreads, 1)
     cluster_sync();
     return;
   }
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Tile::kRegsTeam));
   if (there) {
     const int team = warp / Tile::kTeam, half = warp >> 2 & 1;
     // weights: 16-byte pieces lane & 3 and 4 further of rows w0 and w0 + 8, as tc_st_16x256 wants
@@ -513,6 +520,19 @@ static int launch_f32_tile(const F32Product& p, cudaStream_t s) {
   const int parts = f32_parts(p);
   FK_REQUIRE(n_tiles * row_tiles * parts <= 0x7fffffff, FK_ERR_UNSUPPORTED,
              "fp32 product: too many tiles");
+  // registers a thread of the compiled kernel: the same on every device
+  static std::once_flag regs_once;
+  static cudaError_t regs_err = cudaSuccess;
+  static int launch_regs = 0;
+  std::call_once(regs_once, [] {
+    cudaFuncAttributes f;
+    regs_err = cudaFuncGetAttributes(&f, f32_product_kernel<ACT>);
+    if (regs_err == cudaSuccess) launch_regs = f.numRegs;
+  });
+  FK_CUDA_OK(regs_err);
+  FK_REQUIRE(launch_regs * Tile::kThreads >= Tile::kRegsNeeded, FK_ERR_UNSUPPORTED,
+             "fp32 product: this build of the kernel holds %d registers per thread, fewer than its "
+             "register split needs", launch_regs);
   static PerDeviceOnce once;
   FK_CUDA_OK(set_max_dynamic_smem(once, f32_product_kernel<ACT>, Tile::kSmem));
   cudaLaunchConfig_t cfg{};

@@ -45,3 +45,19 @@ def test_epilogue_threads_of_few_row_products_leave_together(name, mark):
     for m in re.finditer(r"if \(([^{};]*abort_flag[^{};]*)\)\s*(\{)?", body):
         after = _branch(body, m.end() - 1) if m.group(2) else body[m.end():body.index(";", m.end())]
         assert "bar_sync" not in after
+
+
+def test_register_splits_are_checked_before_the_launch():
+    """setmaxnreg.inc waits without end where a CTA was launched with fewer registers than its
+    split adds up to.  Each kernel that has it names its split, and its launch asks the compiled
+    kernel for its registers and refuses."""
+    have = [f.name for f in sorted(CSRC.glob("*.cu*")) if "setmaxnreg.inc" in _code(f.name)]
+    assert have == ["fk_plain.cu", "fk_prefill.cu"]
+    for name in have:
+        text = _code(name)
+        # no number in the instruction itself
+        assert re.findall(r'setmaxnreg\.(?:inc|dec)\.sync\.aligned\.u32 ([^;]*);', text) == ["%0"] * \
+            len(re.findall("setmaxnreg", text))
+        needed = re.search(r"(\w*REGS_?NEEDED) =", text, re.I).group(1)
+        assert re.search(r"FK_REQUIRE\(launch_regs \* [\w:]+ >= (?:Tile::)?%s," % needed, text)
+        assert "cudaFuncGetAttributes(&f, " in text and "f.numRegs" in text
