@@ -20,8 +20,10 @@ namespace fk {
 // exact in fp32, and sums are kept in fp32: 32 k's in tensor memory (whose adder cuts off instead
 // of rounding, so chains there are kept short), smallest parts first, and the blocks of 32 in
 // registers, rounded to nearest.  Off from 64 bits by 1.2 to 1.9e-7 (2-norm; k 2048 to 12288,
-// normal operands), where chains of fp32 multiply-adds are by 2.1 to 5.0e-7.  Numbers below 2^-110
-// are kept to 2^-134, which is as far as bf16 goes.
+// normal operands), where chains of fp32 multiply-adds are by 2.1 to 5.0e-7.  bf16 goes down to
+// 2^-133 and fp32 to 2^-149, so both operands are taken apart times 2^16, and the sums multiplied by
+// 2^-32 when all are added up: exact, and every fp32 number keeps all of its bits (operands of 1e-36
+// as they are were off by 2.6e-5).  It takes 1 to 2 % of the time.
 //
 // A CTA computes 128 weight rows (the M operand) x up to 128 rows of x.  Two teams of eight warps
 // take every other block of k each: they read it ahead, take the numbers apart, and lay the parts
@@ -30,13 +32,15 @@ namespace fk {
 // a block (waits, conversions, loads) follow one another in a warp: sixteen warps on one block go
 // through them in step and take 1800 cycles for it, the teams 1350, the tensor cores alone 770.
 //
-// us, 1 / 100 / 1000 rows (fp32 multiply-adds in register tiles): 24576 x 4096 135 184 1270 (217 644
-// 4542), 2048 x 2048 14 23 96 (36 60 243), 4096 x 12288 68 89 683 (267 317 2540): 160 TFLOP/s.
+// us, 1 / 100 / 1000 rows (fp32 multiply-adds in register tiles), calls apart: 24576 x 4096 136 186
+// 1295 (217 644 4542), 155 TFLOP/s at 1000 rows; 2048 x 2048 14 23 98 (36 60 243); 4096 x 12288 69
+// 90 700 (267 317 2540).  Back to back the power limit has 24576 x 4096, 1000 rows at 1455.
 //
 // A cluster of CTAs shares one tile: each takes a part of k, leaves its sums in its shared
 // memory, and adds up its share of the rows over all parts in their order (f32_parts).  Where a
 // sum is not finite, an operand may not have been either (the parts of an infinity are no
-// numbers), or one too large for bf16: that output is computed again from the operands.
+// numbers), or operands or products may have been too large (from 2^111 and 2^95 on): that output is
+// computed again from the operands, in 64 bits.
 struct F32Tile {
   static constexpr int kRows = 128, kCols = 128;       // rows of x, weight rows
   static constexpr int kBK = 32, kStages = 4, kSums = 2;
@@ -56,6 +60,7 @@ struct F32Tile {
   // tensor memory: two blocks' sums, then the weights' parts, two numbers a cell
   static constexpr int kSumCols = kSums * kRows, kPartCols = kBK / 2, kTmemCols = 512;
   static constexpr int kOutPitch = kCols + 8;
+  static constexpr float kScale = 65536.f;   // of either operand
   static constexpr int kSmem = 128 * 1024;
   static_assert(kSumCols + kStages * 3 * kPartCols <= kTmemCols, "tensor memory");
   static_assert(kStages * kStageBytes + 1024 <= kSmem && kRows * kOutPitch * 4 + 1024 <= kSmem,
@@ -82,6 +87,13 @@ __device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
       : "=f"(c.x), "=f"(c.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return c;
 }
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float b) {
+  float2 c;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\t"
+      "mul.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(c.x), "=f"(c.y) : "f"(a.x), "f"(a.y), "f"(b));
+  return c;
+}
 // One part of two numbers, and what is left of them
 __device__ __forceinline__ uint32_t f32_part(float2& a) {
   const uint32_t p = pack_bf16(a.x, a.y);
@@ -96,18 +108,18 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, int rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
 }
-// One output from the operands
+// One output from the operands, in 64 bits
 __device__ __noinline__ float f32_dot(const float* x, const float* w, int k) {
-  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  double s[2] = {0., 0.};
   for (int i = 0; i < k; i += 4) {
     const float4 a = *reinterpret_cast<const float4*>(x + i);
     const float4 b = *reinterpret_cast<const float4*>(w + i);
-    s[0] = fmaf(a.x, b.x, s[0]);
-    s[1] = fmaf(a.y, b.y, s[1]);
-    s[2] = fmaf(a.z, b.z, s[2]);
-    s[3] = fmaf(a.w, b.w, s[3]);
+    s[0] = fma((double)a.x, (double)b.x, s[0]);
+    s[1] = fma((double)a.y, (double)b.y, s[1]);
+    s[0] = fma((double)a.z, (double)b.z, s[0]);
+    s[1] = fma((double)a.w, (double)b.w, s[1]);
   }
-  return (s[0] + s[1]) + (s[2] + s[3]);
+  return (float)(s[0] + s[1]);
 }
 
 // Row tile `t` of a product with row groups: its group and first row (of the group).
@@ -331,8 +343,10 @@ __global__ void __launch_bounds__(F32Tile::kThreads, 1)
       const uint32_t wto = wdst + stage * 3 * Tile::kPartCols;
 #pragma unroll
       for (int i = 0; i < 4; i += 2) {
-        float2 lo0 = make_float2(wv[i].x, wv[i].y), hi0 = make_float2(wv[i].z, wv[i].w);
-        float2 lo1 = make_float2(wv[i + 1].x, wv[i + 1].y), hi1 = make_float2(wv[i + 1].z, wv[i + 1].w);
+        float2 lo0 = mul_f32x2(make_float2(wv[i].x, wv[i].y), Tile::kScale);
+        float2 hi0 = mul_f32x2(make_float2(wv[i].z, wv[i].w), Tile::kScale);
+        float2 lo1 = mul_f32x2(make_float2(wv[i + 1].x, wv[i + 1].y), Tile::kScale);
+        float2 hi1 = mul_f32x2(make_float2(wv[i + 1].z, wv[i + 1].w), Tile::kScale);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           const uint2 a = make_uint2(f32_part(lo0), f32_part(hi0));
@@ -344,7 +358,8 @@ __global__ void __launch_bounds__(F32Tile::kThreads, 1)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         if (r + 32 * i >= width) continue;
-        float2 lo = make_float2(xv[i].x, xv[i].y), hi = make_float2(xv[i].z, xv[i].w);
+        float2 lo = mul_f32x2(make_float2(xv[i].x, xv[i].y), Tile::kScale);
+        float2 hi = mul_f32x2(make_float2(xv[i].z, xv[i].w), Tile::kScale);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           const uint32_t pl = f32_part(lo), ph = f32_part(hi);
@@ -366,8 +381,9 @@ __global__ void __launch_bounds__(F32Tile::kThreads, 1)
     const uint32_t addr = smem_u32(out + r * Tile::kOutPitch + c);
     float v = ld_cluster_f32(addr, 0);
     for (int q = 1; q < parts; ++q) v += ld_cluster_f32(addr, q);
-    if (!(fabsf(v) <= 3.402823466e38f)) v = f32_dot(f32_rows[Tile::kCols + r], f32_rows[c], p.k);
-    return v;
+    if (!(fabsf(v) <= 3.402823466e38f))
+      return f32_dot(f32_rows[Tile::kCols + r], f32_rows[c], p.k);
+    return v * (1.f / (Tile::kScale * Tile::kScale));
   };
   for (int i = r0 * kOut + tid; i < r1 * kOut; i += 32 * Tile::kWarps) {
     const int r = i / kOut, c = i % kOut;
