@@ -136,6 +136,9 @@ PROTOTYPES = {
     "fk_gemm_f32": (_i32, [_vp, _i64, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp]),
     "fk_paged_attn_any": (_i32, [_vp, _i64, _vp, _i64, _vp, _vp, _i32, _i64, _i32, _vp, _vp, _vp,
                                  _i64, _i32, _i64, _i32, _i32, _i32, _f32, _vp, _vp]),
+    "fk_paged_attn_any_of": (_i32, [_vp, _i64, _vp, _i64, _vp, _vp, _i32, _i64, _i32, _vp, _vp,
+                                    _vp, _i64, _i32, _i64, _i32, _i32, _i32, _f32, _i64, _i64,
+                                    _vp, _vp]),
     "fk_paged_decode_attn_2p": (_i32, [_i32, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _i32, _i64,
                                        _i32, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _f32, _i32,
                                        _vp, _sz, _vp, _vp]),

@@ -591,6 +591,7 @@ struct AnyAttnParams {
   const int32_t* block_tables; int64_t bt_stride;
   int num_seqs, hq, hkv, d, block_size, num_blocks;
   int64_t rows;
+  int64_t least, below;             // sequences of least .. below - 1 queries a KV head are taken
   float scale;
   int32_t* status;
 };
@@ -622,7 +623,8 @@ __device__ __forceinline__ int aa_find(const AnyAttnParams& p, int grp, int64_t&
       a = a < 0 ? 0 : a;
       b = b > p.rows ? p.rows : b;
     }
-    const int64_t mine = b > a ? ((b - a) * grp + QB - 1) / QB : 0;
+    const int64_t n = (b - a) * grp;
+    const int64_t mine = n > 0 && n >= p.least && n < p.below ? (n + QB - 1) / QB : 0;
     int64_t upto = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1096,10 +1098,15 @@ paged_attn_tile_kernel(const AnyAttnParams p, int64_t blocks) {
   }
 }
 
+// Blocks of qb queries at most, over all sequences of a launch
+static int64_t any_blocks(const AnyAttnParams& p, int qb) {
+  const int64_t queries = p.rows * (p.hq / p.hkv), most = (p.below - 1 + qb - 1) / qb;
+  const int64_t all = (queries + qb - 1) / qb + p.num_seqs;
+  return most < all / p.num_seqs ? most * p.num_seqs : all;
+}
 template <typename T, int CH>
 static int launch_attn_tile(const AnyAttnParams& p, cudaStream_t s) {
-  const int64_t queries = p.rows * (p.hq / p.hkv);
-  const int64_t blocks = (queries + AT_QUERIES - 1) / AT_QUERIES + p.num_seqs;
+  const int64_t blocks = any_blocks(p, AT_QUERIES);
   const int64_t cap = (int64_t)sm_count() * 32, want = blocks * p.hkv;
   static PerDeviceOnce once;
   FK_CUDA_OK(set_max_dynamic_smem(once, paged_attn_tile_kernel<T, CH>, AA_MAX_SMEM));
@@ -1111,8 +1118,7 @@ static int launch_attn_tile(const AnyAttnParams& p, cudaStream_t s) {
 }
 template <typename T, int CH, int R>
 static int launch_any_r(const AnyAttnParams& p, cudaStream_t s) {
-  const int64_t queries = p.rows * (p.hq / p.hkv);
-  const int64_t blocks = (queries + AA_WARPS * R - 1) / (AA_WARPS * R) + p.num_seqs;
+  const int64_t blocks = any_blocks(p, AA_WARPS * R);
   const int64_t cap = (int64_t)sm_count() * 32, want = blocks * p.hkv;
   const size_t smem = ((size_t)AA_WARPS * R * p.d + AA_KEYS * aa_pitch(p.d)) * sizeof(float);
   static PerDeviceOnce once;
@@ -1123,37 +1129,49 @@ static int launch_any_r(const AnyAttnParams& p, cudaStream_t s) {
   count_launch();
   return FK_OK;
 }
-// Queries per warp: one while all CTAs are in the first round (or there are no more than eight
-// queries to share a run of keys), then two, which halve the CTAs for 5 to 10 % more time each.
-// Four, in keys of 576 channels, leave one CTA an SM and were behind at every size.  us, one / two /
-// four a warp (and a warp per query that reads its keys from L2): fp32, 576 channels, 4 heads on one
-// KV head, a portion of 5 tokens on 300 keys 131 / 135 / 252 (196); 16 heads, 40 portions of 5
-// 342 / 203 / 232 (1143); one of 900 tokens 1633 / 1031 / 1306 (5827); 128 channels, 16 heads on 4,
-// 64 single tokens on 500 keys 142 / 141 / 145 (346); 64 channels, 16 KV heads, 40 portions of two
-// tokens 72 / 134 / 204 (156) - all before a run's rows came at once.
+// Tiles or warps is chosen for each sequence by its own portion, so that a row comes out with the
+// same bits whatever else is in the batch: tiles from 512 rows x query heads on, and two full ones a KV
+// head, beyond 128 channels (up to there the two are too close for a second form).  Alone that is
+// where they meet on short contexts; on long ones the warps, which spread over more SMs, stay ahead
+// to three times as much, and in a batch the tiles are ahead from the first full one.  us, warps /
+// tiles: fp32, 576 channels, 16 heads on one KV head, one portion of 32 tokens 22 / 22, 64 36 / 36, 128
+// 73 / 64, 333 228 / 161; of 32 behind 300 keys 109 / 157, 128 214 / 200, 333 505 / 326; portions of
+// 40, 120 and 333 271 / 160, 8 of 60 97 / 55, 16 of 20 62 / 34; 256 channels, 8 heads on 2, one of 64
+// tokens 22 / 26, 192 69 / 63, 900 436 / 267, 8 of 60 39 / 25; 192 channels, 16 KV heads, one of 32
+// 15 / 16, 96 40 / 33, 900 631 / 442.
+//
+// Queries per warp, which change no sum's order: one while all CTAs are in the first round (or there
+// are no more than eight queries to share a run of keys), then two, which halve the CTAs.  us, one /
+// two: 576 channels, 4 heads on one KV head, a portion of 5 tokens on 300 keys 108 / 153; 16 heads, 40
+// of them 322 / 218, one of 20 on 700 231 / 319, 8 of 31 49 / 40; 128 channels, 16 heads on 4, 900
+// tokens 394 / 299, 8 portions of 30 on 200 keys 60 / 65, 64 single tokens on 500 95 / 99; 64 channels,
+// 16 KV heads, 40 portions of two tokens 53 / 89.
 template <typename T, int CH>
-static int launch_any_ch(const AnyAttnParams& p, cudaStream_t s) {
-  const int64_t queries = p.rows * (p.hq / p.hkv);
-  const int64_t ctas = ((queries + AA_WARPS - 1) / AA_WARPS) * p.hkv;
+static int launch_any_ch(AnyAttnParams p, int64_t shortest, int64_t longest, cudaStream_t s) {
+  const int64_t grp = p.hq / p.hkv;
+  int64_t rest = p.rows * grp;                  // queries that are left for the warps
   if constexpr (CH == 18) {
-    // Tiles where they are full enough and give the SMs enough to do (us, these / tiles): fp32, 576
-    // channels, 16 heads on one KV head, portions of 40, 120 and 333 tokens 288 / 176, 40 of 5 on 200
-    // keys 162 / 118, one of 20 on 700 233 / 331; 256 channels, 8 heads on 2, 900 tokens 440 / 332,
-    // 20 portions of 9 on 300 111 / 130.  Up to 128 channels the two are too close for a second form.
-    const int64_t tiles = queries / AT_QUERIES * p.hkv;
-    if (queries >= 2 * (int64_t)AT_QUERIES * p.num_seqs &&
-        tiles * p.d >= (int64_t)sm_count() * 288)
-      return launch_attn_tile<T, CH>(p, s);
+    const int64_t full = (512 + p.hkv - 1) / p.hkv;
+    const int64_t least = full > 2 * AT_QUERIES ? full : 2 * AT_QUERIES;
+    if (longest * grp >= least) {
+      p.least = least;
+      const int rc = launch_attn_tile<T, CH>(p, s);
+      if (rc != FK_OK || shortest * grp >= least) return rc;
+      p.least = 0;
+      p.below = least;
+      rest = rest < least * p.num_seqs ? rest : least * p.num_seqs;
+    }
   }
-  if (queries <= (int64_t)AA_WARPS * p.num_seqs || ctas <= sm_count())
+  const int64_t ctas = ((rest + AA_WARPS - 1) / AA_WARPS) * p.hkv;
+  if (rest <= (int64_t)AA_WARPS * p.num_seqs || ctas <= sm_count())
     return launch_any_r<T, CH, 1>(p, s);
   return launch_any_r<T, CH, 2>(p, s);
 }
 template <typename T>
-static int launch_any(const AnyAttnParams& p, cudaStream_t s) {
-  if (p.d <= 64) return launch_any_ch<T, 2>(p, s);
-  if (p.d <= 128) return launch_any_ch<T, 4>(p, s);
-  if (p.d <= 576) return launch_any_ch<T, 18>(p, s);
+static int launch_any(const AnyAttnParams& p, int64_t shortest, int64_t longest, cudaStream_t s) {
+  if (p.d <= 64) return launch_any_ch<T, 2>(p, shortest, longest, s);
+  if (p.d <= 128) return launch_any_ch<T, 4>(p, shortest, longest, s);
+  if (p.d <= 576) return launch_any_ch<T, 18>(p, shortest, longest, s);
   return launch_any_r<T, 36, 1>(p, s);
 }
 
@@ -1181,12 +1199,13 @@ int fk_gemm_f32(const float* x, int64_t x_stride, const float* w, const float* b
   return launch_f32_product(p, static_cast<cudaStream_t>(stream));
 }
 
-int fk_paged_attn_any(const void* q, int64_t q_stride, void* out, int64_t out_stride,
+int fk_paged_attn_any_of(const void* q, int64_t q_stride, void* out, int64_t out_stride,
                       const void* k_cache, const void* v_cache, int is_f32, int64_t num_blocks,
                       int block_size, const int32_t* cu_seqlens_q, const int32_t* kv_lens,
                       const int32_t* block_tables, int64_t block_table_stride, int num_seqs,
                       int64_t rows, int num_q_heads, int num_kv_heads, int head_dim,
-                      float softmax_scale, int32_t* status, fk_stream_t stream) {
+                      float softmax_scale, int64_t shortest, int64_t longest, int32_t* status,
+                      fk_stream_t stream) {
   FK_REQUIRE(rows >= 0 && num_seqs >= 0 && head_dim > 0 && num_q_heads > 0 && num_kv_heads > 0,
              FK_ERR_INVALID_ARG, "fk_paged_attn_any: bad sizes");
   if (rows == 0 || num_seqs == 0) return FK_OK;
@@ -1208,8 +1227,23 @@ int fk_paged_attn_any(const void* q, int64_t q_stride, void* out, int64_t out_st
   p.bt_stride = block_table_stride; p.num_seqs = num_seqs; p.hq = num_q_heads;
   p.hkv = num_kv_heads; p.d = head_dim; p.block_size = block_size; p.num_blocks = (int)num_blocks;
   p.rows = rows; p.scale = softmax_scale; p.status = status;
+  p.below = p.rows * (num_q_heads / num_kv_heads) + 1;
+  if (num_seqs == 1) shortest = longest = rows;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return is_f32 ? launch_any<float>(p, s) : launch_any<uint16_t>(p, s);
+  return is_f32 ? launch_any<float>(p, shortest, longest, s)
+                : launch_any<uint16_t>(p, shortest, longest, s);
+}
+
+int fk_paged_attn_any(const void* q, int64_t q_stride, void* out, int64_t out_stride,
+                      const void* k_cache, const void* v_cache, int is_f32, int64_t num_blocks,
+                      int block_size, const int32_t* cu_seqlens_q, const int32_t* kv_lens,
+                      const int32_t* block_tables, int64_t block_table_stride, int num_seqs,
+                      int64_t rows, int num_q_heads, int num_kv_heads, int head_dim,
+                      float softmax_scale, int32_t* status, fk_stream_t stream) {
+  return fk_paged_attn_any_of(q, q_stride, out, out_stride, k_cache, v_cache, is_f32, num_blocks,
+                              block_size, cu_seqlens_q, kv_lens, block_tables, block_table_stride,
+                              num_seqs, rows, num_q_heads, num_kv_heads, head_dim, softmax_scale,
+                              0, rows, status, stream);
 }
 
 }  // extern "C"

@@ -392,7 +392,7 @@ class DecodeEngine:
                       np.fromiter(accumulate(q, initial=0), np.int32, len(q) + 1),
                       np.fromiter(accumulate(kv, initial=0), np.int32, len(kv) + 1)):
                 put(a)
-            layout.append((cols, max(q), max(kv), sum(kv)))
+            layout.append((cols, max(q), max(kv), sum(kv), min(q)))
         if self.state_slots is not None:
             put(np.repeat(np.array([s.state_slot for s, _, _ in portions], dtype=np.int32), counts))
             put(np.fromiter(accumulate(counts, initial=0), np.int32, len(counts) + 1))

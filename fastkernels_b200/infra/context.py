@@ -37,6 +37,7 @@ class SpanBatch:
     max_seqlen_q: int = 1
     max_seqlen_k: int = 0
     total_k: int = 0            # prefill: keys of all segments
+    min_seqlen_q: int = 0       # no segment has fewer queries
 
 
 @dataclass

@@ -125,7 +125,8 @@ class RotaryAttention:
         heads = out[:, :width].unflatten(1, (self.kv_heads * self.group, self.padded_dim))
         if not self.tensor_cores:
             ops.paged_attn_any(q, kc, vc, span.cu_seqlens_q, span.kv_lens, span.block_tables,
-                               self.scale, out=heads, status=self.status)
+                               self.scale, out=heads, status=self.status,
+                               min_seqlen_q=span.min_seqlen_q, max_seqlen_q=span.max_seqlen_q)
         elif get_context().is_prefill:
             ops.prefill_attn(q, kc, vc, span.cu_seqlens_q, span.cu_seqlens_k, span.max_seqlen_q,
                              self.scale, block_table=span.block_tables, out=heads,
@@ -278,7 +279,8 @@ class LatentAttention:
                                 status=self.status)
         else:
             o = ops.paged_attn_any(q, cache, cache, span.cu_seqlens_q, span.kv_lens,
-                                   span.block_tables, self.scale, status=self.status)
+                                   span.block_tables, self.scale, status=self.status,
+                                   min_seqlen_q=span.min_seqlen_q, max_seqlen_q=span.max_seqlen_q)
         ops.group_gemm(o.view(t, -1), self.w_value, out=out, x_group=o.shape[2],
                        y_group=self.v_pitch, status=self.status)
         return out

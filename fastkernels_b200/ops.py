@@ -843,9 +843,11 @@ def head_norm_gate(o, gate, weight, heads, dim, eps, out):
 
 
 def paged_attn_any(q, k_cache, v_cache, cu_seqlens_q, kv_lens, block_tables, softmax_scale,
-                   out=None, status=None):
+                   out=None, status=None, min_seqlen_q=0, max_seqlen_q=None):
     """Causal attention over the NHD pool without shape restrictions (bf16 or fp32):
-    the path for fp32 and for head sizes / GQA ratios the tensor-core kernels lack."""
+    the path for fp32 and for head sizes / GQA ratios the tensor-core kernels lack.  A row comes
+    out with the same bits whatever other sequences are in the call.  min_seqlen_q and max_seqlen_q:
+    between how many rows every sequence brings, where the caller knows (spares a launch)."""
     f32 = _is_f32(q, "q")
     _need(k_cache, q.dtype, "k_cache")
     _need(v_cache, q.dtype, "v_cache")
@@ -859,11 +861,13 @@ def paged_attn_any(q, k_cache, v_cache, cu_seqlens_q, kv_lens, block_tables, sof
         raise _lib.FkError("paged_attn_any: shape or stride mismatch")
     if out is None:
         out = torch.empty((rows, hq, d), dtype=q.dtype, device=q.device)
-    check(lib.fk_paged_attn_any(
+    longest = rows if max_seqlen_q is None else int(max_seqlen_q)
+    check(lib.fk_paged_attn_any_of(
         _ptr(q), hq * d, _ptr(out), out.stride(0) if rows else hq * d, _ptr(k_cache),
         _ptr(v_cache), f32, nb, bs, _ptr(cu_seqlens_q), _ptr(kv_lens), _ptr(block_tables),
         block_tables.stride(0), cu_seqlens_q.numel() - 1, rows, hq, hkv, d,
-        float(softmax_scale), _status_ptr(status, q), _stream()), "fk_paged_attn_any")
+        float(softmax_scale), int(min_seqlen_q), longest, _status_ptr(status, q), _stream()),
+        "fk_paged_attn_any")
     return out
 
 

@@ -722,13 +722,23 @@ int fk_gemm_f32(const float* x, int64_t x_stride, const float* w, const float* b
 
 /* Causal attention over the NHD pool for any head size up to 1152 (multiple of 4), any
  * query / KV head ratio, bf16 or fp32: sequence i brings query rows cu_seqlens_q[i] ..
- * cu_seqlens_q[i + 1] that end at its kv_lens[i]-th key. */
+ * cu_seqlens_q[i + 1] that end at its kv_lens[i]-th key.  A row comes out with the same bits
+ * whatever other sequences are in the call. */
 int fk_paged_attn_any(const void* q, int64_t q_stride, void* out, int64_t out_stride,
                       const void* k_cache, const void* v_cache, int is_f32, int64_t num_blocks,
                       int block_size, const int32_t* cu_seqlens_q, const int32_t* kv_lens,
                       const int32_t* block_tables, int64_t block_table_stride, int num_seqs,
                       int64_t rows, int num_q_heads, int num_kv_heads, int head_dim,
                       float softmax_scale, int32_t* status, fk_stream_t stream);
+/* The same for callers that know between how many rows the sequences bring: a launch for sequences
+ * there are none of is spared. */
+int fk_paged_attn_any_of(const void* q, int64_t q_stride, void* out, int64_t out_stride,
+                      const void* k_cache, const void* v_cache, int is_f32, int64_t num_blocks,
+                      int block_size, const int32_t* cu_seqlens_q, const int32_t* kv_lens,
+                      const int32_t* block_tables, int64_t block_table_stride, int num_seqs,
+                      int64_t rows, int num_q_heads, int num_kv_heads, int head_dim,
+                      float softmax_scale, int64_t shortest, int64_t longest, int32_t* status,
+                      fk_stream_t stream);
 
 /* fk_paged_decode_attn (planned 0) / _planned (planned 1) and fk_prefill_attn with the
  * fp32 softmax weights taken into P V as two bf16 parts (16 significant bits) instead of

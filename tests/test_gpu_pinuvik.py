@@ -424,6 +424,41 @@ def test_paged_attn_any_of_many_queries(d, hq, hkv, portions, dtype):
     test_paged_attn_any_forms(d, hq, hkv, portions, dtype)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d,hq,hkv", [(576, 16, 1), (256, 8, 2), (132, 16, 16), (128, 8, 2),
+                                      (1152, 4, 1)])
+def test_paged_attn_any_rows_do_not_hang_on_the_batch(d, hq, hkv, dtype):
+    """A sequence's rows have the same bits alone, among others of every length, with empty ones
+    beside them, and whatever the caller says of the lengths."""
+    from fastkernels_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    least = -(-512 // hq)                          # rows from which a sequence goes in tiles
+    portions = [(0, 20), (37, 1), (5, 150), (0, least - 1), (12, least), (0, 0), (3, 2 * least + 7),
+                (64, 1)]
+    lens, page = [a + c for a, c in portions], 16
+    cols = -(-max(lens) // page)
+    bt = torch.randperm(cols * len(lens), generator=gen, device="cuda").int().view(-1, cols)
+
+    def values(*size):
+        return torch.randn(size, generator=gen, device="cuda").to(dtype)
+    k, v = (values(bt.numel(), page, hkv, d) for _ in range(2))
+    q = [values(c, hq, d) for _, c in portions]
+
+    def run(which, **known):
+        cu = np.concatenate([[0], np.cumsum([portions[i][1] for i in which])])
+        out = ops.paged_attn_any(torch.cat([q[i] for i in which]), k, v, i32(cu),
+                                 i32([lens[i] for i in which]), bt[which].contiguous(), d ** -0.5,
+                                 **known)
+        return out.split([portions[i][1] for i in which])
+    every = list(range(len(portions)))
+    want = [run([i])[0] if portions[i][1] else q[i] for i in every]
+    for which in (every, every[::-1], [0, 1, 5], [3, 4], [1, 7], [2, 6, 4]):
+        counts = [portions[i][1] for i in which]
+        for known in ({}, dict(max_seqlen_q=max(counts)),
+                      dict(min_seqlen_q=min(counts), max_seqlen_q=max(counts))):
+            assert all(torch.equal(a, want[i]) for a, i in zip(run(which, **known), which))
+
+
 def test_embed_and_argmax_f32():
     from fastkernels_b200 import ops
     rs = np.random.RandomState(0)
