@@ -42,7 +42,8 @@
 // to the tensor cores.  Five portions of 700 to 2400 tokens, us of prepare / scan, blocks and then
 // chunks: 64 heads of 64 370 / 1174 and 538 / 388, 24 heads of 128 275 / 1311 and 470 / 520; one of
 // 1500, 32 heads of 64 59 / 280 and 79 / 167; 60 of 24 77 / 73 and 101 / 68, of 3 46 / 27 and
-// 60 / 51, so that portions below 32 tokens on average stay with blocks.  Error of o against 64
+// 60 / 51, so that portions below 32 tokens stay with blocks, each by its own length: a row comes out
+// with the same bits whatever else is in the batch.  Error of o against 64
 // bits, of the norm: 2.0 to 2.6e-7 (5.4e-7 with decays that forget nothing in 1500 tokens), blocks
 // 2.7e-7 to 1.6e-6, most of it the decays' (decay_of).
 #include "fk_types.cuh"
@@ -58,6 +59,7 @@ constexpr int DL_STAGES = 3;
 constexpr int DL_STAGE_BLOCKS = 2;
 constexpr int DL_MAX_DIM = 256;
 constexpr int DL_THREADS = 128;
+constexpr int DL_CHUNKS_FROM = 32;   // tokens of a portion that goes in chunks
 constexpr uint32_t DL_WAIT_LIMIT = 1u << 20;
 __host__ __device__ constexpr int dl_block_floats(int dp) { return 21 * dp + 48; }
 
@@ -116,6 +118,7 @@ struct DeltaPrepParams {
   const float* w0; const float* a_bias; // [heads * d]
   float* packed;
   const int32_t* cu; int num_portions;  // blocks only
+  int least, below;                     // portions of least .. below - 1 tokens are taken
   int64_t rows, units; int heads, d, rank, rank_p, heads_per_cta;
   float decay_scale, unit_eps;
 };
@@ -401,7 +404,9 @@ __global__ void __launch_bounds__(DL_THREADS, !CHUNK ? 0 : DP == 64 ? 6 : 4) del
       if (p.cu[mid] / DL_UNIT + mid <= (int)blockIdx.x) lo_i = mid; else hi_i = mid;
     }
     t0 = p.cu[lo_i] + (int64_t)((int)blockIdx.x - (p.cu[lo_i] / DL_UNIT + lo_i)) * DL_UNIT;
-    nt = (int)min((int64_t)DL_UNIT, (int64_t)p.cu[lo_i + 1] - t0);
+    const int n = p.cu[lo_i + 1] - p.cu[lo_i];
+    nt = n < p.least || n >= p.below ? 0
+                                     : (int)min((int64_t)DL_UNIT, (int64_t)p.cu[lo_i + 1] - t0);
   }
   if (nt <= 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -758,6 +763,7 @@ struct DeltaScanParams {
   float* state;                        // [slots][heads][d][dp]
   const int32_t* cu; const int32_t* slots; const int64_t* positions;
   int64_t rows, units; int heads, d, num_slots, num_portions;
+  int least, below;                    // portions of least .. below - 1 tokens are taken
   int32_t* status;
 };
 
@@ -814,6 +820,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_scan_kernel(const DeltaScanP
   pdl_launch_dependents();
   pdl_wait();
   const int64_t begin = p.cu[seq], end = p.cu[seq + 1];
+  if (end - begin < p.least || end - begin >= p.below) return;
   const int slot = begin < end ? p.slots[begin] : -1;
   if (slot >= p.num_slots) {
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
@@ -903,6 +910,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_scan_blocked_kernel(const De
   const int64_t begin = p.cu[seq], end = p.cu[seq + 1];
   const int slot = begin < end ? p.slots[begin] : -1;
   const int64_t n = end - begin;
+  if (n < p.least || n >= p.below) return;
   if (slot >= p.num_slots) {
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
     return;
@@ -1168,6 +1176,7 @@ delta_scan_chunk_kernel(const DeltaScanParams p) {
   __syncthreads();
   const int seq = ranked;
   const int64_t begin = p.cu[seq], end = p.cu[seq + 1];
+  if (end - begin < p.least || end - begin >= p.below) return;
   const int slot = begin < end ? p.slots[begin] : -1;
   if (slot >= p.num_slots) {
     if (threadIdx.x == 0 && p.status) atomicOr(p.status, FK_DEV_BAD_SLOT);
@@ -1480,6 +1489,13 @@ using namespace fk;
 
 extern "C" {
 
+// Portions that a form takes: blocks and chunks take all, 3 the ones below, 4 those from 32 tokens on
+static int delta_form(int blocked, int* least, int* below) {
+  *least = blocked == 4 ? DL_CHUNKS_FROM : 0;
+  *below = blocked == 3 ? DL_CHUNKS_FROM : 0x7fffffff;
+  return blocked == 3 ? 1 : blocked == 4 ? 2 : blocked;
+}
+
 int fk_delta_padded_dim(int dim) {
   return dim <= 0 || dim > DL_MAX_DIM ? 0 : delta_padded(dim);
 }
@@ -1492,7 +1508,7 @@ int fk_delta_chunked(int dim) {
 int64_t fk_delta_packed_floats(int64_t rows, int num_portions, int heads, int dim, int blocked) {
   const int dp = fk_delta_padded_dim(dim);
   if (dp == 0 || rows < 0 || num_portions < 0 || heads <= 0) return 0;
-  if (blocked == 2)
+  if (blocked == 2 || blocked == 4)
     return fk_delta_chunked(dim) ? heads * (rows / DL_UNIT + num_portions) *
                                        (int64_t)(dl_chunk_bytes(dp) / 4) : 0;
   return blocked ? heads * (rows / DL_UNIT + num_portions) * (DL_UNIT / DL_BLK) *
@@ -1511,6 +1527,8 @@ int fk_delta_prepare(const void* r, const void* k, const void* v, const void* a,
   if (rows == 0) return FK_OK;
   FK_REQUIRE(r && k && v && a && y1 && w2 && w0 && a_bias && packed, FK_ERR_INVALID_ARG,
              "fk_delta_prepare: null pointer");
+  DeltaPrepParams p{};
+  blocked = delta_form(blocked, &p.least, &p.below);
   FK_REQUIRE(!blocked || (cu_portions && num_portions > 0), FK_ERR_INVALID_ARG,
              "fk_delta_prepare: blocks need the portions");
   FK_REQUIRE(blocked != 2 || (fk_delta_chunked(dim) && !is_f32), FK_ERR_UNSUPPORTED,
@@ -1519,7 +1537,6 @@ int fk_delta_prepare(const void* r, const void* k, const void* v, const void* a,
              FK_ERR_UNSUPPORTED, "fk_delta_prepare: head size %d or rank %d too large", dim, rank);
   FK_REQUIRE(w2_stride % 4 == 0 && w2_stride >= rank && aligned16(w2) && aligned16(packed),
              FK_ERR_ALIGNMENT, "fk_delta_prepare: w2 rows must be padded to 4 elements");
-  DeltaPrepParams p{};
   p.r = r; p.k = k; p.v = v; p.a = a; p.y1 = y1; p.in_stride = in_stride;
   p.w2 = w2; p.w2_stride = w2_stride; p.w0 = w0; p.a_bias = a_bias; p.packed = packed;
   p.cu = cu_portions; p.num_portions = num_portions;
@@ -1547,11 +1564,12 @@ int fk_delta_scan(const float* packed, int blocked, float* o, float* state, int 
              FK_ERR_INVALID_ARG, "fk_delta_scan: null pointer");
   FK_REQUIRE(dim <= DL_MAX_DIM && heads <= 65535 && num_portions <= 65535, FK_ERR_UNSUPPORTED,
              "fk_delta_scan: head size %d or counts too large", dim);
+  DeltaScanParams p{};
+  blocked = delta_form(blocked, &p.least, &p.below);
   FK_REQUIRE(blocked != 2 || fk_delta_chunked(dim), FK_ERR_UNSUPPORTED,
              "fk_delta_scan: chunks need heads of 33 to 128 channels");
   FK_REQUIRE(aligned16(packed) && aligned16(state), FK_ERR_ALIGNMENT,
              "fk_delta_scan: 16-byte alignment required");
-  DeltaScanParams p{};
   p.packed = packed; p.o = o; p.state = state; p.cu = cu_portions; p.slots = slots;
   p.positions = positions; p.rows = rows; p.units = rows / DL_UNIT + num_portions;
   p.heads = heads; p.d = dim; p.num_slots = num_slots; p.num_portions = num_portions;

@@ -416,7 +416,7 @@ class DecodeEngine:
                     slot_mapping=first.slot_mapping,
                     block_tables=first.block_tables if use_block_tables else None, spans=spans,
                     state_slots=next(parts, None), cu_portions=next(parts, None),
-                    longest_portion=max(counts))
+                    longest_portion=max(counts), shortest_portion=min(counts))
         try:
             hidden = self.model(ids_dev, pos_dev)
         finally:

@@ -165,15 +165,22 @@ class GeneralizedDelta:
 
     def forward(self, cols, positions, run):
         ctx = get_context()
-        chunks = ctx.is_prefill and ops.delta_chunks(
-            self.dim, self.dtype, positions.shape[0], ctx.cu_portions.numel() - 1)
-        packed = ops.delta_prepare(cols["r"], cols["k"], cols["v"], cols["a"], cols["w1"],
-                                   self.w2, self.w0, self.a_bias, self.heads, self.dim,
-                                   self.DECAY_SCALE, self.UNIT_EPS,
-                                   cu_portions=ctx.cu_portions if ctx.is_prefill else None,
-                                   chunks=chunks)
-        o = ops.delta_scan(packed, self.states[run], ctx.cu_portions, ctx.state_slots, positions,
-                           ctx.is_prefill, status=self.status, chunks=chunks)
+        # blocks or chunks, each portion by its own length: (chunks, only the portions they suit)
+        forms = [(False, False)]
+        if ctx.is_prefill:
+            some, every = (ops.delta_chunks(self.dim, self.dtype, n, 1)
+                           for n in (ctx.longest_portion, ctx.shortest_portion))
+            forms = [(True, True), (False, True)] if some and not every else [(some, False)]
+        o = None
+        for chunks, suited in forms:
+            packed = ops.delta_prepare(cols["r"], cols["k"], cols["v"], cols["a"], cols["w1"],
+                                       self.w2, self.w0, self.a_bias, self.heads, self.dim,
+                                       self.DECAY_SCALE, self.UNIT_EPS,
+                                       cu_portions=ctx.cu_portions if ctx.is_prefill else None,
+                                       chunks=chunks, suited=suited)
+            o = ops.delta_scan(packed, self.states[run], ctx.cu_portions, ctx.state_slots,
+                               positions, ctx.is_prefill, out=o, status=self.status,
+                               chunks=chunks, suited=suited)
         out = torch.empty((positions.shape[0], self.out_columns), dtype=self.dtype,
                           device=positions.device)
         return ops.head_norm_gate(o, cols["g"], self.norm, self.heads, self.dim, self.eps, out)

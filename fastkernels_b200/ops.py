@@ -762,10 +762,12 @@ def delta_padded_dim(dim: int) -> int:
 
 
 def delta_prepare(r, k, v, a, y1, w2, w0, a_bias, heads, dim, decay_scale, unit_eps,
-                  cu_portions=None, packed=None, chunks=False):
+                  cu_portions=None, packed=None, chunks=False, suited=False):
     """Operands of the delta rule (fp32, opaque): in blocks of 4 tokens of the portions
-    when cu_portions is given (16 with `chunks`, see delta_chunks), else token by token.  r, k, v, a [T, heads * dim] and
-    y1 [T, rank] are column ranges of the same rows; w2 [heads * dim, padded rank]."""
+    when cu_portions is given (16 with `chunks`, see delta_chunks), else token by token;
+    `suited`: only of the portions that go in blocks, or with `chunks` in chunks, by their own
+    length.  r, k, v, a [T, heads * dim] and y1 [T, rank] are column ranges of the same rows;
+    w2 [heads * dim, padded rank]."""
     f32 = _is_f32(k, "k")
     rows, rank = y1.shape
     for name, t in (("r", r), ("v", v), ("a", a), ("y1", y1), ("w2", w2)):
@@ -781,7 +783,7 @@ def delta_prepare(r, k, v, a, y1, w2, w0, a_bias, heads, dim, decay_scale, unit_
         _need(cu_portions, torch.int32, "cu_portions")
         n_port = cu_portions.numel() - 1
     delta_padded_dim(dim)
-    blocked = (2 if chunks else 1) if n_port > 0 else 0
+    blocked = (2 if chunks else 1) + (2 if suited else 0) if n_port > 0 else 0
     if packed is None:
         n = int(lib.fk_delta_packed_floats(rows, n_port, heads, dim, blocked))
         packed = torch.empty(n, dtype=torch.float32, device=k.device)
@@ -794,15 +796,16 @@ def delta_prepare(r, k, v, a, y1, w2, w0, a_bias, heads, dim, decay_scale, unit_
 
 
 def delta_chunks(dim: int, dtype, rows: int, portions: int) -> bool:
-    """Whether portions of `rows` tokens in all go 16 tokens at a time (prepare and scan with
-    chunks=True): bf16, 33 to 128 channels a head, not mostly padding."""
+    """Whether portions of `rows` tokens in all (a portion of `rows` tokens with portions=1) go 16
+    tokens at a time (prepare and scan with chunks=True): bf16, 33 to 128 channels a head, not
+    mostly padding."""
     return dtype == BF16 and rows >= 32 * portions and bool(lib.fk_delta_chunked(int(dim)))
 
 
 def delta_scan(packed, state, cu_portions, slots, positions, blocked, out=None, status=None,
-               chunks=False):
+               chunks=False, suited=False):
     """The recurrence over prepared operands (`blocked`: prepared with cu_portions, and as there
-    with `chunks`);
+    with `chunks` and `suited`);
     state [slots, heads, dim, padded_dim] fp32 is read and replaced.  Returns
     o [T, heads * dim] fp32."""
     _need(packed, torch.float32, "packed")
@@ -812,7 +815,7 @@ def delta_scan(packed, state, cu_portions, slots, positions, blocked, out=None, 
     _need(positions, torch.int64, "positions")
     rows, heads, dim = positions.shape[0], state.shape[1], state.shape[2]
     n_port = cu_portions.numel() - 1
-    form = (2 if chunks else 1) if blocked else 0
+    form = (2 if chunks else 1) + (2 if suited else 0) if blocked else 0
     if not packed.is_contiguous() or not state.is_contiguous() or \
             state.shape[3] != delta_padded_dim(dim) or packed.numel() < \
             int(lib.fk_delta_packed_floats(rows, n_port, heads, dim, form)):

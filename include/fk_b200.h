@@ -691,7 +691,8 @@ int fk_gemm_bf16_act_mul(const void* x, int64_t x_stride, const void* w, const v
  * [heads][rows][6][padded_dim] fp32 (w, u, a * u, k, r, v), for single tokens;
  * blocked 1: blocks of 4 tokens of a portion (layout: csrc/fk_delta.cu), for portions;
  * blocked 2: chunks of 16 tokens, bf16 and head sizes where fk_delta_chunked is 1 (33 to 128).
- * `packed` is scanned with the `blocked` that it was prepared with.
+ * blocked 3 and 4: blocks of the portions of up to 31 tokens, chunks of the others, and nothing of
+ * the rest.  `packed` is scanned with the `blocked` that it was prepared with.
  * fk_delta_packed_floats: size of `packed` in floats.
  * fk_delta_scan runs the recurrence for every portion from and to
  * state [num_slots][heads][dim (value)][padded_dim (key)] fp32 and writes

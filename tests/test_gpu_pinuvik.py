@@ -715,6 +715,55 @@ def test_delta_rule_in_portions(heads, dim, rank, dtype):
     assert torch.all(state[1] == 3.0) and torch.all(state[3] == 3.0)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,dim,rank", [(3, 64, 33), (2, 100, 8), (2, 24, 4), (2, 136, 8)])
+def test_delta_rows_do_not_hang_on_the_batch(heads, dim, rank, dtype):
+    """A portion's rows and the state it leaves have the same bits alone and beside portions that
+    go another way, on either side of the length from which they go in chunks."""
+    from fastkernels_b200 import ops
+    from fastkernels_b200.infra.context import reset_context, set_context
+    from fastkernels_b200.models.mixers import GeneralizedDelta
+    gen = torch.Generator(device="cuda").manual_seed(dim)
+
+    def values(*size):
+        return torch.randn(size, generator=gen, device="cuda")
+    counts, at = [20, 100, 31, 1, 32, 33, 5, 64], [0, 7, 0, 3, 0, 16, 4, 1]
+    hd = heads * dim
+    mixer = GeneralizedDelta(heads, dim, rank, 1e-6, dtype)
+    mixer.w2 = torch.zeros((hd, (rank + 3) // 4 * 4), dtype=dtype, device="cuda")
+    mixer.w2[:, :rank] = values(hd, rank) / rank ** 0.5
+    mixer.w0, mixer.a_bias, mixer.norm = values(hd) - 2, values(hd), values(hd)
+    mixer.status = ops.new_status("cuda")
+    width = (5 * hd + rank + 7) // 8 * 8
+    rows = [values(c, width).to(dtype) for c in counts]
+    first = values(len(counts), heads, dim, ops.delta_padded_dim(dim))
+    first[..., dim:] = 0
+
+    def run(which):
+        mixer.states = [first.clone()]
+        x, n = torch.cat([rows[i] for i in which]), [counts[i] for i in which]
+        offs = np.cumsum([0] + [hd] * 5 + [rank])
+        cols = {k: x[:, a:b] for k, a, b in zip(("r", "k", "v", "a", "g", "w1"), offs, offs[1:])}
+        set_context(True, state_slots=i32(np.repeat(which, n)),
+                    cu_portions=i32(np.cumsum([0] + n)), longest_portion=max(n),
+                    shortest_portion=min(n))
+        try:
+            out = mixer.forward(cols, i64(np.concatenate([np.arange(counts[i]) + at[i]
+                                                          for i in which])), 0)
+        finally:
+            reset_context()
+        return out.split(n), mixer.states[0]
+    every = list(range(len(counts)))
+    want = [run([i]) for i in every]
+    for which in (every, every[::-1], [0, 1], [2, 4, 6], [3, 6], [1, 5]):
+        out, state = run(which)
+        for i, got in zip(which, out):
+            assert torch.equal(got, want[i][0][0]) and torch.equal(state[i], want[i][1][i])
+        rest = [i for i in every if i not in which]
+        assert torch.equal(state[rest], first[rest])
+    assert int(mixer.status.item()) == 0
+
+
 @pytest.mark.parametrize("heads,dim,rank", [(2, 36, 5), (3, 64, 33), (2, 100, 64), (9, 128, 16)])
 def test_delta_rule_in_chunks(heads, dim, rank):
     """16 tokens at a time on the tensor cores against the plain recurrence: portions that end
