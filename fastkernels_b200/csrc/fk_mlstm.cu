@@ -192,8 +192,9 @@ __device__ __forceinline__ float mc_gates(const MlstmParams& p, int64_t t, int c
   return m;
 }
 
-// RP: rows of S a thread (dim up to 4 RP)
-template <typename T, int RP>
+// RP: rows of S a thread (dim up to 4 RP).  RAGGED: dim below 4 RP; the rows beyond it, whose keys are
+// zero, must not meet a value that is infinite.
+template <typename T, int RP, bool RAGGED>
 __global__ void __launch_bounds__(MC_THREADS + 32) mlstm_scan_kernel(const MlstmParams p) {
   constexpr int NR = (RP * MC_GROUPS + MC_THREADS - 1) / MC_THREADS;   // rows of n a thread
   constexpr int GP = RP + 8, TP = MC_GROUPS * GP;    // row r of a token lies at r % 4 * GP + r / 4
@@ -311,18 +312,27 @@ __global__ void __launch_bounds__(MC_THREADS + 32) mlstm_scan_kernel(const Mlstm
         const float* qr = qs + t * TP + rg * GP;
         const float* kr = ks + t * TP + rg * GP;
         float acc[2] = {0.f, 0.f};
+        if (RAGGED && !(fabsf(vx[t]) <= 3.402823466e38f)) {
 #pragma unroll
-        for (int i = 0; i < RP; i += 4) {
-          const float4 kv = *reinterpret_cast<const float4*>(kr + i);
-          const float4 qv = *reinterpret_cast<const float4*>(qr + i);
-          S[i] = fmaf(kv.x, vx[t], keep * S[i]);
-          S[i + 1] = fmaf(kv.y, vx[t], keep * S[i + 1]);
-          S[i + 2] = fmaf(kv.z, vx[t], keep * S[i + 2]);
-          S[i + 3] = fmaf(kv.w, vx[t], keep * S[i + 3]);
-          acc[0] = fmaf(S[i], qv.x, acc[0]);
-          acc[1] = fmaf(S[i + 1], qv.y, acc[1]);
-          acc[0] = fmaf(S[i + 2], qv.z, acc[0]);
-          acc[1] = fmaf(S[i + 3], qv.w, acc[1]);
+          for (int i = 0; i < RP; ++i)
+            if (i * MC_GROUPS + rg < p.dim) {
+              S[i] = fmaf(kr[i], vx[t], keep * S[i]);
+              acc[i & 1] = fmaf(S[i], qr[i], acc[i & 1]);
+            }
+        } else {
+#pragma unroll
+          for (int i = 0; i < RP; i += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(kr + i);
+            const float4 qv = *reinterpret_cast<const float4*>(qr + i);
+            S[i] = fmaf(kv.x, vx[t], keep * S[i]);
+            S[i + 1] = fmaf(kv.y, vx[t], keep * S[i + 1]);
+            S[i + 2] = fmaf(kv.z, vx[t], keep * S[i + 2]);
+            S[i + 3] = fmaf(kv.w, vx[t], keep * S[i + 3]);
+            acc[0] = fmaf(S[i], qv.x, acc[0]);
+            acc[1] = fmaf(S[i + 1], qv.y, acc[1]);
+            acc[0] = fmaf(S[i + 2], qv.z, acc[0]);
+            acc[1] = fmaf(S[i + 3], qv.w, acc[1]);
+          }
         }
         part[t][rg][lane] = acc[0] + acc[1];
       }
@@ -383,19 +393,25 @@ __global__ void __launch_bounds__(512) mlstm_scan_norm_kernel(const MlstmParams 
   if (r == 0) gN[p.dim] = m;
 }
 
-template <typename T, int RP>
-static int launch_scan_rows(const MlstmParams& p, cudaStream_t s) {
+template <typename T, int RP, bool RAGGED>
+static int launch_scan_one(const MlstmParams& p, cudaStream_t s) {
   constexpr size_t kSmem = 2ull * MC_TOKENS * MC_GROUPS * (RP + 8) * sizeof(float);
   static PerDeviceOnce once;
-  FK_CUDA_OK(set_max_dynamic_smem(once, mlstm_scan_kernel<T, RP>, (int)kSmem));
+  FK_CUDA_OK(set_max_dynamic_smem(once, mlstm_scan_kernel<T, RP, RAGGED>, (int)kSmem));
   const dim3 grid((unsigned)((p.vdim + MC_COLS - 1) / MC_COLS), (unsigned)p.heads,
                   (unsigned)p.num_portions);
-  FK_CUDA_OK(launch_kernel(mlstm_scan_kernel<T, RP>, grid, dim3(MC_THREADS + 32), kSmem, s, p));
+  FK_CUDA_OK(launch_kernel(mlstm_scan_kernel<T, RP, RAGGED>, grid, dim3(MC_THREADS + 32), kSmem, s,
+                           p));
   const dim3 ngrid((unsigned)p.heads, (unsigned)p.num_portions);
   FK_CUDA_OK(launch_kernel(mlstm_scan_norm_kernel<T>, ngrid,
                            dim3((unsigned)((p.dim + 31) / 32 * 32)), 0, s, p));
   count_launch(2);
   return FK_OK;
+}
+template <typename T, int RP>
+static int launch_scan_rows(const MlstmParams& p, cudaStream_t s) {
+  return p.dim < RP * MC_GROUPS ? launch_scan_one<T, RP, true>(p, s)
+                                : launch_scan_one<T, RP, false>(p, s);
 }
 template <typename T>
 static int launch_scan(const MlstmParams& p, cudaStream_t s) {

@@ -614,6 +614,36 @@ def test_matrix_memory_portions_and_tokens(heads, dim, vdim, dtype):
         assert torch.all(S[free] == 3.0) and torch.all(N[free] == 3.0)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("dim", [20, 64, 100, 264])
+def test_matrix_memory_of_infinite_values(dim, dtype):
+    """Token by token: an infinite value is infinite in its own column from its token on, as sums
+    of one sign have it, and nowhere else."""
+    from fastkernels_b200 import ops
+    rs = np.random.RandomState(dim)
+    t, heads, vdim, at = 37, 2, 40, 21
+    q, k = (values(rs, t, heads * dim, dtype=dtype) for _ in range(2))
+    q, k = np.abs(q) + 0.5, np.abs(k) + 0.5
+    v = values(rs, t, heads * vdim, dtype=dtype)
+    z = np.concatenate([rs.randn(t, heads), rs.randn(t, heads) + 5], 1)
+
+    def run(v):
+        x = torch.zeros((t, (2 * dim + vdim) * heads), dtype=dtype, device="cuda")
+        x[:] = dev(np.concatenate([q, k, v], 1), dtype)
+        qd, kd, vd = x.split([heads * dim, heads * dim, heads * vdim], 1)
+        state = [torch.zeros(s, device="cuda") for s in
+                 ops.mlstm_state_shapes(1, heads, dim, vdim)]
+        return ops.mlstm_portions(qd, kd, vd, dev(z), *state, i32([0, t]), i32([0] * t),
+                                  i64(np.arange(t)), heads, dim, vdim, 10.0, 1.0, t, chunked=False)
+    clean, bad = run(v), v.copy()
+    bad[at, 5], bad[at, vdim + 33] = np.inf, -np.inf
+    got = run(bad)
+    assert torch.isfinite(clean).all() and torch.equal(got[:at], clean[:at])
+    assert torch.all(got[at:, 5] == np.inf) and torch.all(got[at:, vdim + 33] == -np.inf)
+    rest = [c for c in range(heads * vdim) if c not in (5, vdim + 33)]
+    assert torch.equal(got[:, rest], clean[:, rest])
+
+
 @pytest.mark.parametrize("chunked", [False, True])
 def test_memory_recalls_a_far_token(chunked):
     """One token with an open input gate, then hundreds with a closed one and hardly any
