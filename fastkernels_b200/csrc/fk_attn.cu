@@ -112,6 +112,12 @@ __device__ __forceinline__ bool att_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// The same for a warp: all lanes get the same answer, and together.
+__device__ __forceinline__ bool att_wait_warp(uint64_t* bar, uint32_t parity,
+                                              volatile int* abort_flag, int32_t* status) {
+  return __all_sync(0xffffffffu, att_wait(bar, parity, abort_flag, status) ? 1 : 0) != 0;
+}
+
 // ---------------------------------------------------------------------------
 // plan
 // ---------------------------------------------------------------------------
@@ -436,7 +442,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_decode_kernel(
   int stage = 0;
   uint32_t phase = 0;
   for (;;) {
-    if (!att_wait(&full[stage], phase, abort_flag, p.status)) break;
+    if (!att_wait_warp(&full[stage], phase, abort_flag, p.status)) break;
     const TileMeta meta = metas[stage];
     if (meta.flags & TILE_END) break;
 

@@ -221,6 +221,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
   return false;
 }
+// The same for a warp: all lanes get the same answer, and together.  Lanes may leave a wait one by
+// one, and what follows (matrix instructions, tensor-memory loads, named barriers: .sync.aligned) wants
+// them converged.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t limit) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit) ? 1 : 0) != 0;
+}
 
 // ---- TMA ------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
@@ -306,7 +312,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// by whole warps
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 

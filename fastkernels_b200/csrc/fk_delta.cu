@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_scan_blocked_kernel(const De
   int si = 0;
   for (; si < nst; ++si) {
     const int sg = si % DL_STAGES;
-    if (!mbar_wait(&full[sg], (uint32_t)(si / DL_STAGES) & 1u, DL_WAIT_LIMIT)) {
+    if (!mbar_wait_warp(&full[sg], (uint32_t)(si / DL_STAGES) & 1u, DL_WAIT_LIMIT)) {
       if (p.status) atomicOr(p.status, FK_DEV_WAIT_TIMEOUT);
       failed = 1;
     }
@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(DL_THREADS) delta_scan_blocked_kernel(const De
   if (failed) {
     // copies that were requested must land before the shared memory goes away
     for (int i = si; i < nst && i < si + DL_STAGES - 1; ++i)
-      (void)mbar_wait(&full[i % DL_STAGES], (uint32_t)(i / DL_STAGES) & 1u, DL_WAIT_LIMIT);
+      (void)mbar_wait_warp(&full[i % DL_STAGES], (uint32_t)(i / DL_STAGES) & 1u, DL_WAIT_LIMIT);
     return;
   }
 #pragma unroll
@@ -1214,7 +1214,7 @@ delta_scan_chunk_kernel(const DeltaScanParams p) {
   const int64_t o_stride = (int64_t)p.heads * p.d;
   int n = 0;
   for (; n < chunks; ++n) {
-    if (!mbar_wait(&full[n % ST], (uint32_t)(n / ST) & 1u, DL_WAIT_LIMIT)) {
+    if (!mbar_wait_warp(&full[n % ST], (uint32_t)(n / ST) & 1u, DL_WAIT_LIMIT)) {
       if (p.status) atomicOr(p.status, FK_DEV_WAIT_TIMEOUT);
       failed = 1;
     }
@@ -1361,7 +1361,7 @@ delta_scan_chunk_kernel(const DeltaScanParams p) {
   if (failed) {
     // copies that were requested must land before the shared memory goes away
     for (int i = n; i < chunks && i < n + ST; ++i)
-      (void)mbar_wait(&full[i % ST], (uint32_t)(i / ST) & 1u, DL_WAIT_LIMIT);
+      (void)mbar_wait_warp(&full[i % ST], (uint32_t)(i / ST) & 1u, DL_WAIT_LIMIT);
     return;
   }
 #pragma unroll

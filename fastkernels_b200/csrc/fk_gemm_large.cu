@@ -244,7 +244,7 @@ gemm_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
     bool ok = true;
     for (int ti = blockIdx.x; ti < total_tiles && ok; ti += gridDim.x) {
       const int mt = ti % p.m_tiles, nt = ti / p.m_tiles;
-      if (!gl_wait(acc_full, tiles_done & 1u, abort_flag, p.status)) { ok = false; break; }
+      if (!gl_wait_warp(acc_full, tiles_done & 1u, abort_flag, p.status)) { ok = false; break; }
       tc_fence_after();
       const int n0 = nt * (ACT ? GL_BN / 2 : GL_BN);
 #pragma unroll 1
@@ -473,7 +473,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x,
       const int mt = ti % p.m_tiles, nt = ti / p.m_tiles;
       const uint32_t buf = tiles_done % Cfg::kBufs;
       const uint32_t use = tiles_done / Cfg::kBufs;
-      if (!gl_wait(&acc_full[buf], use & 1u, abort_flag, p.status)) {
+      if (!gl_wait_warp(&acc_full[buf], use & 1u, abort_flag, p.status)) {
         ok = false;
         break;
       }

@@ -451,7 +451,7 @@ group_large_kernel(const __grid_constant__ CUtensorMap tmap_x,
     for (int ti = blockIdx.x; ti < total; ti += gridDim.x) {
       const GgTile t = gg_tile<Cfg::kRows>(p, first_tile, ti, n_tiles);
       const uint32_t buf = done & 1u, use = done >> 1;
-      if (!gg_wait(&acc_full[buf], use & 1u, abort_flag, p.status)) break;
+      if (!gg_wait_warp(&acc_full[buf], use & 1u, abort_flag, p.status)) break;
       tc_fence_after();
       // rows of this warp that exist
       const int rows = (int)max((int64_t)0, min((int64_t)32, min((int64_t)Cfg::kRows,

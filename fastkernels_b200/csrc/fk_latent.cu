@@ -250,6 +250,7 @@ __host__ __device__ constexpr int la_ring(int subs, int lk) {
 }
 
 __device__ __forceinline__ void named_bar_arrive(int id, int nthreads) {
+  __syncwarp();
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
@@ -329,7 +330,7 @@ latent_attn_kernel(const __grid_constant__ CUtensorMap tmap, const LatentAttnPar
     for (int n = sub; n < tiles; n += SUBS) {
       const int buf = n & 1;
       const int k0 = k_begin + n * LA_KEYS;
-      ok = ok && mbar_wait(&full[st], phase, LA_WAIT_LIMIT);
+      ok = ok && mbar_wait_warp(&full[st], phase, LA_WAIT_LIMIT);
       uint8_t* tile = K + st * tile_bytes;
       if (k0 + LA_KEYS > k_end) {
         // rows behind the last key belong to nobody: their weights are zero, and so must

@@ -545,7 +545,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
       }
       float m_used = -INFINITY, l = 0.f;
       for (int j = 0; j < my_n; ++j) {
-        if (!pf_wait(&s_full[t], (n_sp + (uint32_t)j) & 1u, abort_flag, p.status)) {
+        if (!pf_wait_warp(&s_full[t], (n_sp + (uint32_t)j) & 1u, abort_flag, p.status)) {
           ok = false;
           break;
         }
@@ -635,8 +635,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
           // there; P is zero for them, but 0 * NaN would poison the sum.
           const int vi = kv_base + 2 * j + 1;
           const int vslot = vi % PF_SLOTS;
-          if (!pf_wait(&slot_full[vslot], (uint32_t)(vi / PF_SLOTS) & 1u, abort_flag,
-                       p.status)) {
+          if (!pf_wait_warp(&slot_full[vslot], (uint32_t)(vi / PF_SLOTS) & 1u, abort_flag,
+                            p.status)) {
             ok = false;
             break;
           }
@@ -656,7 +656,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
       if (!ok) break;
       // a row that never saw a key has no reference value: its result is zero
       if (m_used == -INFINITY) l = 0.f;
-      if (!pf_wait(&o_full[t], n_o & 1u, abort_flag, p.status)) {
+      if (!pf_wait_warp(&o_full[t], n_o & 1u, abort_flag, p.status)) {
         ok = false;
         break;
       }

@@ -61,3 +61,41 @@ def test_register_splits_are_checked_before_the_launch():
         needed = re.search(r"(\w*REGS_?NEEDED) =", text, re.I).group(1)
         assert re.search(r"FK_REQUIRE\(launch_regs \* [\w:]+ >= (?:Tile::)?%s," % needed, text)
         assert "cudaFuncGetAttributes(&f, " in text and "f.numRegs" in text
+
+
+def _headers(text, at):
+    """What stands before each brace that is open at `at`, and before the statement itself."""
+    out, depth, i, end = [], 0, at, at
+    while i > 0:
+        i -= 1
+        if text[i] == "}":
+            depth += 1
+        elif text[i] == "{":
+            if depth == 0:
+                j = max(text.rfind(c, 0, i) for c in ";{}")
+                out.append(text[j + 1:i])
+            else:
+                depth -= 1
+    j = max(text.rfind(c, 0, end) for c in ";{}")
+    return out + [text[j + 1:end]]
+
+
+@pytest.mark.parametrize("name", sorted(f.name for f in CSRC.glob("*.cu*")))
+def test_warps_leave_their_waits_together(name):
+    """Lanes may see a barrier's phase one by one, and matrix instructions, tensor-memory accesses and
+    named barriers want whole warps: a wait of more than one lane goes through a form that gives all
+    lanes one answer (*_wait_warp, a vote), or is followed by __syncwarp()."""
+    text = _code(name)
+    for m in re.finditer(r"\b(?:pf|gl|gg|att|gemm|mbar)_wait\(", text):
+        heads = _headers(text, m.start())
+        line = heads[-1]
+        if "__device__" in line or "__all_sync(" in line or "gt_all(" in line:
+            continue
+        one = re.compile(r"lane == 0|threadIdx\.x == (?:0|64)|t128 == 0|feeds")
+        if any(one.search(h) for h in heads):
+            continue
+        rest = text[m.start():]
+        assert re.match(r"[^;]*;\s*(?:__syncwarp\(\);|return __all_sync\()", rest), rest[:200]
+    for m in re.finditer(r'"bar\.(?:sync|arrive) ', text):
+        assert text[:m.start()].rstrip().endswith("__syncwarp();\n  asm volatile(".strip()) or \
+            "__syncwarp();" in text[max(0, m.start() - 60):m.start()]
