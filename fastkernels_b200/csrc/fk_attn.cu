@@ -118,6 +118,29 @@ __device__ __forceinline__ bool att_wait_warp(uint64_t* bar, uint32_t parity,
   return __all_sync(0xffffffffu, att_wait(bar, parity, abort_flag, status) ? 1 : 0) != 0;
 }
 
+// A consumer warp's wait has run out.  It leaves (true) when all of them are here, who meet at named
+// barriers and would wait there for one that left alone; or the tile has come after all, as another
+// one may have seen in the instant in which this one gave up, and it goes on.  `quit` counts the
+// warps that are here; the last one to come closes it, and nobody goes on then.
+__device__ __forceinline__ bool att_give_up(uint64_t* bar, uint32_t parity, int* quit) {
+  constexpr int kClosed = 1 << 16;
+  int leave = 0;
+  if ((threadIdx.x & 31) == 0) {
+    int seen = *(volatile int*)quit, old;
+    while ((old = atomicCAS(quit, seen, seen + 1 == ATT_NW ? kClosed : seen + 1)) != seen)
+      seen = old;
+    for (;;) {
+      if ((leave = (*(volatile int*)quit & kClosed) != 0)) break;
+      if (!mbar_try_wait(bar, parity)) continue;
+      seen = *(volatile int*)quit;
+      while (!(seen & kClosed) && (old = atomicCAS(quit, seen, seen - 1)) != seen) seen = old;
+      leave = (seen & kClosed) != 0;
+      break;
+    }
+  }
+  return __shfl_sync(0xffffffffu, leave, 0) != 0;
+}
+
 // ---------------------------------------------------------------------------
 // plan
 // ---------------------------------------------------------------------------
@@ -251,6 +274,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_decode_kernel(
   uint64_t* empty = full + ATT_STAGES;
   volatile int* abort_flag =
       reinterpret_cast<volatile int*>(smem + AttnSmem::kAbort);
+  int* quit = reinterpret_cast<int*>(smem + AttnSmem::kAbort) + 1;   // consumers that gave up
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -260,6 +284,7 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_decode_kernel(
       mbar_init(&empty[s], ATT_NW);
     }
     *abort_flag = 0;
+    *quit = 0;
     mbar_fence_init();
   }
   pdl_launch_dependents();
@@ -442,7 +467,9 @@ __global__ void __launch_bounds__(ATT_THREADS, 1) attn_decode_kernel(
   int stage = 0;
   uint32_t phase = 0;
   for (;;) {
-    if (!att_wait_warp(&full[stage], phase, abort_flag, p.status)) break;
+    if (!att_wait_warp(&full[stage], phase, abort_flag, p.status) &&
+        att_give_up(&full[stage], phase, quit))
+      break;
     const TileMeta meta = metas[stage];
     if (meta.flags & TILE_END) break;
 

@@ -99,3 +99,70 @@ def test_warps_leave_their_waits_together(name):
     for m in re.finditer(r'"bar\.(?:sync|arrive) ', text):
         assert text[:m.start()].rstrip().endswith("__syncwarp();\n  asm volatile(".strip()) or \
             "__syncwarp();" in text[max(0, m.start() - 60):m.start()]
+
+
+def test_decode_attention_leaves_with_all_its_warps():
+    """Eight warps meet at named barriers when an item's keys are through: one leaves its loop at the
+    end marker, or where att_give_up says that all of them have given up."""
+    text = _code("fk_attn.cu")
+    body = _branch(text, text.index("for (;;) {", text.index("attn_decode_kernel(")))
+    assert "named_bar_sync(1, ATT_NW * 32)" in body and "return" not in body
+    leaves = [" ".join(x.split()) for x in re.findall(r"([^;{}]*)\bbreak\b", body)]
+    assert leaves == ["if (!att_wait_warp(&full[stage], phase, abort_flag, p.status) && "
+                      "att_give_up(&full[stage], phase, quit))", "if (meta.flags & TILE_END)"]
+
+
+@pytest.mark.parametrize("seed", range(40))
+def test_giving_up_is_one_decision(seed):
+    """att_give_up step by step, in any order of its atomic steps: either all eight warps leave, or
+    every one whose tile comes goes on, and none waits for ever."""
+    import random
+    rng = random.Random(seed)
+    closed, warps = 1 << 16, 8
+    state = {"quit": 0, "tile": False, "comes": rng.random() < 0.7}
+
+    def warp():
+        if state["tile"] and rng.random() < 0.5:
+            return False                        # its own wait saw the tile
+        seen = state["quit"]
+        yield
+        while True:
+            old = state["quit"]
+            if old == seen:
+                state["quit"] = closed if seen + 1 == warps else seen + 1
+            yield
+            if old == seen:
+                break
+            seen = old
+        while True:
+            yield
+            if state["quit"] & closed:
+                return True
+            if not state["tile"]:
+                continue
+            seen = state["quit"]
+            yield
+            while not seen & closed:
+                old = state["quit"]
+                if old == seen:
+                    state["quit"] = seen - 1
+                yield
+                if old == seen:
+                    break
+                seen = old
+            return bool(seen & closed)
+    running, left = [warp() for _ in range(warps)], []
+    for step in range(20000):
+        if not running:
+            break
+        if state["comes"] and rng.random() < 0.02:
+            state["tile"] = True
+        w = rng.choice(running)
+        try:
+            next(w)
+        except StopIteration as e:
+            running.remove(w)
+            left.append(e.value)
+            if e.value is False:
+                assert state["tile"]
+    assert not running and len(set(left)) == 1
