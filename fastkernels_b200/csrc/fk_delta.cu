@@ -378,7 +378,8 @@ __device__ void delta_chunk_record(float* vec, float* mats, uint8_t* rec) {
 // 8 channels of a token, one 16-byte load per input, all requested before the decay projection
 // (the first head's before the tanh too); the sum of k^2 stays within the lanes of the token.
 template <typename T, int DP, bool BLOCKED, bool VEC, bool CHUNK>
-__global__ void __launch_bounds__(DL_THREADS, !CHUNK ? 0 : DP == 64 ? 6 : 4) delta_prepare_kernel(const DeltaPrepParams p) {
+__global__ void __launch_bounds__(DL_THREADS, !CHUNK ? 0 : DP == 64 ? 6 : 4)
+delta_prepare_kernel(const DeltaPrepParams p) {
   extern __shared__ __align__(16) uint8_t dl_prep_smem[];
   pdl_launch_dependents();
   if (VEC && !BLOCKED) {

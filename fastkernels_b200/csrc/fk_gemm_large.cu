@@ -652,13 +652,17 @@ static int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const GemmL
 // Which kernel: 0 = single CTAs, 1 = CTA pairs on 256 x 256 tiles, 2 = pairs on 256 x 512.
 //
 // A pair's round is half as long, and its epilogue runs beside the next tile's products, which that
-// of the other two does not: above k = 256 the pairs are ahead or level at all 450 sizes measured (m
-// 257 to 16384, n 1024 to 24576).  us, single / pair / wide: 537 x 2048 x 6144 66 / 37 / 66, 4096 x 3072
-// x 2048 58 / 39 / 60, 8192 x 4096 x 4096 218 / 187 / 219, 8192 x 9472 x 4096 489 / 428 / 547, 16384 x
-// 24576 x 4096 with an activation 3139 / 2555 / 3070; and in prompts, where the power limit sets the
-// clock: 8192 tokens of the 8b Llama sizes 14.1 -> 13.7 ms, five prompts of the 8b Pinuvik sizes 23.5
-// -> 23.1.  Where long k's fill one or two rounds of single CTAs, the estimate below decides as it does
-// for short k (2048 x 4096 x 4096 48 / 47; two full rounds are behind, 2048 x 9472 x 4096 120 / 105).
+// of the other two does not: above k = 256 the pairs were ahead or level at all 450 sizes measured
+// (m 257 to 16384, n 1024 to 24576).  us, single / pair / wide: 537 x 2048 x 6144 66 / 37 / 66,
+// 4096 x 3072 x 2048 58 / 39 / 60, 8192 x 4096 x 4096 218 / 187 / 219, 8192 x 9472 x 4096 489 / 428 /
+// 547, 16384 x 24576 x 4096 with an activation 3139 / 2555 / 3070; and in prompts, where the power
+// limit sets the clock: 8192 tokens of the 8b Llama sizes 14.1 -> 13.7 ms, five prompts of the 8b
+// Pinuvik sizes 23.5 -> 23.1.
+//
+// One window is left to the estimate below: k from 4096 on where the tiles fill one or two rounds of
+// single CTAs.  Its times are older than the pairs' present ones, so it leans to the other two: 2048 x
+// 4096 x 4096 runs single, 48 / 47; 2048 x 9472 x 4096 too, estimated at 117 / 129 and measured at 120
+// / 105; and only here the wide pairs are chosen (3072 x 6144 x 4096).
 //
 // From k = 256 down a round is its epilogue, and the single CTAs' rounds, which store twice as
 // much, are the cheaper ones: 300 x 16384 x 64 9.0 / 10.4, 8192 x 8192 x 256 69 / 80.

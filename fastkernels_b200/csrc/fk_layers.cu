@@ -1,6 +1,8 @@
-// Layers of a prompt portion as one host call (fk_llama_prompt_layers): nothing but the calls of the
-// entry points.  A launch costs the host 20 us where each goes through Python and ctypes, and
-// about 5 here; a short prompt's kernels take 9 on average (61 tokens, 8 layers: 1740 -> 960 us a prompt).
+// Layers of a prompt portion as one host call (fk_llama_prompt_layers): nothing but the calls of
+// the entry points.  A launch costs the host 20 us where each goes through Python and ctypes, and
+// about 5 here; a short prompt's kernels take 9 on average (61 tokens, 8 layers: 1740 -> 960 us a
+// prompt).  Both structs are read between the launches: the caller keeps them until the call
+// returns.
 #include "fk_common.cuh"
 
 using namespace fk;

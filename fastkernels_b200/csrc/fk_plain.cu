@@ -40,7 +40,7 @@ namespace fk {
 // memory, and adds up its share of the rows over all parts in their order (f32_parts).  Where a
 // sum is not finite, an operand may not have been either (the parts of an infinity are no
 // numbers), or operands or products may have been too large (from 2^111 and 2^95 on): that output is
-// computed again from the operands, in 64 bits.
+// computed again from the operands, in 64 bits (a matrix full of them: 40 to 70 times as long).
 struct F32Tile {
   static constexpr int kRows = 128, kCols = 128;       // rows of x, weight rows
   static constexpr int kBK = 32, kStages = 4, kSums = 2;
@@ -1130,22 +1130,22 @@ static int launch_any_r(const AnyAttnParams& p, cudaStream_t s) {
   return FK_OK;
 }
 // Tiles or warps is chosen for each sequence by its own portion, so that a row comes out with the
-// same bits whatever else is in the batch: tiles from 512 rows x query heads on, and two full ones a KV
-// head, beyond 128 channels (up to there the two are too close for a second form).  Alone that is
-// where they meet on short contexts; on long ones the warps, which spread over more SMs, stay ahead
-// to three times as much, and in a batch the tiles are ahead from the first full one.  us, warps /
-// tiles: fp32, 576 channels, 16 heads on one KV head, one portion of 32 tokens 22 / 22, 64 36 / 36, 128
-// 73 / 64, 333 228 / 161; of 32 behind 300 keys 109 / 157, 128 214 / 200, 333 505 / 326; portions of
-// 40, 120 and 333 271 / 160, 8 of 60 97 / 55, 16 of 20 62 / 34; 256 channels, 8 heads on 2, one of 64
-// tokens 22 / 26, 192 69 / 63, 900 436 / 267, 8 of 60 39 / 25; 192 channels, 16 KV heads, one of 32
-// 15 / 16, 96 40 / 33, 900 631 / 442.
+// same bits whatever else is in the batch: tiles from 512 rows x query heads on, and two full ones
+// a KV head, beyond 128 channels (up to there the two are too close for a second form).  Alone that
+// is where they meet on short contexts; on long ones the warps, which spread over more SMs, stay
+// ahead to three times as much, and in a batch the tiles are ahead from the first full one.  us,
+// warps / tiles: fp32, 576 channels, 16 heads on one KV head, one portion of 32 tokens 22 / 22, 64
+// 36 / 36, 128 73 / 64, 333 228 / 161; of 32 behind 300 keys 109 / 157, 128 214 / 200, 333 505 / 326;
+// portions of 40, 120 and 333 271 / 160, 8 of 60 97 / 55, 16 of 20 62 / 34; 256 channels, 8 heads on
+// 2, one of 64 tokens 22 / 26, 192 69 / 63, 900 436 / 267, 8 of 60 39 / 25; 192 channels, 16 KV heads,
+// one of 32 15 / 16, 96 40 / 33, 900 631 / 442.
 //
-// Queries per warp, which change no sum's order: one while all CTAs are in the first round (or there
-// are no more than eight queries to share a run of keys), then two, which halve the CTAs.  us, one /
-// two: 576 channels, 4 heads on one KV head, a portion of 5 tokens on 300 keys 108 / 153; 16 heads, 40
-// of them 322 / 218, one of 20 on 700 231 / 319, 8 of 31 49 / 40; 128 channels, 16 heads on 4, 900
-// tokens 394 / 299, 8 portions of 30 on 200 keys 60 / 65, 64 single tokens on 500 95 / 99; 64 channels,
-// 16 KV heads, 40 portions of two tokens 53 / 89.
+// Queries per warp, which change no sum's order: one while all CTAs are in the first round (or
+// there are no more than eight queries to share a run of keys), then two, which halve the CTAs.
+// us, one / two: 576 channels, 4 heads on one KV head, a portion of 5 tokens on 300 keys 108 / 153;
+// 16 heads, 40 of them 322 / 218, one of 20 on 700 231 / 319, 8 of 31 49 / 40; 128 channels, 16 heads
+// on 4, 900 tokens 394 / 299, 8 portions of 30 on 200 keys 60 / 65, 64 single tokens on 500 95 / 99;
+// 64 channels, 16 KV heads, 40 portions of two tokens 53 / 89.
 template <typename T, int CH>
 static int launch_any_ch(AnyAttnParams p, int64_t shortest, int64_t longest, cudaStream_t s) {
   const int64_t grp = p.hq / p.hkv;

@@ -31,8 +31,9 @@
 //                 overlaps the other tile's matrix work.
 //   warps 0-3     softmax of tile 0, one thread per query row (TMEM lane):
 //   warps 4-7     softmax of tile 1.  Row max / exp2 / row sum in registers,
-//                 P written back to TMEM as bf16, O rescaled in TMEM only when a row's running max grew by more than 2^8
-//                 (the final division by the row sum makes this exact).
+//                 P written back to TMEM as bf16, O rescaled in TMEM only when a row's
+//                 running max grew by more than 2^8 (the final division by the row sum
+//                 makes this exact).
 //
 // The softmax warpgroups hold a whole score row in registers, so they take 208
 // registers per thread (setmaxnreg) and the third warpgroup (TMA, MMA, two idle
@@ -317,7 +318,8 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap tmap_q,
   if (ORDER)
     total_items = p.hq * pf_order_blocks(p, reinterpret_cast<uint32_t*>(smem + PF_OFF_LIST),
                                          reinterpret_cast<int*>(smem + PF_OFF_KV));
-  // rounds of items, every other one backwards: who takes the first of one takes the last of the next
+  // rounds of items, every other one backwards: who takes the first of one takes the last of the
+  // next
   const int ctas = gridDim.x;
   auto item_of = [&](int round) {
     return round * ctas + (round & 1 ? ctas - 1 - (int)blockIdx.x : (int)blockIdx.x);

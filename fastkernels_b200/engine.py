@@ -764,7 +764,12 @@ class DecodeEngine:
         With sync=True the sampled ids come back to the host before returning
         and feed the next step from the host (on one GPU, a device-side anomaly up
         to here raises); with sync=False the next step reads them from the device
-        buffer and the host copy is deferred."""
+        buffer and the host copy is deferred.
+
+        A step with sync=True leaves the next one's positions, lengths, slots and page tables in
+        graph_vars (copied ahead, on this stream) beside its own tokens, hidden rows and logits;
+        where the sequences or their tokens change before the next step, or it runs on another
+        stream, that one's inputs are copied again."""
         n = self.prepare_decode(use_host_ids=sync)
         bs = self.graph_batch_size(n)
         # staged behind the step before, which has also left its tokens on the device
